@@ -35,21 +35,21 @@ YARN = {"factor": 4.0, "original": 4096, "fast": 32.0, "slow": 1.0}
 def listed():
     return [
         # one user's chat on the small model: the smallest step there is, all launches and latency
-        dict(name="decode 0.6B, 1 sequence", task="decode", model="qwen3_0_6b", dtype="bfloat16", seqs=1, shortest=300, longest=300),
+        dict(name="decode 0.6B x 1", task="decode", model="qwen3_0_6b", dtype="bfloat16", seqs=1, shortest=300, longest=300),
         # a small server of the small model: more sequences than the few-row kernels take, lengths that do not line up
-        dict(name="decode 0.6B, 24 sequences", task="decode", model="qwen3_0_6b", dtype="bfloat16", seqs=24, shortest=16, longest=2048),
+        dict(name="decode 0.6B x 24", task="decode", model="qwen3_0_6b", dtype="bfloat16", seqs=24, shortest=16, longest=2048),
         # the benchmark's step: eight long conversations on the 8B shape, bound by its weights
-        dict(name="decode 8B, 8 sequences", task="decode", model="qwen3_8b", dtype="bfloat16", seqs=8, shortest=4000, longest=4090),
+        dict(name="decode 8B x 8", task="decode", model="qwen3_8b", dtype="bfloat16", seqs=8, shortest=4000, longest=4090),
         # a full batch with conversations of every length, half of the traffic is cache
-        dict(name="decode 8B, 64 sequences", task="decode", model="qwen3_8b", dtype="bfloat16", seqs=64, shortest=16, longest=4096),
+        dict(name="decode 8B x 64", task="decode", model="qwen3_8b", dtype="bfloat16", seqs=64, shortest=16, longest=4096),
         # the benchmark's prompt
-        dict(name="prompt 8B, 2048 tokens", task="prompt", model="qwen3_8b", dtype="bfloat16", seqs=1, shortest=2048, longest=2048, past=0),
+        dict(name="prompt 8B 2048 tokens", task="prompt", model="qwen3_8b", dtype="bfloat16", seqs=1, shortest=2048, longest=2048, past=0),
         # a one-line question: time to the first token of a short chat turn
-        dict(name="prompt 8B, 45 tokens", task="prompt", model="qwen3_8b", dtype="bfloat16", seqs=1, shortest=45, longest=45, past=0),
+        dict(name="prompt 8B 45 tokens", task="prompt", model="qwen3_8b", dtype="bfloat16", seqs=1, shortest=45, longest=45, past=0),
         # the next turn of two conversations: some hundred new tokens behind a long cached past
-        dict(name="prompt 8B, next turns", task="prompt", model="qwen3_8b", dtype="bfloat16", seqs=2, shortest=200, longest=350, past=3100),
+        dict(name="next turns 8B", task="prompt", model="qwen3_8b", dtype="bfloat16", seqs=2, shortest=200, longest=350, past=3100),
         # a batch of prompts of very unequal lengths in one step (the 0.6B configuration of the benchmarks: 16 to 2,048 tokens)
-        dict(name="prompts 0.6B, 16 ragged", task="prompt", model="qwen3_0_6b", dtype="bfloat16", seqs=16, shortest=16, longest=2048, past=0),
+        dict(name="prompts 0.6B ragged", task="prompt", model="qwen3_0_6b", dtype="bfloat16", seqs=16, shortest=16, longest=2048, past=0),
         # scoring texts in float32: logits at every position, the precision that parity runs use
         dict(name="score 0.6B float32", task="score", model="qwen3_0_6b", dtype="float32", seqs=3, shortest=5, longest=333, past=0),
         # a reply of a model with a linear recurrence beside attention: the prompt, then single tokens
@@ -57,7 +57,7 @@ def listed():
         # two replies of a model with a gated delta rule beside window attention, and matrix memories
         dict(name="reply Lunadra", task="reply", model="lunadra", dtype="bfloat16", seqs=2, shortest=400, longest=1100, steps=8),
         # drawing the next token of a full batch with the usual filters
-        dict(name="sample, 64 rows", task="sample", seqs=64, vocab=151936, temperature=0.8, top_k=50, top_p=0.95, min_p=0.0),
+        dict(name="sample 64 rows", task="sample", seqs=64, vocab=151936, temperature=0.8, top_k=50, top_p=0.95, min_p=0.0),
     ]
 
 
