@@ -12,11 +12,15 @@
 // the batch a request runs in.  (The reference draws with torch.multinomial, engine.py:149.)
 //
 // Two kernels when the caller lends scratch memory and the row is greedy or has a small top-k: the
-// first cuts every row into chunks of kChunk entries, one block each, and leaves each chunk's
-// candidates (its own top-k, found by a threshold search on the ordered keys in shared memory; or
-// its largest entry); the second runs the filter chain on the candidates of a row, which hold
-// every entry that the row's top-k can keep.  A threshold search takes 8 sweeps of 4 bits with
-// per-thread counters (no atomics, fixed summation order) instead of 32 sweeps of one bit.
+// first cuts every row into chunks, one block each, and leaves each chunk's candidates (a set that
+// holds its own top-k; or its largest entry); the second runs the filter chain on the candidates
+// of a row, which hold every entry that the row's top-k can keep.
+//   top-k up to kTopMax: chunks of kTopChunk entries held in registers, candidates above a lower
+//     bound of the chunk's k-th value that costs one comparison of 256 group maxima with each other
+//     (sample_top_kernel); the second kernel finds the row's k-th value bit by bit on keys in registers.
+//   larger top-k: chunks of kChunk entries in shared memory, threshold search (sample_chunks_kernel).
+// A threshold search over a row takes 8 sweeps of 4 bits with per-thread counters (no atomics, fixed
+// summation order) instead of 32 sweeps of one bit.
 #include "api.h"
 #include "common.cuh"
 
@@ -28,6 +32,14 @@ constexpr int kChunk = 4096;        // entries of a row per block of the first k
 constexpr int kChunkThreads = 256;
 constexpr int kMaxChunks = 64;
 constexpr int kMaxCandidates = 3072;  // candidates of a row that the second kernel takes
+constexpr int kTopThreads = 512;
+constexpr int kTopPer = 32;           // entries a thread of sample_top_kernel holds in registers
+constexpr int kTopChunk = kTopThreads * kTopPer;
+constexpr int kTopGroups = 256;       // groups of a chunk whose maxima bound its k-th value from below
+// Largest top-k for sample_top_kernel.  Of 256 group maxima the k-th largest has about 256 ln(256 / (256 - k))
+// entries at or above it: 56 for k = 50, 532 for k = 224, 1,567 for k = 256, where the bound says nothing any more.
+constexpr int kTopMax = 224;
+static_assert(kTopGroups * 2 == kTopThreads, "a group is a pair of threads");
 
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
   z += 0x9E3779B97F4A7C15ull;
@@ -44,6 +56,9 @@ __device__ __forceinline__ unsigned ordered_key(float v) {
   const unsigned u = __float_as_uint(v);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
+
+// The smallest key above that of -infinity: entries below it weigh nothing and are never drawn.
+constexpr unsigned kFirstKey = 0x00800000u;
 
 struct ArgBest {
   float v;
@@ -157,6 +172,7 @@ struct SampleArgs {
   const int* row_request;
   const int* row_step;
   int* out_tokens;
+  int vec;                    // rows start on 16-byte boundaries
   // scratch of the two-kernel path (null: one kernel does everything)
   int n_chunks, cand_cap;     // chunks per row; room for candidates per chunk
   float* cand_val;            // [rows][chunks][cap] values / temperature, in index order
@@ -169,7 +185,148 @@ __device__ __forceinline__ float scaled(float v, float mult) {
   return v == v ? v : -INFINITY;   // NaN sorts lowest
 }
 
-// First kernel of the two-kernel path.  grid: (chunks, rows).
+// Entries i .. i + 3 of a row's n; those beyond it come as -infinity.
+__device__ __forceinline__ float4 load_quad(const float* src, int i, int n, int vec) {
+  if (vec && i + 3 < n) return *reinterpret_cast<const float4*>(src + i);
+  float4 q;
+  q.x = i < n ? src[i] : -INFINITY;
+  q.y = i + 1 < n ? src[i + 1] : -INFINITY;
+  q.z = i + 2 < n ? src[i + 2] : -INFINITY;
+  q.w = i + 3 < n ? src[i + 3] : -INFINITY;
+  return q;
+}
+
+// Sum over the block's threads; every thread gets it.  scratch: one int a warp.
+__device__ __forceinline__ int block_count(int v, int* scratch) {
+  v = __reduce_add_sync(0xffffffffu, v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
+  __syncthreads();
+  int r = (threadIdx.x & 31) < (blockDim.x >> 5) ? scratch[threadIdx.x & 31] : 0;
+  return __reduce_add_sync(0xffffffffu, r);
+}
+
+// A key with at least k of the block's entries at or above it, and exactly those of the k largest
+// unless entries tie with the k-th (then its own key): one bit a step, ended early by a count of k.
+// Each thread holds N keys; a key of 0 is no entry.
+template <int N>
+__device__ __forceinline__ unsigned block_kth_key(const unsigned (&key)[N], int k, int* scratch) {
+  unsigned K = 0u;
+  for (int bit = 31; bit >= 0; --bit) {
+    const unsigned cand = K | (1u << bit);
+    int mine = 0;
+#pragma unroll
+    for (int j = 0; j < N; ++j) mine += key[j] >= cand;
+    const int count = block_count(mine, scratch);
+    if (count >= k) K = cand;
+    if (count == k) break;
+  }
+  return K;
+}
+
+// Where a thread's `mine` entries begin in a list over the block's threads; the list's length.
+__device__ __forceinline__ int block_offset(int mine, int* scratch, int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  int incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int add = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += add;
+  }
+  __syncthreads();
+  if (lane == 31) scratch[warp] = incl;
+  __syncthreads();
+  const int w = lane < nwarps ? scratch[lane] : 0;
+  *total = __reduce_add_sync(0xffffffffu, w);
+  return __reduce_add_sync(0xffffffffu, lane < warp ? w : 0) + incl - mine;
+}
+
+// First kernel for top-k up to kTopMax.  grid: (chunks of kTopChunk, rows).
+// The chunk stays in registers.  The k-th largest of the maxima of 256 groups of 64 entries has k
+// entries at or above it, so nothing below it can be among the chunk's k largest; what is left is
+// little more than k entries and goes out as it is.  Where it is more than the room (ties, or k near
+// the number of groups) the k-th key is searched bit by bit.  64 rows of 151,936 entries, top-k 50, take
+// 26 us (39 MB, 1.5 TB/s: the ranking, not the reads); the threshold search of sample_chunks_kernel, which
+// reads every entry eight times from shared memory with sixteen conditional adds each, took 186 us.
+__global__ void __launch_bounds__(kTopThreads) sample_top_kernel(SampleArgs a) {
+  __shared__ __align__(16) unsigned top[kTopGroups];
+  __shared__ int red[32];
+  __shared__ unsigned bound;
+  pdl_wait_block();
+  pdl_launch_dependents();
+  const int row = blockIdx.y, chunk = blockIdx.x, tid = threadIdx.x;
+  const int lo = chunk * kTopChunk, n = min(kTopChunk, a.vocab - lo);
+  const float* src = a.logits + (size_t)row * a.ld + lo;
+  const size_t slot = (size_t)row * a.n_chunks + chunk;
+  float* out_val = a.cand_val + slot * a.cand_cap;
+  int* out_idx = a.cand_idx + slot * a.cand_cap;
+  const float mult = 1.0f / a.temperature;
+  const int k = min(a.top_k, n);
+
+  unsigned key[kTopPer];   // 0: beyond the row
+  {
+    float4 q[kTopPer / 4];
+#pragma unroll
+    for (int j = 0; j < kTopPer / 4; ++j) q[j] = load_quad(src, (j * kTopThreads + tid) * 4, n, a.vec);
+#pragma unroll
+    for (int j = 0; j < kTopPer; ++j) {
+      const int i = (j / 4 * kTopThreads + tid) * 4 + j % 4;
+      key[j] = i < n ? ordered_key(scaled((&q[j / 4].x)[j % 4], mult)) : 0u;
+    }
+  }
+  unsigned m = 0u;
+#pragma unroll
+  for (int j = 0; j < kTopPer; ++j) m = max(m, key[j]);
+  m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+  const int group = tid >> 1;
+  if ((tid & 1) == 0) top[group] = m;
+  if (tid == 0) bound = 0u;
+  __syncthreads();
+  {
+    // a pair of threads ranks its group: each against one half of the groups
+    const int j0 = (tid & 1) * (kTopGroups / 2);
+    int rank = 0;
+#pragma unroll 8
+    for (int j = 0; j < kTopGroups / 2; j += 4) {
+      const uint4 t = *reinterpret_cast<const uint4*>(&top[j0 + j]);
+      rank += (t.x > m || (t.x == m && j0 + j < group));
+      rank += (t.y > m || (t.y == m && j0 + j + 1 < group));
+      rank += (t.z > m || (t.z == m && j0 + j + 2 < group));
+      rank += (t.w > m || (t.w == m && j0 + j + 3 < group));
+    }
+    rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+    if (rank == k - 1) bound = m;   // one group has this rank; none where k exceeds the groups
+  }
+  __syncthreads();
+  unsigned K = max(bound, kFirstKey);
+  int mine = 0;
+#pragma unroll
+  for (int j = 0; j < kTopPer; ++j) mine += key[j] >= K;
+  int total;
+  int pos = block_offset(mine, red, &total);
+  if (total > a.cand_cap) {
+    K = max(block_kth_key(key, k, red), kFirstKey);
+    mine = 0;
+#pragma unroll
+    for (int j = 0; j < kTopPer; ++j) mine += key[j] >= K;
+    pos = block_offset(mine, red, &total);
+    if (total > a.cand_cap) {   // ties beyond the room: the second kernel reads the whole row instead
+      if (tid == 0) a.cand_cnt[slot] = -1;
+      return;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < kTopPer; ++j)
+    if (key[j] >= K) {
+      // the value back from its key
+      out_val[pos] = __uint_as_float((key[j] & 0x80000000u) ? (key[j] & 0x7fffffffu) : ~key[j]);
+      out_idx[pos] = lo + (j / 4 * kTopThreads + tid) * 4 + j % 4;
+      ++pos;
+    }
+  if (tid == 0) a.cand_cnt[slot] = total;
+}
+
+// First kernel of the two-kernel path otherwise.  grid: (chunks, rows).
 __global__ void __launch_bounds__(kChunkThreads) sample_chunks_kernel(SampleArgs a) {
   __shared__ float vals[kChunk];
   __shared__ int red_i[33 * 16];
@@ -190,10 +347,21 @@ __global__ void __launch_bounds__(kChunkThreads) sample_chunks_kernel(SampleArgs
     const unsigned long long key =
         mix64(a.seed ^ mix64(((unsigned long long)(unsigned)a.row_request[row] << 32) | (unsigned)a.row_step[row]));
     ArgBest best{-INFINITY, 0x7fffffff};
-    for (int i = tid; i < n; i += blockDim.x) {
-      float v = scaled(src[i], mult);
-      if (!greedy && v != -INFINITY) v += -logf(-logf(uniform_of(key, lo + i)));
-      best = better(best, ArgBest{v, lo + i});
+    // all 16 loads of a thread in flight at once, 16 bytes each where rows allow it
+    constexpr int kQuads = kChunk / (4 * kChunkThreads);
+    float4 q[kQuads];
+#pragma unroll
+    for (int j = 0; j < kQuads; ++j) q[j] = load_quad(src, (j * kChunkThreads + tid) * 4, n, a.vec);
+#pragma unroll
+    for (int j = 0; j < kQuads; ++j) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int i = (j * kChunkThreads + tid) * 4 + c;
+        if (i >= n) continue;
+        float v = scaled((&q[j].x)[c], mult);
+        if (!greedy && v != -INFINITY) v += -logf(-logf(uniform_of(key, lo + i)));
+        best = better(best, ArgBest{v, lo + i});
+      }
     }
     best = block_argbest(best, red_b);
     if (tid == 0) {
@@ -244,6 +412,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleArgs a) {
   __shared__ int scan[kSampleThreads];
   __shared__ float l_val[kMaxCandidates];
   __shared__ int l_idx[kMaxCandidates];
+  __shared__ int chunk_base[kMaxChunks], chunk_cnt[kMaxChunks];
   pdl_wait_block();
   pdl_launch_dependents();
   const int row = blockIdx.x;
@@ -259,25 +428,26 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleArgs a) {
   float mult = greedy ? 1.0f : 1.0f / a.temperature;
   int n = V;
   if (a.cand_cnt != nullptr) {
-    // gather the chunks' candidates (index order is kept); a chunk that overflowed sends us to the row
+    // gather the chunks' candidates, a warp per chunk; a chunk that overflowed sends us to the row
     const int* cnt = a.cand_cnt + (size_t)row * a.n_chunks;
-    int total = 0;
-    bool ok = true;
-    for (int c = 0; c < a.n_chunks; ++c) {
-      const int m = cnt[c];
-      if (m < 0) ok = false;
-      total += max(m, 0);
+    static_assert(kMaxChunks <= kSampleThreads, "a thread per chunk");
+    const int m = tid < a.n_chunks ? cnt[tid] : 0;
+    const bool ok = __syncthreads_and(m >= 0);
+    int total;
+    const int base = block_offset(max(m, 0), red_i, &total);
+    if (tid < kMaxChunks) {
+      chunk_base[tid] = base;
+      chunk_cnt[tid] = m;
     }
+    __syncthreads();
     if (ok && total <= kMaxCandidates) {
-      int base = 0;
-      for (int c = 0; c < a.n_chunks; ++c) {
-        const int m = cnt[c];
+      for (int c = tid >> 5; c < a.n_chunks; c += kSampleThreads / 32) {
+        const int b = chunk_base[c];
         const size_t slot = ((size_t)row * a.n_chunks + c) * a.cand_cap;
-        for (int i = tid; i < m; i += blockDim.x) {
-          l_val[base + i] = a.cand_val[slot + i];
-          l_idx[base + i] = a.cand_idx[slot + i];
+        for (int i = tid & 31; i < chunk_cnt[c]; i += 32) {
+          l_val[b + i] = a.cand_val[slot + i];
+          l_idx[b + i] = a.cand_idx[slot + i];
         }
-        base += m;
       }
       __syncthreads();
       vals = l_val;
@@ -303,10 +473,42 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleArgs a) {
   for (int i = tid; i < n; i += blockDim.x) mx = fmaxf(mx, scaled(vals[i], mult));
   mx = block_max(mx, red_f);
 
-  if (a.top_k > 0 && a.top_k < V) {
+  bool listed = false;   // the kept entries are the list in c_val, at most one a thread
+  if (a.top_k > 0 && a.top_k < V && idxs != nullptr && a.top_k <= kTopMax) {
+    // candidates of the first kernel: three a thread at most, their keys in registers (with the list's masses
+    // below: 17 us for 64 rows at top-k 50 and top-p 0.95, against 90 us for threshold searches in shared memory)
+    constexpr int kPer = kMaxCandidates / kSampleThreads;
+    unsigned key[kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int i = j * kSampleThreads + tid;
+      key[j] = i < n ? ordered_key(l_val[i]) : 0u;
+    }
+    const unsigned K = max(block_kth_key(key, min(a.top_k, n), red_i), kFirstKey);
+    int mine = 0, total;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) mine += key[j] >= K;
+    int pos = block_offset(mine, red_i, &total);
+    keep_key = K;
+    if (total <= kMaxCompact) {   // always, but for hundreds of entries that tie with the k-th
+#pragma unroll
+      for (int j = 0; j < kPer; ++j)
+        if (key[j] >= K) {
+          c_val[pos] = l_val[j * kSampleThreads + tid];
+          c_idx[pos] = l_idx[j * kSampleThreads + tid];
+          ++pos;
+        }
+      __syncthreads();
+      vals = c_val;
+      idxs = c_idx;
+      n = total;
+      listed = true;
+    }
+  } else if (a.top_k > 0 && a.top_k < V) {
     // k-th largest value: the largest key K with count(key >= K) >= k
-    const unsigned K = search16<false, int>(
-        n, min(a.top_k, n), [&](int i, unsigned& key, int& w) { key = ordered_key(scaled(vals[i], mult)); w = 1; }, red_i);
+    // (masked entries stay out: with fewer than k others they would all tie with the k-th and fill the list)
+    const unsigned K = max(kFirstKey, search16<false, int>(
+        n, min(a.top_k, n), [&](int i, unsigned& key, int& w) { key = ordered_key(scaled(vals[i], mult)); w = 1; }, red_i));
     keep_key = K;
     if (a.top_k <= kMaxCompact) {
       // compact the candidates in index order (deterministic): count, scan, write
@@ -364,7 +566,25 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleArgs a) {
     // cannot be: the whole mass exceeds it)
     const float limit = a.top_p * z;
     const unsigned kk = keep_key;
-    const unsigned J = search16<true, float>(
+    unsigned J = 0u;
+    if (listed) {
+      // few entries: each adds up the mass above itself; J is the smallest key that stays
+      if (tid < n) {
+        const float v = vals[tid];
+        l_val[tid] = ordered_key(v) >= kk ? expf(v - mx) : 0.f;
+        l_idx[tid] = (int)ordered_key(v);
+      }
+      if (tid == 0) red_i[0] = -1;   // as unsigned the largest key there is
+      __syncthreads();
+      if (tid < n) {
+        const unsigned own = (unsigned)l_idx[tid];
+        float mass = 0.f;
+        for (int j = 0; j < n; ++j) mass += (unsigned)l_idx[j] > own ? l_val[j] : 0.f;
+        if (!(mass > limit)) atomicMin(reinterpret_cast<unsigned*>(red_i), own);
+      }
+      __syncthreads();
+      J = (unsigned)red_i[0];
+    } else J = search16<true, float>(
         n, limit,
         [&](int i, unsigned& key, float& w) {
           const float v = scaled(vals[i], mult);
@@ -423,25 +643,35 @@ __global__ void repetition_penalty_kernel(float* logits, long long ld, int vocab
 
 }  // namespace pe
 
-// Room for ties at a chunk's k-th value beyond its k candidates.
 static bool unfiltered(float temperature, int top_k, float top_p, float min_p) {
   return temperature <= 1e-5f || ((top_k <= 0) && !(top_p > 0.f && top_p < 1.f) && !(min_p > 0.f));
 }
-static int cand_cap_of(float temperature, int top_k, float top_p, float min_p) {
-  return unfiltered(temperature, top_k, top_p, min_p) ? 1 : top_k + 8;
-}
-static bool two_kernels(int vocab, float temperature, int top_k, float top_p, float min_p) {
-  const int chunks = (vocab + pe::kChunk - 1) / pe::kChunk;
-  if (chunks < 2 || chunks > pe::kMaxChunks) return false;
-  if (unfiltered(temperature, top_k, top_p, min_p)) return true;
-  return top_k > 0 && top_k < vocab && (long long)chunks * top_k <= pe::kMaxCandidates;
+
+// How a row is cut for the first kernel: chunks of how many entries, with room for how many candidates each.
+struct SamplePlan {
+  int chunk, n_chunks, cap;   // n_chunks 0: one kernel does everything
+};
+static SamplePlan sample_plan(int vocab, float temperature, int top_k, float top_p, float min_p) {
+  const SamplePlan none{0, 0, 0};
+  const int small = (vocab + pe::kChunk - 1) / pe::kChunk, large = (vocab + pe::kTopChunk - 1) / pe::kTopChunk;
+  if (small < 2) return none;
+  if (unfiltered(temperature, top_k, top_p, min_p))
+    return small <= pe::kMaxChunks ? SamplePlan{pe::kChunk, small, 1} : none;
+  if (top_k <= 0 || top_k >= vocab) return none;
+  if (top_k <= pe::kTopMax && large <= pe::kMaxChunks) {
+    const int cap = top_k + top_k / 4 + 16;   // the bound of a chunk's k-th entry lets about k / 8 more pass at k = 50
+    if (large * cap <= pe::kMaxCandidates) return SamplePlan{pe::kTopChunk, large, cap};
+  }
+  if (small <= pe::kMaxChunks && (long long)small * top_k <= pe::kMaxCandidates)
+    return SamplePlan{pe::kChunk, small, top_k + 8};   // 8: ties with a chunk's k-th value
+  return none;
 }
 
 // Bytes of scratch with which pe_sample takes its two-kernel path for these settings (0: it has none).
 extern "C" long long pe_sample_scratch_bytes(int n_rows, int vocab, float temperature, int top_k, float top_p, float min_p) {
-  if (n_rows <= 0 || !two_kernels(vocab, temperature, top_k, top_p, min_p)) return 0;
-  const long long chunks = (vocab + pe::kChunk - 1) / pe::kChunk;
-  return (long long)n_rows * chunks * (cand_cap_of(temperature, top_k, top_p, min_p) * 8ll + 4ll);
+  if (n_rows <= 0 || vocab <= 0) return 0;
+  const SamplePlan plan = sample_plan(vocab, temperature, top_k, top_p, min_p);
+  return (long long)n_rows * plan.n_chunks * (plan.cap * 8ll + 4ll);
 }
 
 // scratch: null, or at least pe_sample_scratch_bytes(...) bytes, 4-byte aligned.
@@ -454,16 +684,21 @@ extern "C" int pe_sample(const float* logits, long long ld, int n_rows, int voca
   a.logits = logits; a.ld = ld; a.n_rows = n_rows; a.vocab = vocab; a.temperature = temperature; a.top_k = top_k;
   a.top_p = top_p; a.min_p = min_p; a.seed = seed; a.row_request = row_request; a.row_step = row_step;
   a.out_tokens = out_tokens;
+  a.vec = ((uintptr_t)logits % 16) == 0 && ld % 4 == 0;
   a.n_chunks = 0; a.cand_cap = 0; a.cand_val = nullptr; a.cand_idx = nullptr; a.cand_cnt = nullptr;
   const long long need = pe_sample_scratch_bytes(n_rows, vocab, temperature, top_k, top_p, min_p);
   if (scratch != nullptr && need > 0 && scratch_bytes >= need && ((uintptr_t)scratch % 4) == 0) {
-    a.n_chunks = (vocab + pe::kChunk - 1) / pe::kChunk;
-    a.cand_cap = cand_cap_of(temperature, top_k, top_p, min_p);
+    const SamplePlan plan = sample_plan(vocab, temperature, top_k, top_p, min_p);
+    a.n_chunks = plan.n_chunks;
+    a.cand_cap = plan.cap;
     const size_t slots = (size_t)n_rows * a.n_chunks;
     a.cand_val = reinterpret_cast<float*>(scratch);
     a.cand_idx = reinterpret_cast<int*>(a.cand_val + slots * a.cand_cap);
     a.cand_cnt = a.cand_idx + slots * a.cand_cap;
-    pe::launch(pe::sample_chunks_kernel, dim3(a.n_chunks, n_rows), pe::kChunkThreads, 0, stream, a);
+    if (plan.chunk == pe::kTopChunk)
+      pe::launch(pe::sample_top_kernel, dim3(a.n_chunks, n_rows), pe::kTopThreads, 0, stream, a);
+    else
+      pe::launch(pe::sample_chunks_kernel, dim3(a.n_chunks, n_rows), pe::kChunkThreads, 0, stream, a);
     PE_LAUNCH_CHECK();
   }
   pe::launch(pe::sample_kernel, n_rows, pe::kSampleThreads, 0, stream, a);

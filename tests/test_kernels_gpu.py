@@ -788,6 +788,36 @@ def test_sampler_with_scratch_matches_the_plain_draw_and_the_single_kernel(ops, 
     assert ops.sample_scratch_bytes(rows, V, 0.8, 0, 0.9) == 0 and ops.sample_scratch_bytes(rows, 3000, 0.8, 40) == 0
 
 
+@pytest.mark.parametrize("V,k", [(4097, 50), (16384, 224), (16385, 200), (16387, 225), (50001, 17), (151936, 200)])
+def test_sampler_top_k_at_the_edges_of_its_chunks(ops, V, k):
+    """A last chunk of one entry or with fewer entries than k, rows without 16-byte alignment, k at the largest that
+    the register kernel takes and beyond it, masked rows, ties: the same draws as one kernel over the whole row."""
+    torch.manual_seed(14)
+    rows = 8
+    logits = torch.randn(rows, V, device=DEV) * 2.5
+    logits[1, k // 2:] = -float("inf")                        # fewer finite entries than k
+    logits[2, ::3] = float("nan")
+    logits[3, V - 1] = 30.0
+    logits[4, :3 * k] = 8.0                                   # 3 k entries tie at the top: more than a chunk has room for
+    logits[5] = -float("inf")
+    logits[6, 7] = float("inf")
+    req = torch.arange(rows, dtype=torch.int32, device=DEV)
+    step = torch.zeros(rows, dtype=torch.int32, device=DEV)
+    need = ops.sample_scratch_bytes(rows, V, 0.8, k, 0.95, 0.0)
+    assert need > 0
+    scratch = torch.empty(need, dtype=torch.uint8, device=DEV)
+    for top_p, min_p in ((1.0, 0.0), (0.95, 0.0), (0.7, 0.02)):
+        a, b = (torch.empty(rows, dtype=torch.int32, device=DEV) for _ in range(2))
+        ops.sample(logits, 0.8, k, top_p, min_p, 3, req, step, a, scratch=scratch)
+        ops.sample(logits, 0.8, k, top_p, min_p, 3, req, step, b)
+        assert a.tolist() == b.tolist(), (top_p, min_p)
+        for r in (0, 1, 2, 3):
+            row = logits[r].cpu()
+            row[row.isnan()] = -float("inf")                  # where the kernels sort them
+            _, probs = plain.filter_logits(row, temperature=0.8, top_k=k, top_p=top_p, min_p=min_p)
+            assert probs[a[r]] > 0
+
+
 def test_sampler_with_scratch_unfiltered_draw_is_the_single_kernels(ops):
     torch.manual_seed(13)
     rows, V = 12, 30000
