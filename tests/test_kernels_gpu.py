@@ -403,6 +403,30 @@ def test_attention_umma_prefill(ops, nh, nkv, window):
     assert rel_err(out.float().cpu().view(N, nh, d), want) < ATT_TOL[dtype]
 
 
+def test_attention_umma_prefill_rows_beyond_a_sequences_last(ops):
+    """A tile's spare rows hold the next sequence's queries: whatever those are, the sequence's own rows do not see them."""
+    torch.manual_seed(26)
+    nh, nkv, d, dtype = 32, 8, 128, torch.bfloat16
+    q_lens, pasts = [33, 31, 1, 40], [70, 0, 300, 128]
+    ps = PagedSetup([a + b for a, b in zip(q_lens, pasts)], nkv, d, dtype, seed=26)
+    N = sum(q_lens)
+    q_all = torch.randn(N, (nh + 2 * nkv) * d, device=DEV).to(dtype)
+    qstart = torch.tensor([0] + list(torch.tensor(q_lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    past_t = torch.tensor(pasts, dtype=torch.int32, device=DEV)
+    outs = []
+    for bad in (None, float("nan"), float("inf")):
+        q = q_all.clone()
+        if bad is not None:
+            q[33:64] = bad
+        out = torch.zeros(N, nh * d, device=DEV, dtype=dtype)
+        st = _status()
+        ops.attention_umma_prefill(q, out, 4, max(q_lens), nh, nkv, d, d ** -0.5, 0, qstart, past_t, ps.seq_slot, ps.table,
+                                   ps.num_pages, ps.k_pages, ps.v_pages, st)
+        assert st.tolist()[0] == 0
+        outs.append(torch.cat([out[:33], out[64:]]))
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
 def test_attention_umma_prefill_blocks_of_two_pages_again_and_again(ops):
     """Blocks that see two or three pages only (a short window) end a few barrier phases after they
     start; a wait that names a phase by its parity must not pass because the barrier is two phases
