@@ -237,6 +237,39 @@ def test_attention_prefill(ops, dtype, nh, nkv, d, window):
     assert rel_err(out.float().cpu().view(N, nh, d), want) < ATT_TOL[dtype]
 
 
+@pytest.mark.parametrize("nh,nkv,d", [(16, 8, 128), (3, 3, 128), (10, 2, 64), (33, 1, 64)])
+@pytest.mark.parametrize("window,sink", [(0, False), (37, False), (0, True)])
+def test_attention_prefill_float32_tiles(ops, nh, nkv, d, window, sink):
+    """The tiled float32 kernel (head sizes 64 and 128) at the edges of its 32-row tiles and 64-key pages, against 64 bits."""
+    torch.manual_seed(27)
+    q_lens, pasts = [1, 15, 16, 17, 65, 200], [0, 64, 63, 128, 7, 0]
+    ps = PagedSetup([a + b for a, b in zip(q_lens, pasts)], nkv, d, torch.float32, seed=27, key_scale=2.0)
+    N = sum(q_lens)
+    q_all = torch.randn(N, nh * d + 32, device=DEV)
+    out = torch.zeros(N, nh * d, device=DEV)
+    qstart = torch.tensor([0] + list(torch.tensor(q_lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    past_t = torch.tensor(pasts, dtype=torch.int32, device=DEV)
+    st = _status()
+    ops.attention_generic_ex(False, q_all, out, len(q_lens), max(q_lens), nh, nkv, d, d, d ** -0.5, window, sink, None, None, 0,
+                             False, qstart, past_t, ps.seq_slot, ps.table, ps.num_pages, ps.k_pages, ps.v_pages, None, 0, 0, st)
+    assert st.tolist()[0] == 0
+    o = 0
+    for b, (n, past) in enumerate(zip(q_lens, pasts)):
+        L = n + past
+        idx = ps.table[ps.slots[b], :-(-L // 64)].long()
+        k, v = (t[idx].permute(1, 0, 2, 3).reshape(nkv, -1, d)[:, :L].double().repeat_interleave(nh // nkv, 0) for t in (ps.k_pages, ps.v_pages))
+        q = q_all[o:o + n, :nh * d].double().view(n, nh, d).transpose(0, 1)
+        i, j = torch.arange(n, device=DEV)[:, None] + past, torch.arange(L, device=DEV)[None]
+        hidden = (j > i) | ((i - j >= window) if window else False)
+        s = (q @ k.transpose(1, 2) * d ** -0.5).masked_fill(hidden, -math.inf)
+        if sink:
+            s = torch.cat([s, torch.zeros(nh, n, 1, device=DEV, dtype=torch.float64)], -1)
+        want = (torch.softmax(s, -1)[..., :L] @ v).transpose(0, 1).reshape(n, -1)
+        # 2 d sums and as many roundings of the scores (which grow to about 2 * 5 here) before the exponential
+        assert float((out[o:o + n].double() - want).norm() / want.norm()) < ATT_TOL[torch.float32]
+        o += n
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("nh,nkv,d", [(4, 2, 16), (6, 2, 32), (5, 5, 48), (32, 8, 128), (4, 1, 256), (16, 2, 64)])
 @pytest.mark.parametrize("window", [0, 300])
