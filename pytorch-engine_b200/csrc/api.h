@@ -235,6 +235,11 @@ int pe_mlstm_recurrence(int dtype, const void* q, const void* k, const void* v, 
     const float* gates, const float* gate_bias, const float* norm_w, float cap, float eps, float q_scale, void* out,
     float* S, float* n, float* m, const int* seq_slot, const int* seq_qstart, int n_seqs, int max_q, int heads, int d,
     int dv, int n_slots, int chunk, int max_chunks, float* scratch, int* status, cudaStream_t stream);
+long long pe_mlstm_walk_scratch_floats(int n_tokens, int heads, int d, int dv);
+int pe_mlstm_walk(int dtype, const void* q, const void* k, const void* v, const void* g, long long ld, const float* gates,
+    const float* gate_bias, const float* norm_w, float cap, float eps, float q_scale, void* out, float* S, float* n, float* m,
+    const int* seq_slot, const int* seq_qstart, int n_tokens, int n_seqs, int heads, int d, int dv, int n_slots, float* scratch,
+    int* status, cudaStream_t stream);
 long long pe_mlstm_scratch_floats(int n_seqs, int heads, int d, int dv, int max_chunks);
 
 // delta_rule.cu
@@ -246,6 +251,11 @@ int pe_delta_rule_recurrence(int dtype, const void* qkv, const float* a, const f
     const int* seq_slot, const int* seq_qstart, int n_seqs, int max_q, int heads, int kv_heads, int d, int dv, int n_slots,
     int chunk, int max_chunks, float* scratch, int head_decay, int gate_silu, long long a_ld, long long b_ld, int* status,
     cudaStream_t stream);
+long long pe_delta_rule_walk_scratch_floats(int n_tokens, int heads, int kv_heads, int d, int dv);
+int pe_delta_rule_walk(int dtype, const void* qkv, const float* a, const float* dt_bias, const float* A_log, const float* b,
+    const void* gate, long long gate_ld, const float* norm_w, float eps, float q_scale, void* out, float* S, const int* seq_slot,
+    const int* seq_qstart, int n_tokens, int n_seqs, int heads, int kv_heads, int d, int dv, int n_slots, float* scratch,
+    int head_decay, int gate_silu, long long a_ld, long long b_ld, int* status, cudaStream_t stream);
 long long pe_delta_rule_scratch_floats(int n_seqs, int heads, int d, int dv, int max_chunks);
 
 // moe.cu

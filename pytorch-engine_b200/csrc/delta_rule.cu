@@ -13,6 +13,7 @@
 // the run dtype.
 #include "api.h"
 #include "common.cuh"
+#include "walk.cuh"
 
 namespace pe {
 
@@ -493,6 +494,89 @@ __global__ void __launch_bounds__(1024) delta_chain_kernel(DeltaArgs a, int col_
   }
 }
 
+// ---- the walk over columns (walk.cuh): what comes before and behind it --------------------------------------------------
+// A step's vectors, once a token: k and q at unit length (q times q_scale), the decays, beta.  grid: tokens; a warp per key
+// head, then per head.
+template <typename T>
+__global__ void __launch_bounds__(256) delta_prepare_kernel(DeltaArgs a, float* kq, float* g, float* num) {
+  pdl_wait_block();
+  pdl_launch_dependents();
+  const int t = blockIdx.x, lane = threadIdx.x & 31, d = a.d;
+  const int channels = 2 * a.kv_heads * d + a.heads * a.dv;
+  const T* row = (const T*)a.qkv + (size_t)t * channels;
+  for (int unit = threadIdx.x >> 5; unit < a.kv_heads + a.heads; unit += blockDim.x >> 5) {
+    if (unit < a.kv_heads) {
+      float* dst = kq + ((size_t)t * a.kv_heads + unit) * 2 * d;
+      float k[4], q[4], k2 = 0.f, q2 = 0.f;          // d <= 128
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int i = lane + 32 * r;
+        k[r] = i < d ? to_f32<T>(row[(a.kv_heads + unit) * d + i]) : 0.f;
+        q[r] = i < d ? to_f32<T>(row[unit * d + i]) : 0.f;
+        k2 = fmaf(k[r], k[r], k2);
+        q2 = fmaf(q[r], q[r], q2);
+      }
+      const float kn = rsqrtf(warp_sum(k2) + 1e-6f), qn = rsqrtf(warp_sum(q2) + 1e-6f) * a.q_scale;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int i = lane + 32 * r;
+        if (i < d) {
+          dst[i] = k[r] * kn;
+          dst[d + i] = q[r] * qn;
+        }
+      }
+    } else {
+      const int h = unit - a.kv_heads;
+      const float rate = expf(a.A_log[h]);
+      for (int i = lane; i < d; i += 32) {
+        const float z = a.head_decay ? a.a[(size_t)t * a.a_ld + h] + a.dt_bias[h] : a.a[(size_t)t * a.a_ld + h * d + i] + a.dt_bias[h * d + i];
+        const float softplus = z > 20.f ? z : log1pf(expf(z));
+        g[((size_t)t * a.heads + h) * d + i] = expf(-rate * softplus);
+      }
+      if (lane == 0) num[((size_t)t * a.heads + h) * 2] = 1.f / (1.f + expf(-a.b[(size_t)t * a.b_ld + h]));
+    }
+  }
+}
+
+// The per-head norm and the gate.  grid: tokens; a warp per head.
+template <typename T>
+__global__ void __launch_bounds__(256) delta_finish_kernel(DeltaArgs a, const float* o) {
+  pdl_wait_block();
+  pdl_launch_dependents();
+  const int t = blockIdx.x, lane = threadIdx.x & 31, dv = a.dv;
+  for (int h = threadIdx.x >> 5; h < a.heads; h += blockDim.x >> 5) {
+    const float* src = o + ((size_t)t * a.heads + h) * dv;
+    float ss = 0.f;
+    for (int j = lane; j < dv; j += 32) ss = fmaf(src[j], src[j], ss);
+    const float inv = rsqrtf(warp_sum(ss) / (float)dv + a.eps);
+    for (int j = lane; j < dv; j += 32) {
+      const float gate = to_f32<T>(((const T*)a.gate)[(size_t)t * a.gate_ld + h * dv + j]);
+      const float y = src[j] * inv * a.norm_w[j] * (a.gate_silu ? gate : 1.f) / (1.f + expf(-gate));
+      ((T*)a.out)[((size_t)t * a.heads + h) * dv + j] = from_f32<T>(y);
+    }
+  }
+}
+
+template <typename T>
+static int delta_walk(const DeltaArgs& a, int n_tokens, float* scratch, cudaStream_t stream) {
+  float* kq = scratch;
+  float* g = kq + (size_t)n_tokens * a.kv_heads * 2 * a.d;
+  float* o = g + (size_t)n_tokens * a.heads * a.d;
+  float* num = o + (size_t)n_tokens * a.heads * a.dv;
+  launch(delta_prepare_kernel<T>, n_tokens, 256, 0, stream, a, kq, g, num);
+  PE_LAUNCH_CHECK();
+  WalkArgs w{};
+  const int channels = 2 * a.kv_heads * a.d + a.heads * a.dv;
+  w.kq = kq; w.g = g; w.num = num; w.v = (const T*)a.qkv + 2 * a.kv_heads * a.d; w.v_ld = channels; w.o = o; w.o_ld = a.dv;
+  w.S = a.S; w.n = nullptr; w.seq_slot = a.seq_slot; w.seq_qstart = a.seq_qstart;
+  w.heads = a.heads; w.key_heads = a.kv_heads; w.dv = a.dv; w.n_slots = a.n_slots; w.status = a.status;
+  launch_walk<T, kWalkDelta>(w, a.d, a.n_seqs, stream);
+  PE_LAUNCH_CHECK();
+  launch(delta_finish_kernel<T>, n_tokens, 256, 0, stream, a, (const float*)o);
+  PE_LAUNCH_CHECK();
+  return PE_OK;
+}
+
 template <typename T, int DREG, int SPLIT>
 static int delta_run(const DeltaArgs& a, cudaStream_t stream) {
   const int d = a.d, dv = a.dv;
@@ -576,6 +660,31 @@ extern "C" int pe_short_conv_silu(int dtype, const void* x, long long ld, int co
 // Floats of scratch that the chunked form needs for `max_chunks` chunks per sequence.
 extern "C" long long pe_delta_rule_scratch_floats(int n_seqs, int heads, int d, int dv, int max_chunks) {
   return (long long)n_seqs * max_chunks * heads * (long long)pe::delta_unit(d, dv);
+}
+
+// Floats of scratch for pe_delta_rule_walk; 0: these sizes are not taken.
+extern "C" long long pe_delta_rule_walk_scratch_floats(int n_tokens, int heads, int kv_heads, int d, int dv) {
+  if (!pe::walk_takes(d, dv) || n_tokens <= 0) return 0;
+  return (long long)n_tokens * (2ll * kv_heads * d + (long long)heads * (d + dv + 2));
+}
+
+// The same step as pe_delta_rule_recurrence, with each head's columns spread over the chip (walk.cuh): key sizes of 32, 64
+// and 128, value sizes that are multiples of 16.  scratch: pe_delta_rule_walk_scratch_floats floats; it and qkv 16-byte aligned.
+extern "C" int pe_delta_rule_walk(int dtype, const void* qkv, const float* a, const float* dt_bias, const float* A_log,
+                                  const float* b, const void* gate, long long gate_ld, const float* norm_w, float eps,
+                                  float q_scale, void* out, float* S, const int* seq_slot, const int* seq_qstart, int n_tokens,
+                                  int n_seqs, int heads, int kv_heads, int d, int dv, int n_slots, float* scratch, int head_decay,
+                                  int gate_silu, long long a_ld, long long b_ld, int* status, cudaStream_t stream) {
+  if (n_seqs <= 0 || n_tokens <= 0) return PE_OK;
+  if (heads <= 0 || kv_heads <= 0 || heads % kv_heads || n_seqs > 65535) return PE_ERR_BAD_ARGUMENT;
+  if (!pe::walk_takes(d, dv) || dv / pe::kWalkCols > 65535) return PE_ERR_UNSUPPORTED_SIZE;
+  if (!scratch || ((uintptr_t)scratch % 16) || ((uintptr_t)qkv % 16)) return PE_ERR_BAD_ARGUMENT;
+  pe::DeltaArgs args{qkv, a, dt_bias, A_log, b, gate, gate_ld, norm_w, eps, q_scale, out, S, seq_slot, seq_qstart,
+                     n_seqs, heads, kv_heads, d, dv, n_slots, 0, 1, nullptr, status, head_decay, gate_silu,
+                     a_ld > 0 ? a_ld : (long long)(head_decay ? heads : heads * d), b_ld > 0 ? b_ld : (long long)heads};
+  if (dtype == PE_F32) return pe::delta_walk<float>(args, n_tokens, scratch, stream);
+  if (dtype == PE_BF16) return pe::delta_walk<__nv_bfloat16>(args, n_tokens, scratch, stream);
+  return PE_ERR_UNSUPPORTED_DTYPE;
 }
 
 // chunk > 0: prompts cut into chunks of that many tokens (scratch from pe_delta_rule_scratch_floats, max_chunks >=

@@ -13,6 +13,7 @@
 // pre-activations from a product that writes float32.
 #include "api.h"
 #include "common.cuh"
+#include "walk.cuh"
 
 namespace pe {
 
@@ -309,6 +310,106 @@ __global__ void mlstm_chain_kernel(MlstmArgs a) {
   }
 }
 
+// ---- the walk over columns (walk.cuh): what comes before and behind it --------------------------------------------------
+// The first heads * n_seqs blocks take a head's gates and the chain of its maxima through a sequence; one more block a token
+// leaves k and q as float32 (q with its factor).
+constexpr int kGateTile = 1024;
+
+template <typename T>
+__global__ void __launch_bounds__(256) mlstm_prepare_kernel(MlstmArgs a, float* kq, float* num, float* em) {
+  __shared__ float s_i[kGateTile], s_f[kGateTile], s_m[kGateTile + 1];
+  pdl_wait_block();
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, H = a.heads, d = a.d;
+  if ((int)blockIdx.x >= H * a.n_seqs) {
+    const int t = (int)blockIdx.x - H * a.n_seqs;
+    const T* q = (const T*)a.q + (size_t)t * a.ld;
+    const T* k = (const T*)a.k + (size_t)t * a.ld;
+    float* dst = kq + (size_t)t * H * 2 * d;
+    for (int i = tid; i < H * d; i += blockDim.x) {
+      const int h = i / d, c = i - h * d;
+      dst[(size_t)h * 2 * d + c] = to_f32<T>(k[i]);
+      dst[(size_t)h * 2 * d + d + c] = to_f32<T>(q[i]) * a.q_scale;
+    }
+    return;
+  }
+  const int head = blockIdx.x % H, b = blockIdx.x / H;
+  const int slot = a.seq_slot[b];
+  if (slot < 0 || slot >= a.n_slots) return;       // the walk reports it
+  const int q0 = a.seq_qstart[b], q1 = a.seq_qstart[b + 1];
+  const float bi = a.gate_bias[head], bf = a.gate_bias[H + head];
+  float m = a.m[(size_t)slot * H + head];          // followed by thread 0
+  for (int tb = q0; tb < q1; tb += kGateTile) {
+    const int nb = min(kGateTile, q1 - tb);
+    __syncthreads();
+    for (int i = tid; i < nb; i += blockDim.x) {
+      const float* row = a.gates + (size_t)(tb + i) * 2 * H;
+      s_i[i] = a.cap * tanhf((row[head] + bi) / a.cap);
+      s_f[i] = log_sigmoid(a.cap * tanhf((row[H + head] + bf) / a.cap));
+    }
+    __syncthreads();
+    if (tid == 0) {
+      s_m[0] = m;
+#pragma unroll 8
+      for (int i = 0; i < nb; ++i) {
+        m = fmaxf(s_f[i] + m, s_i[i]);
+        s_m[i + 1] = m;
+      }
+    }
+    __syncthreads();
+    for (int i = tid; i < nb; i += blockDim.x) {
+      const float m_old = s_m[i], m_new = s_m[i + 1];
+      const size_t at = (size_t)(tb + i) * H + head;
+      num[at * 2] = expf(s_f[i] + m_old - m_new);
+      num[at * 2 + 1] = expf(s_i[i] - m_new);
+      em[at] = expf(-m_new);
+    }
+  }
+  if (tid == 0) a.m[(size_t)slot * H + head] = m;
+}
+
+// The read's denominator, the per-head norm and the gate.  grid: tokens; a warp per head.
+template <typename T>
+__global__ void __launch_bounds__(256) mlstm_finish_kernel(MlstmArgs a, const float* o, int o_ld, const float* em) {
+  pdl_wait_block();
+  pdl_launch_dependents();
+  const int t = blockIdx.x, lane = threadIdx.x & 31, dv = a.dv;
+  for (int h = threadIdx.x >> 5; h < a.heads; h += blockDim.x >> 5) {
+    const float* src = o + ((size_t)t * a.heads + h) * o_ld;
+    const float den = fmaxf(fabsf(src[dv]), em[(size_t)t * a.heads + h]) + 1e-6f;
+    float ss = 0.f;
+    for (int j = lane; j < dv; j += 32) {
+      const float x = src[j] / den;
+      ss = fmaf(x, x, ss);
+    }
+    const float inv = rsqrtf(warp_sum(ss) / (float)dv + a.eps);
+    for (int j = lane; j < dv; j += 32) {
+      const float gate = to_f32<T>(((const T*)a.g)[(size_t)t * a.ld + h * dv + j]);
+      ((T*)a.out)[((size_t)t * a.heads + h) * dv + j] = from_f32<T>(src[j] / den * inv * a.norm_w[h * dv + j] / (1.f + expf(-gate)));
+    }
+  }
+}
+
+template <typename T>
+static int mlstm_walk(const MlstmArgs& a, int n_tokens, float* scratch, cudaStream_t stream) {
+  const int o_ld = a.dv + 4;
+  float* kq = scratch;
+  float* o = kq + (size_t)n_tokens * a.heads * 2 * a.d;
+  float* num = o + (size_t)n_tokens * a.heads * o_ld;
+  float* em = num + (size_t)n_tokens * a.heads * 2;
+  launch(mlstm_prepare_kernel<T>, a.heads * a.n_seqs + n_tokens, 256, 0, stream, a, kq, num, em);
+  PE_LAUNCH_CHECK();
+  WalkArgs w{};
+  w.kq = kq; w.g = nullptr; w.num = num; w.v = a.v; w.v_ld = a.ld; w.o = o; w.o_ld = o_ld;
+  w.S = a.S; w.n = a.n; w.seq_slot = a.seq_slot; w.seq_qstart = a.seq_qstart;
+  w.heads = a.heads; w.key_heads = a.heads; w.dv = a.dv; w.n_slots = a.n_slots; w.status = a.status;
+  launch_walk<T, kWalkGated>(w, a.d, a.n_seqs, stream);
+  PE_LAUNCH_CHECK();
+  launch(mlstm_finish_kernel<T>, n_tokens, 256, 0, stream, a, (const float*)o, o_ld, (const float*)em);
+  PE_LAUNCH_CHECK();
+  return PE_OK;
+}
+
 template <typename T, int DREG, int SPLIT>
 static int mlstm_run(const MlstmArgs& a, int max_q, cudaStream_t stream) {
   const int d = a.d, dv = a.dv;
@@ -348,6 +449,28 @@ static int mlstm_run(const MlstmArgs& a, int max_q, cudaStream_t stream) {
 // Floats of scratch that the chunked form needs for `max_chunks` chunks per sequence.
 extern "C" long long pe_mlstm_scratch_floats(int n_seqs, int heads, int d, int dv, int max_chunks) {
   return (long long)n_seqs * max_chunks * heads * (long long)pe::mlstm_unit(d, dv);
+}
+
+// Floats of scratch for pe_mlstm_walk; 0: these sizes are not taken.
+extern "C" long long pe_mlstm_walk_scratch_floats(int n_tokens, int heads, int d, int dv) {
+  if (!pe::walk_takes(d, dv) || n_tokens <= 0) return 0;
+  return (long long)n_tokens * heads * (2ll * d + dv + 4 + 3);
+}
+
+// The same step as pe_mlstm_recurrence, with each head's columns spread over the chip (walk.cuh): key sizes of 32, 64 and
+// 128, value sizes that are multiples of 16.  scratch: pe_mlstm_walk_scratch_floats floats; it, v and v's rows 16-byte aligned.
+extern "C" int pe_mlstm_walk(int dtype, const void* q, const void* k, const void* v, const void* g, long long ld,
+                             const float* gates, const float* gate_bias, const float* norm_w, float cap, float eps, float q_scale,
+                             void* out, float* S, float* n, float* m, const int* seq_slot, const int* seq_qstart, int n_tokens,
+                             int n_seqs, int heads, int d, int dv, int n_slots, float* scratch, int* status, cudaStream_t stream) {
+  if (n_seqs <= 0 || n_tokens <= 0) return PE_OK;
+  if (heads <= 0 || !(cap > 0.f) || n_seqs > 65535) return PE_ERR_BAD_ARGUMENT;
+  if (!pe::walk_takes(d, dv) || dv / pe::kWalkCols + 1 > 65535) return PE_ERR_UNSUPPORTED_SIZE;
+  if (dtype != PE_F32 && dtype != PE_BF16) return PE_ERR_UNSUPPORTED_DTYPE;
+  if (!scratch || ((uintptr_t)scratch % 16) || ((uintptr_t)v % 16) || (ld * (dtype == PE_F32 ? 4 : 2)) % 16) return PE_ERR_BAD_ARGUMENT;
+  pe::MlstmArgs a{q, k, v, g, ld, gates, gate_bias, norm_w, cap, eps, q_scale, out, S, n, m, seq_slot, seq_qstart,
+                  n_seqs, heads, d, dv, n_slots, 0, 1, nullptr, status};
+  return dtype == PE_F32 ? pe::mlstm_walk<float>(a, n_tokens, scratch, stream) : pe::mlstm_walk<__nv_bfloat16>(a, n_tokens, scratch, stream);
 }
 
 // chunk > 0: prompts cut into chunks of that many tokens (scratch from pe_mlstm_scratch_floats, max_chunks >=

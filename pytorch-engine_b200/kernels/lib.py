@@ -84,6 +84,8 @@ _SIGNATURES = {
     "pe_rmsnorm_residual_sum": [I, P, P, P, I, P, P, P, I, I, F, P],
     "pe_mlstm_recurrence": [I, P, P, P, P, L, P, P, P, F, F, F, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P, P, P],
     "pe_short_conv_silu": [I, P, L, I, P, P, I, P, P, P, P, P, I, I, I, I, P, P],
+    "pe_mlstm_walk": [I, P, P, P, P, L, P, P, P, F, F, F, P, P, P, P, P, P, I, I, I, I, I, I, P, P, P],
+    "pe_delta_rule_walk": [I, P, P, P, P, P, P, L, P, F, F, P, P, P, P, I, I, I, I, I, I, I, P, I, I, L, L, P, P],
     "pe_delta_rule_recurrence": [I, P, P, P, P, P, P, L, P, F, F, P, P, P, P, I, I, I, I, I, I, I, I, I, P, I, I, L, L, P, P],
     "pe_moe_route": [P, P, I, I, I, P, P, P, I, P],
     "pe_moe_group": [P, I, I, I, P, P, P, P, P, P],
@@ -130,6 +132,8 @@ _SIGNATURES = {
 _RESTYPES = {"pe_wait_limit_polls": (L, []),
              "pe_attention_generic_scratch_floats": (L, [I, I, I, I]),
              "pe_wkv_scratch_floats": (L, [I, I, I, I]),
+             "pe_mlstm_walk_scratch_floats": (L, [I, I, I, I]),
+             "pe_delta_rule_walk_scratch_floats": (L, [I, I, I, I, I]),
              "pe_mlstm_scratch_floats": (L, [I, I, I, I, I]),
              "pe_delta_rule_scratch_floats": (L, [I, I, I, I, I]),
              "pe_ssd_scratch_floats": (L, [I, I, I, I, I]),

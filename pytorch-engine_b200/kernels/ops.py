@@ -785,6 +785,27 @@ def mlstm_recurrence(q, k, v, g, gates: torch.Tensor, gate_bias: torch.Tensor, n
     _count(3 if chunk > 0 else 1)
 
 
+def mlstm_walk_scratch_floats(n_tokens: int, heads: int, d: int, dv: int) -> int:
+    """Floats of scratch for ``mlstm_walk``; 0 if it does not take these sizes."""
+    return int(library().pe_mlstm_walk_scratch_floats(n_tokens, heads, d, dv))
+
+
+def mlstm_walk(q, k, v, g, gates: torch.Tensor, gate_bias: torch.Tensor, norm_w: torch.Tensor, cap: float, eps: float,
+               q_scale: float, out: torch.Tensor, S: torch.Tensor, n: torch.Tensor, m: torch.Tensor, seq_slot: torch.Tensor,
+               seq_qstart: torch.Tensor, n_seqs: int, heads: int, d: int, dv: int, status: torch.Tensor, scratch: torch.Tensor) -> None:
+    """``mlstm_recurrence`` with each head's columns spread over the chip (csrc/walk.cuh): for steps of several tokens a sequence."""
+    ld, n_tokens = q.stride(0), q.shape[0]
+    _need(all(t.stride(0) == ld and t.stride(1) == 1 and t.dtype == q.dtype for t in (q, k, v, g)), "mlstm: q, k, v, g share a row stride")
+    _need(gates.dtype == torch.float32 and gates.is_contiguous() and S.dtype == torch.float32 and S.is_contiguous()
+          and n.is_contiguous() and m.is_contiguous() and out.is_contiguous() and out.dtype == q.dtype, "mlstm: layouts")
+    _need(scratch.dtype == torch.float32 and scratch.numel() >= mlstm_walk_scratch_floats(n_tokens, heads, d, dv), "mlstm_walk: scratch")
+    check(library().pe_mlstm_walk(dtype_tag(q.dtype), _ptr(q), _ptr(k), _ptr(v), _ptr(g), ld, _ptr(gates), _ptr(gate_bias),
+                                  _ptr(norm_w), float(cap), float(eps), float(q_scale), _ptr(out), _ptr(S), _ptr(n), _ptr(m),
+                                  _ptr(seq_slot), _ptr(seq_qstart), n_tokens, n_seqs, heads, d, dv, S.shape[0], _ptr(scratch),
+                                  _ptr(status), _stream()), "mlstm_walk")
+    _count(3)
+
+
 def mlstm_scratch_floats(n_seqs: int, heads: int, d: int, dv: int, max_chunks: int) -> int:
     return int(library().pe_mlstm_scratch_floats(n_seqs, heads, d, dv, max_chunks))
 
@@ -825,6 +846,32 @@ def delta_rule_recurrence(qkv: torch.Tensor, a: torch.Tensor, dt_bias: torch.Ten
                                              1 if gate_silu else 0, a.stride(0), b.stride(0), _ptr(status), _stream()),
           "delta_rule_recurrence")
     _count(3 if chunk > 0 else 1)
+
+
+def delta_rule_walk_scratch_floats(n_tokens: int, heads: int, kv_heads: int, d: int, dv: int) -> int:
+    """Floats of scratch for ``delta_rule_walk``; 0 if it does not take these sizes."""
+    return int(library().pe_delta_rule_walk_scratch_floats(n_tokens, heads, kv_heads, d, dv))
+
+
+def delta_rule_walk(qkv: torch.Tensor, a: torch.Tensor, dt_bias: torch.Tensor, A_log: torch.Tensor, b: torch.Tensor,
+                    gate: torch.Tensor, norm_w: torch.Tensor, eps: float, q_scale: float, out: torch.Tensor, S: torch.Tensor,
+                    seq_slot: torch.Tensor, seq_qstart: torch.Tensor, n_seqs: int, heads: int, kv_heads: int, d: int, dv: int,
+                    status: torch.Tensor, scratch: torch.Tensor, head_decay: bool = False, gate_silu: bool = False) -> None:
+    """``delta_rule_recurrence`` with each head's columns spread over the chip (csrc/walk.cuh): for steps of several tokens a
+    sequence."""
+    n_tokens = qkv.shape[0]
+    _need(a.shape[1] == (heads if head_decay else heads * d) and dt_bias.numel() == a.shape[1], "delta_rule: the decay's layout")
+    _need(qkv.is_contiguous() and qkv.shape[1] == 2 * kv_heads * d + heads * dv, "delta_rule: q|k|v layout")
+    _need(a.dtype == torch.float32 and a.stride(1) == 1 and b.dtype == torch.float32 and b.stride(1) == 1, "delta_rule: a, b f32")
+    _need(gate.stride(1) == 1 and gate.dtype == qkv.dtype and out.is_contiguous() and S.is_contiguous(), "delta_rule: layouts")
+    _need(scratch.dtype == torch.float32 and scratch.numel() >= delta_rule_walk_scratch_floats(n_tokens, heads, kv_heads, d, dv),
+          "delta_rule_walk: scratch")
+    check(library().pe_delta_rule_walk(dtype_tag(qkv.dtype), _ptr(qkv), _ptr(a), _ptr(dt_bias), _ptr(A_log), _ptr(b), _ptr(gate),
+                                       gate.stride(0), _ptr(norm_w), float(eps), float(q_scale), _ptr(out), _ptr(S), _ptr(seq_slot),
+                                       _ptr(seq_qstart), n_tokens, n_seqs, heads, kv_heads, d, dv, S.shape[0], _ptr(scratch),
+                                       1 if head_decay else 0, 1 if gate_silu else 0, a.stride(0), b.stride(0), _ptr(status),
+                                       _stream()), "delta_rule_walk")
+    _count(3)
 
 
 def delta_rule_scratch_floats(n_seqs: int, heads: int, d: int, dv: int, max_chunks: int) -> int:

@@ -929,3 +929,98 @@ def test_a_bounded_wait_gives_up_within_seconds(ops):
     assert 1e-7 < poll < 2e-5, f"one failing poll took {poll * 1e6:.2f} us"
     limit = ops.wait_limit_seconds(DEV)
     assert 0.5 < limit < 10.0, f"a wait that nothing ends would last {limit:.1f} s"
+
+
+def _near(got, want, tol):
+    return float((got.double() - want).norm() / want.norm()) < tol
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 5e-6), (torch.bfloat16, 6e-3)])   # float32 chains of 25 tokens; one rounding
+@pytest.mark.parametrize("heads,kv_heads,d,dv", [(4, 2, 128, 128), (2, 2, 64, 48), (3, 1, 32, 16), (2, 1, 128, 256)])
+@pytest.mark.parametrize("head_decay", [False, True])
+def test_delta_rule_walk(ops, dtype, tol, heads, kv_heads, d, dv, head_decay):
+    """Sequences that end before, at and behind a stage of eight tokens, from states that are not zero, against 64 bits and
+    against the kernel that keeps a head in one block."""
+    torch.manual_seed(40)
+    lens, slots = [1, 7, 8, 9, 25], [3, 0, 5, 1, 2]
+    N, n = sum(lens), len(lens)
+    qkv = torch.randn(N, 2 * kv_heads * d + heads * dv, device=DEV).to(dtype)
+    a = torch.randn(N, heads if head_decay else heads * d, device=DEV)
+    dt = torch.randn(a.shape[1], device=DEV) - 3.0
+    A_log, b = torch.randn(heads, device=DEV) * 0.5, torch.randn(N, heads, device=DEV)
+    gate, w = torch.randn(N, heads * dv, device=DEV).to(dtype), torch.rand(dv, device=DEV) + 0.5
+    S0 = torch.randn(6, heads, d, dv, device=DEV)
+    qstart = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    slot = torch.tensor(slots, dtype=torch.int32, device=DEV)
+    floats = ops.delta_rule_walk_scratch_floats(N, heads, kv_heads, d, dv)
+    assert floats > 0 and ops.delta_rule_walk_scratch_floats(N, heads, kv_heads, 96, dv) == 0 and ops.delta_rule_walk_scratch_floats(N, heads, kv_heads, d, 24) == 0
+    S, S1, st = S0.clone(), S0.clone(), _status()
+    out, out1 = (torch.zeros(N, heads * dv, device=DEV, dtype=dtype) for _ in range(2))
+    args = (qkv, a, dt, A_log, b, gate, w, 1e-5, d ** -0.5)
+    form = dict(head_decay=head_decay, gate_silu=head_decay)
+    ops.delta_rule_walk(*args, out, S, slot, qstart, n, heads, kv_heads, d, dv, st, torch.full((floats,), float("nan"), device=DEV), **form)
+    ops.delta_rule_recurrence(*args, out1, S1, slot, qstart, n, max(lens), heads, kv_heads, d, dv, st, **form)
+    assert st.tolist()[0] == 0
+    q, k, v = qkv.double().split([kv_heads * d, kv_heads * d, heads * dv], 1)
+    q, k = (x.view(N, kv_heads, d).repeat_interleave(heads // kv_heads, 1) for x in (q, k))
+    q = q / (q.pow(2).sum(-1, keepdim=True) + 1e-6).sqrt() * d ** -0.5
+    k = k / (k.pow(2).sum(-1, keepdim=True) + 1e-6).sqrt()
+    z = (a.double() + dt.double()).view(N, heads, -1)
+    g = torch.exp(-A_log.double().exp()[None, :, None] * torch.nn.functional.softplus(z)).expand(N, heads, d)
+    o, end = torch.empty(N, heads, dv, dtype=torch.float64, device=DEV), S0.double()
+    t = 0
+    for L, s in zip(lens, slots):
+        M = end[s]
+        for _ in range(L):
+            M = g[t][:, :, None] * M
+            u = torch.sigmoid(b[t].double())[:, None] * (v[t].view(heads, dv) - torch.einsum("hij,hi->hj", M, k[t]))
+            M = M + k[t][:, :, None] * u[:, None]
+            o[t] = torch.einsum("hij,hi->hj", M, q[t])
+            t += 1
+        end[s] = M
+    gd = gate.double().view(N, heads, dv)
+    y = o / (o.pow(2).mean(-1, keepdim=True) + 1e-5).sqrt() * w.double() * torch.sigmoid(gd) * (gd if head_decay else 1.0)
+    assert _near(out, y.reshape(N, -1), tol) and _near(S, end, 5e-6)
+    assert _near(out1, y.reshape(N, -1), tol) and torch.equal(S[4], S0[4])     # the slot that no sequence has
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 6e-3)])   # (a small denominator magnifies its sum's rounding)
+@pytest.mark.parametrize("heads,d,dv", [(3, 128, 256), (2, 64, 48), (5, 32, 16)])
+def test_mlstm_walk(ops, dtype, tol, heads, d, dv):
+    """As above for the matrix memory with exponential gates; one sequence is longer than a tile of its gates."""
+    torch.manual_seed(41)
+    lens, slots = [1, 8, 9, 23, 1030], [3, 0, 5, 1, 2]
+    N, n = sum(lens), len(lens)
+    rows = torch.randn(N, 2 * heads * (d + dv), device=DEV).to(dtype)
+    q, k, v, g = rows.split([heads * d, heads * d, heads * dv, heads * dv], 1)
+    gates, bias = torch.randn(N, 2 * heads, device=DEV), torch.cat([torch.randn(heads), torch.randn(heads) + 4.0]).to(DEV)
+    w = torch.rand(heads * dv, device=DEV) + 0.5
+    S0, n0, m0 = torch.randn(6, heads, d, dv, device=DEV), torch.randn(6, heads, d, device=DEV), torch.randn(6, heads, device=DEV)
+    qstart = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    slot = torch.tensor(slots, dtype=torch.int32, device=DEV)
+    floats = ops.mlstm_walk_scratch_floats(N, heads, d, dv)
+    assert floats > 0 and ops.mlstm_walk_scratch_floats(N, heads, 96, dv) == 0
+    S, nv, m, st = S0.clone(), n0.clone(), m0.clone(), _status()
+    out = torch.zeros(N, heads * dv, device=DEV, dtype=dtype)
+    ops.mlstm_walk(q, k, v, g, gates, bias, w, 15.0, 1e-5, d ** -0.5, out, S, nv, m, slot, qstart, n, heads, d, dv, st,
+                   torch.full((floats,), float("nan"), device=DEV))
+    assert st.tolist()[0] == 0
+    z = 15.0 * torch.tanh((gates.double() + bias.double()) / 15.0)
+    gi, gf = z[:, :heads], torch.nn.functional.logsigmoid(z[:, heads:])
+    qd, kd, vd = q.double().view(N, heads, d) * d ** -0.5, k.double().view(N, heads, d), v.double().view(N, heads, dv)
+    o, eS, en, em = torch.empty(N, heads, dv, dtype=torch.float64, device=DEV), S0.double(), n0.double(), m0.double()
+    t = 0
+    for L, s in zip(lens, slots):
+        M, nn, mm = eS[s], en[s], em[s]
+        for _ in range(L):
+            new = torch.maximum(gf[t] + mm, gi[t])
+            keep, take = torch.exp(gf[t] + mm - new)[:, None], torch.exp(gi[t] - new)[:, None]
+            M = keep[..., None] * M + (take * kd[t])[:, :, None] * vd[t][:, None]
+            nn, mm = keep * nn + take * kd[t], new
+            den = torch.maximum((nn * qd[t]).sum(-1).abs(), torch.exp(-mm)) + 1e-6
+            o[t] = torch.einsum("hij,hi->hj", M, qd[t]) / den[:, None]
+            t += 1
+        eS[s], en[s], em[s] = M, nn, mm
+    y = o / (o.pow(2).mean(-1, keepdim=True) + 1e-5).sqrt() * w.double().view(heads, dv) * torch.sigmoid(g.double().view(N, heads, dv))
+    assert _near(out, y.reshape(N, -1), tol) and _near(S, eS, 1e-5) and _near(nv, en, 1e-5) and _near(m, em, 1e-5)
+    assert torch.equal(S[4], S0[4])
