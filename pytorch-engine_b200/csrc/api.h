@@ -138,6 +138,13 @@ int pe_gemm_umma_glu(const void* x, long long ldx, const void* w, void* y, long 
 int pe_gemm_umma(const void* x, long long ldx, const void* w, void* y, long long ldy, int M, int N, int K,
     int out_f32, int pair_offset, int n_sms, int* status, cudaStream_t stream);
 
+// gemm_split32.cu
+int pe_gemm_split32_supported(int M, int N, int K);
+long long pe_gemm_split32_scratch_floats(int M, int N, int K, int n_sms);
+int pe_gemm_split32_launches(int M, int N, int K, int n_sms);
+int pe_gemm_split32(const float* x, long long ldx, const float* w, float* y, long long ldy, int M, int N, int K,
+    float* scratch, int n_sms, int* status, cudaStream_t stream);
+
 // gemm_umma2.cu
 int pe_gemm_umma2_supported(int M, int N, int K, int pair_offset);
 int pe_gemm_umma2_glu(const void* x, long long ldx, const void* w, void* y, long long ldy, int M, int N, int K,

@@ -52,6 +52,9 @@ _SIGNATURES = {
     "pe_gemm_smallm": [P, L, P, P, L, I, I, I, I, I, I, P],
     "pe_gemm_smallm_supported": [I, I, I],
     "pe_gemm_smallm_grouped": [P, L, L, I, I, P, P, L, I, I, I, I, P],
+    "pe_gemm_split32_supported": [I, I, I],
+    "pe_gemm_split32_launches": [I, I, I, I],
+    "pe_gemm_split32": [P, L, P, P, L, I, I, I, P, I, P, P],
     "pe_gemm_umma": [P, L, P, P, L, I, I, I, I, I, I, P, P],
     "pe_gemm_umma_supported": [I, I, I, I],
     "pe_gemm_umma2": [P, L, P, P, L, I, I, I, I, I, I, P, P],
@@ -131,6 +134,7 @@ _SIGNATURES = {
 }
 _RESTYPES = {"pe_wait_limit_polls": (L, []),
              "pe_attention_generic_scratch_floats": (L, [I, I, I, I]),
+             "pe_gemm_split32_scratch_floats": (L, [I, I, I, I]),
              "pe_wkv_scratch_floats": (L, [I, I, I, I]),
              "pe_mlstm_walk_scratch_floats": (L, [I, I, I, I]),
              "pe_delta_rule_walk_scratch_floats": (L, [I, I, I, I, I]),

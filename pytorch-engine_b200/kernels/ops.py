@@ -544,6 +544,27 @@ def gemm_umma(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, status: 
     _count(1)
 
 
+def gemm_split32_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether csrc/gemm_split32.cu takes ``x [M, K] @ weight^T``: float32, K % 4 == 0, 16-byte aligned rows."""
+    return (x.dtype == torch.float32 and weight.dtype == torch.float32 and x.dim() == 2 and x.stride(1) == 1
+            and x.stride(0) % 4 == 0 and x.stride(0) >= x.shape[1] and x.data_ptr() % 16 == 0 and weight.is_contiguous()
+            and weight.data_ptr() % 16 == 0 and bool(library().pe_gemm_split32_supported(x.shape[0], weight.shape[0], x.shape[1])))
+
+
+def gemm_split32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, status: torch.Tensor) -> None:
+    """``out[M, N] = x @ weight^T`` in float32 on the tcgen05 tensor cores, each operand split into three bfloat16 parts."""
+    _need(gemm_split32_supported(x, weight), "gemm_split32: needs float32, K % 4 == 0, aligned and dense rows")
+    m, k = x.shape
+    n = weight.shape[0]
+    _need(out.dtype == torch.float32 and out.shape == (m, n) and out.stride(1) == 1 and out.stride(0) >= n
+          and out.stride(0) % 4 == 0 and out.data_ptr() % 16 == 0 and weight.shape[1] == k, "gemm_split32: out float32 [M, N], aligned rows")
+    sms = sm_count(x.device)
+    scratch = torch.empty(int(library().pe_gemm_split32_scratch_floats(m, n, k, sms)), dtype=torch.float32, device=x.device)
+    check(library().pe_gemm_split32(_ptr(x), x.stride(0), _ptr(weight), _ptr(out), out.stride(0), m, n, k, _ptr(scratch), sms,
+                                    _ptr(status), _stream()), "gemm_split32")
+    _count(int(library().pe_gemm_split32_launches(m, n, k, sms)))
+
+
 def gemm_umma2_supported(x: torch.Tensor, weight: torch.Tensor, pair_offset: int = 0) -> bool:
     """Whether csrc/gemm_umma2.cu takes the product: as ``gemm_umma_supported``, and K % 64 == 0."""
     if not gemm_umma_supported(x, weight, pair_offset):

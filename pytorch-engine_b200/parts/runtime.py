@@ -87,6 +87,9 @@ class Runtime:
         self.own_large_gemm = True
         self.large_gemm_rows = 1024
         self.large_gemm_min_fill = 0.8   # least share of the waves of tiles that does work (see takes_large_gemm)
+        # float32 products with at least this many rows run on csrc/gemm_split32.cu (16 rows: 12-15 us against the library's
+        # 19-24 on the 0.6B shape; single tokens stay with the library)
+        self.split32_rows = 16
         self.pair_gemm = True       # large products on tcgen05 cta_group::2
         # q/k-norm, rotation and cache append in the epilogue of the q|k|v product where the pair kernel runs it
         # (PE_B200_FUSE_QKV_ROPE=0 keeps them kernels of their own, for comparisons)
@@ -129,6 +132,14 @@ class Runtime:
         # library, which has smaller tiles to choose from (8B shape, 1,536 rows, down projection: 96 tiles
         # on 74 pairs took 133 us against 103 us).
         return bool(pair_offset) or large_gemm_fill(x.shape[0], weight.shape[0], ops.sm_count(x.device)) >= self.large_gemm_min_fill
+
+    def takes_split32_gemm(self, x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor], out_dtype) -> bool:
+        """Whether a float32 product runs on csrc/gemm_split32.cu (float32's precision on the tensor cores)."""
+        return (x.dtype == torch.float32 and self.own_large_gemm and x.dim() == 2 and x.shape[0] >= self.split32_rows
+                and out_dtype in (None, torch.float32) and ops.gemm_split32_supported(x, weight)
+                and (out is None or (out.dtype == torch.float32 and out.stride(1) == 1 and out.stride(0) % 4 == 0
+                                     and out.stride(0) >= weight.shape[0] and out.data_ptr() % 16 == 0))
+                and (out is not None or weight.shape[0] % 4 == 0))
 
     def fetch_tokens(self, n: int):
         """The first ``n`` ints of ``token_area`` as a list, after checking the status word: one
@@ -197,6 +208,11 @@ class Runtime:
             if out is None:
                 out = torch.empty((x.shape[0], weight.shape[0]), dtype=out_dtype or x.dtype, device=x.device)
             ops.gemm_smallm(x, weight, out)
+            return out
+        if self.takes_split32_gemm(x, weight, out, out_dtype):
+            if out is None:
+                out = torch.empty((x.shape[0], weight.shape[0]), dtype=torch.float32, device=x.device)
+            ops.gemm_split32(x, weight, out, self.status)
             return out
         if x.dtype == torch.float32:
             prev = torch.backends.cuda.matmul.allow_tf32

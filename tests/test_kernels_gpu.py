@@ -642,6 +642,37 @@ def test_gemm_umma(ops, M, N, K, kernel):
     assert st.tolist()[0] == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 1, 4), (16, 128, 64), (63, 127, 60), (65, 132, 68), (129, 260, 1000), (200, 1024, 3072),
+                                   (600, 4096, 1024), (40, 256, 8192)])
+def test_gemm_split32(ops, M, N, K):
+    """Float32 products on the tensor cores at the edges of tiles, chunks and ranges of K: no further from 64 bits than float32
+    multiply-adds, for rows of any scale and next to numbers that have no bfloat16 parts."""
+    torch.manual_seed(32)
+    wide = torch.randn(M, K + 8, device=DEV) * torch.logspace(-18, 18, M, device=DEV)[:, None]
+    x, w = wide[:, :K], torch.randn(N, K, device=DEV) * 0.5
+    assert ops.gemm_split32_supported(x, w)
+    out = torch.full((M, -(-N // 4) * 4 + 4), float("nan"), device=DEV)
+    st = _status()
+    ops.gemm_split32(x, w, out[:, :N], st)
+    assert st.tolist()[0] == 0 and bool(out[:, N:].isnan().all())
+    want = x.double() @ w.double().t()
+    row_err = ((out[:, :N].double() - want).norm(dim=1) / want.norm(dim=1)).max()
+    # parts: 3 dropped products of 2^-27; sums: 64 of K in the tensor core (2^-23 a step at worst, 4 large steps) and a chain
+    # of K / 64 roundings of 2^-24
+    scale = (x.double().norm(dim=1)[:, None] * w.double().norm(dim=1)[None]).norm(dim=1) / want.norm(dim=1)
+    assert float(row_err) < (4 * 2.0 ** -23 + (1 + (K / 64) ** 0.5) * 2.0 ** -24) * max(1.0, float(scale.max()) / 8)
+    if M >= 16 and K >= 64:
+        x = x.contiguous().clone()
+        x[3, 5], x[7, 0], x[9, 9], x[11, 1] = float("inf"), float("nan"), 3.4e38, -float("inf")
+        w = w.clone()
+        w[N // 2, 2] = float("inf")
+        ops.gemm_split32(x, w, out[:, :N], st)
+        ref = torch.mm(x, w.t())
+        assert torch.equal(out[:, :N].isnan(), ref.isnan()) and torch.equal(out[:, :N].isinf(), ref.isinf())
+        fin = ref.isfinite()
+        assert rel_err(out[:, :N][fin].cpu() / ref[fin].abs().max().cpu(), ref[fin].cpu() / ref[fin].abs().max().cpu()) < 1e-5
+
+
 @pytest.mark.parametrize("M,I,K", [(128, 128, 64), (200, 384, 200), (1000, 1280, 1024), (5, 256, 4096)])
 @pytest.mark.parametrize("kernel", ["gemm_umma", "gemm_umma2"])
 def test_gemm_umma_with_the_gate_fused(ops, M, I, K, kernel):
