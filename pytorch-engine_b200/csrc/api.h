@@ -36,6 +36,7 @@ int pe_attention_decode_noalloc(int dtype, const void* q, long long q_ld, void* 
     const void* v_pages, int split_keys, int max_splits, int* status, cudaStream_t stream);
 
 // attention_mma.cu
+int pe_attention_mma_decode_launches(int pairs, int split_keys, int max_splits);
 int pe_attention_mma_decode_blocks_per_sm(int head_dim, int v_dim);
 int pe_attention_mma_dims_supported(int head_dim, int v_dim, int n_heads, int n_kv_heads);
 int pe_attention_mma_supported(int head_dim, int n_heads, int n_kv_heads);

@@ -474,8 +474,26 @@ __device__ __forceinline__ int range_keys(const Args& a, int len) {
   return max(max(BN, a.min_range_keys), (per + BN - 1) / BN * BN);
 }
 
+// A cluster's blocks: its barrier (every thread of a block that is still there takes part) and a float of another block's
+// shared memory.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
+}
+__device__ __forceinline__ float cluster_load(const float* p, int rank) {
+  uint32_t at;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(at) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(at) : "memory");
+  return v;
+}
+// Ranges that one cluster holds at most (the portable size), blocks up to which a step's ranges are clusters.
+constexpr int kClusterRanges = 8, kClusterBlocks = 64;
+
 // grid: (max_splits, n_kv_heads, n_seqs); block: 128 threads; STAGES pages in flight.
-template <int HD, int VD, int STAGES, bool SPLIT_P, bool PAD>
+// CLUSTER: the ranges of a (sequence, kv head) are one cluster, and its blocks put them together through each other's shared
+// memory, a share of the outputs each: no partial results in global memory and no second kernel, which a step waits for
+// once a layer.
+template <int HD, int VD, int STAGES, bool SPLIT_P, bool PAD, bool CLUSTER>
 __global__ void __launch_bounds__(128) decode_split_kernel(Args a, const __grid_constant__ CUtensorMap kmap,
                                                            const __grid_constant__ CUtensorMap vmap) {
   extern __shared__ char smem_raw[];
@@ -554,19 +572,30 @@ __global__ void __launch_bounds__(128) decode_split_kernel(Args a, const __grid_
     const int nxt = it + STAGES - 1;
     if (tid == 0 && nxt < n_tiles)
       issue_page<HD, VD>(a, &kmap, &vmap, slot, kvh, tile_k0(nxt), smem + (nxt % STAGES) * STAGE, &bars[nxt % STAGES]);
-    if (!tma::mbar_wait(&bars[it % STAGES], (it / STAGES) & 1)) {
+    const bool there = tma::mbar_wait(&bars[it % STAGES], (it / STAGES) & 1);
+    if (!CLUSTER && !there) {
       give_up(a, bars, STAGES, 2);
       return;
     }
     const int k0 = tile_k0(it);
     decode_fold_page<HD, VD, SPLIT_P>(smem_u32(smem + (it % STAGES) * STAGE), smem_u32(smem + (it % STAGES) * STAGE) + BN * HD * 2,
                          warp * 16, k0, k_first, k_hi, hole_lo, hole_hi, a.scale_log2, qf, o, m_lo, m_hi, l_lo, l_hi, lane);
-    __syncthreads();
+    if (CLUSTER) {
+      // the whole block leaves the loop together, and stays for the cluster's barriers: others read its shared memory
+      if (__syncthreads_or(!there)) {
+        give_up(a, bars, STAGES, 2);
+        break;
+      }
+    } else {
+      __syncthreads();
+    }
   }
   pdl_launch_dependents();
   // merge the four warps (fixed order) through shared memory laid over the stages
   float* ml = reinterpret_cast<float*>(smem);            // [4 warps][16 rows][2]
   float* acc = ml + 4 * 16 * 2;                          // [4 warps][16 rows][VD]
+  float* res = acc + 4 * 16 * VD;                        // CLUSTER: [16 rows][VD] sums of the block, then
+  float* res_ml = res + 16 * VD;                         // [16 rows] maximum and denominator
   if (t == 0) {
     ml[(warp * 16 + g) * 2] = m_lo;     ml[(warp * 16 + g) * 2 + 1] = l_lo;
     ml[(warp * 16 + g + 8) * 2] = m_hi; ml[(warp * 16 + g + 8) * 2 + 1] = l_hi;
@@ -594,10 +623,64 @@ __global__ void __launch_bounds__(128) decode_split_kernel(Args a, const __grid_
         aa += acc[(size_t)(w * 16 + r) * VD + c] * f;
       }
     }
+    if (CLUSTER) {
+      res[r * VD + c] = aa;
+      if (c == 0) {
+        res_ml[2 * r] = mm;
+        res_ml[2 * r + 1] = ll;
+      }
+      continue;
+    }
     const size_t pidx = ((size_t)b * a.n_heads + (kvh * group + r)) * a.max_splits + split;
     a.part_acc[pidx * vd + c] = (ll > 0.f) ? aa / ll : 0.f;
     // log-sum-exp in natural units, as the merge kernel expects: (m + log2 l) * ln 2
     if (c == 0) a.part_lse[pidx] = (ll > 0.f) ? (mm + log2f(ll)) * 0.6931471805599453f : -INFINITY;
+  }  if (CLUSTER) {
+    // the ranges that hold something, and this one's place among them (as in the merge kernel below)
+    const int n_splits = (len + per_range - 1) / per_range;
+    const int first = min(win_lo / per_range, n_splits), kept = min((keep + per_range - 1) / per_range, first);
+    const int n_live = kept + n_splits - first, mine = split < kept ? split : kept + split - first;
+    if (n_live > 1) cluster_sync();
+    else __syncthreads();
+    for (int i = mine * 128 + tid; i < group * vd; i += n_live * 128) {
+      const int r = i / vd, c = i - r * vd, h = kvh * group + r;
+      float m[kClusterRanges], l[kClusterRanges], x[kClusterRanges];
+      float mx = a.sink ? 0.f : -INFINITY;
+#pragma unroll
+      for (int k = 0; k < kClusterRanges; ++k) {
+        const bool live = k < n_live;
+        const int rank = k < kept ? k : first + k - kept;
+        m[k] = live ? cluster_load(res_ml + 2 * r, rank) : -INFINITY;
+        l[k] = live ? cluster_load(res_ml + 2 * r + 1, rank) : 0.f;
+        x[k] = live ? cluster_load(res + r * VD + c, rank) : 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < kClusterRanges; ++k) mx = fmaxf(mx, m[k]);
+      float denom = a.sink ? exp2f(-mx) : 0.f, v = 0.f;
+#pragma unroll
+      for (int k = 0; k < kClusterRanges; ++k) {
+        const float f = m[k] == -INFINITY ? 0.f : exp2f(m[k] - mx);
+        denom = fmaf(l[k], f, denom);
+        v = fmaf(x[k], f, v);
+      }
+      v /= fmaxf(denom, 1e-20f);
+      if (a.gate) v *= gate_of(a, tq, h);
+      if (a.out_cos) {
+        // features c and c ^ 1 are one interleaved pair in adjacent lanes (turned outputs: 64 or 128 features)
+        const float other = __shfl_xor_sync(0xffffffffu, v, 1);
+        const int pos = len - 1;
+        if (pos < 0 || pos >= a.out_rows) {
+          if (c == 0) report(a.status, kStatusPositionOutOfRange, tq, pos, a.out_rows);
+          continue;
+        }
+        const float cs = a.out_cos[(size_t)pos * (vd / 2) + (c >> 1)], sn = a.out_sin[(size_t)pos * (vd / 2) + (c >> 1)];
+        v = (c & 1) ? v * cs - other * sn : v * cs + other * sn;
+      }
+      const size_t at = (size_t)tq * a.out_ld + (size_t)h * vd + c;
+      if (a.out_f32) reinterpret_cast<float*>(a.out)[at] = v;
+      else a.out[at] = __float2bfloat16_rn(v);
+    }
+    if (n_live > 1) cluster_sync();    // nobody leaves while its shared memory is read
   }
 }
 
@@ -677,6 +760,26 @@ __global__ void decode_merge_kernel(Args a) {
   }
 }
 
+// The tile sizes that rows of these sizes run in.
+static int tile_of(int dim) { return (dim + 63) / 64 * 64; }
+
+// Decode blocks that one SM holds at a time (shared memory bound).
+static int decode_blocks_per_sm(int head_dim, int v_dim) {
+  const size_t hd = tile_of(head_dim), vd = tile_of(v_dim);
+  const size_t stage = (size_t)BN * (hd + vd) * 2;
+  const size_t smem = 3 * stage + 16 * hd * 2 + 1024 + 1024;   // + the block's static and reserved part
+  const int n = (int)((227 * 1024) / smem);
+  return n < 1 ? 1 : n;
+}
+// Whether a decode step's ranges are put together inside clusters: cut by the sequences' own lengths, and few.  One sequence
+// of 300 keys, 8 kv heads: 7.1 -> 5.7 us, a step of the 0.6B shape 750 -> 723 us.  With more blocks the second kernel is better:
+// 64 pairs of four ranges take 26.8 instead of 28.7 us by themselves, but the product behind them, which then starts while
+// they drain, loses twice that (8B shape, 8 sequences of 4,090 keys: 1,488 -> 1,535 us a step), and with more blocks than the
+// chip holds clusters wait for room (64 sequences of up to 4,096 keys: 94 -> 112 us).
+static bool cluster_ranges(int pairs, int split_keys, int max_splits) {
+  return split_keys == 0 && max_splits <= kClusterRanges && (long long)pairs * max_splits <= kClusterBlocks;
+}
+
 template <typename K>
 static int opt_in(K kernel, size_t bytes) {
   if (bytes > 227 * 1024) return PE_ERR_UNSUPPORTED_SIZE;
@@ -709,18 +812,37 @@ static int launch(const Args& a, bool decode, int n_seqs, int max_q, cudaStream_
   }
   dim3 grid(a.max_splits, a.n_kv_heads, n_seqs);
   if (grid.y > 65535 || grid.z > 65535) return PE_ERR_UNSUPPORTED_SIZE;
-  auto go = [&](auto kern, int STAGES) -> int {
+  auto go = [&](auto kern, int STAGES, int cluster) -> int {
     size_t smem = STAGES * STAGE + 16 * HD * 2;
-    const size_t merge = (4 * 16 * 2 + 4 * 16 * VD) * sizeof(float);
+    const size_t merge = (4 * 16 * 2 + 4 * 16 * VD + (cluster ? 16 * VD + 16 * 2 : 0)) * sizeof(float);
     if (merge > smem) smem = merge;
     smem += 1024;
     int e = opt_in(kern, smem);
     if (e) return e;
-    pe::launch(kern, grid, 128, smem, stream, a, kmap, vmap);
-    return 0;
+    if (!cluster) {
+      pe::launch(kern, grid, 128, smem, stream, a, kmap, vmap);
+      return 0;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = dim3(128); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    const cudaError_t ce = cudaLaunchKernelEx(&cfg, kern, a, kmap, vmap);
+    return ce == cudaSuccess ? 0 : (int)ce;
   };
+  if (cluster_ranges(n_seqs * a.n_kv_heads, a.split_keys, a.max_splits)) {
+    const int e = go(decode_split_kernel<HD, VD, 3, SPLIT_P, PAD, true>, 3, a.max_splits);
+    if (e) return e;
+    PE_LAUNCH_CHECK();
+    return PE_OK;
+  }
   // three stages: two blocks per SM, two pages in flight per block (measured best of 2, 3, 4)
-  const int e = go(decode_split_kernel<HD, VD, 3, SPLIT_P, PAD>, 3);
+  const int e = go(decode_split_kernel<HD, VD, 3, SPLIT_P, PAD, false>, 3, 0);
   if (e) return e;
   PE_LAUNCH_CHECK();
   // The merge starts when the split kernel has completed, not while it drains: with the early start a
@@ -737,17 +859,13 @@ static int launch(const Args& a, bool decode, int n_seqs, int max_q, cudaStream_
 }  // namespace fa
 }  // namespace pe
 
-// The tile sizes that rows of these sizes run in.
-static int tile_of(int dim) { return (dim + 63) / 64 * 64; }
-
 // Decode blocks that one SM holds at a time (shared memory bound): the caller sizes the number of
 // ranges per sequence so that one wave of blocks covers the batch.
-extern "C" int pe_attention_mma_decode_blocks_per_sm(int head_dim, int v_dim) {
-  const size_t hd = tile_of(head_dim), vd = tile_of(v_dim);
-  const size_t stage = (size_t)pe::fa::BN * (hd + vd) * 2;
-  const size_t smem = 3 * stage + 16 * hd * 2 + 1024 + 1024;   // + the block's static and reserved part
-  const int n = (int)((227 * 1024) / smem);
-  return n < 1 ? 1 : n;
+extern "C" int pe_attention_mma_decode_blocks_per_sm(int head_dim, int v_dim) { return pe::fa::decode_blocks_per_sm(head_dim, v_dim); }
+
+// Kernels of a decode step of so many (sequence, kv head) pairs.
+extern "C" int pe_attention_mma_decode_launches(int pairs, int split_keys, int max_splits) {
+  return pe::fa::cluster_ranges(pairs, split_keys, max_splits) ? 1 : 2;
 }
 
 // 1 if this file's kernels take the shape (bfloat16 only), else 0: the caller then uses the generic path.
@@ -859,7 +977,7 @@ extern "C" int pe_attention_mma_gated(int decode, const void* q, long long q_ld,
     return launch<128, 128, false, false>(a, dec, n_seqs, max_q, stream);
   }
   const bool wide = v_dim > 64;
-  switch (tile_of(head_dim)) {
+  switch (pe::fa::tile_of(head_dim)) {
     case 64: return wide ? launch<64, 128, false, true>(a, dec, n_seqs, max_q, stream) : launch<64, 64, false, true>(a, dec, n_seqs, max_q, stream);
     case 128: return wide ? launch<128, 128, false, true>(a, dec, n_seqs, max_q, stream) : launch<128, 64, false, true>(a, dec, n_seqs, max_q, stream);
     case 192: return wide ? launch<192, 128, false, true>(a, dec, n_seqs, max_q, stream) : launch<192, 64, false, true>(a, dec, n_seqs, max_q, stream);

@@ -190,6 +190,21 @@ def test_decode_attention_ranges(pe):
         assert sk == 0 and 1 <= n <= max(1, -(-kv // 512)) and least in (512, 2048)
 
 
+def test_decode_attention_ranges_on_the_tensor_core_kernel(pe):
+    """The rule of csrc/attention_mma.cu: every length is covered, one wave where there is room, whole pages."""
+    f = pe.kernels.ops.mma_decode_ranges
+    assert f(296, 8, 320, 512) == (0, 3, 128) and f(296, 8, 3968, 512) == (0, 16, 128) and f(296, 8, 40960, 512) == (0, 37, 128)
+    assert f(296, 64, 4096, 512) == (0, 4, 128) and f(296, 192, 2112, 512) == (0, 3, 704) and f(296, 512, 4096, 512) == (0, 2, 2048)
+    for slots, pairs, cap in [(296, 7, 5000), (296, 148, 64), (296, 149, 64), (296, 296, 40960), (296, 200, 1000), (10, 1000, 64), (592, 100, 70000)]:
+        sk, n, least = f(slots, pairs, cap, 512)
+        assert sk == 0 and n >= 1 and least > 0 and least % 64 == 0
+        if slots // pairs >= 2:
+            assert n * pairs <= slots
+        for length in {1, 63, 64, 65, cap // 2, cap}:
+            per = max(least, -(-(-(-length // n)) // 64) * 64)       # as the kernel cuts it
+            assert -(-length // per) <= n
+
+
 def test_reset_forgets_everything_and_loses_nothing(pe):
     c = _cache(pe, window=100, with_state=True)
     slots = [c.alloc_slot() for _ in range(3)]

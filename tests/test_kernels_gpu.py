@@ -543,6 +543,38 @@ def test_attention_mma_decode(ops, nh, nkv, d, window, split_keys, max_splits, l
     assert rel_err(out.float().cpu().view(B, nh, d), want) < ATT_TOL[dtype]
 
 
+@pytest.mark.parametrize("nh,nkv,d", [(8, 4, 128), (32, 2, 64), (10, 2, 128)])
+@pytest.mark.parametrize("B,splits", [(8, 1), (8, 2), (4, 3), (3, 5), (2, 8)])
+@pytest.mark.parametrize("window,keep,sink", [(0, 0, False), (100, 0, True), (100, 70, False), (0, 0, True)])
+def test_attention_mma_decode_clusters(ops, nh, nkv, d, B, splits, window, keep, sink):
+    """The ranges of a sequence as one cluster, among them ranges that hold nothing (short sequences, keys before the window),
+    against fixed ranges of a page merged by the second kernel, and against the plain formula."""
+    torch.manual_seed(18)
+    lens = [700, 257, 33, 513, 1, 256, 64, 65][:B]
+    ps = PagedSetup(lens, nkv, d, torch.bfloat16, seed=18, key_scale=2.0)
+    q = torch.randn(B, nh * d, device=DEV).to(torch.bfloat16)
+    gate = torch.randn(B, nh, device=DEV).to(torch.bfloat16)
+    qstart = torch.arange(B + 1, dtype=torch.int32, device=DEV)
+    past = torch.tensor([L - 1 for L in lens], dtype=torch.int32, device=DEV)
+    st = _status()
+    outs = []
+    for split_keys, n, least in ((0, splits, 64), (0, splits, 128), (64, 11, 0)):   # 700 keys: 11 pages
+        out = torch.full((B, nh * d), float("nan"), device=DEV, dtype=torch.bfloat16)
+        scratch = torch.full((ops.attention_generic_scratch_floats(B, nh, d, n),), float("nan"), device=DEV)
+        before = ops.launch_count()
+        ops.attention_mma_gated(True, q, out, B, 1, nh, nkv, d, d, d ** -0.5, window, qstart, past, ps.seq_slot, ps.table, ps.num_pages,
+                                ps.k_pages, ps.v_pages, scratch, split_keys, n, st, min_range_keys=least, sink=sink, gate=gate,
+                                keep_first=keep)
+        assert ops.launch_count() - before == (2 if split_keys else 1)
+        outs.append(out.float().cpu())
+    assert st.tolist()[0] == 0
+    assert rel_err(outs[0], outs[2]) < 2 * ATT_TOL[torch.bfloat16] and rel_err(outs[1], outs[2]) < 2 * ATT_TOL[torch.bfloat16]
+    if not keep and not sink:
+        want = _plain_attention(ps, [q[b:b + 1].cpu().view(1, nh, d) for b in range(B)], [L - 1 for L in lens], nh, d ** -0.5, window or None)
+        want = want * torch.sigmoid(gate.float().cpu())[:, :, None]
+        assert rel_err(outs[0].view(B, nh, d), want) < ATT_TOL[torch.bfloat16]
+
+
 @pytest.mark.parametrize("decode", [False, True])
 def test_attention_mma_finds_a_far_key_and_ignores_what_lies_beyond_the_length(ops, decode):
     nh, nkv, d = 8, 2, 128
