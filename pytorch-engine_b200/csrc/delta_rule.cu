@@ -8,6 +8,8 @@
 //   step         S <- diag(g) S ;  u = beta (v - S^T k) ;  S <- S + k u^T ;  o = S^T q            beta = sigmoid(b)
 //   out          = o / rms(o) * w * sigmoid(gate)  (or * silu(gate))        per head, eps inside the root, w of size dv
 //
+// Steps of several tokens a sequence, with sizes that it takes, spread a head's columns over the chip (walk.cuh and
+// pe_delta_rule_walk); single tokens and other sizes run here:
 // A block owns one head's S [d, dv] of one sequence (in registers or in shared memory) and walks the sequence's tokens
 // of this step in order; thread j owns column j.  State, decay, beta, the unit vectors and the head norm are float32 whatever
 // the run dtype.

@@ -7,6 +7,8 @@
 //   read      o    = S'^T q / (max(|n' . q|, e^(-m')) + 1e-6)     q already carries its factor d^(-1/2)
 //   out       = o / rms(o) * w * sigmoid(g)                 per head, eps inside the root
 //
+// Steps of several tokens a sequence, with sizes that it takes, spread a head's columns over the chip (walk.cuh and
+// pe_mlstm_walk); single tokens and other sizes run here:
 // A block owns one head's S [d, dv], n [d] and m of one sequence (S in registers or in shared memory) and walks the
 // sequence's tokens of this step in order; thread j owns column j of S.  Gates, state, the read's denominator and the head norm are
 // float32 whatever the run dtype; q, k, v, g come from matrix products in the run dtype, the two gate

@@ -3,8 +3,8 @@
 ``Runtime.linear`` is the one place where ``y = x W^T`` is computed.  The reference computes its
 unquantised linears with a library call (``F.linear``, pygguf_engine/quant_kernels.py:1836); here
 the library product (cuBLAS through ``torch.mm``) stands wherever the package's own tensor-core
-kernels do not take the shape, and the float32 mode always runs in true float32 (TF32 is switched
-off around the call).
+kernels do not take the shape, and the float32 mode never computes in less than float32 (TF32 is
+switched off around the call; from 16 rows on each operand is three bfloat16 parts, csrc/gemm_split32.cu).
 """
 from __future__ import annotations
 
