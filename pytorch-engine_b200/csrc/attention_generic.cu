@@ -1,6 +1,7 @@
 // Causal grouped-query attention over the paged cache, for every head size, group size and
 // window, in float32 arithmetic (inputs float32 or bfloat16).  This is the exact path (the whole
-// model in float32 runs through it; prompts with head sizes of 64 and 128 on a kernel with larger tiles) and the fallback for head sizes the tensor-core kernels refuse.
+// model in float32 runs through it; prompts with head sizes of 64 and 128 on a kernel with larger
+// tiles) and the fallback for head sizes the tensor-core kernels refuse.
 //
 // Reference formulas: scores q.k * scale; key visible iff kpos <= qpos (pygguf_engine/kv_cache.py:833,
 // 2192) and, with a window, kpos > qpos - window (2189-2190); query head h reads kv head h / group
@@ -16,6 +17,8 @@
 // sequence's own length, never on what else is in the batch.
 #include "api.h"
 #include "common.cuh"
+
+#include <type_traits>
 
 namespace pe {
 
@@ -260,7 +263,8 @@ __global__ void __launch_bounds__(256) attn_prefill_kernel(AttnArgs a) {
 // padded by 16 bytes (the 16 keys that a warp reads at once then lie in distinct banks).  K of the next page is
 // fetched (cp.async) while the values of this one are summed, V while the scores are computed; two blocks fit on an SM.
 // Three sequences of 333, 200 and 100 tokens, 16 heads over 8 of 128: 207 -> 57 us; one of 2,048: 2,893 -> 663 us (52
-// TFLOP/s).  Sums run in the order of the features and of the keys, as in the kernel above; masked keys weigh exactly zero.
+// TFLOP/s).  Sums run in the order of the features and of the keys, as in the kernel above; a key that a row does not see takes no
+// part in its sums, whatever its value.
 constexpr int kFRows = 32;
 constexpr int kFThreads = 128;
 
@@ -339,11 +343,16 @@ __global__ void __launch_bounds__(kFThreads, 2) attn_prefill_f32_kernel(AttnArgs
   constexpr int kF = D / 64;                     // 16-byte groups of output features a lane: 4 kg + 64 f
   float m[4], l[4], acc[4][kF * 4];
   int qpos[4], lo[4];
+  int all_from = 0, all_to = 0x7fffffff;                   // the keys that each of this lane's rows sees
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int row = row0 + warp * 8 + rg * 4 + i;
     qpos[i] = row < n_rows ? past + row / group : -1;      // a row that is not there sees nothing
     lo[i] = row < n_rows ? first_visible(a, qpos[i]) : 0;
+    if (row < n_rows) {
+      all_from = max(all_from, lo[i]);
+      all_to = min(all_to, qpos[i]);
+    }
     m[i] = -INFINITY;
     l[i] = 0.f;
 #pragma unroll
@@ -403,26 +412,36 @@ __global__ void __launch_bounds__(kFThreads, 2) attn_prefill_f32_kernel(AttnArgs
     }
     cp_async_wait<1>();          // V of this page (K of the next may still be on its way)
     __syncthreads();
+    // A key that a row does not see is left out of its sum (its weight is zero, but zero times an infinity or a NaN is not);
+    // pages that every row of the warp sees whole, all but the last one or two, go without the selects.
+    const int page0 = (p_begin + j) * kPageTokens;
+    auto fold = [&](auto masked) {
+      const int keys = decltype(masked)::value ? min(kPageTokens, k_end - page0) : kPageTokens;
 #pragma unroll 2
-    for (int k = 0; k < kPageTokens; k += 4) {
-      float4 p[4];
+      for (int k = 0; k < keys; k += 4) {
+        float4 p[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(p_row + i * L::kPLd + k);
+        for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(p_row + i * L::kPLd + k);
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk)
+        for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-        for (int f = 0; f < kF; ++f) {
-          const float4 v = *reinterpret_cast<const float4*>(Vs + (k + kk) * D + kg * 4 + 64 * f);
+          for (int f = 0; f < kF; ++f) {
+            const float4 v = *reinterpret_cast<const float4*>(Vs + (k + kk) * D + kg * 4 + 64 * f);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float w = (&p[i].x)[kk];
-            acc[i][f * 4] = fmaf(w, v.x, acc[i][f * 4]);
-            acc[i][f * 4 + 1] = fmaf(w, v.y, acc[i][f * 4 + 1]);
-            acc[i][f * 4 + 2] = fmaf(w, v.z, acc[i][f * 4 + 2]);
-            acc[i][f * 4 + 3] = fmaf(w, v.w, acc[i][f * 4 + 3]);
+            for (int i = 0; i < 4; ++i) {
+              const float w = (&p[i].x)[kk];
+              const int kpos = page0 + k + kk;
+              const bool sees = !decltype(masked)::value || (kpos <= qpos[i] && kpos >= lo[i]);
+              acc[i][f * 4] = sees ? fmaf(w, v.x, acc[i][f * 4]) : acc[i][f * 4];
+              acc[i][f * 4 + 1] = sees ? fmaf(w, v.y, acc[i][f * 4 + 1]) : acc[i][f * 4 + 1];
+              acc[i][f * 4 + 2] = sees ? fmaf(w, v.z, acc[i][f * 4 + 2]) : acc[i][f * 4 + 2];
+              acc[i][f * 4 + 3] = sees ? fmaf(w, v.w, acc[i][f * 4 + 3]) : acc[i][f * 4 + 3];
+            }
           }
-        }
-    }
+      }
+    };
+    if (__all_sync(0xffffffffu, page0 >= all_from && page0 + kPageTokens - 1 <= all_to)) fold(std::false_type{});
+    else fold(std::true_type{});
     __syncthreads();             // V and P have been read
     if (j + 1 < n_pages) load_page(a.v_pages, D, Vs, j + 1);
     else cp_async_commit();

@@ -270,6 +270,33 @@ def test_attention_prefill_float32_tiles(ops, nh, nkv, d, window, sink):
         o += n
 
 
+@pytest.mark.parametrize("nh,nkv,d", [(16, 8, 128), (4, 4, 64), (33, 1, 64)])
+@pytest.mark.parametrize("window", [0, 37])
+def test_attention_prefill_float32_tiles_leave_out_what_a_row_does_not_see(ops, nh, nkv, d, window):
+    """Keys and values that are infinite or not numbers, behind a token or in front of its window, change no bit of its output."""
+    torch.manual_seed(28)
+    n, past = 50, 130
+    ps = PagedSetup([n + past], nkv, d, torch.float32, seed=28)
+    q = torch.randn(n, nh * d, device=DEV)
+    qstart = torch.tensor([0, n], dtype=torch.int32, device=DEV)
+    past_t = torch.tensor([past], dtype=torch.int32, device=DEV)
+    at = past + 20                                          # the key that is spoilt: seen by tokens 20 .. 20 + window - 1
+    page = int(ps.table[ps.slots[0], at // 64])
+    outs = []
+    for bad in (None, float("nan"), float("inf")):
+        k, v = ps.k_pages.clone(), ps.v_pages.clone()
+        if bad is not None:
+            k[page, :, at % 64], v[page, :, at % 64] = bad, bad
+        out, st = torch.zeros(n, nh * d, device=DEV), _status()
+        ops.attention_generic(False, q, out, 1, n, nh, nkv, d, d ** -0.5, window, qstart, past_t, ps.seq_slot, ps.table, ps.num_pages,
+                              k, v, None, 0, 0, st)
+        assert st.tolist()[0] == 0
+        outs.append(out)
+    unseen = torch.tensor([i < 20 or (window > 0 and i - 20 >= window) for i in range(n)], device=DEV)
+    assert bool(outs[0].isfinite().all()) and bool(outs[1][~unseen].isnan().all())
+    assert torch.equal(outs[0][unseen], outs[1][unseen]) and torch.equal(outs[0][unseen], outs[2][unseen])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("nh,nkv,d", [(4, 2, 16), (6, 2, 32), (5, 5, 48), (32, 8, 128), (4, 1, 256), (16, 2, 64)])
 @pytest.mark.parametrize("window", [0, 300])
