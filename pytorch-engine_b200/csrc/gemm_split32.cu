@@ -1,7 +1,7 @@
 // y[M, N] = x[M, K] . W[N, K]^T in float32 on the bfloat16 tensor cores (tcgen05.mma), without giving up float32's precision.
 //
 // Every operand is the sum of three bfloat16 numbers: x = hi + mid + lo, each the rounding of what is left, 8 bits apiece,
-// so that the three hold float32's 24 bits.  Of the nine products of two such sums the six largest are formed (hi hi, hi mid,
+// so that the three hold float32's 24 bits (from 2^-110 on; what lies below is dealt with in second_look).  Of the nine products of two such sums the six largest are formed (hi hi, hi mid,
 // mid hi, hi lo, lo hi, mid mid); what the other three would add is below 2^-25 of the product.  The products are exact in
 // the tensor core; its sums are not rounded to nearest, so they are kept short: the accumulator in tensor memory covers 64 of
 // K, small terms first, and is then added to float32 registers with ordinary rounding.  Against 64 bits the result is closer
@@ -18,8 +18,8 @@
 //   8-15   accumulators: add each chunk's sums to their registers, store at the end;
 //   16     issues the MMAs;
 //   17     TMA producer: the three parts of the x tile.
-// A range of K whose operands hold an infinity, a NaN or a number that bfloat16 rounds to infinity leaves NaN in the sums of
-// its rows (inf - inf in the split): such outputs are computed again as a plain chain of multiply-adds.
+// Operands that three parts cannot hold (infinities, NaN, numbers next to either end of float32's range) and results as small or
+// as large are noticed, and what they touch is computed again as a plain chain of multiply-adds (second_look).
 // What bounds it: the issue of 24 MMAs a chunk and shared memory (96 KB written and 192 KB read per 64 of K of a 128 x 128 tile:
 // 1.2 of the 1.5 us that a chunk takes).  600 rows against the library's float32 product: 4,096 x 1,024 weights 57 against
 // 121 us, 1,024 x 3,072 36 against 125, 151,936 x 1,024 1,113 against 3,173 (168 TFLOP/s); 16 rows 12-15 against 19-24.
@@ -48,6 +48,7 @@ struct Tile {
 
 struct Params {
   const float* x; long long ldx;
+  const float* x_top; int segments;   // [M][segments]: a row's largest magnitude; infinity where its parts cut a value off
   const float* w;
   float* y; long long ldy;      // splits > 1: partial sums [splits][M][N]
   int M, N, K;
@@ -100,6 +101,13 @@ __device__ __forceinline__ uint32_t take_part(float& a, float& b) {
   b -= __uint_as_float(u & 0xFFFF0000u);
   return u;
 }
+// Values that three parts do not hold whole: what bfloat16's smallest subnormal, 2^-133, cuts off (see second_look).
+constexpr float kCutOff = 7.7037198e-34f;       // 2^-110
+__device__ __forceinline__ bool cut_off(float v) { return fabsf(v) < kCutOff && v != 0.f; }
+__device__ __forceinline__ bool cut_off(float4 v) { return cut_off(v.x) || cut_off(v.y) || cut_off(v.z) || cut_off(v.w); }
+__device__ __forceinline__ float largest(float m, float4 v) {
+  return fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+}
 // Four rows' four neighbouring values into the three parts' tiles, `bytes` apart, rows 16 apart: part by part over all four,
 // so that eight conversions run side by side.
 __device__ __forceinline__ void store_parts(float4* v, char* dst, int bytes) {
@@ -113,22 +121,161 @@ __device__ __forceinline__ void store_parts(float4* v, char* dst, int bytes) {
   }
 }
 
-// x [M, K] into planes [3][M][Kp] of bfloat16, Kp = K up to a multiple of 64, the rest zeros.
-__global__ void __launch_bounds__(256) gemm_split32_parts_kernel(const float* x, long long ldx, __nv_bfloat16* parts, int M, int K, int Kp) {
+// x [M, K] into planes [3][M][Kp] of bfloat16, Kp = K up to a multiple of 64, the rest zeros; x_top as in Params.  A warp takes
+// kSegment values of a row at a time.
+constexpr int kSegment = 512;
+__global__ void __launch_bounds__(256) gemm_split32_parts_kernel(const float* x, long long ldx, __nv_bfloat16* parts, float* x_top, int M, int K,
+                                                                 int Kp) {
   pdl_wait_block();
   pdl_launch_dependents();
-  const int quads = Kp / 4;
-  const size_t total = (size_t)M * quads, plane = (size_t)M * Kp;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t m = i / quads;
-    const int k = (int)(i - m * quads) * 4;
-    float4 v = k < K ? *reinterpret_cast<const float4*>(x + m * ldx + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const int segments = (Kp + kSegment - 1) / kSegment, lane = threadIdx.x & 31;
+  const size_t total = (size_t)M * segments, plane = (size_t)M * Kp;
+  for (size_t i = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); i < total; i += (size_t)gridDim.x * 8) {
+    const size_t m = i / segments;
+    const int k0 = (int)(i - m * segments) * kSegment + lane * 4;
+    float4 v[kSegment / 128];
 #pragma unroll
-    for (int p = 0; p < kParts; ++p) {
-      const uint32_t lo = take_part(v.x, v.y), hi = take_part(v.z, v.w);
-      *reinterpret_cast<uint2*>(parts + p * plane + m * Kp + k) = make_uint2(lo, hi);
+    for (int j = 0; j < kSegment / 128; ++j) {
+      const int k = k0 + j * 128;
+      v[j] = k < K ? *reinterpret_cast<const float4*>(x + m * ldx + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    bool cut = false;
+    float top = 0.f;
+#pragma unroll
+    for (int j = 0; j < kSegment / 128; ++j) {
+      cut = cut || cut_off(v[j]);
+      top = largest(top, v[j]);
+      const int k = k0 + j * 128;
+      if (k >= Kp) continue;
+#pragma unroll
+      for (int p = 0; p < kParts; ++p) {
+        const uint32_t lo = take_part(v[j].x, v[j].y), hi = take_part(v[j].z, v[j].w);
+        *reinterpret_cast<uint2*>(parts + p * plane + m * Kp + k) = make_uint2(lo, hi);
+      }
+    }
+    // magnitudes are ordered as their bits
+    const unsigned bits = __reduce_max_sync(0xffffffffu, cut ? 0x7f800000u : __float_as_uint(top));
+    if (lane == 0) x_top[i] = __uint_as_float(bits);
+  }
+}
+
+// ---- outputs whose products the parts do not carry -------------------------------------------------------------------
+// Three parts hold a float32 value whole from 2^-110 to the largest that rounds to a finite bfloat16.  Below, the smallest
+// subnormal of bfloat16 (2^-133) cuts the value off, by at most 2^-134; above, and for infinities and NaN, the parts give NaN.
+// The tensor core's products and sums keep float32's subnormals but do not round to nearest, so results next to them suffer too.
+// Such outputs are computed again as a plain chain of float32 multiply-adds.  Which they are:
+//   * those that are infinite or NaN;
+//   * those of magnitude below kSmall, and zeros whose operands' largest product is that small;
+//   * those that a row's cut-off values could move by more than 2^-24 of the output: |y| < K 2^-110 (largest |w| if x was
+//     cut off, plus largest |x| if w was).
+// The product kernel only asks whether some output could be one: W's values may have been cut off (the converters have no time
+// to look), x's not, or the row's largest magnitude says infinity.  Then the tile's operands are read again to decide.
+constexpr float kSmall = 1.2037062e-35f;        // 2^-116
+constexpr float kLargest = 3.4028235e38f;
+constexpr int kExactK = 32;                     // values of K a step
+constexpr int kExactWarps = kConvWarps + kAccWarps, kExactThreads = kExactWarps * 32;
+
+__device__ __forceinline__ int exact_any(int v) {        // a barrier of these warps; whether any thread has v
+  int any;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.s32 p, %1, 0;\n"
+      "barrier.cta.red.or.pred q, 1, %2, p;\n"
+      "selp.s32 %0, 1, 0, q;\n"
+      "}\n" : "=r"(any) : "r"(v), "n"(kExactThreads) : "memory");
+  return any;
+}
+
+// Every warp but the last two; a thread has one column and a quarter of the rows.  The tile's results are in y, shared memory is
+// free.  A tile in which nothing is computed again reads its operands once more; otherwise the whole tile's chains run side by side.
+// 600 x 4,096 outputs, K = 1,024, 59 us: 73 with one zero row of W (the tiles of its 128 rows look), 134 where every tile looks,
+// 713 where everything is NaN (one NaN row of W took 4,519 when its outputs were one thread's).
+template <int NT>
+__device__ __noinline__ void second_look(const Params p) {      // (takes nothing that the product would have to keep for it)
+  constexpr int kRows = NT / 4;
+  extern __shared__ char smem_raw[];
+  const int m0 = blockIdx.x * NT, n0 = blockIdx.y * BM;
+  const int k_first = blockIdx.z * p.chunks_per_split * BK, k_last = min(p.K, k_first + p.chunks_per_split * BK);
+  float* y = p.y + (gridDim.z > 1 ? (size_t)blockIdx.z * p.M * p.N : 0);
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int col = t % BM, row0 = t / BM * kRows, n = n0 + col;
+  float* top = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(smem_raw) + 15) & ~static_cast<uintptr_t>(15));
+  int* cut = reinterpret_cast<int*>(top + NT + BM);          // [NT + BM] whether a row of x, of W has values that were cut off;
+  float* xs = reinterpret_cast<float*>(cut + NT + BM);       // top: its largest magnitude.  [kExactK][NT + 4]
+  float* ws = xs + kExactK * (NT + 4);                       // [kExactK][BM + 4]
+  auto row_of = [&](int r) -> const float* {                 // the r-th row of x, then of W; null: not there
+    if (r < NT) return m0 + r < p.M ? p.x + (size_t)(m0 + r) * p.ldx : nullptr;
+    return n0 + r - NT < p.N ? p.w + (size_t)(n0 + r - NT) * p.K : nullptr;
+  };
+  for (int r = warp * 4; r < NT + BM; r += kExactWarps * 4) {
+    const float* row[4];
+    float mx[4] = {0.f, 0.f, 0.f, 0.f};
+    bool low[4] = {false, false, false, false};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) row[i] = row_of(r + i);
+#pragma unroll 4
+    for (int k = k_first + lane * 4; k < k_last; k += 128)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (row[i] != nullptr) {
+          const float4 v = *reinterpret_cast<const float4*>(row[i] + k);
+          mx[i] = largest(mx[i], v);
+          low[i] = low[i] || cut_off(v);
+        }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const unsigned bits = __reduce_max_sync(0xffffffffu, __float_as_uint(mx[i]));   // magnitudes are ordered as their bits
+      const int any = __any_sync(0xffffffffu, low[i]);
+      if (lane == 0) {
+        top[r + i] = __uint_as_float(bits);
+        cut[r + i] = any;
+      }
     }
   }
+  exact_any(0);
+  uint32_t again = 0;
+  const float len = (float)(k_last - k_first), w_top = top[NT + col], w_cut = cut[NT + col] ? 1.f : 0.f;
+  if (n < p.N)
+    for (int j = 0; j < kRows && m0 + row0 + j < p.M; ++j) {
+      const float v = fabsf(y[(size_t)(m0 + row0 + j) * p.ldy + n]), x_top = top[row0 + j];
+      const float lost = len * kCutOff * ((cut[row0 + j] ? w_top : 0.f) + w_cut * x_top);
+      const bool tiny = v > 0.f ? v < kSmall : x_top > 0.f && w_top > 0.f && x_top * w_top * len < kSmall;
+      if (!(v <= kLargest) || tiny || v < lost) again |= 1u << j;
+    }
+  if (!exact_any(again != 0)) return;
+  const bool mine = __any_sync(0xffffffffu, again != 0);
+  float e[kRows];
+#pragma unroll
+  for (int j = 0; j < kRows; ++j) e[j] = 0.f;
+  for (int k0 = k_first; k0 < k_last; k0 += kExactK) {
+    exact_any(0);                // the step before has been read
+    for (int i = t; i < (NT + BM) * (kExactK / 4); i += kExactThreads) {
+      const int r = i / (kExactK / 4), q = i % (kExactK / 4) * 4;
+      const float* row = row_of(r);
+      const float4 v = row != nullptr && k0 + q < k_last ? *reinterpret_cast<const float4*>(row + k0 + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+      float* dst = r < NT ? xs + q * (NT + 4) + r : ws + q * (BM + 4) + r - NT;
+      const int step = r < NT ? NT + 4 : BM + 4;
+      dst[0] = v.x; dst[step] = v.y; dst[2 * step] = v.z; dst[3 * step] = v.w;
+    }
+    exact_any(0);
+    if (!mine) continue;
+#pragma unroll 1
+    for (int k = 0; k < kExactK && k0 + k < k_last; ++k) {
+      const float w = ws[k * (BM + 4) + col];
+#pragma unroll
+      for (int j = 0; j < kRows; j += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(xs + k * (NT + 4) + row0 + j);
+        e[j] = fmaf(x.x, w, e[j]);
+        e[j + 1] = fmaf(x.y, w, e[j + 1]);
+        e[j + 2] = fmaf(x.z, w, e[j + 2]);
+        e[j + 3] = fmaf(x.w, w, e[j + 3]);
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < kRows; ++j)
+    if ((again >> j) & 1) y[(size_t)(m0 + row0 + j) * p.ldy + n] = e[j];
 }
 
 // grid: (tiles of x rows, tiles of W rows, splits of K).  xmap: the planes as [3 M, Kp], boxes of NT rows.
@@ -138,6 +285,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split32_kernel(Params p, con
   extern __shared__ char smem_raw[];
   __shared__ uint64_t full_bar[T::kStages], empty_bar[T::kStages], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_holder;
+  __shared__ uint64_t drain_bar;
   __shared__ volatile int failed;
   char* smem = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -155,6 +303,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split32_kernel(Params p, con
       tma::mbar_init(&acc_full[b], 1);
       tma::mbar_init(&acc_empty[b], kAccWarps);
     }
+    tma::mbar_init(&drain_bar, 1);
     failed = 0;
     tma::fence_barrier_init();
   }
@@ -179,6 +328,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split32_kernel(Params p, con
   fence_after_sync();
   const uint32_t tmem_base = tmem_holder;
   pdl_wait_block();
+  bool look = false;             // whether this thread's outputs call for a second look
 
   if (warp < kConvWarps) {
     int stage = 0;
@@ -212,8 +362,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split32_kernel(Params p, con
 #pragma unroll
     for (int j = 0; j < T::kAcc; ++j) acc[j] = 0.f;
     bool ok = true;
+    // the largest magnitude of this warp's rows, some of their segments a chunk while the tensor core works
+    const float* tops = p.x_top + (size_t)(m0 + half * T::kAcc) * p.segments;
+    const int n_tops = min(T::kAcc, p.M - m0 - half * T::kAcc) * p.segments;
+    float top = 0.f;
     for (int c = 0; c < chunks; ++c) {
-      const int b = c & 1;
+      const int b = c & 1, at = c * 128 + lane;
+      float seen[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) seen[i] = at + 32 * i < n_tops ? tops[at + 32 * i] : 0.f;
       if (failed || !tma::mbar_wait(&acc_full[b], (c >> 1) & 1)) {
         if (lane == 0 && !failed) report(p.status, kStatusWaitTimedOut, 51, (int)blockIdx.y, c);
         failed = 1;
@@ -232,8 +389,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split32_kernel(Params p, con
       fence_before_sync();
       __syncwarp();
       if (lane == 0) tma::mbar_arrive(&acc_empty[b]);
+      top = fmaxf(fmaxf(top, fmaxf(seen[0], seen[1])), fmaxf(seen[2], seen[3]));
     }
     pdl_launch_dependents();
+    for (int i = chunks * 128 + lane; i < n_tops; i += 32) top = fmaxf(top, tops[i]);     // (a short last range of K)
+    // the least magnitude that an output has without a second look
+    const float least = fmaxf(kSmall, __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(top))) * kCutOff * (float)p.K);
     const int n = n0 + quarter * 32 + lane;
     if (ok && n < p.N) {
       float* y = p.y + (gridDim.z > 1 ? (size_t)blockIdx.z * p.M * p.N : 0);
@@ -241,15 +402,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split32_kernel(Params p, con
       for (int j = 0; j < T::kAcc; ++j) {
         const int m = m0 + half * T::kAcc + j;
         if (m >= p.M) break;
-        float v = acc[j];
-        if (v != v) {
-          const float* wr = p.w + (size_t)n * p.K;
-          const float* xr = p.x + (size_t)m * p.ldx;
-          v = 0.f;
-#pragma unroll 1
-          for (int k = k_first; k < k_last; ++k) v = fmaf(xr[k], wr[k], v);
-        }
-        y[(size_t)m * p.ldy + n] = v;
+        y[(size_t)m * p.ldy + n] = acc[j];
+        look = look || !(fabsf(acc[j]) >= least && fabsf(acc[j]) <= kLargest);
       }
     }
   } else if (warp == kMmaWarp) {
@@ -297,11 +451,22 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split32_kernel(Params p, con
     }
   }
   fence_before_sync();
-  __syncthreads();
+  const int again = __syncthreads_or(look);
+  if (failed) {
+    // Products in flight still use shared and tensor memory: wait for them; copies in flight get as long as a wait lasts at most
+    // (nothing completes that phase) to land before the block gives its shared memory back.
+    if (warp == kMmaWarp && lane == 0) {
+      umma_commit(&drain_bar);
+      tma::mbar_wait(&drain_bar, 0);
+      tma::mbar_wait(&drain_bar, 1);
+    }
+    __syncthreads();
+  }
   if (warp == kMmaWarp) {
     fence_after_sync();
     tmem_dealloc(tmem_base, T::kCols);
   }
+  if (again && !failed && warp < kMmaWarp) second_look<NT>(p);
 }
 
 // y[m, n] = the ranges' partial sums, added in their order.
@@ -341,6 +506,8 @@ static Plan plan_for(int M, int N, int K, int n_sms) {
 }
 static long long padded_k(int K) { return (K + BK - 1) / BK * (long long)BK; }
 static long long parts_floats(int M, int K) { return (kParts * (long long)M * padded_k(K) + 1) / 2; }   // a multiple of 32 (K's padding)
+static int segments_of(int K) { return (int)((padded_k(K) + kSegment - 1) / kSegment); }
+static long long top_floats(int M, int K) { return ((long long)M * segments_of(K) + 3) / 4 * 4; }
 
 }  // namespace umma32
 }  // namespace pe
@@ -353,7 +520,7 @@ extern "C" int pe_gemm_split32_supported(int M, int N, int K) {
 extern "C" long long pe_gemm_split32_scratch_floats(int M, int N, int K, int n_sms) {
   if (!pe_gemm_split32_supported(M, N, K)) return 0;
   const pe::umma32::Plan plan = pe::umma32::plan_for(M, N, K, n_sms);
-  return pe::umma32::parts_floats(M, K) + (plan.splits > 1 ? (long long)plan.splits * M * N : 0);
+  return pe::umma32::parts_floats(M, K) + pe::umma32::top_floats(M, K) + (plan.splits > 1 ? (long long)plan.splits * M * N : 0);
 }
 
 // Kernels that one call launches.
@@ -374,16 +541,17 @@ extern "C" int pe_gemm_split32(const float* x, long long ldx, const float* w, fl
   if (scratch == nullptr || ((uintptr_t)scratch % 16) || (sums && ldy % 4)) return PE_ERR_BAD_ARGUMENT;
   const int Kp = (int)padded_k(K);
   __nv_bfloat16* parts = reinterpret_cast<__nv_bfloat16*>(scratch);
-  float* partial = scratch + parts_floats(M, K);
+  float* x_top = scratch + parts_floats(M, K);
+  float* partial = scratch + parts_floats(M, K) + top_floats(M, K);
   CUtensorMap xmap;
   const int e = pe::tma::make_map_2d_bf16(&xmap, parts, Kp, (uint64_t)kParts * M, Kp, BK, plan.nt);
   if (e != 0) return e < 0 ? e : PE_ERR_BAD_ARGUMENT;
-  const long long quads = (long long)M * Kp / 4;
-  const int blocks = (int)((quads + 255) / 256 < 8ll * n_sms ? (quads + 255) / 256 : 8ll * n_sms);
-  pe::launch(gemm_split32_parts_kernel, blocks, 256, 0, stream, x, ldx, parts, M, K, Kp);
+  // eight segments a block; no more blocks than fit at a time, each with as many rounds as the others
+  const long long units = ((long long)M * segments_of(K) + 7) / 8, rounds = (units + 8ll * n_sms - 1) / (8ll * n_sms);
+  pe::launch(gemm_split32_parts_kernel, (int)((units + rounds - 1) / rounds), 256, 0, stream, x, ldx, parts, x_top, M, K, Kp);
   PE_LAUNCH_CHECK();
   Params p;
-  p.x = x; p.ldx = ldx; p.w = w; p.y = sums ? partial : y; p.ldy = sums ? N : ldy; p.M = M; p.N = N; p.K = K;
+  p.x = x; p.ldx = ldx; p.x_top = x_top; p.segments = segments_of(K); p.w = w; p.y = sums ? partial : y; p.ldy = sums ? N : ldy; p.M = M; p.N = N; p.K = K;
   p.chunks_per_split = plan.chunks_per_split; p.status = status;
   auto kern = plan.nt == 128 ? gemm_split32_kernel<128> : gemm_split32_kernel<64>;
   const size_t smem = 1024 + (plan.nt == 128 ? (size_t)Tile<128>::kStages * Tile<128>::kStage : (size_t)Tile<64>::kStages * Tile<64>::kStage);

@@ -732,6 +732,46 @@ def test_gemm_split32(ops, M, N, K):
         assert rel_err(out[:, :N][fin].cpu() / ref[fin].abs().max().cpu(), ref[fin].cpu() / ref[fin].abs().max().cpu()) < 1e-5
 
 
+@pytest.mark.parametrize("M,N,K", [(40, 200, 1000), (50, 132, 68), (150, 130, 60)])
+def test_gemm_split32_at_the_ends_of_float32s_range(ops, M, N, K):
+    """Operands and results that bfloat16 parts do not hold: as close as a chain of float32 multiply-adds."""
+    torch.manual_seed(33)
+    near_one = lambda *shape: (torch.rand(*shape, device=DEV) + 0.5) * torch.randn(*shape, device=DEV).sign()
+    st = _status()
+
+    def check(x, w):
+        x, w = x.contiguous(), w.contiguous()
+        out = torch.full((M, -(-N // 4) * 4), float("nan"), device=DEV)[:, :N]
+        ops.gemm_split32(x, w, out, st)
+        want, size = x.double() @ w.double().t(), (x.double().abs() @ w.double().abs().t())
+        # a chain of K multiply-adds: K roundings of 2^-24 of a partial sum or, below 2^-126, of half the smallest subnormal; as
+        # independent errors sqrt(K) of them, partial sums sqrt(K) products high
+        bound = 3 * (K ** 0.5 * 2.0 ** -24 * size / K ** 0.5 + K ** 0.5 * 2.0 ** -150)
+        assert bool(((out.double() - want).abs() <= bound.clamp(min=2.0 ** -149)).all()), float(((out.double() - want).abs() / bound).max())
+
+    steps = lambda n, lo, hi: 2.0 ** torch.linspace(lo, hi, n, device=DEV, dtype=torch.float64).round()[:, None]
+    check((near_one(M, K) * steps(M, -148, -90)).float(), near_one(N, K))           # small rows of x, of w, of both
+    check(near_one(M, K), (near_one(N, K) * steps(N, -148, -90)).float())
+    check((near_one(M, K) * steps(M, -80, -50)).float(), (near_one(N, K) * steps(N, -80, -40)).float())
+    x, w = near_one(M, K), near_one(N, K)                                          # small values where the weights are large, and
+    x[:, ::2] *= 2.0 ** -122                                                        # ordinary ones where there are none
+    w[:, ::2] *= 2.0 ** 110
+    w[:, 1::2] = 0
+    check(x, w)
+    check(x * torch.tensor([1.0, 0.0], device=DEV).repeat(K // 2), w)
+    x, w = torch.zeros(M, K, device=DEV), torch.zeros(N, K, device=DEV)             # one product a sum, close to the largest number
+    x[:, 4], w[:, 4] = 3.4028e38, 0.999
+    check(x, w)
+    x[:, 4], w[:, 4] = 1.9999 * 2.0 ** 63, 1.9999 * 2.0 ** 63
+    check(x, w)
+    assert st.tolist()[0] == 0
+    bad = near_one(M, K)                                                            # nothing but NaN
+    bad[:] = float("nan")
+    out = torch.zeros(M, -(-N // 4) * 4, device=DEV)[:, :N]
+    ops.gemm_split32(bad, near_one(N, K), out, st)
+    assert bool(out.isnan().all()) and st.tolist()[0] == 0
+
+
 @pytest.mark.parametrize("M,I,K", [(128, 128, 64), (200, 384, 200), (1000, 1280, 1024), (5, 256, 4096)])
 @pytest.mark.parametrize("kernel", ["gemm_umma", "gemm_umma2"])
 def test_gemm_umma_with_the_gate_fused(ops, M, I, K, kernel):
