@@ -664,9 +664,20 @@ extern "C" long long pe_delta_rule_scratch_floats(int n_seqs, int heads, int d, 
   return (long long)n_seqs * max_chunks * heads * (long long)pe::delta_unit(d, dv);
 }
 
-// Floats of scratch for pe_delta_rule_walk; 0: these sizes are not taken.
+// Where a block keeps a head's columns: the register tile (128: two threads a column with 64 rows each, where the columns then
+// fill whole half-warps), 0 for shared memory, -1 for sizes that fit neither.
+static int delta_tile(int d, int dv) {
+  if (d <= 0 || dv <= 0 || dv > 1024 || d > 1024) return -1;
+  const int widest = dv > d ? dv : d;
+  if (d <= 32 && widest <= 512) return 32;
+  if (d <= 64 && widest <= 512) return 64;
+  if (d <= 128 && widest <= 256 && dv % 16 == 0 && d % 16 == 0) return 128;
+  return ((size_t)d * widest + 3 * (size_t)d + 2 * (size_t)dv) * sizeof(float) > 200 * 1024 ? -1 : 0;
+}
+
+// Floats of scratch for pe_delta_rule_walk; 0: these sizes are not taken (nor those that single tokens could not have).
 extern "C" long long pe_delta_rule_walk_scratch_floats(int n_tokens, int heads, int kv_heads, int d, int dv) {
-  if (!pe::walk_takes(d, dv) || n_tokens <= 0) return 0;
+  if (!pe::walk_takes(d, dv) || delta_tile(d, dv) < 0 || n_tokens <= 0) return 0;
   return (long long)n_tokens * (2ll * kv_heads * d + (long long)heads * (d + dv + 2));
 }
 
@@ -679,7 +690,7 @@ extern "C" int pe_delta_rule_walk(int dtype, const void* qkv, const float* a, co
                                   int gate_silu, long long a_ld, long long b_ld, int* status, cudaStream_t stream) {
   if (n_seqs <= 0 || n_tokens <= 0) return PE_OK;
   if (heads <= 0 || kv_heads <= 0 || heads % kv_heads || n_seqs > 65535) return PE_ERR_BAD_ARGUMENT;
-  if (!pe::walk_takes(d, dv) || dv / pe::kWalkCols > 65535) return PE_ERR_UNSUPPORTED_SIZE;
+  if (!pe::walk_takes(d, dv) || delta_tile(d, dv) < 0) return PE_ERR_UNSUPPORTED_SIZE;
   if (!scratch || ((uintptr_t)scratch % 16) || ((uintptr_t)qkv % 16)) return PE_ERR_BAD_ARGUMENT;
   pe::DeltaArgs args{qkv, a, dt_bias, A_log, b, gate, gate_ld, norm_w, eps, q_scale, out, S, seq_slot, seq_qstart,
                      n_seqs, heads, kv_heads, d, dv, n_slots, 0, 1, nullptr, status, head_decay, gate_silu,
@@ -699,7 +710,8 @@ extern "C" int pe_delta_rule_recurrence(int dtype, const void* qkv, const float*
                                         long long b_ld, int* status, cudaStream_t stream) {
   if (n_seqs <= 0) return PE_OK;
   if (heads <= 0 || kv_heads <= 0 || heads % kv_heads || d <= 0 || dv <= 0) return PE_ERR_BAD_ARGUMENT;
-  if (dv > 1024 || d > 1024) return PE_ERR_UNSUPPORTED_SIZE;
+  const int reg = delta_tile(d, dv);
+  if (reg < 0) return PE_ERR_UNSUPPORTED_SIZE;
   if (dtype != PE_F32 && dtype != PE_BF16) return PE_ERR_UNSUPPORTED_DTYPE;
   pe::DeltaArgs args{qkv, a, dt_bias, A_log, b, gate, gate_ld, norm_w, eps, q_scale, out, S, seq_slot, seq_qstart,
                      n_seqs, heads, kv_heads, d, dv, n_slots, 0, 1, nullptr, status, head_decay, gate_silu,
@@ -708,11 +720,6 @@ extern "C" int pe_delta_rule_recurrence(int dtype, const void* qkv, const float*
     if (!scratch || max_chunks <= 0 || (long long)max_chunks * chunk < max_q || max_chunks > 32767) return PE_ERR_BAD_ARGUMENT;
     args.chunk = chunk; args.max_chunks = max_chunks; args.scratch = scratch;
   }
-  const int widest = dv > d ? dv : d;
-  // 128: two threads a column with 64 rows each (the columns then fill whole half-warps)
-  const int reg = (d <= 32 && widest <= 512) ? 32
-                  : (d <= 64 && widest <= 512 ? 64 : (d <= 128 && widest <= 256 && dv % 16 == 0 && d % 16 == 0 ? 128 : 0));
-  if (reg == 0 && ((size_t)d * widest + 3 * (size_t)d + 2 * (size_t)dv) * sizeof(float) > 200 * 1024) return PE_ERR_UNSUPPORTED_SIZE;
   int rc;
 #define PE_DELTA(T)                                                       \
   (reg == 32 ? pe::delta_run<T, 32, 1>(args, stream)                      \

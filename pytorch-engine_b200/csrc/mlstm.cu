@@ -453,9 +453,20 @@ extern "C" long long pe_mlstm_scratch_floats(int n_seqs, int heads, int d, int d
   return (long long)n_seqs * max_chunks * heads * (long long)pe::mlstm_unit(d, dv);
 }
 
-// Floats of scratch for pe_mlstm_walk; 0: these sizes are not taken.
+// Where a block keeps a head's columns: in registers where a column fits (key sizes up to 128, value sizes up to the block;
+// returned is the register tile, and 128 stands for two threads a column with 64 rows each, where the value size then fills
+// whole half-warps), else in shared memory (0).  -1: neither.
+static int mlstm_tile(int d, int dv) {
+  if (d <= 0 || dv <= 0 || dv > 1024) return -1;
+  if (d <= 32) return 32;
+  if (d <= 64 && dv <= 512) return 64;
+  if (d <= 128 && dv <= 256 && dv % 16 == 0) return 128;
+  return ((size_t)d * dv + 3 * (size_t)d) * sizeof(float) + 2 * (size_t)dv * 4 > 200 * 1024 ? -1 : 0;
+}
+
+// Floats of scratch for pe_mlstm_walk; 0: these sizes are not taken (nor those that single tokens could not have).
 extern "C" long long pe_mlstm_walk_scratch_floats(int n_tokens, int heads, int d, int dv) {
-  if (!pe::walk_takes(d, dv) || n_tokens <= 0) return 0;
+  if (!pe::walk_takes(d, dv) || mlstm_tile(d, dv) < 0 || n_tokens <= 0) return 0;
   return (long long)n_tokens * heads * (2ll * d + dv + 4 + 3);
 }
 
@@ -467,7 +478,7 @@ extern "C" int pe_mlstm_walk(int dtype, const void* q, const void* k, const void
                              int n_seqs, int heads, int d, int dv, int n_slots, float* scratch, int* status, cudaStream_t stream) {
   if (n_seqs <= 0 || n_tokens <= 0) return PE_OK;
   if (heads <= 0 || !(cap > 0.f) || n_seqs > 65535) return PE_ERR_BAD_ARGUMENT;
-  if (!pe::walk_takes(d, dv) || dv / pe::kWalkCols + 1 > 65535) return PE_ERR_UNSUPPORTED_SIZE;
+  if (!pe::walk_takes(d, dv) || mlstm_tile(d, dv) < 0) return PE_ERR_UNSUPPORTED_SIZE;
   if (dtype != PE_F32 && dtype != PE_BF16) return PE_ERR_UNSUPPORTED_DTYPE;
   if (!scratch || ((uintptr_t)scratch % 16) || ((uintptr_t)v % 16) || (ld * (dtype == PE_F32 ? 4 : 2)) % 16) return PE_ERR_BAD_ARGUMENT;
   pe::MlstmArgs a{q, k, v, g, ld, gates, gate_bias, norm_w, cap, eps, q_scale, out, S, n, m, seq_slot, seq_qstart,
@@ -484,7 +495,8 @@ extern "C" int pe_mlstm_recurrence(int dtype, const void* q, const void* k, cons
                                    int chunk, int max_chunks, float* scratch, int* status, cudaStream_t stream) {
   if (n_seqs <= 0) return PE_OK;
   if (heads <= 0 || d <= 0 || dv <= 0 || !(cap > 0.f)) return PE_ERR_BAD_ARGUMENT;
-  if (dv > 1024) return PE_ERR_UNSUPPORTED_SIZE;
+  const int reg = mlstm_tile(d, dv);
+  if (reg < 0) return PE_ERR_UNSUPPORTED_SIZE;
   if (dtype != PE_F32 && dtype != PE_BF16) return PE_ERR_UNSUPPORTED_DTYPE;
   pe::MlstmArgs a{q, k, v, g, ld, gates, gate_bias, norm_w, cap, eps, q_scale, out, S, n, m, seq_slot, seq_qstart,
                   n_seqs, heads, d, dv, n_slots, 0, 1, nullptr, status};
@@ -492,11 +504,6 @@ extern "C" int pe_mlstm_recurrence(int dtype, const void* q, const void* k, cons
     if (!scratch || max_chunks <= 0 || (long long)max_chunks * chunk < max_q || max_chunks > 65535) return PE_ERR_BAD_ARGUMENT;
     a.chunk = chunk; a.max_chunks = max_chunks; a.scratch = scratch;
   }
-  // the state's columns in registers where a column fits (key sizes up to 128, value sizes up to the block), in shared
-  // memory otherwise
-  // 128: two threads a column with 64 rows each (the value size then fills whole half-warps)
-  const int reg = (d <= 32) ? 32 : (d <= 64 && dv <= 512 ? 64 : (d <= 128 && dv <= 256 && dv % 16 == 0 ? 128 : 0));
-  if (reg == 0 && ((size_t)d * dv + 3 * (size_t)d) * sizeof(float) + 2 * (size_t)dv * 4 > 200 * 1024) return PE_ERR_UNSUPPORTED_SIZE;
   int rc;
 #define PE_MLSTM(T)                                                          \
   (reg == 32 ? pe::mlstm_run<T, 32, 1>(a, max_q, stream)                     \

@@ -123,3 +123,12 @@ def test_router_of_the_plain_implementation():
     chosen, weight = plain.router(h, w, "p", 2)
     s = torch.softmax(torch.tensor([2.0, 0.0, 1.0], dtype=torch.float64), 0)
     assert chosen.tolist() == [[2, 0]] and torch.allclose(weight, s[[2, 0]][None])
+
+
+def test_prompts_take_no_sizes_that_single_tokens_refuse(pe):
+    """The walk over columns keeps no head in a block; the step that follows a prompt does."""
+    ops = pe.kernels.ops
+    for d, dv, taken in [(128, 256, True), (128, 384, True), (128, 400, False), (64, 768, True), (64, 784, False), (32, 1024, True),
+                         (32, 1040, False), (96, 128, False), (64, 24, False)]:
+        assert (ops.mlstm_walk_scratch_floats(8, 4, d, dv) > 0) == taken, (d, dv)
+        assert (ops.delta_rule_walk_scratch_floats(8, 4, 4, d, dv) > 0) == taken, (d, dv)
