@@ -265,6 +265,11 @@ def lunadra_kernel_pairs(pe, torch, s, hbm_gbs, prompt, batch, context):
     flush = torch.zeros(96 * 2 ** 20, device=dev)
     status = torch.zeros(4, dtype=torch.int32, device=dev)
     out = {}
+    walk = importlib.import_module(pe.__name__ + ".parts.walk")
+    areas = {}
+
+    def scratch_of(name, floats):
+        return areas.setdefault((name, floats), torch.empty(floats, device=dev))
 
     def us_of(fn):
         return 1e3 * timed(torch, fn, 20, 5, flush, graph=True)
@@ -285,7 +290,6 @@ def lunadra_kernel_pairs(pe, torch, s, hbm_gbs, prompt, batch, context):
         token_seq = torch.arange(n_seqs, dtype=torch.int32, device=dev).repeat_interleave(q_len).contiguous()
         token_pos = torch.arange(q_len, dtype=torch.int32, device=dev).repeat(n_seqs).contiguous() + (0 if q_len > 1 else 5)
         chunked = q_len > 128
-        dchunk = 128 if chunked else 0
         max_chunks = -(-q_len // 64) if chunked else 1
         # the like kernel: the wkv recurrence at its own shape (state heads x 64 x 64)
         WH, wd = s["wkv_heads"], s["wkv_dim"]
@@ -310,10 +314,9 @@ def lunadra_kernel_pairs(pe, torch, s, hbm_gbs, prompt, batch, context):
         gbias, nw = torch.zeros(2 * H, device=dev), torch.ones(vv, device=dev)
         o = torch.empty(n, vv, dtype=bf, device=dev)
         S, nn, mm = torch.zeros(n_seqs, H, d, dv, device=dev), torch.zeros(n_seqs, H, d, device=dev), torch.zeros(n_seqs, H, device=dev)
-        scratch_m = torch.empty(ops.mlstm_scratch_floats(n_seqs, H, d, dv, max_chunks), device=dev) if chunked else None
-        us = us_of(lambda: ops.mlstm_recurrence(qkvg[:, :qk], qkvg[:, qk:2 * qk], qkvg[:, 2 * qk:2 * qk + vv], qkvg[:, 2 * qk + vv:], gates,
-                                                gbias, nw, 15.0, 1e-6, d ** -0.5, o, S, nn, mm, slots, qstart, n_seqs, q_len, H, d, dv,
-                                                status, 64 if chunked else 0, max_chunks, scratch_m))
+        memory = (qkvg[:, :qk], qkvg[:, qk:2 * qk], qkvg[:, 2 * qk:2 * qk + vv], qkvg[:, 2 * qk + vv:], gates, gbias, nw, 15.0, 1e-6,
+                  d ** -0.5, o, S, nn, mm, slots, qstart)
+        us = us_of(lambda: walk.run_mlstm(memory, n_seqs, q_len, H, d, dv, status, scratch_of))
         entry(f"{what}: mlstm recurrence, head norm, gate", us, roof_us(n * (2 * qk + 3 * vv) * 2 + n_seqs * H * d * dv * 8, n * H * d * dv * 5.0),
               "wkv_recurrence", us_wkv, roof_wkv)
         # gated delta rule
@@ -325,10 +328,8 @@ def lunadra_kernel_pairs(pe, torch, s, hbm_gbs, prompt, batch, context):
         gate = torch.randn(n, DH * ddv, device=dev).to(bf)
         o2 = torch.empty(n, DH * ddv, dtype=bf, device=dev)
         S2 = torch.zeros(n_seqs, DH, dd, ddv, device=dev)
-        dmax = -(-q_len // 128) if chunked else 1
-        scratch_d = torch.empty(ops.delta_rule_scratch_floats(n_seqs, DH, dd, ddv, dmax), device=dev) if chunked else None
-        us = us_of(lambda: ops.delta_rule_recurrence(qkv, a_lin, dtb, alog, beta, gate, nw2, 1e-6, dd ** -0.5, o2, S2, slots, qstart, n_seqs,
-                                                     q_len, DH, DG, dd, ddv, status, dchunk, dmax, scratch_d))
+        rule = (qkv, a_lin, dtb, alog, beta, gate, nw2, 1e-6, dd ** -0.5, o2, S2, slots, qstart)
+        us = us_of(lambda: walk.run_delta_rule(rule, n_seqs, q_len, DH, DG, dd, ddv, status, scratch_of))
         entry(f"{what}: gated delta recurrence, head norm, gate", us,
               roof_us(n * (ch * 2 + DH * dd * 4 + DH * ddv * 4) + n_seqs * DH * dd * ddv * 8, n * DH * dd * ddv * 7.0),
               "wkv_recurrence", us_wkv, roof_wkv)
@@ -633,6 +634,11 @@ def zonevik_kernel_pairs(pe, torch, s, peaks, prompt, batch, context):
     flush = torch.zeros(96 * 2 ** 20, device=dev)
     status = torch.zeros(4, dtype=torch.int32, device=dev)
     out = {}
+    walk = importlib.import_module(pe.__name__ + ".parts.walk")
+    areas = {}
+
+    def scratch_of(name, floats):
+        return areas.setdefault((name, floats), torch.empty(floats, device=dev))
 
     def us_of(fn):
         return 1e3 * timed(torch, fn, 20, 5, flush, graph=True)
@@ -660,16 +666,13 @@ def zonevik_kernel_pairs(pe, torch, s, peaks, prompt, batch, context):
         gate = torch.randn(n, DH * ddv, device=dev).to(bf)
         o2 = torch.empty(n, DH * ddv, dtype=bf, device=dev)
         S2 = torch.zeros(n_seqs, DH, dd, ddv, device=dev)
-        dmax = -(-q_len // 128) if chunked else 1
-        scratch_d = torch.empty(ops.delta_rule_scratch_floats(n_seqs, DH, dd, ddv, dmax), device=dev) if chunked else None
-        us_delta = us_of(lambda: ops.delta_rule_recurrence(qkv, a_lin, dtb, alog, beta, gate, nw2, 1e-6, dd ** -0.5, o2, S2, slots, qstart,
-                                                           n_seqs, q_len, DH, DG, dd, ddv, status, 128 if chunked else 0, dmax, scratch_d))
+        rule = (qkv, a_lin, dtb, alog, beta, gate, nw2, 1e-6, dd ** -0.5, o2, S2, slots, qstart)
+        us_delta = us_of(lambda: walk.run_delta_rule(rule, n_seqs, q_len, DH, DG, dd, ddv, status, scratch_of))
         roof_delta = roof_us(n * (ch * 2 + DH * dd * 4 + DH * ddv * 4) + n_seqs * DH * dd * ddv * 8, n * DH * dd * ddv * 7.0)
         # the same kernel with one decay a head and the silu gate (what Zonevik's delta layers run)
         a_head, dtb_h = torch.randn(n, DH, device=dev), torch.zeros(DH, device=dev)
-        us = us_of(lambda: ops.delta_rule_recurrence(qkv, a_head, dtb_h, alog, beta, gate, nw2, 1e-6, dd ** -0.5, o2, S2, slots, qstart,
-                                                     n_seqs, q_len, DH, DG, dd, ddv, status, 128 if chunked else 0, dmax, scratch_d,
-                                                     head_decay=True, gate_silu=True))
+        rule_h = (qkv, a_head, dtb_h, alog, beta, gate, nw2, 1e-6, dd ** -0.5, o2, S2, slots, qstart)
+        us = us_of(lambda: walk.run_delta_rule(rule_h, n_seqs, q_len, DH, DG, dd, ddv, status, scratch_of, head_decay=True, gate_silu=True))
         entry(f"{what}: gated delta recurrence with one decay a head, silu gate", us,
               roof_us(n * (ch * 2 + DH * 8 + DH * ddv * 4) + n_seqs * DH * dd * ddv * 8, n * DH * dd * ddv * 7.0),
               "delta_rule_recurrence (decay per channel)", us_delta, roof_delta)

@@ -28,16 +28,7 @@ from ..kernels import ops
 from .linear import fuse_rows
 from .registry import register
 from .spec import CacheRequest, WeightDecl
-
-
-# steps whose longest sequence brings at least this many tokens spread each head's columns over the chip (csrc/walk.cuh), where
-# its sizes are taken; fewer tokens are over before its two further launches have paid
-WALK_TOKENS = 4
-
-# otherwise: tokens per chunk when a prompt is cut into chunks that run side by side (the chain from chunk to chunk costs a product
-# with a d x d matrix per chunk, so the chunks are longer than the mlstm's); steps whose longest sequence has no more
-# tokens than one chunk walk each sequence in one go
-CHUNK_TOKENS = 128
+from .walk import run_delta_rule
 
 
 @register("mixer", "gated_delta")
@@ -166,20 +157,11 @@ class GatedDeltaMixer:
     def recur(self, qkv, decay, beta, gate, out, ctx, view) -> None:
         """The recurrence over the step's tokens, from the convolved q | k | v to the gated, normed head outputs."""
         rt = self.runtime
-        n, nh, nkv, d, dv = qkv.shape[0], self.n_heads, self.n_kv_heads, self.head_dim, self.v_dim
-        args = (qkv, decay, self.dt_bias, self.A_log, beta, gate, self.norm, self.eps, d ** -0.5, out, view.state("S"), ctx.seq_slot,
-                ctx.seq_qstart, ctx.n_seqs)
-        form = dict(head_decay=self.head_decay, gate_silu=self.gate_silu)
-        walk = ops.delta_rule_walk_scratch_floats(n, nh, nkv, d, dv) if ctx.max_q >= WALK_TOKENS else 0
-        if walk:
-            ops.delta_rule_walk(*args, nh, nkv, d, dv, rt.status, ctx.buffer("delta.walk", (walk,), torch.float32), **form)
-            return
-        chunk, max_chunks, scratch = 0, 1, None
-        if ctx.max_q > CHUNK_TOKENS:
-            chunk = CHUNK_TOKENS
-            max_chunks = -(-ctx.max_q // chunk)
-            scratch = ctx.buffer("delta.scratch", (ops.delta_rule_scratch_floats(ctx.n_seqs, nh, d, dv, max_chunks),), torch.float32)
-        ops.delta_rule_recurrence(*args, ctx.max_q, nh, nkv, d, dv, rt.status, chunk, max_chunks, scratch, **form)
+        d, dv = self.head_dim, self.v_dim
+        run_delta_rule((qkv, decay, self.dt_bias, self.A_log, beta, gate, self.norm, self.eps, d ** -0.5, out, view.state("S"), ctx.seq_slot,
+                        ctx.seq_qstart), ctx.n_seqs, ctx.max_q, self.n_heads, self.n_kv_heads, d, dv, rt.status,
+                       lambda name, floats: ctx.buffer(name, (floats,), torch.float32), head_decay=self.head_decay,
+                       gate_silu=self.gate_silu)
 
     def forward_full_rank(self, x, wide, qkv, ctx, view) -> torch.Tensor:
         """The form with one decay per head and a silu gate of full rank: beta | decay are the float32 outputs of one product,

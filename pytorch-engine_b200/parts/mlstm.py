@@ -19,19 +19,10 @@ from typing import Dict, Optional
 
 import torch
 
-from ..kernels import ops
 from .linear import fuse_rows
 from .registry import register
 from .spec import CacheRequest, WeightDecl
-
-
-# steps whose longest sequence brings at least this many tokens spread each head's columns over the chip (csrc/walk.cuh), where
-# its sizes are taken; fewer tokens are over before its two further launches have paid
-WALK_TOKENS = 4
-
-# otherwise: tokens per chunk when a prompt is cut into chunks that run side by side; steps whose longest sequence has no more
-# tokens than two chunks walk each sequence in one go
-CHUNK_TOKENS = 64
+from .walk import run_mlstm
 
 
 @register("mixer", "mlstm")
@@ -89,24 +80,10 @@ class MlstmMixer:
         if y.data_ptr() != gates.data_ptr():
             gates.copy_(y)
         out = ctx.buffer("mlstm.out", (n, vv), rt.dtype)
-        chunk, max_chunks, scratch = 0, 1, None
-        views = (qkvg[:, :qk], qkvg[:, qk:2 * qk], qkvg[:, 2 * qk:2 * qk + vv], qkvg[:, 2 * qk + vv:])
-        walk = ops.mlstm_walk_scratch_floats(n, self.n_heads, self.head_dim, self.v_dim) if ctx.max_q >= WALK_TOKENS else 0
-        if walk:
-            ops.mlstm_walk(*views, gates, self.gate_bias, self.norm, self.cap, self.eps, self.head_dim ** -0.5, out, view.state("S"),
-                           view.state("n"), view.state("m"), ctx.seq_slot, ctx.seq_qstart, ctx.n_seqs, self.n_heads, self.head_dim,
-                           self.v_dim, rt.status, ctx.buffer("mlstm.walk", (walk,), torch.float32))
-            delta = ctx.buffer("mlstm.delta", (n, self.hidden), rt.dtype)
-            rt.linear(out, self.o_proj, out=delta)
-            return delta
-        if ctx.max_q > 2 * CHUNK_TOKENS:
-            chunk = CHUNK_TOKENS
-            max_chunks = -(-ctx.max_q // chunk)
-            scratch = ctx.buffer("mlstm.scratch", (ops.mlstm_scratch_floats(ctx.n_seqs, self.n_heads, self.head_dim, self.v_dim,
-                                                                          max_chunks),), torch.float32)
-        ops.mlstm_recurrence(*views, gates, self.gate_bias, self.norm, self.cap, self.eps, self.head_dim ** -0.5, out, view.state("S"),
-                             view.state("n"), view.state("m"), ctx.seq_slot, ctx.seq_qstart, ctx.n_seqs, ctx.max_q, self.n_heads,
-                             self.head_dim, self.v_dim, rt.status, chunk, max_chunks, scratch)
+        run_mlstm((qkvg[:, :qk], qkvg[:, qk:2 * qk], qkvg[:, 2 * qk:2 * qk + vv], qkvg[:, 2 * qk + vv:], gates, self.gate_bias, self.norm,
+                   self.cap, self.eps, self.head_dim ** -0.5, out, view.state("S"), view.state("n"), view.state("m"), ctx.seq_slot,
+                   ctx.seq_qstart), ctx.n_seqs, ctx.max_q, self.n_heads, self.head_dim, self.v_dim, rt.status,
+                  lambda name, floats: ctx.buffer(name, (floats,), torch.float32))
         delta = ctx.buffer("mlstm.delta", (n, self.hidden), rt.dtype)
         rt.linear(out, self.o_proj, out=delta)
         return delta

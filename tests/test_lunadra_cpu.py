@@ -132,3 +132,19 @@ def test_prompts_take_no_sizes_that_single_tokens_refuse(pe):
                          (32, 1040, False), (96, 128, False), (64, 24, False)]:
         assert (ops.mlstm_walk_scratch_floats(8, 4, d, dv) > 0) == taken, (d, dv)
         assert (ops.delta_rule_walk_scratch_floats(8, 4, 4, d, dv) > 0) == taken, (d, dv)
+
+
+# sizes of a step, and what the form with a head in one block and the walk over columns took on a B200 (us)
+@pytest.mark.parametrize("kind,d,dv,heads,seqs,tokens,block,walk", [
+    ("mlstm", 128, 256, 4, 1, 2048, 185, 300), ("mlstm", 128, 256, 4, 1, 8192, 746, 1189), ("mlstm", 128, 256, 4, 1, 512, 173, 81),
+    ("mlstm", 128, 256, 8, 1, 2048, 360, 315), ("mlstm", 128, 256, 8, 2, 1024, 355, 251), ("mlstm", 128, 256, 8, 32, 4, 30, 47),
+    ("mlstm", 64, 128, 8, 1, 1024, 97, 113), ("mlstm", 64, 128, 8, 1, 2048, 123, 233), ("mlstm", 64, 128, 16, 32, 64, 109, 138),
+    ("mlstm", 128, 256, 4, 8, 16, 35, 19), ("delta", 128, 128, 8, 1, 2048, 604, 393), ("delta", 128, 128, 4, 1, 8192, 1178, 1538),
+    ("delta", 64, 64, 4, 1, 4096, 443, 573), ("delta", 128, 128, 8, 2, 1024, 596, 206), ("delta", 128, 128, 8, 32, 4, 19, 29),
+    ("delta", 128, 128, 4, 1, 4, 13, 8)])
+def test_steps_of_several_tokens_take_the_faster_form_of_the_recurrence(pe, kind, d, dv, heads, seqs, tokens, block, walk):
+    rule = import_module("pytorch-engine_b200.parts.walk")
+    cost, chunk, whole = (rule.MLSTM, 64, 128) if kind == "mlstm" else (rule.DELTA, 128, 128)
+    took = walk if rule.takes_walk(cost, seqs * tokens, seqs, tokens, heads, d, dv, chunk, whole, 148) else block
+    assert took <= 1.15 * min(block, walk)
+    assert not rule.takes_walk(cost, seqs, seqs, 1, heads, d, dv, chunk, whole, 148)      # single tokens: one launch
