@@ -635,7 +635,8 @@ __global__ void __launch_bounds__(128) decode_split_kernel(Args a, const __grid_
     a.part_acc[pidx * vd + c] = (ll > 0.f) ? aa / ll : 0.f;
     // log-sum-exp in natural units, as the merge kernel expects: (m + log2 l) * ln 2
     if (c == 0) a.part_lse[pidx] = (ll > 0.f) ? (mm + log2f(ll)) * 0.6931471805599453f : -INFINITY;
-  }  if (CLUSTER) {
+  }
+  if (CLUSTER) {
     // the ranges that hold something, and this one's place among them (as in the merge kernel below)
     const int n_splits = (len + per_range - 1) / per_range;
     const int first = min(win_lo / per_range, n_splits), kept = min((keep + per_range - 1) / per_range, first);
@@ -771,11 +772,13 @@ static int decode_blocks_per_sm(int head_dim, int v_dim) {
   const int n = (int)((227 * 1024) / smem);
   return n < 1 ? 1 : n;
 }
-// Whether a decode step's ranges are put together inside clusters: cut by the sequences' own lengths, and few.  One sequence
-// of 300 keys, 8 kv heads: 7.1 -> 5.7 us, a step of the 0.6B shape 750 -> 723 us.  With more blocks the second kernel is better:
-// 64 pairs of four ranges take 26.8 instead of 28.7 us by themselves, but the product behind them, which then starts while
-// they drain, loses twice that (8B shape, 8 sequences of 4,090 keys: 1,488 -> 1,535 us a step), and with more blocks than the
-// chip holds clusters wait for room (64 sequences of up to 4,096 keys: 94 -> 112 us).
+// Whether a decode step's ranges are put together inside clusters: cut by the sequences' own lengths, and few.  The number of
+// ranges follows the cache's limit, so this is for caches of few keys: up to 1,024 for 4 to 8 pairs of sequence and kv head, 512
+// for 16, 256 for 32, 128 for 64.  One sequence of 300 keys, 8 kv heads: 4.4 us, with the second kernel 5.8 (and so in a cache for
+// more than 1,024 keys, which gets 16 ranges and up); a step of the 0.6B shape in a cache for 320 keys 750 -> 723 us.
+// With more blocks the second kernel is better: 64 pairs of four ranges take 26.8 instead of 28.7 us by themselves, but the
+// product behind them, which then starts while they drain, loses twice that (8B shape, 8 sequences of 4,090 keys: 1,488 -> 1,535
+// us a step), and with more blocks than the chip holds clusters wait for room (64 sequences of up to 4,096 keys: 94 -> 112 us).
 static bool cluster_ranges(int pairs, int split_keys, int max_splits) {
   return split_keys == 0 && max_splits <= kClusterRanges && (long long)pairs * max_splits <= kClusterBlocks;
 }

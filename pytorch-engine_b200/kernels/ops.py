@@ -1,7 +1,6 @@
 """Tensor-level wrappers of the CUDA entry points.  Every op requires CUDA tensors."""
 from __future__ import annotations
 
-import math
 from typing import Optional
 
 import torch
@@ -661,27 +660,26 @@ def attention_mma_decode_ranges(device: torch.device, head_dim: int, n_seqs: int
 
 
 def mma_decode_ranges(slots: int, pairs: int, max_kv_len: int, split_keys: int) -> tuple:
-    """``decode_ranges`` with two cases of its own.  How a sequence's keys are cut depends on its own length, the cache's limit
-    and the number of sequences, never on the other sequences' lengths.
+    """``decode_ranges`` with a case of its own.  How a sequence's keys are cut depends on its own length, the cache's limit
+    ``max_kv_len`` and the number of sequences, never on the other sequences' lengths.
 
-    Room for two or more ranges a pair: a block takes about 0.8 us a page and the chip is mostly empty, so up to 16 ranges of
-    two pages or more, while one wave holds them (one sequence, 8 kv heads: 300 keys 8.9 -> 7.1 us, 3,900 keys 11.3 -> 9.2).
+    Room for two or more ranges a pair: a block takes about 0.8 us a page and the chip is mostly empty, so ranges of two pages
+    or more, 16 of them or as many as ranges of ``split_keys`` keys would be, whichever is more, while one wave holds them.
+    In a cache for 40,960 keys, 8 kv heads, against ``decode_ranges``: one sequence of 300 keys 8.1 -> 5.8 us, of 2,048 keys 10.3
+    -> 7.3; four of 2,048 13.5 -> 11.5; eight of 300 10.3 -> 8.1, of 2,048 16.4 and 16.5.  (15 batches of one to 32 sequences of equal
+    and of unequal lengths, caches for 4,096 and 40,960 keys: 0.58 to 1.02 times the time.)  A cache for few keys gets few ranges,
+    and few ranges need no second kernel (csrc/attention_mma.cu, ``cluster_ranges``): one sequence of 300 keys in a cache for up
+    to 1,024, 4.4 us.
 
-    Pairs fill between half of the slots and all of them: ranges of 512 to 1,024 keys, as many as fill their last wave best.
-    One range a pair leaves the chip to the longest sequences (24 sequences of 16 to 2,048 keys, 8 kv heads: 36.4 us with one,
-    28 with three; all of 2,048 keys: 36.9 and 38.6).  With more pairs than slots the waves even that out (64 sequences: 93.7
-    against 95.5)."""
+    Less room: as there.  (Ranges of 512 to 1,024 keys in two or three waves helped unequal lengths and cost equal ones: 24
+    sequences of 16 to 2,048 keys 34.3 -> 32.6 us, all of 2,048 keys 36.3 -> 38.1, 30 of 2,048 43.6 -> 51; and in a cache for many
+    keys their empty blocks alone cost more than that: 24 sequences of 300 keys, 40,960 in the cache, 16.9 -> 21.8 us.)"""
     pairs = max(1, pairs)
     per_pair = slots // pairs
+    if per_pair < 2:
+        return decode_ranges(slots, pairs, max_kv_len, split_keys)
     fixed = -(-max_kv_len // split_keys)
-    if per_pair >= 2:
-        return 0, max(1, min(per_pair, max(16, fixed), -(-max_kv_len // 128))), 128
-    if per_pair == 1:
-        fewest, most = max(1, -(-max_kv_len // (2 * split_keys))), max(1, max_kv_len // split_keys)
-        waves = lambda s: pairs * s / slots
-        splits = max(range(fewest, max(fewest, min(most, fewest + 8)) + 1), key=lambda s: (waves(s) / math.ceil(waves(s)), -s))
-        return 0, splits, max(64, -(-max_kv_len // (64 * splits)) * 64)
-    return decode_ranges(slots, pairs, max_kv_len, split_keys)
+    return 0, max(1, min(per_pair, max(16, fixed), -(-max_kv_len // 128))), 128
 
 
 def attention_umma_supported(dtype: torch.dtype, head_dim: int, n_heads: int, n_kv_heads: int) -> bool:

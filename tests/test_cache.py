@@ -194,7 +194,10 @@ def test_decode_attention_ranges_on_the_tensor_core_kernel(pe):
     """The rule of csrc/attention_mma.cu: every length is covered, one wave where there is room, whole pages."""
     f = pe.kernels.ops.mma_decode_ranges
     assert f(296, 8, 320, 512) == (0, 3, 128) and f(296, 8, 3968, 512) == (0, 16, 128) and f(296, 8, 40960, 512) == (0, 37, 128)
-    assert f(296, 64, 4096, 512) == (0, 4, 128) and f(296, 192, 2112, 512) == (0, 3, 704) and f(296, 512, 4096, 512) == (0, 2, 2048)
+    assert f(296, 64, 4096, 512) == (0, 4, 128) and f(296, 512, 4096, 512) == (0, 2, 2048)
+    # one range a pair in a wave: no more ranges than the general rule's, whatever the cache's limit
+    for pairs, cap in [(152, 1024), (192, 2112), (192, 40960), (240, 8192), (296, 4096)]:
+        assert f(296, pairs, cap, 512) == pe.kernels.ops.decode_ranges(296, pairs, cap, 512)
     for slots, pairs, cap in [(296, 7, 5000), (296, 148, 64), (296, 149, 64), (296, 296, 40960), (296, 200, 1000), (10, 1000, 64), (592, 100, 70000)]:
         sk, n, least = f(slots, pairs, cap, 512)
         assert sk == 0 and n >= 1 and least > 0 and least % 64 == 0
