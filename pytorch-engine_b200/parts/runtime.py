@@ -4,7 +4,8 @@
 unquantised linears with a library call (``F.linear``, pygguf_engine/quant_kernels.py:1836); here
 the library product (cuBLAS through ``torch.mm``) stands wherever the package's own tensor-core
 kernels do not take the shape, and the float32 mode never computes in less than float32 (TF32 is
-switched off around the call; from 16 rows on each operand is three bfloat16 parts, csrc/gemm_split32.cu).
+switched off around the call; larger products of 16 rows and more split each operand into three
+bfloat16 parts, csrc/gemm_split32.cu).
 """
 from __future__ import annotations
 
@@ -60,6 +61,20 @@ def large_gemm_fill(rows: int, cols: int, sms: int) -> float:
     return tiles / (waves * pairs)
 
 
+def split32_pays(rows: int, cols: int, depth: int) -> bool:
+    """Whether a float32 product of 16 rows or more is faster on csrc/gemm_split32.cu than in the library.  It has two or three
+    launches and a long start, so sums of few terms pay only where the outputs are many; up to 16 rows the library has a
+    short-cut for narrow weights.  This kernel and the library, us: 24 rows, 4,096 x 1,024 weights 13 and 27; 16 rows, 151,936 x
+    1,024 222 and 238, 256 x 1,024 10.4 and 8.6; 128 rows, 4,096 x 512 12 and 17, 1,024 x 512 11.2 and 10.9; 512 rows, 1,024 x 64 5.8
+    and 4.4; 2,048 rows, 4,096 x 64 25 and 35.  Over 1,430 sizes (16 to 4,096 rows, 16 to 32,768 columns, 32 to 1,536 terms) the
+    choice is nowhere more than 4 % slower than the library, and misses a gain of 10 % or more in one of 36."""
+    if depth < 64:
+        return False
+    if depth < 768:
+        return rows >= 96 and rows * cols >= 3 << (19 if depth < 128 else 18 if depth < 512 else 17)
+    return depth >= 1536 or ((rows > 16 or cols >= 2048) and (cols >= 128 or rows <= 1024))
+
+
 class Runtime:
     def __init__(self, device, dtype: torch.dtype) -> None:
         self.device = torch.device(device)
@@ -87,8 +102,7 @@ class Runtime:
         self.own_large_gemm = True
         self.large_gemm_rows = 1024
         self.large_gemm_min_fill = 0.8   # least share of the waves of tiles that does work (see takes_large_gemm)
-        # float32 products with at least this many rows run on csrc/gemm_split32.cu (16 rows: 12-15 us against the library's
-        # 19-24 on the 0.6B shape; single tokens stay with the library)
+        # float32 products with at least this many rows may run on csrc/gemm_split32.cu (see split32_pays)
         self.split32_rows = 16
         self.pair_gemm = True       # large products on tcgen05 cta_group::2
         # q/k-norm, rotation and cache append in the epilogue of the q|k|v product where the pair kernel runs it
@@ -136,7 +150,7 @@ class Runtime:
     def takes_split32_gemm(self, x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor], out_dtype) -> bool:
         """Whether a float32 product runs on csrc/gemm_split32.cu (float32's precision on the tensor cores)."""
         return (x.dtype == torch.float32 and self.own_large_gemm and x.dim() == 2 and x.shape[0] >= self.split32_rows
-                and out_dtype in (None, torch.float32) and ops.gemm_split32_supported(x, weight)
+                and out_dtype in (None, torch.float32) and split32_pays(x.shape[0], weight.shape[0], x.shape[1]) and ops.gemm_split32_supported(x, weight)
                 and (out is None or (out.dtype == torch.float32 and out.stride(1) == 1 and out.stride(0) % 4 == 0
                                      and out.stride(0) >= weight.shape[0] and out.data_ptr() % 16 == 0))
                 and (out is not None or weight.shape[0] % 4 == 0))

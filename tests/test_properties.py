@@ -2,6 +2,7 @@
 decisions for any mix of prompt lengths, limits and stop tokens, and (on the GPU) the logits of a prompt cut into
 steps in any way."""
 import random
+from importlib import import_module
 
 import pytest
 import torch
@@ -223,3 +224,13 @@ def test_any_cut_of_a_prompt_gives_the_same_logits(pe, model_folders, tmp_path, 
 
     run()
     eng.cache.check()
+
+
+# rows, columns and terms of float32 products, and what csrc/gemm_split32.cu and the library took on a B200 (us)
+@pytest.mark.parametrize("rows,cols,depth,own,library", [
+    (24, 4096, 1024, 13.1, 27.3), (16, 151936, 1024, 222.0, 238.0), (16, 256, 1024, 10.4, 8.6), (17, 256, 1024, 10.6, 13.1),
+    (128, 4096, 512, 12.0, 17.0), (128, 1024, 512, 11.2, 10.9), (512, 1024, 64, 5.8, 4.4), (2048, 4096, 64, 24.7, 35.4),
+    (64, 64, 64, 5.3, 3.6), (4096, 16, 768, 15.9, 15.1), (16, 16, 2048, 10.8, 14.2)])
+def test_float32_products_take_the_faster_kernel(pe, rows, cols, depth, own, library):
+    pays = import_module("pytorch-engine_b200.parts.runtime").split32_pays(rows, cols, depth)
+    assert (own if pays else library) <= 1.05 * min(own, library)
