@@ -37,7 +37,10 @@ constexpr int kTopPer = 32;           // entries a thread of sample_top_kernel h
 constexpr int kTopChunk = kTopThreads * kTopPer;
 constexpr int kTopGroups = 256;       // groups of a chunk whose maxima bound its k-th value from below
 // Largest top-k for sample_top_kernel.  Of 256 group maxima the k-th largest has about 256 ln(256 / (256 - k))
-// entries at or above it: 56 for k = 50, 532 for k = 224, 1,567 for k = 256, where the bound says nothing any more.
+// entries at or above it: 56 for k = 50, 532 for k = 224, 1,567 for k = 256, where the bound says nothing any more.  From
+// about k = 130 on that is more than the room (k + k / 4 + 16 candidates), and chunks search their k-th key bit by bit: both
+// kernels together take 36 us at k = 50 (64 rows of 151,936, top-p 0.95), 38 at 100, 58 at 128, 68 at 150 and 70 at 200 and 224,
+// where the form for larger k takes 247 at 50 and 460 from 81 on.
 constexpr int kTopMax = 224;
 static_assert(kTopGroups * 2 == kTopThreads, "a group is a pair of threads");
 
@@ -244,8 +247,8 @@ __device__ __forceinline__ int block_offset(int mine, int* scratch, int* total) 
 // First kernel for top-k up to kTopMax.  grid: (chunks of kTopChunk, rows).
 // The chunk stays in registers.  The k-th largest of the maxima of 256 groups of 64 entries has k
 // entries at or above it, so nothing below it can be among the chunk's k largest; what is left is
-// little more than k entries and goes out as it is.  Where it is more than the room (ties, or k near
-// the number of groups) the k-th key is searched bit by bit.  64 rows of 151,936 entries, top-k 50, take
+// little more than k entries and goes out as it is.  Where it is more than the room (ties, or k from
+// about 130 on) the k-th key is searched bit by bit.  64 rows of 151,936 entries, top-k 50, take
 // 26 us (39 MB, 1.5 TB/s: the ranking, not the reads); the threshold search of sample_chunks_kernel, which
 // reads every entry eight times from shared memory with sixteen conditional adds each, took 186 us.
 __global__ void __launch_bounds__(kTopThreads) sample_top_kernel(SampleArgs a) {
