@@ -20,9 +20,11 @@
 //   17     TMA producer: the three parts of the x tile.
 // Operands that three parts cannot hold (infinities, NaN, numbers next to either end of float32's range) and results as small or
 // as large are noticed, and what they touch is computed again as a plain chain of multiply-adds (second_look).
-// What bounds it: the issue of 24 MMAs a chunk and shared memory (96 KB written and 192 KB read per 64 of K of a 128 x 128 tile:
-// 1.2 of the 1.5 us that a chunk takes).  600 rows against the library's float32 product: 4,096 x 1,024 weights 57 against
-// 121 us, 1,024 x 3,072 36 against 125, 151,936 x 1,024 1,113 against 3,173 (168 TFLOP/s); 16 rows 12-15 against 19-24.
+// What bounds it: no unit (600 x 30,720 outputs, K = 1,024, 261 us, 145 TFLOP/s: tensor pipe 46 % busy, loads and stores of shared
+// memory 43 %, issue slots 38 %).  A block takes 32 us for its 16 chunks; about 3 lie before the first chunk's sums and behind the
+// last's, where nothing overlaps, and in between conversion, MMAs and addition of a chunk follow one another over two stages.
+// 600 rows against the library's float32 product: 4,096 x 1,024 weights 55 against 122 us, 1,024 x 3,072 35 against 125, 151,936 x
+// 1,024 1,137 against 3,349 (164 TFLOP/s); 24 rows, 4,096 x 1,024 13 against 27.
 // All waits are bounded.
 #include "api.h"
 #include "common.cuh"
