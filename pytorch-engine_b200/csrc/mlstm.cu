@@ -427,7 +427,7 @@ static int mlstm_run(const MlstmArgs& a, int max_q, cudaStream_t stream) {
   auto k0 = mlstm_kernel<T, 0, DREG, SPLIT>;
   auto k1 = mlstm_kernel<T, 1, DREG, SPLIT>;
   auto k3 = mlstm_kernel<T, 3, DREG, SPLIT>;
-  if (smem > 48 * 1024) {
+  if (smem > 47 * 1024) {      // beside it the kernels have static shared memory of their own
     cudaError_t e = cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

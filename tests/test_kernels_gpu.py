@@ -602,6 +602,35 @@ def test_attention_mma_decode_clusters(ops, nh, nkv, d, B, splits, window, keep,
         assert rel_err(outs[0].view(B, nh, d), want) < ATT_TOL[torch.bfloat16]
 
 
+@pytest.mark.parametrize("d,dv,kind", [(36, 96, "delta"), (64, 126, "mlstm")])
+def test_recurrences_just_below_48_kb(ops, d, dv, kind):
+    """Heads whose dynamic shared memory stays below 48 KB only without the kernel's static part: two tokens in one call as in two."""
+    torch.manual_seed(26)
+    H, B, slots = 2, 2, 3
+    slot, rand = torch.tensor([2, 0], dtype=torch.int32, device=DEV), (lambda *shape: torch.randn(*shape, device=DEV))
+    rows, gates, bias = rand(2 * B, H * (2 * d + 2 * dv)), rand(2 * B, 2 * H), rand(2 * H)
+    S0, n0, m0, w = rand(slots, H, d, dv), rand(slots, H, d), rand(slots, H), 1 + 0.2 * rand(H * dv)
+
+    def run(rows, gates, per, S, n, m):
+        rows, gates = rows.contiguous(), gates.contiguous()
+        out, st = torch.full((per * B, H * dv), float("nan"), device=DEV), _status()
+        qstart = torch.arange(0, per * B + 1, per, dtype=torch.int32, device=DEV)
+        q, k, v, g = (rows[:, lo:hi] for lo, hi in ((0, H * d), (H * d, 2 * H * d), (2 * H * d, H * (2 * d + dv)), (H * (2 * d + dv), rows.shape[1])))
+        if kind == "delta":
+            ops.delta_rule_recurrence(rows[:, :H * (2 * d + dv)].contiguous(), gates[:, :H].contiguous(), bias[:H], bias[H:], gates[:, H:].contiguous(), g, w[:dv],
+                                      1e-6, d ** -0.5, out, S, slot, qstart, B, per, H, H, d, dv, st, head_decay=True)
+        else:
+            ops.mlstm_recurrence(q, k, v, g, gates, bias, w, 15.0, 1e-6, d ** -0.5, out, S, n, m, slot, qstart, B, per, H, d, dv, st)
+        assert st.tolist()[0] == 0
+        return out
+
+    once, twice = [t.clone() for t in (S0, n0, m0)], [t.clone() for t in (S0, n0, m0)]
+    whole = run(rows, gates, 2, *once)
+    for i in range(2):
+        assert rel_err(run(rows[i::2], gates[i::2], 1, *twice), whole[i::2]) < 2e-5
+    assert all(rel_err(x, y) < 5e-6 for x, y in zip(once, twice))
+
+
 @pytest.mark.parametrize("decode", [False, True])
 def test_attention_mma_finds_a_far_key_and_ignores_what_lies_beyond_the_length(ops, decode):
     nh, nkv, d = 8, 2, 128
