@@ -15,9 +15,9 @@
 // first cuts every row into chunks, one block each, and leaves each chunk's candidates (a set that
 // holds its own top-k; or its largest entry); the second runs the filter chain on the candidates
 // of a row, which hold every entry that the row's top-k can keep.
-//   top-k up to kTopMax: chunks of kTopChunk entries held in registers, candidates above a lower
-//     bound of the chunk's k-th value that costs one comparison of 256 group maxima with each other
-//     (sample_top_kernel); the second kernel finds the row's k-th value bit by bit on keys in registers.
+//   top-k up to kTopMax: the first leaves the largest value of every group of 8 to 512 neighbouring entries and nothing else
+//     (sample_maxima_kernel); the second bounds the row's k-th value by the k-th of the maxima, which has k entries at or above
+//     it, and reads again only the groups whose maximum reaches it.
 //   larger top-k: chunks of kChunk entries in shared memory, threshold search (sample_chunks_kernel).
 // A threshold search over a row takes 8 sweeps of 4 bits with per-thread counters (no atomics, fixed
 // summation order) instead of 32 sweeps of one bit.
@@ -32,17 +32,16 @@ constexpr int kChunk = 4096;        // entries of a row per block of the first k
 constexpr int kChunkThreads = 256;
 constexpr int kMaxChunks = 64;
 constexpr int kMaxCandidates = 3072;  // candidates of a row that the second kernel takes
-constexpr int kTopThreads = 512;
-constexpr int kTopPer = 32;           // entries a thread of sample_top_kernel holds in registers
-constexpr int kTopChunk = kTopThreads * kTopPer;
-constexpr int kTopGroups = 256;       // groups of a chunk whose maxima bound its k-th value from below
-// Largest top-k for sample_top_kernel.  Of 256 group maxima the k-th largest has about 256 ln(256 / (256 - k))
-// entries at or above it: 56 for k = 50, 532 for k = 224, 1,567 for k = 256, where the bound says nothing any more.  From
-// about k = 130 on that is more than the room (k + k / 4 + 16 candidates), and chunks search their k-th key bit by bit: both
-// kernels together take 36 us at k = 50 (64 rows of 151,936, top-p 0.95), 38 at 100, 58 at 128, 68 at 150 and 70 at 200 and 224,
-// where the form for larger k takes 247 at 50 and 460 from 81 on.
+constexpr int kGroupThreads = 512;      // threads of the second kernel where the first left groups' maxima
+constexpr int kGroupsPer = 5;           // maxima a thread of it holds
+constexpr int kMaxGroups = kGroupThreads * kGroupsPer;
+constexpr int kMaximaThreads = 256;
+constexpr int kMaximaTask = 1024;       // entries a warp of the first kernel takes: eight 16-byte loads a lane
+constexpr int kMaxGroupList = 1024;     // groups that the second kernel reads again
+constexpr int kMaxRanked = 640;         // candidates up to which each is compared with every other
+// Largest top-k for the groups.  They are at least 512 (see group_size), and the k-th largest of g maxima has about g ln(g / (g - k))
+// entries at or above it: 56 for k = 50 and 295 for k = 224 where g = 512, 229 where g = 2,374 (a row of 151,936 entries).
 constexpr int kTopMax = 224;
-static_assert(kTopGroups * 2 == kTopThreads, "a group is a pair of threads");
 
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
   z += 0x9E3779B97F4A7C15ull;
@@ -177,7 +176,8 @@ struct SampleArgs {
   int* out_tokens;
   int vec;                    // rows start on 16-byte boundaries
   // scratch of the two-kernel path (null: one kernel does everything)
-  int n_chunks, cand_cap;     // chunks per row; room for candidates per chunk
+  int n_chunks, cand_cap;     // chunks (groups) per row; room for candidates per chunk
+  int group;                  // entries of a group whose maximum the first kernel left in cand_val [rows][groups], 0: chunks
   float* cand_val;            // [rows][chunks][cap] values / temperature, in index order
   int* cand_idx;              // [rows][chunks][cap]
   int* cand_cnt;              // [rows][chunks]; -1: more than cap entries tie for the chunk's top-k
@@ -244,89 +244,49 @@ __device__ __forceinline__ int block_offset(int mine, int* scratch, int* total) 
   return __reduce_add_sync(0xffffffffu, lane < warp ? w : 0) + incl - mine;
 }
 
-// First kernel for top-k up to kTopMax.  grid: (chunks of kTopChunk, rows).
-// The chunk stays in registers.  The k-th largest of the maxima of 256 groups of 64 entries has k
-// entries at or above it, so nothing below it can be among the chunk's k largest; what is left is
-// little more than k entries and goes out as it is.  Where it is more than the room (ties, or k from
-// about 130 on) the k-th key is searched bit by bit.  64 rows of 151,936 entries, top-k 50, take
-// 26 us (39 MB, 1.5 TB/s: the ranking, not the reads); the threshold search of sample_chunks_kernel, which
-// reads every entry eight times from shared memory with sixteen conditional adds each, took 186 us.
-__global__ void __launch_bounds__(kTopThreads) sample_top_kernel(SampleArgs a) {
-  __shared__ __align__(16) unsigned top[kTopGroups];
-  __shared__ int red[32];
-  __shared__ unsigned bound;
+// First kernel for top-k up to kTopMax.  grid: (tasks of eight warps, rows).  The largest value of every group, as it is in the row
+// (NaN counts as -infinity); the reads are all it does.  A call for 64 rows of 151,936
+// entries, top-k 50, its copies included: 100 -> 84.5 us (a kernel that took its chunk's k-th value and candidates, too, was 26 of them).
+__global__ void __launch_bounds__(kMaximaThreads) sample_maxima_kernel(SampleArgs a) {
   pdl_wait_block();
   pdl_launch_dependents();
-  const int row = blockIdx.y, chunk = blockIdx.x, tid = threadIdx.x;
-  const int lo = chunk * kTopChunk, n = min(kTopChunk, a.vocab - lo);
-  const float* src = a.logits + (size_t)row * a.ld + lo;
-  const size_t slot = (size_t)row * a.n_chunks + chunk;
-  float* out_val = a.cand_val + slot * a.cand_cap;
-  int* out_idx = a.cand_idx + slot * a.cand_cap;
-  const float mult = 1.0f / a.temperature;
-  const int k = min(a.top_k, n);
-
-  unsigned key[kTopPer];   // 0: beyond the row
-  {
-    float4 q[kTopPer / 4];
+  const int row = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lo = (blockIdx.x * (kMaximaThreads / 32) + warp) * kMaximaTask;
+  if (lo >= a.vocab) return;
+  const float* src = a.logits + (size_t)row * a.ld;
+  constexpr int kLoads = kMaximaTask / 128;
+  float m[kLoads];
 #pragma unroll
-    for (int j = 0; j < kTopPer / 4; ++j) q[j] = load_quad(src, (j * kTopThreads + tid) * 4, n, a.vec);
-#pragma unroll
-    for (int j = 0; j < kTopPer; ++j) {
-      const int i = (j / 4 * kTopThreads + tid) * 4 + j % 4;
-      key[j] = i < n ? ordered_key(scaled((&q[j / 4].x)[j % 4], mult)) : 0u;
-    }
+  for (int j = 0; j < kLoads; ++j) {
+    const float4 q = load_quad(src, lo + j * 128 + lane * 4, a.vocab, a.vec);
+    m[j] = fmaxf(fmaxf(fmaxf(q.x, q.y), fmaxf(q.z, q.w)), -INFINITY);      // (the maximum of two NaN is NaN)
   }
-  unsigned m = 0u;
+  // a group is `lanes` lanes of a load, or all of `loads` loads
+  const int lanes = min(32, a.group / 4), loads = max(1, a.group / 128);
 #pragma unroll
-  for (int j = 0; j < kTopPer; ++j) m = max(m, key[j]);
-  m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
-  const int group = tid >> 1;
-  if ((tid & 1) == 0) top[group] = m;
-  if (tid == 0) bound = 0u;
-  __syncthreads();
-  {
-    // a pair of threads ranks its group: each against one half of the groups
-    const int j0 = (tid & 1) * (kTopGroups / 2);
-    int rank = 0;
-#pragma unroll 8
-    for (int j = 0; j < kTopGroups / 2; j += 4) {
-      const uint4 t = *reinterpret_cast<const uint4*>(&top[j0 + j]);
-      rank += (t.x > m || (t.x == m && j0 + j < group));
-      rank += (t.y > m || (t.y == m && j0 + j + 1 < group));
-      rank += (t.z > m || (t.z == m && j0 + j + 2 < group));
-      rank += (t.w > m || (t.w == m && j0 + j + 3 < group));
+  for (int j = 0; j < kLoads; ++j)
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+      if (o < lanes) m[j] = fmaxf(m[j], __shfl_xor_sync(0xffffffffu, m[j], o));
+  float* out = a.cand_val + (size_t)row * a.n_chunks;
+  if (loads == 1) {
+#pragma unroll
+    for (int j = 0; j < kLoads; ++j) {
+      const int g = (lo + j * 128 + lane * 4) / a.group;
+      if (lane % lanes == 0 && g < a.n_chunks) out[g] = m[j];
     }
-    rank += __shfl_xor_sync(0xffffffffu, rank, 1);
-    if (rank == k - 1) bound = m;   // one group has this rank; none where k exceeds the groups
-  }
-  __syncthreads();
-  unsigned K = max(bound, kFirstKey);
-  int mine = 0;
-#pragma unroll
-  for (int j = 0; j < kTopPer; ++j) mine += key[j] >= K;
-  int total;
-  int pos = block_offset(mine, red, &total);
-  if (total > a.cand_cap) {
-    K = max(block_kth_key(key, k, red), kFirstKey);
-    mine = 0;
-#pragma unroll
-    for (int j = 0; j < kTopPer; ++j) mine += key[j] >= K;
-    pos = block_offset(mine, red, &total);
-    if (total > a.cand_cap) {   // ties beyond the room: the second kernel reads the whole row instead
-      if (tid == 0) a.cand_cnt[slot] = -1;
-      return;
-    }
+    return;
   }
 #pragma unroll
-  for (int j = 0; j < kTopPer; ++j)
-    if (key[j] >= K) {
-      // the value back from its key
-      out_val[pos] = __uint_as_float((key[j] & 0x80000000u) ? (key[j] & 0x7fffffffu) : ~key[j]);
-      out_idx[pos] = lo + (j / 4 * kTopThreads + tid) * 4 + j % 4;
-      ++pos;
-    }
-  if (tid == 0) a.cand_cnt[slot] = total;
+  for (int o = 1; o < kLoads; o <<= 1)
+    if (o < loads)
+#pragma unroll
+      for (int j = 0; j < kLoads; j += 2 * o) m[j] = fmaxf(m[j], m[j + o]);
+#pragma unroll
+  for (int j = 0; j < kLoads; ++j) {
+    const int g = (lo + j * 128) / a.group;
+    if (lane == 0 && j % loads == 0 && g < a.n_chunks) out[g] = m[j];
+  }
 }
 
 // First kernel of the two-kernel path otherwise.  grid: (chunks, rows).
@@ -406,13 +366,16 @@ __global__ void __launch_bounds__(kChunkThreads) sample_chunks_kernel(SampleArgs
   if (tid == 0) a.cand_cnt[slot] = total;
 }
 
-__global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleArgs a) {
+// The second kernel, or the only one.  GROUPS: the first left groups' maxima.
+template <int THREADS, bool GROUPS>
+__global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
+  constexpr int kSampleThreads = THREADS;
   __shared__ float red_f[33 * 16];
   __shared__ int red_i[33 * 16];
   __shared__ ArgBest red_b[32];
   __shared__ float c_val[kMaxCompact];
   __shared__ int c_idx[kMaxCompact];
-  __shared__ int scan[kSampleThreads];
+  __shared__ int scan[kMaxGroupList > kSampleThreads ? kMaxGroupList : kSampleThreads];
   __shared__ float l_val[kMaxCandidates];
   __shared__ int l_idx[kMaxCandidates];
   __shared__ int chunk_base[kMaxChunks], chunk_cnt[kMaxChunks];
@@ -430,7 +393,74 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleArgs a) {
   const int* idxs = nullptr;
   float mult = greedy ? 1.0f : 1.0f / a.temperature;
   int n = V;
-  if (a.cand_cnt != nullptr) {
+  if (GROUPS) {
+    // a bound of the row's k-th value: the largest key found bit by bit that k of the maxima reach, or a few more
+    const float* maxima = a.cand_val + (size_t)row * a.n_chunks;
+    unsigned gkey[kGroupsPer];
+#pragma unroll
+    for (int j = 0; j < kGroupsPer; ++j) {
+      const int g = j * THREADS + tid;
+      gkey[j] = g < a.n_chunks ? ordered_key(scaled(maxima[g], mult)) : 0u;
+    }
+    const int k = min(a.top_k, V), slack = k / 8 + 8;
+    unsigned bound = 0u;
+    for (int bit = 31; bit >= 0; --bit) {
+      const unsigned cand = bound | (1u << bit);
+      int mine = 0;
+#pragma unroll
+      for (int j = 0; j < kGroupsPer; ++j) mine += gkey[j] >= cand;
+      const int count = block_count(mine, red_i);
+      if (count < k) continue;
+      bound = cand;
+      if (count <= k + slack) break;
+    }
+    bound = max(bound, kFirstKey);
+    int mine = 0, n_list, total;
+#pragma unroll
+    for (int j = 0; j < kGroupsPer; ++j) mine += gkey[j] >= bound;
+    int pos = block_offset(mine, red_i, &n_list);
+    if (n_list <= kMaxGroupList) {      // (more only where groups tie)
+      int* list = scan;                 // in c_idx's place would do as well: neither is in use yet
+#pragma unroll
+      for (int j = 0; j < kGroupsPer; ++j)
+        if (gkey[j] >= bound) list[pos++] = j * THREADS + tid;
+      __syncthreads();
+      // the groups' entries that reach the bound, a thread's quads one after the other: counted, then written (from the L1)
+      const int quads = a.group / 4, n_quads = n_list * quads;
+      auto quad_at = [&](int e, int& i) {
+        i = list[e / quads] * a.group + e % quads * 4;
+        return load_quad(src, i, V, a.vec);
+      };
+      mine = 0;
+      for (int e = tid; e < n_quads; e += THREADS) {
+        int i;
+        const float4 q = quad_at(e, i);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) mine += i + c < V && ordered_key(scaled((&q.x)[c], mult)) >= bound;
+      }
+      pos = block_offset(mine, red_i, &total);
+      if (total <= kMaxCandidates) {
+        for (int e = tid; e < n_quads; e += THREADS) {
+          int i;
+          const float4 q = quad_at(e, i);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const float v = scaled((&q.x)[c], mult);
+            if (i + c < V && ordered_key(v) >= bound) {
+              l_val[pos] = v;
+              l_idx[pos] = i + c;
+              ++pos;
+            }
+          }
+        }
+        __syncthreads();
+        vals = l_val;
+        idxs = l_idx;
+        mult = 1.0f;
+        n = total;
+      }
+    }
+  } else if (a.cand_cnt != nullptr) {
     // gather the chunks' candidates, a warp per chunk; a chunk that overflowed sends us to the row
     const int* cnt = a.cand_cnt + (size_t)row * a.n_chunks;
     static_assert(kMaxChunks <= kSampleThreads, "a thread per chunk");
@@ -476,10 +506,36 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleArgs a) {
   for (int i = tid; i < n; i += blockDim.x) mx = fmaxf(mx, scaled(vals[i], mult));
   mx = block_max(mx, red_f);
 
-  bool listed = false;   // the kept entries are the list in c_val, at most one a thread
-  if (a.top_k > 0 && a.top_k < V && idxs != nullptr && a.top_k <= kTopMax) {
-    // candidates of the first kernel: three a thread at most, their keys in registers (with the list's masses
-    // below: 17 us for 64 rows at top-k 50 and top-p 0.95, against 90 us for threshold searches in shared memory)
+  bool listed = false;   // the kept entries are the list in c_val
+  if (GROUPS && idxs != nullptr && n <= kMaxRanked) {
+    // few candidates: the k-th key is the smallest that fewer than k others exceed
+    if (tid == 0) red_i[0] = -1;        // as unsigned the largest key there is
+    for (int i = tid; i < n; i += THREADS) c_idx[i] = (int)ordered_key(l_val[i]);
+    __syncthreads();
+    const int k = min(a.top_k, n);
+    for (int i = tid; i < n; i += THREADS) {
+      const unsigned own = (unsigned)c_idx[i];
+      int more = 0;
+      for (int j = 0; j < n; ++j) more += (unsigned)c_idx[j] > own;
+      if (more < k) atomicMin(reinterpret_cast<unsigned*>(red_i), own);
+    }
+    __syncthreads();
+    keep_key = max((unsigned)red_i[0], kFirstKey);
+    int mine = 0, total;
+    for (int i = tid; i < n; i += THREADS) mine += (unsigned)c_idx[i] >= keep_key;
+    int pos = block_offset(mine, red_i, &total);
+    for (int i = tid; i < n; i += THREADS)
+      if ((unsigned)c_idx[i] >= keep_key) {
+        c_val[pos] = l_val[i];
+        scan[pos++] = l_idx[i];
+      }
+    __syncthreads();
+    vals = c_val;
+    idxs = scan;
+    n = total;
+    listed = true;
+  } else if (a.top_k > 0 && a.top_k < V && idxs != nullptr && a.top_k <= kTopMax) {
+    // more of them: a few a thread, their keys in registers
     constexpr int kPer = kMaxCandidates / kSampleThreads;
     unsigned key[kPer];
 #pragma unroll
@@ -572,15 +628,15 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleArgs a) {
     unsigned J = 0u;
     if (listed) {
       // few entries: each adds up the mass above itself; J is the smallest key that stays
-      if (tid < n) {
-        const float v = vals[tid];
-        l_val[tid] = ordered_key(v) >= kk ? expf(v - mx) : 0.f;
-        l_idx[tid] = (int)ordered_key(v);
+      for (int i = tid; i < n; i += THREADS) {
+        const float v = vals[i];
+        l_val[i] = ordered_key(v) >= kk ? expf(v - mx) : 0.f;
+        l_idx[i] = (int)ordered_key(v);
       }
       if (tid == 0) red_i[0] = -1;   // as unsigned the largest key there is
       __syncthreads();
-      if (tid < n) {
-        const unsigned own = (unsigned)l_idx[tid];
+      for (int i = tid; i < n; i += THREADS) {
+        const unsigned own = (unsigned)l_idx[i];
         float mass = 0.f;
         for (int j = 0; j < n; ++j) mass += (unsigned)l_idx[j] > own ? l_val[j] : 0.f;
         if (!(mass > limit)) atomicMin(reinterpret_cast<unsigned*>(red_i), own);
@@ -652,18 +708,24 @@ static bool unfiltered(float temperature, int top_k, float top_p, float min_p) {
 
 // How a row is cut for the first kernel: chunks of how many entries, with room for how many candidates each.
 struct SamplePlan {
-  int chunk, n_chunks, cap;   // n_chunks 0: one kernel does everything
+  int chunk, n_chunks, cap;   // n_chunks 0: one kernel does everything; cap 0: groups of `chunk` entries, their maxima only
 };
+// Entries of a group: as few as keep a row's maxima in the second kernel's registers (so that a row has more than 512 groups).
+static int group_size(int vocab) {
+  int size = 8;
+  while (size < 512 && (vocab + size - 1) / size > pe::kMaxGroups) size *= 2;
+  return size;
+}
 static SamplePlan sample_plan(int vocab, float temperature, int top_k, float top_p, float min_p) {
   const SamplePlan none{0, 0, 0};
-  const int small = (vocab + pe::kChunk - 1) / pe::kChunk, large = (vocab + pe::kTopChunk - 1) / pe::kTopChunk;
+  const int small = (vocab + pe::kChunk - 1) / pe::kChunk;
   if (small < 2) return none;
   if (unfiltered(temperature, top_k, top_p, min_p))
     return small <= pe::kMaxChunks ? SamplePlan{pe::kChunk, small, 1} : none;
   if (top_k <= 0 || top_k >= vocab) return none;
-  if (top_k <= pe::kTopMax && large <= pe::kMaxChunks) {
-    const int cap = top_k + top_k / 4 + 16;   // the bound of a chunk's k-th entry lets about k / 8 more pass at k = 50
-    if (large * cap <= pe::kMaxCandidates) return SamplePlan{pe::kTopChunk, large, cap};
+  if (top_k <= pe::kTopMax) {
+    const int size = group_size(vocab), groups = (vocab + size - 1) / size;
+    if (groups <= pe::kMaxGroups) return SamplePlan{size, groups, 0};
   }
   if (small <= pe::kMaxChunks && (long long)small * top_k <= pe::kMaxCandidates)
     return SamplePlan{pe::kChunk, small, top_k + 8};   // 8: ties with a chunk's k-th value
@@ -674,7 +736,7 @@ static SamplePlan sample_plan(int vocab, float temperature, int top_k, float top
 extern "C" long long pe_sample_scratch_bytes(int n_rows, int vocab, float temperature, int top_k, float top_p, float min_p) {
   if (n_rows <= 0 || vocab <= 0) return 0;
   const SamplePlan plan = sample_plan(vocab, temperature, top_k, top_p, min_p);
-  return (long long)n_rows * plan.n_chunks * (plan.cap * 8ll + 4ll);
+  return (long long)n_rows * plan.n_chunks * (plan.cap * 8ll + 4ll);   // (a group's maximum: four bytes)
 }
 
 // scratch: null, or at least pe_sample_scratch_bytes(...) bytes, 4-byte aligned.
@@ -688,7 +750,7 @@ extern "C" int pe_sample(const float* logits, long long ld, int n_rows, int voca
   a.top_p = top_p; a.min_p = min_p; a.seed = seed; a.row_request = row_request; a.row_step = row_step;
   a.out_tokens = out_tokens;
   a.vec = ((uintptr_t)logits % 16) == 0 && ld % 4 == 0;
-  a.n_chunks = 0; a.cand_cap = 0; a.cand_val = nullptr; a.cand_idx = nullptr; a.cand_cnt = nullptr;
+  a.n_chunks = 0; a.cand_cap = 0; a.group = 0; a.cand_val = nullptr; a.cand_idx = nullptr; a.cand_cnt = nullptr;
   const long long need = pe_sample_scratch_bytes(n_rows, vocab, temperature, top_k, top_p, min_p);
   if (scratch != nullptr && need > 0 && scratch_bytes >= need && ((uintptr_t)scratch % 4) == 0) {
     const SamplePlan plan = sample_plan(vocab, temperature, top_k, top_p, min_p);
@@ -698,13 +760,19 @@ extern "C" int pe_sample(const float* logits, long long ld, int n_rows, int voca
     a.cand_val = reinterpret_cast<float*>(scratch);
     a.cand_idx = reinterpret_cast<int*>(a.cand_val + slots * a.cand_cap);
     a.cand_cnt = a.cand_idx + slots * a.cand_cap;
-    if (plan.chunk == pe::kTopChunk)
-      pe::launch(pe::sample_top_kernel, dim3(a.n_chunks, n_rows), pe::kTopThreads, 0, stream, a);
-    else
-      pe::launch(pe::sample_chunks_kernel, dim3(a.n_chunks, n_rows), pe::kChunkThreads, 0, stream, a);
+    if (plan.cap == 0) {
+      a.group = plan.chunk;
+      const int tasks = (vocab + pe::kMaximaTask - 1) / pe::kMaximaTask, warps = pe::kMaximaThreads / 32;
+      pe::launch(pe::sample_maxima_kernel, dim3((tasks + warps - 1) / warps, n_rows), pe::kMaximaThreads, 0, stream, a);
+      PE_LAUNCH_CHECK();
+      pe::launch(pe::sample_kernel<pe::kGroupThreads, true>, n_rows, pe::kGroupThreads, 0, stream, a);
+      PE_LAUNCH_CHECK();
+      return PE_OK;
+    }
+    pe::launch(pe::sample_chunks_kernel, dim3(a.n_chunks, n_rows), pe::kChunkThreads, 0, stream, a);
     PE_LAUNCH_CHECK();
   }
-  pe::launch(pe::sample_kernel, n_rows, pe::kSampleThreads, 0, stream, a);
+  pe::launch(pe::sample_kernel<pe::kSampleThreads, false>, n_rows, pe::kSampleThreads, 0, stream, a);
   PE_LAUNCH_CHECK();
   return PE_OK;
 }

@@ -164,3 +164,16 @@ def test_reference_arm_and_plain_baseline_of_the_benchmark_run(pe):
     assert out["impl"] == "reference" and "unavailable" not in out
     assert out["e2e"]["tokens"] == 12 and out["value"] > 0 and out["config"]["layers"] == 3
     assert "pytorch-engine_b200" not in open(os.path.join(ROOT, "baseline", "reference_arm.py")).read().split('"""', 2)[2]
+def test_scratch_of_the_sampler_with_groups(pe):
+    """Rows with a small top-k leave one float a group of entries: more than 512 groups, and no more than a block holds."""
+    f = pe.kernels.lib.library().pe_sample_scratch_bytes
+    for vocab in (4097, 4100, 20479, 20480, 20481, 32768, 50001, 151936, 163840, 163841, 1000000, 1310720):
+        for k in (1, 50, 224):
+            groups, rest = divmod(f(3, vocab, 0.8, k, 0.95, 0.0), 12)
+            assert rest == 0 and 512 < groups <= 2560, vocab
+            size = -(-vocab // groups)                  # the smallest power of two from 8 on with no more groups than that
+            assert min(s for s in (8, 16, 32, 64, 128, 256, 512) if -(-vocab // s) <= 2560) >= size
+    assert f(3, 4096, 0.8, 50, 0.95, 0.0) == 0 and f(3, 151936, 0.8, 0, 0.95, 0.0) == 0
+    assert f(3, 20000, 0.8, 225, 0.95, 0.0) > 0         # chunks and their candidates beyond
+
+
