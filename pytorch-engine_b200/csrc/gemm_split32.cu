@@ -12,7 +12,7 @@
 // split in here as well a thread had to hold twice as many values and could not ask for them early enough: a chunk of
 // 128 x 128 x 64 took 1.95 us, of which the tensor core worked 0.8.)
 //
-// A block owns a tile of 128 rows of W (the MMA's M side, so that a thread's accumulators are one column of y for 64 or 32
+// A block owns a tile of 128 rows of W (the MMA's M side, so that a thread's accumulators are one column of y for 80, 64 or 32
 // rows, and a warp stores 32 neighbouring floats) and NT rows of x, and a range of K.  Its warps:
 //   0-7    converters of W: 16-byte loads, split, stores as K-major tiles with the 128-byte swizzle;
 //   8-15   accumulators: add each chunk's sums to their registers, store at the end;
@@ -43,9 +43,10 @@ template <int NT>
 struct Tile {
   static constexpr int kA = BM * 128, kB = NT * 128;       // bytes of one part
   static constexpr int kStage = kParts * (kA + kB);
-  static constexpr int kStages = NT == 128 ? 2 : 3;
-  static constexpr int kCols = 2 * NT;                     // two accumulators
+  static constexpr int kStages = NT >= 96 ? 2 : 3;
+  static constexpr int kCols = NT <= 64 ? 128 : NT <= 128 ? 256 : 512;   // two accumulators of NT columns, in a power of two
   static constexpr int kAcc = NT / 2;                      // accumulators a thread
+  static constexpr int kLd = NT > 128 ? 8 : 16;            // sums of a chunk that it reads at a time
 };
 
 struct Params {
@@ -85,6 +86,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
+}
+// ... and 8
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 // K-major tile with the 128-byte swizzle (see gemm_umma.cu): rows of 64 bfloat16, groups of 8 rows 1,024 bytes apart.
@@ -236,14 +242,14 @@ __device__ __noinline__ void second_look(const Params p) {      // (takes nothin
     }
   }
   exact_any(0);
-  uint32_t again = 0;
+  uint64_t again = 0;
   const float len = (float)(k_last - k_first), w_top = top[NT + col], w_cut = cut[NT + col] ? 1.f : 0.f;
   if (n < p.N)
     for (int j = 0; j < kRows && m0 + row0 + j < p.M; ++j) {
       const float v = fabsf(y[(size_t)(m0 + row0 + j) * p.ldy + n]), x_top = top[row0 + j];
       const float lost = len * kCutOff * ((cut[row0 + j] ? w_top : 0.f) + w_cut * x_top);
       const bool tiny = v > 0.f ? v < kSmall : x_top > 0.f && w_top > 0.f && x_top * w_top * len < kSmall;
-      if (!(v <= kLargest) || tiny || v < lost) again |= 1u << j;
+      if (!(v <= kLargest) || tiny || v < lost) again |= 1ull << j;
     }
   if (!exact_any(again != 0)) return;
   const bool mine = __any_sync(0xffffffffu, again != 0);
@@ -381,12 +387,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split32_kernel(Params p, con
       }
       fence_after_sync();
 #pragma unroll
-      for (int h = 0; h < T::kAcc / 16; ++h) {
-        uint32_t v[16];
-        tmem_ld16(t_row + b * NT + h * 16, v);
+      for (int h = 0; h < T::kAcc / T::kLd; ++h) {
+        uint32_t v[T::kLd];
+        if constexpr (T::kLd == 16) tmem_ld16(t_row + b * NT + h * 16, v);
+        else tmem_ld8(t_row + b * NT + h * 8, v);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 16; ++j) acc[h * 16 + j] += __uint_as_float(v[j]);
+        for (int j = 0; j < T::kLd; ++j) acc[h * T::kLd + j] += __uint_as_float(v[j]);
       }
       fence_before_sync();
       __syncwarp();
@@ -493,13 +500,13 @@ static Plan plan_for(int M, int N, int K, int n_sms) {
   const int chunks = (K + BK - 1) / BK, n_tiles = (N + BM - 1) / BM;
   Plan best{128, 1, chunks};
   double best_t = 1e30;
-  for (int nt = 64; nt <= 128; nt += 64) {
+  for (int nt : {64, 128, 160}) {
     const long long tiles = (long long)((M + nt - 1) / nt) * n_tiles;
     for (int s = 1; s == 1 || (s <= 8 && s * 4 <= chunks); ++s) {
-      if (s > 1 && (N % 4 || (double)s * M * N * 4 > 64e6)) break;   // (the sums' memory is bounded, too)
+      if (s > 1 && (nt == 160 || N % 4 || (double)s * M * N * 4 > 64e6)) break;   // (the sums' memory is bounded, too)
       const int cps = (chunks + s - 1) / s, splits = (chunks + cps - 1) / cps;
       const long long waves = (tiles * splits + n_sms - 1) / n_sms;
-      double t = waves * (cps * (nt == 128 ? 1.5 : 1.3) + 3.0);
+      double t = waves * (cps * (nt == 160 ? 1.95 : nt == 128 ? 1.5 : 1.3) + 3.0);
       if (splits > 1) t += 3.0 + (double)(splits + 1) * M * N * 4 / 4e6;
       if (t < best_t) { best_t = t; best = Plan{nt, splits, cps}; }
     }
@@ -555,8 +562,9 @@ extern "C" int pe_gemm_split32(const float* x, long long ldx, const float* w, fl
   Params p;
   p.x = x; p.ldx = ldx; p.x_top = x_top; p.segments = segments_of(K); p.w = w; p.y = sums ? partial : y; p.ldy = sums ? N : ldy; p.M = M; p.N = N; p.K = K;
   p.chunks_per_split = plan.chunks_per_split; p.status = status;
-  auto kern = plan.nt == 128 ? gemm_split32_kernel<128> : gemm_split32_kernel<64>;
-  const size_t smem = 1024 + (plan.nt == 128 ? (size_t)Tile<128>::kStages * Tile<128>::kStage : (size_t)Tile<64>::kStages * Tile<64>::kStage);
+  auto kern = plan.nt == 160 ? gemm_split32_kernel<160> : plan.nt == 128 ? gemm_split32_kernel<128> : gemm_split32_kernel<64>;
+  const size_t smem = 1024 + (plan.nt == 160 ? (size_t)Tile<160>::kStages * Tile<160>::kStage : plan.nt == 128 ? (size_t)Tile<128>::kStages * Tile<128>::kStage
+                              : (size_t)Tile<64>::kStages * Tile<64>::kStage);
   cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (ce != cudaSuccess) return (int)ce;
   dim3 grid((M + plan.nt - 1) / plan.nt, (N + BM - 1) / BM, plan.splits);

@@ -810,6 +810,14 @@ def test_gemm_split32_at_the_ends_of_float32s_range(ops, M, N, K):
     assert bool(out.isnan().all()) and st.tolist()[0] == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(257, 9468, 68), (300, 9472, 1000), (320, 9472, 128)])
+def test_gemm_split32_tiles_of_160_rows(ops, M, N, K):
+    """Tiles of 160 rows (where they save a wave of blocks): a last tile of 97 rows, of 140, and whole ones."""
+    test_gemm_split32(ops, M, N, K)
+    if K == 68:
+        test_gemm_split32_at_the_ends_of_float32s_range(ops, M, N, K)
+
+
 @pytest.mark.parametrize("M,I,K", [(128, 128, 64), (200, 384, 200), (1000, 1280, 1024), (5, 256, 4096)])
 @pytest.mark.parametrize("kernel", ["gemm_umma", "gemm_umma2"])
 def test_gemm_umma_with_the_gate_fused(ops, M, I, K, kernel):
