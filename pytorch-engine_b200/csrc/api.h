@@ -84,6 +84,11 @@ int pe_attention_umma_prefill_gated(const void* q, long long q_ld, long long n_t
     const float* out_cos, const float* out_sin, int out_rows, const void* gate, long long gate_ld, const int* seq_qstart,
     const int* seq_past, const int* seq_slot, const int* page_table, int table_stride, int num_pages, const void* k_pages,
     const void* v_pages, int n_sms, int* work_counter, int* status, cudaStream_t stream);
+int pe_attention_umma_prefill_parts(const void* q, long long q_ld, long long n_tokens, void* out, long long out_ld,
+    int n_seqs, int max_q, int n_heads, int n_kv_heads, int head_dim, int v_dim, float scale, int window, int sink,
+    const float* out_cos, const float* out_sin, int out_rows, const void* gate, long long gate_ld, const int* seq_qstart,
+    const int* seq_past, const int* seq_slot, const int* page_table, int table_stride, int num_pages, const void* k_pages,
+    const void* v_pages, int n_sms, int* work_counter, int parts, float* scratch, int* status, cudaStream_t stream);
 int pe_attention_umma_prefill_ex(const void* q, long long q_ld, long long n_tokens, void* out, long long out_ld,
     int n_seqs, int max_q, int n_heads, int n_kv_heads, int head_dim, float scale, int window, int sink,
     const float* out_cos, const float* out_sin, int out_rows, const int* seq_qstart, const int* seq_past,

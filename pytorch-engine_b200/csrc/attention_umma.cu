@@ -57,6 +57,7 @@ constexpr int kPageBytes = 2 * kKPart;        // 16 KB: a V page (a K page: KH p
 constexpr int kKStages = 2, kVStages = 3;     // K is spent once S is there, V only after P.V: V needs the deeper ring
 constexpr int kTmemCols = 256;                // S0 [0,64) S1 [64,128) O [128,256)
 constexpr float kRescaleThreshold = 8.0f;     // in log2 units
+constexpr int kMaxParts = 8;                  // items that a row tile's pages may be shared out over
 
 struct Args {
   __nv_bfloat16* out; long long out_ld;
@@ -75,16 +76,22 @@ struct Args {
   int vd, v_halves;       // size of a value row; 64-feature halves of a V page (1 or 2)
   // each head's output times sigmoid(gate[token, head]) (rows of the step's tokens, gate_ld apart); null: no gate
   const __nv_bfloat16* gate; long long gate_ld;
+  // parts > 1: a row tile's pages are shared out over so many items, whose outputs ([parts][token, head][vd], float32, each divided by
+  // its own denominator) and log-sums ([parts][token, head], in log2 units, -inf: no key) a second kernel puts together
+  int parts; long long part_rows;
+  float* part_out; float* part_lse;
 };
 
 // One work item: the rows [row0, row0 + rows_blk) of sequence b's (token, head) rows for kv head kvh.
 struct Item {
-  int b, kvh, row0, n_rows, q0, past, slot, tok0, k_begin, n_tiles;
+  int b, kvh, row0, n_rows, q0, past, slot, tok0, k_begin, n_tiles, part;
 };
 // Rank -> item (late row tiles first, then sequences, then kv heads); false if the sequence has no such rows.
 __device__ __forceinline__ bool item_at(const Args& a, int rank, int rows_blk, Item& w) {
-  w.kvh = rank % a.n_kv_heads;
-  const int r2 = rank / a.n_kv_heads;
+  w.part = rank % a.parts;
+  const int r1 = rank / a.parts;
+  w.kvh = r1 % a.n_kv_heads;
+  const int r2 = r1 / a.n_kv_heads;
   w.b = r2 % a.n_seqs;
   const int tile = a.tiles - 1 - r2 / a.n_seqs;
   w.q0 = a.seq_qstart[w.b];
@@ -100,6 +107,11 @@ __device__ __forceinline__ bool item_at(const Args& a, int rank, int rows_blk, I
   w.k_begin = 0;
   if (a.window > 0) w.k_begin = max(0, first_pos - a.window + 1) / BN * BN;
   w.n_tiles = (last_pos + 1 - w.k_begin + BN - 1) / BN;
+  if (a.parts > 1) {      // even shares in whole pages (none for the last ones where there are fewer pages than parts)
+    const int first = (int)((long long)w.n_tiles * w.part / a.parts), end = (int)((long long)w.n_tiles * (w.part + 1) / a.parts);
+    w.k_begin += first * BN;
+    w.n_tiles = end - first;
+  }
   return true;
 }
 // Every block calls this once, when it takes no more ranks: the last of the G blocks through leaves the work
@@ -319,7 +331,7 @@ prefill_umma_kernel(Args a, const __grid_constant__ CUtensorMap qmap, const __gr
   const int group = a.group;
   const int rows_blk = (BM / group) * group;                  // whole tokens only
   const int G = (int)gridDim.x, me = (int)blockIdx.x;
-  const int total = a.tiles * a.n_seqs * a.n_kv_heads;
+  const int total = a.tiles * a.n_seqs * a.n_kv_heads * a.parts;
 
   if (tid == 0) {
     tma::mbar_init(&q_full, 1);
@@ -384,7 +396,7 @@ prefill_umma_kernel(Args a, const __grid_constant__ CUtensorMap qmap, const __gr
         tma::mbar_arrive(&w_full[f & 1]);
         if (rank < 0) break;
         Item w;
-        if (rank >= total || !item_at(a, rank, rows_blk, w)) continue;
+        if (rank >= total || !item_at(a, rank, rows_blk, w) || w.n_tiles == 0) continue;
         // Q of the item before must have been read by its last S product
         if (!tma::mbar_wait(&q_empty, (it & 1) ^ 1)) {
           report(a.status, kStatusWaitTimedOut, 25, me, (int)it);
@@ -461,7 +473,7 @@ prefill_umma_kernel(Args a, const __grid_constant__ CUtensorMap qmap, const __gr
         tma::mbar_arrive(&w_empty[f & 1]);
         if (rank < 0) break;
         Item w;
-        if (rank >= total || !item_at(a, rank, rows_blk, w)) continue;
+        if (rank >= total || !item_at(a, rank, rows_blk, w) || w.n_tiles == 0) continue;
         const int n_tiles = w.n_tiles;
         // S of the item's page j; its K page is there (the caller has waited for the barrier that counts it)
         auto issue_qk = [&](int j) {
@@ -526,6 +538,12 @@ prefill_umma_kernel(Args a, const __grid_constant__ CUtensorMap qmap, const __gr
       if (rank < 0) break;
       Item w;
       if (rank >= total || !item_at(a, rank, rows_blk, w)) continue;
+      if (w.n_tiles == 0) {      // a part without pages
+        const int tok = (w.row0 + tid) / group, head = w.kvh * group + (w.row0 + tid) % group;
+        if (tid < rows_blk && w.row0 + tid < w.n_rows)
+          a.part_lse[(size_t)w.part * a.part_rows + (size_t)(w.q0 + tok) * a.n_heads + head] = -INFINITY;
+        continue;
+      }
       const int row0 = w.row0, n_rows = w.n_rows, past = w.past, n_tiles = w.n_tiles;
       const int row = row0 + r;
       const bool live = r < rows_blk && row < n_rows;
@@ -624,10 +642,35 @@ prefill_umma_kernel(Args a, const __grid_constant__ CUtensorMap qmap, const __gr
       }
       if (ok && tma::mbar_wait(&o_done, it & 1)) {
         fence_after_sync();
+        const int tok = row / group, head = w.kvh * group + row % group;
+        if (a.parts > 1) {
+          const float inv = l > 0.f ? 1.f / l : 0.f;
+          const size_t at = (size_t)w.part * a.part_rows + (size_t)(w.q0 + tok) * a.n_heads + head;
+          if (live) a.part_lse[at] = l > 0.f ? m_ref + log2f(l) : -INFINITY;
+          float* dst = a.part_out + at * a.vd;
+#pragma unroll 1
+          for (int c = 0; c < a.vd; c += 32) {
+            uint32_t ov[32];
+            tmem_ld32(tmem_o + c + lane_off, ov);
+            tmem_ld_wait();
+            if (live) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+                if (c + 4 * i < a.vd)
+                  *reinterpret_cast<float4*>(dst + c + 4 * i) =
+                      make_float4(__uint_as_float(ov[4 * i]) * inv, __uint_as_float(ov[4 * i + 1]) * inv,
+                                  __uint_as_float(ov[4 * i + 2]) * inv, __uint_as_float(ov[4 * i + 3]) * inv);
+            }
+          }
+          fence_before_sync();
+          tma::mbar_arrive(&o_free);
+          n += n_tiles;
+          ++it;
+          continue;
+        }
         // the sink's score is 0: its weight relative to the reference that the row's weights were taken against
         if (a.sink) l += fast_exp2(-((m_ref == -INFINITY) ? 0.f : m_ref));
         float inv = 1.f / fmaxf(l, 1e-20f);
-        const int tok = row / group, head = w.kvh * group + row % group;
         if (a.gate && live) inv /= 1.f + expf(-__bfloat162float(a.gate[(size_t)(w.q0 + tok) * a.gate_ld + head]));
         __nv_bfloat16* dst = a.out + (size_t)(w.q0 + tok) * a.out_ld + (size_t)head * a.vd;
         const bool turn = a.out_cos != nullptr;
@@ -688,6 +731,52 @@ prefill_umma_kernel(Args a, const __grid_constant__ CUtensorMap qmap, const __gr
   if (tid == 0) leave_work_counter(a.work_counter, G);
 }
 
+// Put the parts of every (token, head) row together: a warp a row, four features a lane.
+__global__ void __launch_bounds__(256) merge_parts_kernel(Args a) {
+  pdl_wait_block();
+  pdl_launch_dependents();
+  const int lane = threadIdx.x & 31;
+  const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (r >= a.part_rows) return;
+  const int tok = (int)(r / a.n_heads), head = (int)(r - (long long)tok * a.n_heads);
+  float lse[kMaxParts], mx = a.sink ? 0.f : -INFINITY;
+#pragma unroll
+  for (int p = 0; p < kMaxParts; ++p) {
+    lse[p] = p < a.parts ? a.part_lse[(size_t)p * a.part_rows + r] : -INFINITY;
+    mx = fmaxf(mx, lse[p]);
+  }
+  float4 x[kMaxParts];
+#pragma unroll
+  for (int p = 0; p < kMaxParts; ++p)
+    x[p] = lse[p] != -INFINITY && 4 * lane < a.vd ? *reinterpret_cast<const float4*>(a.part_out + ((size_t)p * a.part_rows + r) * a.vd + 4 * lane)
+                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+  float denom = a.sink ? exp2f(-mx) : 0.f;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int p = 0; p < kMaxParts; ++p) {
+    const float f = lse[p] == -INFINITY ? 0.f : exp2f(lse[p] - mx);
+    denom += f;
+    v.x = fmaf(x[p].x, f, v.x); v.y = fmaf(x[p].y, f, v.y); v.z = fmaf(x[p].z, f, v.z); v.w = fmaf(x[p].w, f, v.w);
+  }
+  float inv = 1.f / fmaxf(denom, 1e-20f);
+  if (a.gate) inv /= 1.f + expf(-__bfloat162float(a.gate[(size_t)tok * a.gate_ld + head]));
+  v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
+  if (4 * lane >= a.vd) return;
+  if (a.out_cos) {
+    int b = 0;      // the token's sequence, for its position
+    while (b + 1 < a.n_seqs && a.seq_qstart[b + 1] <= tok) ++b;
+    const int pos = a.seq_past[b] + tok - a.seq_qstart[b];
+    if (pos < 0 || pos >= a.out_rows) {
+      if (lane == 0) report(a.status, kStatusPositionOutOfRange, tok, pos, a.out_rows);
+      return;
+    }
+    const float2 c = *reinterpret_cast<const float2*>(a.out_cos + (size_t)pos * (HD / 2) + 2 * lane);
+    const float2 s = *reinterpret_cast<const float2*>(a.out_sin + (size_t)pos * (HD / 2) + 2 * lane);
+    v = make_float4(v.x * c.x + v.y * s.x, v.y * c.x - v.x * s.x, v.z * c.y + v.w * s.y, v.w * c.y - v.z * s.y);
+  }
+  *reinterpret_cast<uint2*>(a.out + (size_t)tok * a.out_ld + (size_t)head * a.vd + 4 * lane) = make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
+}
+
 }  // namespace fau
 }  // namespace pe
 
@@ -740,11 +829,27 @@ extern "C" int pe_attention_umma_prefill_gated(const void* q, long long q_ld, lo
                                                const int* seq_past, const int* seq_slot, const int* page_table,
                                                int table_stride, int num_pages, const void* k_pages, const void* v_pages,
                                                int n_sms, int* work_counter, int* status, cudaStream_t stream) {
+  return pe_attention_umma_prefill_parts(q, q_ld, n_tokens, out, out_ld, n_seqs, max_q, n_heads, n_kv_heads, head_dim, v_dim, scale, window,
+                                         sink, out_cos, out_sin, out_rows, gate, gate_ld, seq_qstart, seq_past, seq_slot, page_table,
+                                         table_stride, num_pages, k_pages, v_pages, n_sms, work_counter, 1, nullptr, status, stream);
+}
+
+// The same with a row tile's pages shared out over `parts` (1 to 8) blocks and a second kernel that puts their results together, for
+// steps of few tiles behind a long past.  parts > 1: scratch of parts * n_tokens * n_heads * (v_dim + 1) floats, 16-byte aligned.
+extern "C" int pe_attention_umma_prefill_parts(const void* q, long long q_ld, long long n_tokens, void* out, long long out_ld,
+                                               int n_seqs, int max_q, int n_heads, int n_kv_heads, int head_dim, int v_dim,
+                                               float scale, int window, int sink, const float* out_cos, const float* out_sin,
+                                               int out_rows, const void* gate, long long gate_ld, const int* seq_qstart,
+                                               const int* seq_past, const int* seq_slot, const int* page_table,
+                                               int table_stride, int num_pages, const void* k_pages, const void* v_pages,
+                                               int n_sms, int* work_counter, int parts, float* scratch, int* status,
+                                               cudaStream_t stream) {
   using namespace pe::fau;
   if (n_seqs <= 0) return PE_OK;
   if ((out_cos == nullptr) != (out_sin == nullptr) || ((uintptr_t)out_cos % 16) || ((uintptr_t)out_sin % 16)) return PE_ERR_BAD_ARGUMENT;
   if (!pe_attention_umma_dims_supported(head_dim, v_dim, n_heads, n_kv_heads)) return PE_ERR_UNSUPPORTED_SIZE;
   if (out_cos && (head_dim != 128 || v_dim != 128)) return PE_ERR_UNSUPPORTED_SIZE;
+  if (parts < 1 || parts > kMaxParts || (parts > 1 && (!scratch || (uintptr_t)scratch % 16))) return PE_ERR_BAD_ARGUMENT;
   if (((uintptr_t)q % 16) || (q_ld * 2) % 16 || ((uintptr_t)out % 16) || (out_ld * 2) % 16) return PE_ERR_BAD_ARGUMENT;
   Args a;
   a.out = (__nv_bfloat16*)out; a.out_ld = out_ld; a.n_heads = n_heads; a.n_kv_heads = n_kv_heads;
@@ -753,6 +858,8 @@ extern "C" int pe_attention_umma_prefill_gated(const void* q, long long q_ld, lo
   a.page_table = page_table; a.table_stride = table_stride; a.num_pages = num_pages; a.status = status;
   a.sink = sink; a.out_cos = out_cos; a.out_sin = out_sin; a.out_rows = out_rows;
   a.vd = v_dim; a.v_halves = v_dim > 64 ? 2 : 1; a.gate = (const __nv_bfloat16*)gate; a.gate_ld = gate_ld;
+  a.parts = parts; a.part_rows = n_tokens * n_heads;
+  a.part_out = scratch; a.part_lse = parts > 1 ? scratch + (size_t)parts * a.part_rows * v_dim : nullptr;
   pe::tma::EncodeTiledFn fn = pe::tma::encode_fn();
   if (fn == nullptr) return -5;
   CUtensorMap qmap, kmap, vmap;
@@ -782,7 +889,7 @@ extern "C" int pe_attention_umma_prefill_gated(const void* q, long long q_ld, lo
   }
   const int rows_blk = (BM / a.group) * a.group;
   const long long tiles = ((long long)max_q * a.group + rows_blk - 1) / rows_blk;
-  const long long total = tiles * n_kv_heads * n_seqs;
+  const long long total = tiles * n_kv_heads * n_seqs * parts;
   if (total <= 0 || total > (1ll << 30)) return PE_ERR_UNSUPPORTED_SIZE;
   a.tiles = (int)tiles; a.n_seqs = n_seqs; a.work_counter = work_counter;
   // two blocks fit on an SM (shared memory, tensor memory columns), or one with wider keys; no more blocks than items
@@ -790,5 +897,9 @@ extern "C" int pe_attention_umma_prefill_gated(const void* q, long long q_ld, lo
   dim3 grid((unsigned)(total < slots ? total : slots));
   pe::launch(kern, grid, 192, smem, stream, a, qmap, kmap, vmap);
   PE_LAUNCH_CHECK();
+  if (parts > 1) {
+    pe::launch(merge_parts_kernel, dim3((unsigned)((a.part_rows + 7) / 8)), dim3(256), 0, stream, a);
+    PE_LAUNCH_CHECK();
+  }
   return PE_OK;
 }

@@ -107,6 +107,7 @@ _SIGNATURES = {
                                P, P],
     "pe_attention_umma_dims_supported": [I, I, I, I],
     "pe_attention_umma_prefill_gated": [P, L, L, P, L, I, I, I, I, I, I, F, I, I, P, P, I, P, L, P, P, P, P, I, I, P, P, I, P, P, P],
+    "pe_attention_umma_prefill_parts": [P, L, L, P, L, I, I, I, I, I, I, F, I, I, P, P, I, P, L, P, P, P, P, I, I, P, P, I, P, I, P, P, P],
     "pe_moe_route_logits": [P, P, I, I, I, P, P, P, I, P],
     "pe_attention_generic_masked": [I, I, P, L, P, L, I, I, I, I, I, I, F, I, I, I, I, I, I, I, P, P, P, I, I, I, P, P, P, P, I, I,
                                     P, P, P, I, I, P, P],

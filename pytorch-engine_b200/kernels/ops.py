@@ -490,6 +490,9 @@ def gemm_smallm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, pair_o
     _count(1)
 
 
+    _count(1)
+
+
 def gemm_smallm_grouped_supported(xs: torch.Tensor, weight: torch.Tensor, group_rows: int) -> bool:
     """Whether csrc/gemm_smallm.cu takes ``xs [G, M, K]`` (any strides of G and M that keep rows on 16-byte boundaries)
     times ``weight [G * group_rows, K]`` in one launch."""
@@ -706,27 +709,44 @@ def _work_counter(device: torch.device) -> torch.Tensor:
     return t
 
 
+def attention_umma_parts(slots: int, items: int, pages: int) -> int:
+    """How many blocks a row tile's pages (``pages`` at most) are shared out over, for ``items`` (row tile, sequence, kv head) items
+    on ``slots`` places: as many as fill the places once, of six pages or more, where tiles are long (every part costs its output
+    written and read in float32, and a second kernel).  Microseconds with one block a tile and with this rule, 32 heads on 8: 16
+    tokens behind 3,500 cached ones 53, 18; 128 tokens 55, 28; 256 behind 2,000 38, 29; 512 behind 3,500 61, 53; 16 heads on 8: 512
+    behind 3,500 60, 36.  With fewer pages a tile it loses: 8 x 64 tokens behind 1,000 (17 pages) 24, 26; 700 behind 700 (22 pages) 26, 28;
+    and with the places nearly full: 676 tokens of two sequences behind 3,100, 32 heads, 63 with one block and 69 with three."""
+    if items <= 0 or 2 * items > slots or pages < 32:
+        return 1
+    return min(8, slots // items, pages // 6)
+
+
 def attention_umma_prefill(q: torch.Tensor, out: torch.Tensor, n_seqs: int, max_q: int, n_heads: int, n_kv_heads: int,
                            head_dim: int, scale: float, window: int, seq_qstart: torch.Tensor, seq_past: torch.Tensor,
                            seq_slot: torch.Tensor, page_table: torch.Tensor, num_pages: int, k_pages: torch.Tensor,
                            v_pages: torch.Tensor, status: torch.Tensor, sink: bool = False,
                            out_cos: Optional[torch.Tensor] = None, out_sin: Optional[torch.Tensor] = None,
-                           v_dim: Optional[int] = None, gate: Optional[torch.Tensor] = None) -> None:
+                           v_dim: Optional[int] = None, gate: Optional[torch.Tensor] = None, parts: int = 1,
+                           scratch: Optional[torch.Tensor] = None) -> None:
     """Prefill attention on tcgen05 (bfloat16, head size 128, groups up to 32; or key and value sizes that
     ``attention_umma_dims_supported`` takes, with ``gate`` as for ``attention_mma_gated``); ``q`` holds the step's
     query rows (the first ``n_heads * head_dim`` features of each row of the fused q|k|v buffer).  ``sink``,
-    ``out_cos``, ``out_sin``: as for ``attention_mma``."""
+    ``out_cos``, ``out_sin``: as for ``attention_mma``.  ``parts`` > 1: a row tile's pages over so many blocks
+    (``attention_umma_parts``), with ``scratch`` of ``parts * q.shape[0] * n_heads * (v_dim + 1)`` floats."""
+    _need(parts == 1 or (scratch is not None and scratch.dtype == torch.float32
+                         and scratch.numel() >= parts * q.shape[0] * n_heads * ((head_dim if v_dim is None else int(v_dim)) + 1)),
+          "attention_umma: scratch of the parts")
     _need(q.stride(-1) == 1 and out.stride(-1) == 1, "attention: rows must be contiguous")
     _need(q.dtype == out.dtype == k_pages.dtype == torch.bfloat16, "attention_umma: bfloat16 tensors only")
     _check_out_tables(out_cos, out_sin, head_dim)
     _need(gate is None or (gate.dtype == torch.bfloat16 and gate.stride(-1) == 1 and gate.shape[-1] >= n_heads), "attention_umma: gate rows")
-    check(library().pe_attention_umma_prefill_gated(
+    check(library().pe_attention_umma_prefill_parts(
         _ptr(q), q.stride(0), q.shape[0], _ptr(out), out.stride(0), n_seqs, max_q, n_heads, n_kv_heads, head_dim,
         head_dim if v_dim is None else int(v_dim), float(scale), int(window), 1 if sink else 0, _ptr(out_cos), _ptr(out_sin),
         0 if out_cos is None else out_cos.shape[0], _ptr(gate), 0 if gate is None else gate.stride(0), _ptr(seq_qstart), _ptr(seq_past), _ptr(seq_slot), _ptr(page_table),
-        page_table.shape[1], num_pages, _ptr(k_pages), _ptr(v_pages), sm_count(q.device), _ptr(_work_counter(q.device)), _ptr(status), _stream()),
+        page_table.shape[1], num_pages, _ptr(k_pages), _ptr(v_pages), sm_count(q.device), _ptr(_work_counter(q.device)), parts, _ptr(scratch), _ptr(status), _stream()),
         "attention_umma_prefill")
-    _count(1)
+    _count(1 if parts == 1 else 2)
 
 
 def sample_scratch_bytes(n_rows: int, vocab: int, temperature: float, top_k: int, top_p: float = 1.0,

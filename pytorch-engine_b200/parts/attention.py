@@ -308,7 +308,7 @@ class GQAttention:
         gate = self.gate_columns(q) if self.gate_in_kernel(ctx) else None
         if self.use_umma_prefill and not ctx.decode and not self.generic_attention:
             ops.attention_umma_prefill(q, out, ctx.n_seqs, ctx.max_q, self.n_heads, self.n_kv_heads, self.head_dim, self.scale,
-                                       self.window, *where, self.runtime.status, v_dim=self.v_dim, gate=gate, **extra)
+                                       self.window, *where, self.runtime.status, v_dim=self.v_dim, gate=gate, **self.in_parts(q, ctx), **extra)
             return
         if self.use_mma and not self.generic_attention:
             scratch = None
@@ -391,7 +391,7 @@ class GQAttention:
             ops.attention_umma_prefill(
                 q, out, ctx.n_seqs, ctx.max_q, self.n_heads, self.n_kv_heads, self.head_dim, self.scale, self.window,
                 ctx.seq_qstart, ctx.seq_past, ctx.seq_slot, view.page_table, view.num_pages, view.k_pages, view.v_pages,
-                self.runtime.status)
+                self.runtime.status, **self.in_parts(q, ctx))
             return
         scratch = None
         max_splits = 0
@@ -413,3 +413,15 @@ class GQAttention:
             ctx.decode, q, out, ctx.n_seqs, ctx.max_q, self.n_heads, self.n_kv_heads, self.head_dim, self.scale,
             self.window, ctx.seq_qstart, ctx.seq_past, ctx.seq_slot, view.page_table, view.num_pages, view.k_pages,
             view.v_pages, scratch, split_keys, max_splits, self.runtime.status, **extra)
+
+    def in_parts(self, q: torch.Tensor, ctx) -> dict:
+        """How many blocks a tile of queries is shared out over (``ops.attention_umma_parts``), and their scratch."""
+        group = self.n_heads // self.n_kv_heads
+        whole = 128 // group                   # tokens of a tile
+        items = -(-ctx.max_q // whole) * ctx.n_seqs * self.n_kv_heads
+        seen = min(ctx.max_kv_len, self.window + whole) if self.window else ctx.max_kv_len
+        parts = ops.attention_umma_parts(ops.sm_count(q.device) * (2 if self.head_dim <= 128 else 1), items, -(-seen // 64))
+        if parts == 1:
+            return {}
+        return dict(parts=parts, scratch=ctx.buffer("attn.parts", (parts * q.shape[0] * self.n_heads * (self.v_dim + 1),), torch.float32))
+

@@ -631,6 +631,36 @@ def test_recurrences_just_below_48_kb(ops, d, dv, kind):
     assert all(rel_err(x, y) < 5e-6 for x, y in zip(once, twice))
 
 
+@pytest.mark.parametrize("nh,nkv,d,dv", [(8, 2, 128, 128), (5, 1, 128, 128), (6, 2, 192, 64)])
+@pytest.mark.parametrize("parts", [2, 3, 8])
+@pytest.mark.parametrize("window,sink,extra", [(0, False, ""), (200, True, "gate"), (0, True, "turn")])
+def test_attention_umma_prefill_in_parts(ops, nh, nkv, d, dv, parts, window, sink, extra):
+    """A row tile's pages over several blocks against one block a tile: new tokens behind a long past, tiles with fewer pages than
+    parts, rows whose keys all lie in one part."""
+    if extra == "turn" and (d, dv) != (128, 128):
+        pytest.skip("turned outputs: heads of 128 features")
+    torch.manual_seed(26)
+    bf = torch.bfloat16
+    q_lens, pasts = [70, 1, 33, 130], [900, 70, 0, 512]
+    lens, N = [a + b for a, b in zip(q_lens, pasts)], sum(q_lens)
+    kp, vp = PagedSetup(lens, nkv, d, bf, seed=26, key_scale=2.0), PagedSetup(lens, nkv, dv, bf, seed=26)
+    q = torch.randn(N, (nh + nkv) * d, device=DEV).to(bf)
+    gate = torch.randn(N, nh, device=DEV).to(bf) if extra == "gate" else None
+    angles = torch.rand(1024, 64, device=DEV) * 6
+    turn = dict(out_cos=angles.cos(), out_sin=angles.sin()) if extra == "turn" else {}
+    qstart = torch.tensor([0] + list(torch.tensor(q_lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    past, st = torch.tensor(pasts, dtype=torch.int32, device=DEV), _status()
+    outs = []
+    for n in (1, parts):
+        out = torch.full((N, nh * dv), float("nan"), device=DEV, dtype=bf)
+        scratch = torch.full((n * N * nh * (dv + 1) + 64,), float("nan"), device=DEV)
+        ops.attention_umma_prefill(q, out, 4, max(q_lens), nh, nkv, d, d ** -0.5, window, qstart, past, kp.seq_slot, kp.table, kp.num_pages,
+                                   kp.k_pages, vp.v_pages, st, sink=sink, v_dim=dv, gate=gate, parts=n, scratch=scratch, **turn)
+        assert st.tolist()[0] == 0 and bool(scratch[n * N * nh * (dv + 1):].isnan().all())
+        outs.append(out.float())
+    assert rel_err(outs[1], outs[0]) < 2 * ATT_TOL[bf]
+
+
 @pytest.mark.parametrize("decode", [False, True])
 def test_attention_mma_finds_a_far_key_and_ignores_what_lies_beyond_the_length(ops, decode):
     nh, nkv, d = 8, 2, 128
