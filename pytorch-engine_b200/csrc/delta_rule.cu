@@ -141,6 +141,51 @@ __global__ void conv_tail_kernel(const T* x, long long ld, int col0, float* tail
   }
 }
 
+// Both for steps with as many tokens as sequences, which is one a sequence: a thread owns a channel of a sequence, so its output and
+// its new tail need no kernel between them.  (Any other split of as many tokens over the sequences takes the loop.)  2,048 channels of
+// two sequences: 2.3 us.
+template <typename T>
+__global__ void __launch_bounds__(128) short_conv_step_kernel(const T* x, long long ld, int col0, const float* __restrict__ w,
+                                                              const float* __restrict__ bias, int taps, float* tail, const int* seq_slot,
+                                                              const int* seq_qstart, T* __restrict__ out, int channels, int n_slots, int* status) {
+  const int c = blockIdx.x * 128 + threadIdx.x, b = blockIdx.y;
+  constexpr int kTaps = 8;
+  float wr[kTaps], br = 0.f;
+#pragma unroll
+  for (int j = 0; j < kTaps; ++j) wr[j] = c < channels && j < taps ? w[(size_t)c * taps + j] : 0.f;
+  if (bias && c < channels) br = bias[c];
+  pdl_wait_block();
+  pdl_launch_dependents();
+  const int slot = seq_slot[b], t0 = seq_qstart[b], t1 = seq_qstart[b + 1];
+  if (t1 <= t0) return;
+  if (slot < 0 || slot >= n_slots) {
+    if (c == 0) report(status, kStatusSlotOutOfRange, t0, slot, n_slots);
+    return;
+  }
+  if (c >= channels) return;
+  float* mine = tail + (size_t)slot * (taps - 1) * channels + c;
+  float v[kTaps];
+#pragma unroll
+  for (int j = 0; j < kTaps; ++j) v[j] = j + 1 < taps ? mine[(size_t)j * channels] : 0.f;
+  for (int t = t0; t < t1; ++t) {
+    const float now = to_f32<T>(x[(size_t)t * ld + col0 + c]);
+    float acc = br;
+#pragma unroll
+    for (int j = 0; j < kTaps; ++j)
+      if (j < taps) {
+        if (j + 1 == taps) v[j] = now;
+        acc = fmaf(wr[j], v[j], acc);
+      }
+    out[(size_t)t * channels + c] = from_f32<T>(acc / (1.f + expf(-acc)));
+#pragma unroll
+    for (int j = 0; j + 1 < kTaps; ++j)
+      if (j + 1 < taps) v[j] = v[j + 1];
+  }
+#pragma unroll
+  for (int j = 0; j + 1 < kTaps; ++j)
+    if (j + 1 < taps) mine[(size_t)j * channels] = v[j];
+}
+
 // ---- the recurrence -----------------------------------------------------------------------------------------------
 struct DeltaArgs {
   const void* qkv;          // [n_tokens, channels] after the convolution: q (kv_heads * d) | k (kv_heads * d) | v (heads * dv)
@@ -415,6 +460,121 @@ __global__ void __launch_bounds__(DREG == 0 ? 1024 : 512) delta_rule_kernel(Delt
   }
 }
 
+// One token a sequence (walk.cuh): S' = diag(g) S + k u^T with u = beta (v - (diag(g) S)^T k), and S'^T q = (diag(g) S)^T q + u (k.q).
+// Eight heads of 128 x 128, two sequences: 4.8 us, 10.9 in one block a head (8 of 148 SMs a sequence, and a
+// chain of d / 64 rounds of loads from global memory).
+template <typename T, int CV>
+__global__ void __launch_bounds__(kStepThreads) delta_step_kernel(DeltaArgs a) {
+  __shared__ __align__(16) float s_sum[4][2][16 * CV];
+  __shared__ float s_k[128], s_q[128], s_g[128], s_dot[4][3], s_o[16 * CV], s_ss;
+  constexpr int COLS = 16 * CV;
+  const int ranks = a.dv / COLS, head = blockIdx.x / ranks, rank = blockIdx.x % ranks, b = blockIdx.y;
+  const int d = a.d, dv = a.dv, col0 = rank * COLS, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rg = warp * 8 + (lane >> 2), cg = lane & 3, kvh = head / (a.heads / a.kv_heads);
+  const int slot = a.seq_slot[b], t = a.seq_qstart[b], tokens = a.seq_qstart[b + 1] - t;
+  const bool there = slot >= 0 && slot < a.n_slots;
+  float* S = a.S + ((size_t)(there ? slot : 0) * a.heads + head) * d * dv;
+  const float rate = expf(a.A_log[head]);
+  const float dt = tid < d ? a.dt_bias[a.head_decay ? head : head * d + tid] : 0.f;
+  const float nw = tid < COLS ? a.norm_w[col0 + tid] : 0.f;
+  pdl_wait_block();
+  pdl_launch_dependents();
+  if (!there) {
+    if (tid == 0 && blockIdx.x == 0) report(a.status, kStatusSlotOutOfRange, b, slot, a.n_slots);
+    return;      // the whole cluster
+  }
+  if (tokens <= 0) return;
+  StepState<CV> st;
+  st.load(S, d, dv, col0, rg, cg);
+  const int channels = 2 * a.kv_heads * d + a.heads * dv;
+  const T* x = (const T*)a.qkv + (size_t)t * channels;
+  float k = 0.f, q = 0.f, vj = 0.f, gate = 0.f;
+  if (tid < d) {
+    q = to_f32<T>(x[kvh * d + tid]);
+    k = to_f32<T>(x[a.kv_heads * d + kvh * d + tid]);
+    const float z = a.a[(size_t)t * a.a_ld + (a.head_decay ? head : head * d + tid)] + dt;
+    s_g[tid] = expf(-rate * (z > 20.f ? z : log1pf(expf(z))));
+    s_k[tid] = k;
+    s_q[tid] = q;
+  }
+  if (tid < COLS) {
+    vj = to_f32<T>(x[2 * a.kv_heads * d + head * dv + col0 + tid]);
+    gate = to_f32<T>(((const T*)a.gate)[(size_t)t * a.gate_ld + head * dv + col0 + tid]);
+    s_o[tid] = vj;
+  }
+  const float beta = 1.f / (1.f + expf(-a.b[(size_t)t * a.b_ld + head]));
+  const float kk = warp_sum(k * k), qq = warp_sum(q * q), kq = warp_sum(k * q);
+  if (lane == 0) {
+    s_dot[warp][0] = kk;
+    s_dot[warp][1] = qq;
+    s_dot[warp][2] = kq;
+  }
+  __syncthreads();
+  const float kn = rsqrtf((s_dot[0][0] + s_dot[1][0]) + (s_dot[2][0] + s_dot[3][0]) + 1e-6f);
+  const float qn = rsqrtf((s_dot[0][1] + s_dot[1][1]) + (s_dot[2][1] + s_dot[3][1]) + 1e-6f) * a.q_scale;
+  const float k_q = (s_dot[0][2] + s_dot[1][2]) + (s_dot[2][2] + s_dot[3][2]);
+  float kr[4];
+#pragma unroll
+  for (int v = 0; v < CV; ++v) {
+    float4 sk = make_float4(0.f, 0.f, 0.f, 0.f), sq = sk;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int i = rg + 32 * r;
+      const bool live = i < d;
+      const float g = live ? s_g[i] : 0.f, ki = live ? s_k[i] : 0.f, qi = live ? s_q[i] : 0.f;
+      kr[r] = ki;
+      float4& c = st.s[r][v];
+      c.x *= g; c.y *= g; c.z *= g; c.w *= g;
+      sk.x = fmaf(c.x, ki, sk.x); sk.y = fmaf(c.y, ki, sk.y); sk.z = fmaf(c.z, ki, sk.z); sk.w = fmaf(c.w, ki, sk.w);
+      sq.x = fmaf(c.x, qi, sq.x); sq.y = fmaf(c.y, qi, sq.y); sq.z = fmaf(c.z, qi, sq.z); sq.w = fmaf(c.w, qi, sq.w);
+    }
+    sk = step_rows_sum(sk);
+    sq = step_rows_sum(sq);
+    if (lane < 4) {
+      *reinterpret_cast<float4*>(&s_sum[warp][0][16 * v + 4 * cg]) = sk;
+      *reinterpret_cast<float4*>(&s_sum[warp][1][16 * v + 4 * cg]) = sq;
+    }
+  }
+  __syncthreads();
+  auto total = [&](int what, int c) { return (s_sum[0][what][c] + s_sum[1][what][c]) + (s_sum[2][what][c] + s_sum[3][what][c]); };
+  // the block's outputs, a column a thread of the first warp, and their squares' sum for the head norm
+  float o = 0.f;
+  if (tid < COLS) {
+    const float uk = beta * (vj - total(0, tid) * kn) * kn;
+    o = fmaf(uk, k_q, total(1, tid)) * qn;
+  }
+  if (warp == 0) {
+    const float ss = warp_sum(o * o);
+    if (lane == 0) s_ss = ss;
+  }
+  cluster_arrive();
+#pragma unroll
+  for (int v = 0; v < CV; ++v) {
+    float u[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int c = 16 * v + 4 * cg + e;
+      u[e] = beta * (s_o[c] - total(0, c) * kn) * kn;
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      float4& c = st.s[r][v];
+      c.x = fmaf(kr[r], u[0], c.x); c.y = fmaf(kr[r], u[1], c.y); c.z = fmaf(kr[r], u[2], c.z); c.w = fmaf(kr[r], u[3], c.w);
+    }
+  }
+  st.store(S, d, dv, col0, rg, cg);
+  cluster_wait();
+  if (tid < COLS) {
+    float ss = 0.f;
+    for (int r = 0; r < ranks; ++r) ss += cluster_read(&s_ss, r);
+    const float y = o * rsqrtf(ss / (float)dv + a.eps) * nw * (a.gate_silu ? gate : 1.f) / (1.f + expf(-gate));
+    ((T*)a.out)[(size_t)t * a.heads * dv + head * dv + col0 + tid] = from_f32<T>(y);
+  }
+  __syncwarp();
+  cluster_arrive();      // nobody leaves while its shared memory is read
+  cluster_wait();
+}
+
 // Chain the chunks: on entry scratch[c] holds chunk c's end state from zero and its transition matrix (every chunk
 // but the sequence's last); on exit its S part holds chunk c's true start state, chunk 0's being the slot's state.
 // A block takes a few columns of one head's state: thread (i, col) keeps element i of its column, the chunk's
@@ -629,6 +789,17 @@ extern "C" int pe_short_conv_silu(int dtype, const void* x, long long ld, int co
   if (channels <= 0 || taps <= 0 || taps > 64 || col0 < 0 || col0 + channels > ld) return PE_ERR_BAD_ARGUMENT;
   const int threads = channels >= 1024 ? 256 : 128;
   if (dtype != PE_F32 && dtype != PE_BF16) return PE_ERR_UNSUPPORTED_DTYPE;
+  if (n_tokens == n_seqs && taps >= 2 && taps <= 8 && n_seqs <= 65535) {      // one token a sequence
+    const dim3 grid((channels + 127) / 128, n_seqs);
+    if (dtype == PE_F32)
+      pe::launch(pe::short_conv_step_kernel<float>, grid, dim3(128), 0, stream, (const float*)x, ld, col0, w, bias, taps, tail, seq_slot,
+                 seq_qstart, (float*)out, channels, n_slots, status);
+    else
+      pe::launch(pe::short_conv_step_kernel<__nv_bfloat16>, grid, dim3(128), 0, stream, (const __nv_bfloat16*)x, ld, col0, w, bias, taps,
+                 tail, seq_slot, seq_qstart, (__nv_bfloat16*)out, channels, n_slots, status);
+    PE_LAUNCH_CHECK();
+    return PE_OK;
+  }
   const bool vec8 = dtype == PE_BF16 && taps >= 2 && taps <= 4 && channels % 8 == 0 && ld % 8 == 0 && col0 % 8 == 0 &&
                     (uintptr_t)x % 16 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)tail % 16 == 0;   // (taps == 1: no tail is read)
   if (vec8) {
@@ -719,6 +890,16 @@ extern "C" int pe_delta_rule_recurrence(int dtype, const void* qkv, const float*
   if (chunk > 0) {
     if (!scratch || max_chunks <= 0 || (long long)max_chunks * chunk < max_q || max_chunks > 32767) return PE_ERR_BAD_ARGUMENT;
     args.chunk = chunk; args.max_chunks = max_chunks; args.scratch = scratch;
+  }
+  // single tokens: a head's columns over a cluster, where the state's rows are 16-byte pieces
+  if (chunk <= 0 && max_q == 1 && pe::step_takes(d, dv) && (uintptr_t)S % 16 == 0 && n_seqs <= 65535) {
+    const int cols = pe::step_columns(dv), ranks = dv / cols;
+    cudaError_t ce;
+    if (dtype == PE_F32) ce = pe::launch_step(cols == 16 ? pe::delta_step_kernel<float, 1> : pe::delta_step_kernel<float, 2>, heads, ranks, n_seqs, stream, args);
+    else ce = pe::launch_step(cols == 16 ? pe::delta_step_kernel<__nv_bfloat16, 1> : pe::delta_step_kernel<__nv_bfloat16, 2>, heads, ranks, n_seqs, stream, args);
+    if (ce != cudaSuccess) return (int)ce;
+    PE_LAUNCH_CHECK();
+    return PE_OK;
   }
   int rc;
 #define PE_DELTA(T)                                                       \

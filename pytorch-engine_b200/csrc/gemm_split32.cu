@@ -20,11 +20,11 @@
 //   17     TMA producer: the three parts of the x tile.
 // Operands that three parts cannot hold (infinities, NaN, numbers next to either end of float32's range) and results as small or
 // as large are noticed, and what they touch is computed again as a plain chain of multiply-adds (second_look).
-// What bounds it: no unit (600 x 30,720 outputs, K = 1,024, 261 us, 145 TFLOP/s: tensor pipe 46 % busy, loads and stores of shared
-// memory 43 %, issue slots 38 %).  A block takes 32 us for its 16 chunks; about 3 lie before the first chunk's sums and behind the
+// What bounds it: no unit (600 x 30,720 outputs, K = 1,024, 240 us, 158 TFLOP/s; in tiles of 128 rows 261 us: tensor pipe 46 % busy,
+// loads and stores of shared memory 43 %, issue slots 38 %).  A block takes 32 us for its 16 chunks; about 3 lie before the first chunk's sums and behind the
 // last's, where nothing overlaps, and in between conversion, MMAs and addition of a chunk follow one another over two stages.
-// 600 rows against the library's float32 product: 4,096 x 1,024 weights 55 against 122 us, 1,024 x 3,072 35 against 125, 151,936 x
-// 1,024 1,137 against 3,349 (164 TFLOP/s); 24 rows, 4,096 x 1,024 13 against 27.
+// 600 rows against the library's float32 product: 4,096 x 1,024 weights 37 against 123 us, 1,024 x 3,072 35 against 127, 151,936 x
+// 1,024 1,106 against 3,204 (169 TFLOP/s); 24 rows, 4,096 x 1,024 13 against 27.
 // All waits are bounded.
 #include "api.h"
 #include "common.cuh"
@@ -197,8 +197,8 @@ __device__ __forceinline__ int exact_any(int v) {        // a barrier of these w
 
 // Every warp but the last two; a thread has one column and a quarter of the rows.  The tile's results are in y, shared memory is
 // free.  A tile in which nothing is computed again reads its operands once more; otherwise the whole tile's chains run side by side.
-// 600 x 4,096 outputs, K = 1,024, 59 us: 73 with one zero row of W (the tiles of its 128 rows look), 134 where every tile looks,
-// 713 where everything is NaN (one NaN row of W took 4,519 when its outputs were one thread's).
+// 600 x 4,096 outputs, K = 1,024, 37 us: 86 with one zero row of W (the tiles of its 128 rows look), 87 where every tile looks,
+// 486 where everything is NaN (one NaN row of W took 4,519 when its outputs were one thread's).
 template <int NT>
 __device__ __noinline__ void second_look(const Params p) {      // (takes nothing that the product would have to keep for it)
   constexpr int kRows = NT / 4;
@@ -495,7 +495,9 @@ __global__ void __launch_bounds__(256) gemm_split32_add_kernel(const float* part
 
 struct Plan { int nt, splits, chunks_per_split; };
 // Tile and ranges of K by how many blocks come after one another on an SM.  Times in microseconds, measured on a B200: a chunk
-// of a tile of 128 or 64 rows, what a block costs beyond its chunks, the addition of partial sums.
+// of a tile of 160, 128 or 64 rows, what a block costs beyond its chunks, the addition of partial sums.  Tiles of 160 rows are for
+// one wave less: 527 x 4,096 outputs, K = 1,024, are 160 tiles of 128 rows (59 us) or 288 of 64 (63) but 128 of 160 (37); with 400 rows
+// of 4,096 outputs, 128 tiles of 128 rows, 31 us against 37.
 static Plan plan_for(int M, int N, int K, int n_sms) {
   const int chunks = (K + BK - 1) / BK, n_tiles = (N + BM - 1) / BM;
   Plan best{128, 1, chunks};

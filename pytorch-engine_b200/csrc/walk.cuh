@@ -225,4 +225,70 @@ inline void launch_walk(const WalkArgs& a, int d, int n_seqs, cudaStream_t strea
 }
 inline bool walk_takes(int d, int dv) { return (d == 32 || d == 64 || d == 128) && dv > 0 && dv % kWalkCols == 0; }
 
+// ---- one token a sequence --------------------------------------------------------------------------------------------
+// A step of single tokens is a pass over the states: a head's S is read once and written once, and the block that owned a whole
+// head (a token's staging, three barriers, one column a thread) took 11 us for 64 KB.  Here a head's columns are shared out over
+// a cluster of blocks of 16 or 32 columns each, whose 128 threads hold four neighbouring columns of every 32nd row: all of the
+// state is on its way at once, and one pass of sums over the rows is enough, since what a token adds to S adds a known multiple of
+// k.q to the read.  The head norm's sum goes through the cluster's shared memory.
+constexpr int kStepThreads = 128;
+inline bool step_takes(int d, int dv) {      // rows: up to four a thread; blocks of a head: one cluster of up to eight
+  return d >= 8 && d <= 128 && dv % 16 == 0 && (dv <= 128 || (dv % 32 == 0 && dv <= 256));
+}
+inline int step_columns(int dv) { return dv <= 128 ? 16 : 32; }
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
+__device__ __forceinline__ float cluster_read(const float* p, int rank) {
+  uint32_t at;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(at) : "memory");
+  return v;
+}
+
+// A thread's part of S: rows rg + 32 r, columns 4 cg .. + 3 of the block's (and 16 further on with CV == 2).
+template <int CV> struct StepState {
+  float4 s[4][CV];
+  __device__ __forceinline__ void load(const float* S, int d, int dv, int col0, int rg, int cg) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int v = 0; v < CV; ++v)
+        s[r][v] = rg + 32 * r < d ? *reinterpret_cast<const float4*>(S + (size_t)(rg + 32 * r) * dv + col0 + 16 * v + 4 * cg)
+                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  __device__ __forceinline__ void store(float* S, int d, int dv, int col0, int rg, int cg) const {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int v = 0; v < CV; ++v)
+        if (rg + 32 * r < d) *reinterpret_cast<float4*>(S + (size_t)(rg + 32 * r) * dv + col0 + 16 * v + 4 * cg) = s[r][v];
+  }
+};
+// Sums over the rows a warp holds (lanes of one column group: every fourth).
+__device__ __forceinline__ float4 step_rows_sum(float4 v) {
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o); v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+    v.z += __shfl_xor_sync(0xffffffffu, v.z, o); v.w += __shfl_xor_sync(0xffffffffu, v.w, o);
+  }
+  return v;
+}
+
+// One block a cluster rank: grid (heads * ranks, n_seqs), cluster (ranks, 1, 1).
+template <typename K, typename A>
+inline cudaError_t launch_step(K kernel, int heads, int ranks, int n_seqs, cudaStream_t stream, const A& args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(heads * ranks, n_seqs); cfg.blockDim = dim3(kStepThreads); cfg.dynamicSmemBytes = 0; cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ranks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args);
+}
+
 }  // namespace pe

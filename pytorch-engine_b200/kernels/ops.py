@@ -892,7 +892,7 @@ def short_conv_silu(x: torch.Tensor, col0: int, w: torch.Tensor, tail: torch.Ten
     check(library().pe_short_conv_silu(dtype_tag(x.dtype), _ptr(x), x.stride(0), int(col0), _ptr(w), _ptr(bias), taps, _ptr(tail),
                                        _ptr(token_seq), _ptr(seq_slot), _ptr(seq_qstart), _ptr(out), x.shape[0], n_seqs, channels,
                                        tail.shape[0] if taps > 1 else (1 << 30), _ptr(status), _stream()), "short_conv_silu")
-    _count(2 if taps > 1 else 1)
+    _count(2 if taps > 1 and not (taps <= 8 and x.shape[0] == n_seqs) else 1)
 
 
 def delta_rule_recurrence(qkv: torch.Tensor, a: torch.Tensor, dt_bias: torch.Tensor, A_log: torch.Tensor, b: torch.Tensor,

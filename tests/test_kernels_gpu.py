@@ -631,6 +631,70 @@ def test_recurrences_just_below_48_kb(ops, d, dv, kind):
     assert all(rel_err(x, y) < 5e-6 for x, y in zip(once, twice))
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d,dv", [(128, 128), (128, 256), (64, 64), (8, 16), (100, 48), (32, 160), (36, 96)])
+def test_recurrences_of_single_tokens_over_a_cluster(ops, dtype, d, dv):
+    """A step of one token a sequence with a head's columns over a cluster against the same step in one block a head (which runs where
+    a step says that it may bring two tokens): outputs and every part of the state; a sequence's slot out of range is left out."""
+    torch.manual_seed(24)
+    H, G, B, slots, f32 = 4, 2, 3, 5, torch.float32
+    slot, qstart = torch.tensor([4, 0, 2], dtype=torch.int32, device=DEV), torch.arange(B + 1, dtype=torch.int32, device=DEV)
+    rand = lambda *shape: torch.randn(*shape, device=DEV)  # noqa: E731
+    qkv, gate = rand(B, 2 * G * d + H * dv).to(dtype), rand(B, H * dv + 8).to(dtype)[:, :H * dv]
+    a, b, dt, A, nw, S0 = rand(B, H * d), rand(B, H), rand(H * d) - 2, rand(H) * 0.3, 1 + 0.2 * rand(dv), rand(slots, H, d, dv)
+    tol = 2e-5 if dtype == f32 else 1e-2
+    for head_decay, gate_silu in ((False, False), (True, True)):
+        got = []
+        for max_q in (1, 2):
+            out, S, st = torch.full((B, H * dv), float("nan"), device=DEV, dtype=dtype), S0.clone(), _status()
+            ops.delta_rule_recurrence(qkv, a[:, :H].contiguous() if head_decay else a, dt[:H] if head_decay else dt, A, b, gate, nw, 1e-6, d ** -0.5,
+                                      out, S, slot, qstart, B, max_q, H, G, d, dv, st, head_decay=head_decay, gate_silu=gate_silu)
+            assert st.tolist()[0] == 0
+            got.append((out.float(), S))
+        assert rel_err(got[0][0], got[1][0]) < tol and rel_err(got[0][1], got[1][1]) < 2e-6
+    rows = rand(B, H * (2 * d + 2 * dv)).to(dtype)
+    q, k, v, g = (rows[:, lo:hi] for lo, hi in ((0, H * d), (H * d, 2 * H * d), (2 * H * d, H * (2 * d + dv)), (H * (2 * d + dv), H * (2 * d + 2 * dv))))
+    gates, bias, mw, n0, m0 = 3 * rand(B, 2 * H), rand(2 * H), 1 + 0.2 * rand(H * dv), rand(slots, H, d), rand(slots, H)
+    got = []
+    for max_q in (1, 2):
+        out, S, n, mx, st = torch.full((B, H * dv), float("nan"), device=DEV, dtype=dtype), S0.clone(), n0.clone(), m0.clone(), _status()
+        ops.mlstm_recurrence(q, k, v, g, gates, bias, mw, 15.0, 1e-6, d ** -0.5, out, S, n, mx, slot, qstart, B, max_q, H, d, dv, st)
+        assert st.tolist()[0] == 0
+        got.append((out.float(), S, n, mx))
+    assert rel_err(got[0][0], got[1][0]) < tol
+    for i in (1, 2, 3):
+        assert rel_err(got[0][i], got[1][i]) < 2e-6
+    S, st = S0.clone(), _status()
+    ops.mlstm_recurrence(q, k, v, g, gates, bias, mw, 15.0, 1e-6, d ** -0.5, out, S, n, mx, slot + 2, qstart, B, 1, H, d, dv, st)
+    assert st.tolist()[0] == 5 and torch.equal(S[[0, 1, 3]], S0[[0, 1, 3]])
+    some, S, st = torch.tensor([0, 1, 1, 2], dtype=torch.int32, device=DEV), S0.clone(), _status()      # a sequence without a token
+    ops.mlstm_recurrence(q, k, v, g, gates, bias, mw, 15.0, 1e-6, d ** -0.5, out, S, n, mx, slot, some, B, 1, H, d, dv, st)
+    ops.delta_rule_recurrence(qkv, a, dt, A, b, gate, nw, 1e-6, d ** -0.5, out, S, slot, some, B, 1, H, G, d, dv, st)
+    assert st.tolist()[0] == 0 and torch.equal(S[0], S0[0]) and not torch.equal(S[2], S0[2]) and not torch.equal(S[4], S0[4])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("taps,channels", [(2, 40), (4, 2048), (8, 129), (9, 64)])
+@pytest.mark.parametrize("lengths", [(1, 1, 1), (2, 0, 1), (0, 0, 3)])
+def test_short_conv_of_single_tokens(ops, dtype, taps, channels, lengths):
+    """As many tokens as sequences (up to eight taps: one kernel) against the sum over the tail and the tokens, and the tail moved on."""
+    torch.manual_seed(25)
+    B, slots = 3, 5
+    slot, ends = torch.tensor([4, 0, 2], dtype=torch.int32, device=DEV), [0, lengths[0], lengths[0] + lengths[1], B]
+    qstart, of = torch.tensor(ends, dtype=torch.int32, device=DEV), [b for b in range(B) for _ in range(lengths[b])]
+    x, w, bias = torch.randn(B, channels + 16, device=DEV).to(dtype), torch.randn(channels, taps, device=DEV), torch.randn(channels, device=DEV)
+    tail = torch.randn(slots, taps - 1, channels, device=DEV)
+    before, out, st = tail.clone(), torch.empty(B, channels, device=DEV, dtype=dtype), _status()
+    ops.short_conv_silu(x, 8, w, tail, torch.tensor(of, dtype=torch.int32, device=DEV), slot, qstart, out, B, st, bias)
+    want = before.clone()
+    for t, s in enumerate(slot[of].tolist()):
+        rows = torch.cat([want[s], x[t:t + 1, 8:8 + channels].float()])
+        y = (rows.double() * w.t().double()).sum(0) + bias.double()
+        assert rel_err(out[t].float(), (y / (1 + (-y).exp())).float()) < (2e-6 if dtype == torch.float32 else 1e-2)
+        want[s] = rows[1:]
+    assert torch.equal(tail, want) and st.tolist()[0] == 0
+
+
 @pytest.mark.parametrize("nh,nkv,d,dv", [(8, 2, 128, 128), (5, 1, 128, 128), (6, 2, 192, 64)])
 @pytest.mark.parametrize("parts", [2, 3, 8])
 @pytest.mark.parametrize("window,sink,extra", [(0, False, ""), (200, True, "gate"), (0, True, "turn")])
