@@ -37,7 +37,7 @@ constexpr int STAGES = 3;
 constexpr int kTileA = BM * BK * 2, kTileB = BNH * BK * 2;   // one k block of each operand
 constexpr int kBytesA = KBS * kTileA, kBytesB = KBS * kTileB, kStage = kBytesA + kBytesB;
 constexpr int kTmemCols = 512;
-constexpr int kThreads = 192;
+constexpr int kThreads = 192, kRopeThreads = 320;   // four or eight epilogue warps
 
 // Mode 3: the product is the fused q|k|v projection of an attention layer with head size 128, and the epilogue
 // does what csrc/rope_append.cu does in a kernel of its own: per-head q/k RMSNorm, rotary encoding, q written to
@@ -159,6 +159,13 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 
 // K-major tile, 128-byte swizzle: rows of 64 bfloat16, groups of 8 rows 1024 bytes apart (see gemm_umma.cu)
@@ -185,92 +192,86 @@ __device__ __forceinline__ float bf16_round(uint32_t bits) {
   return __bfloat162float(__float2bfloat16_rn(__uint_as_float(bits)));
 }
 
-// The epilogue of mode 3 for one token row of a 256-column tile (two heads of 128 features).  Formulas and order
-// as csrc/rope_append.cu (pygguf_engine/model.py:471-474 q/k-norm before RoPE, not on v; 232-241 split-half
+// What a warp of mode 3's epilogue has in shared memory: 32 features of each of its 32 rows on their way out.  Rows are 80 bytes, so
+// that the 16-byte accesses of eight lanes to eight rows fall into different banks.
+constexpr int kRopeRow = 80, kRopeWarp = 32 * kRopeRow;
+
+// The epilogue of mode 3 for the 32 token rows of a warp (`row`: this lane's) of one head of 128 features.
+// Formulas and order as csrc/rope_append.cu (pygguf_engine/model.py:471-474 q/k-norm before RoPE, not on v; 232-241 split-half
 // rotation; 482-483 append): the accumulator is rounded to bfloat16 first (the value the projection would have
 // stored), the norm's sum runs over those values, norm and rotation are one float32 computation, the result is
 // rounded once.  Every thread of the warp runs every tensor-memory load; only live rows store.
-__device__ __forceinline__ void rope_epilogue(const Params& p, int row, int n0, uint32_t t_row) {
+//
+// Eight warps, two a scheduler, share a tile of two heads: with four, one a scheduler and both heads, each instruction waited for
+// the one before.  A lane owns a row, and rows lie far apart in the outputs, so results go out four lanes a row, through shared
+// memory, 16 pairs of features at a time (a lane that stored its own row touched 32 of them with each instruction).  16 prompts of 16
+// to 2,048 tokens, 4,096 x 1,024 weights: 192 -> 174 us (the new stores alone gained nothing).  With K = 4,096 the epilogue is
+// hidden behind the next tile's MMAs either way, but for the last tile of a block.
+__device__ __forceinline__ void rope_epilogue(const Params& p, int row, int n0, uint32_t t_row, char* stage, int lane) {
   const RopeFuse& r = p.rope;
-  constexpr int D = 128, HALF = 64;
+  constexpr int D = 128, HALF = 64, C = 16, H = 1;
+  char* out_s = stage;
   const bool live = row < p.M;
+  const int n_cached = r.n_heads + 2 * r.n_kv_heads;      // heads of q|k|v
   int pos = 0;
   if (live) pos = r.token_pos[row];
-  const bool rotates = r.cos_table != nullptr;
-  const bool pos_ok = !rotates || (pos >= 0 && pos < r.table_rows);
+  const bool rotates = r.cos_table != nullptr && n0 / D < r.n_heads + r.n_kv_heads;
+  const bool pos_ok = r.cos_table == nullptr || (pos >= 0 && pos < r.table_rows);
   if (live && !pos_ok) report(p.status, kStatusPositionOutOfRange, row, pos, r.table_rows);
-#pragma unroll 1
-  for (int h = 0; h < BN / D; ++h) {
-    const int col0 = n0 + h * D;
-    if (col0 >= p.N) break;
-    const int head = col0 / D;
-    if (head >= r.n_heads + 2 * r.n_kv_heads) {           // columns behind q|k|v
-#pragma unroll 1
-      for (int c = 0; c < D && col0 + c < p.N; c += 32) {
-        uint32_t v[32];
-        __syncwarp();
-        tmem_ld32(t_row + h * D + c, v);
-        tmem_ld_wait();
-        if (live) {
-          __nv_bfloat16* yrow = reinterpret_cast<__nv_bfloat16*>(p.y) + (size_t)row * p.ldy + col0 + c;
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (col0 + c + j < p.N) yrow[j] = __float2bfloat16_rn(__uint_as_float(v[j]));
-        }
-      }
-      continue;
-    }
-    const bool is_q = head < r.n_heads;
-    const bool is_k = !is_q && head < r.n_heads + r.n_kv_heads;
-    const int kv_head = is_q ? 0 : (is_k ? head - r.n_heads : head - r.n_heads - r.n_kv_heads);
-    const uint32_t t_head = t_row + h * D;
-    const float* w = is_q ? r.q_norm_w : (is_k ? r.k_norm_w : nullptr);
-    const bool is_v = !is_q && !is_k;
-    const bool unit = r.qk_unit != 0 && !is_v;
-    const float4* bias = r.bias ? reinterpret_cast<const float4*>(r.bias + col0) : nullptr;
-    const size_t v_off = ((size_t)row * r.n_kv_heads + kv_head) * D;
-    const __nv_bfloat16* mix = is_v && r.v_mix && live ? r.v_mix + v_off : nullptr;
-    __nv_bfloat16* keep = is_v && r.v_keep && live ? r.v_keep + v_off : nullptr;
-    const bool wanted = is_q || r.write_cache;            // k and v of a layer that only reads a cache go nowhere
-    // where the row goes: q into the output rows, k and v into their page of the cache
-    __nv_bfloat16* dst = nullptr;
-    if (live && pos_ok && wanted) {
-      if (is_q) {
-        dst = reinterpret_cast<__nv_bfloat16*>(p.y) + (size_t)row * p.ldy + col0;
+  // the row's place in a page of the cache, and how much of the page behind it is to be cleared: rows of a page beyond the
+  // sequence's last key must hold finite values, so the sequence's last token of this step clears the rest of its page when it
+  // starts the page or ends a multi-token step
+  long long place = -1;
+  int rest = 0;
+  if (live && pos_ok && r.write_cache && n0 / D + H > r.n_heads && n0 / D < n_cached) {
+    const int seq = r.token_seq[row];
+    const int slot = r.seq_slot[seq], q_begin = r.seq_qstart[seq], q_end = r.seq_qstart[seq + 1];
+    const int logical = pos / kPageTokens;
+    if (pos < 0 || logical >= r.table_stride) {
+      report(p.status, kStatusPositionOutOfRange, row, pos, r.table_stride * kPageTokens);
+    } else {
+      const int page = r.page_table[(size_t)slot * r.table_stride + logical];
+      if (page < 0 || page >= r.num_pages) {
+        report(p.status, kStatusPageOutOfRange, row, page, r.num_pages);
       } else {
-        const int seq = r.token_seq[row];
-        const int slot = r.seq_slot[seq];
-        const int logical = pos / kPageTokens;
-        if (pos < 0 || logical >= r.table_stride) {
-          report(p.status, kStatusPositionOutOfRange, row, pos, r.table_stride * kPageTokens);
-        } else {
-          const int page = r.page_table[(size_t)slot * r.table_stride + logical];
-          if (page < 0 || page >= r.num_pages) {
-            report(p.status, kStatusPageOutOfRange, row, page, r.num_pages);
-          } else {
-            const int off = pos % kPageTokens;
-            dst = (is_k ? r.k_pages : r.v_pages) + (((size_t)page * r.n_kv_heads + kv_head) * kPageTokens + off) * D;
-            // rows of the page beyond the sequence's last key must hold finite values: the sequence's last token of
-            // this step clears the rest of its page when it starts the page or ends a multi-token step
-            const int q_begin = r.seq_qstart[seq], q_end = r.seq_qstart[seq + 1];
-            if (row + 1 == q_end && off + 1 < kPageTokens && (off == 0 || q_end - q_begin > 1)) {
-              uint4* rest = reinterpret_cast<uint4*>(dst + D);
-              const int n16 = (kPageTokens - 1 - off) * D / 8;
-              for (int i = 0; i < n16; ++i) rest[i] = make_uint4(0, 0, 0, 0);
-            }
-          }
-        }
+        const int off = pos % kPageTokens;
+        place = ((long long)page * r.n_kv_heads * kPageTokens + off) * D;
+        if (row + 1 == q_end && (off == 0 || q_end - q_begin > 1)) rest = kPageTokens - 1 - off;
+      }
+    }
+  }
+  __nv_bfloat16* dst[H];
+  float inv[H];
+#pragma unroll
+  for (int h = 0; h < H; ++h) {
+    const int col0 = n0 + h * D, head = col0 / D;
+    dst[h] = nullptr;
+    inv[h] = 1.f;
+    if (col0 >= p.N || head >= n_cached) continue;
+    const bool is_q = head < r.n_heads, is_k = !is_q && head < r.n_heads + r.n_kv_heads, is_v = !is_q && !is_k;
+    // q goes into the output rows, k and v into their page of the cache (those of a layer that only reads a cache nowhere)
+    if (is_q) {
+      if (live && pos_ok) dst[h] = reinterpret_cast<__nv_bfloat16*>(p.y) + (size_t)row * p.ldy + col0;
+    } else {
+      const int kv_head = is_k ? head - r.n_heads : head - r.n_heads - r.n_kv_heads;
+      if (place >= 0) dst[h] = (is_k ? r.k_pages : r.v_pages) + place + (size_t)kv_head * kPageTokens * D;
+      for (unsigned who = __ballot_sync(0xffffffffu, place >= 0 && rest > 0); who != 0; who &= who - 1) {
+        const int from = __ffs(who) - 1;
+        uint4* to = reinterpret_cast<uint4*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(dst[h] + D), from));
+        const int n16 = __shfl_sync(0xffffffffu, rest, from) * (D / 8);
+        for (int i = lane; i < n16; i += 32) to[i] = make_uint4(0, 0, 0, 0);
       }
     }
     // the norm's scale: sum of squares over the head, in four chains added up in a fixed order
-    float inv = 1.f;
-    if (w != nullptr || unit) {
+    const bool normed = is_q ? r.q_norm_w != nullptr : (is_k && r.k_norm_w != nullptr);
+    if (normed || (r.qk_unit != 0 && !is_v)) {
+      const float4* bias = r.bias ? reinterpret_cast<const float4*>(r.bias + col0) : nullptr;
       float ss[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
       for (int c = 0; c < D; c += 32) {
         uint32_t v[32];
         __syncwarp();
-        tmem_ld32(t_head + c, v);
+        tmem_ld32(t_row + h * D + c, v);
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -283,95 +284,139 @@ __device__ __forceinline__ void rope_epilogue(const Params& p, int row, int n0, 
           }
         }
       }
-      inv = rsqrtf(((ss[0] + ss[1]) + (ss[2] + ss[3])) / (float)D + r.eps);
+      inv[h] = rsqrtf(((ss[0] + ss[1]) + (ss[2] + ss[3])) / (float)D + r.eps);
     }
-    // features j and j + 64 together, 32 pairs at a time
+  }
+  // this lane's part of the rows that it stores: rows 8 i + lane / 4, 16 bytes of each half
+  const int sub = lane >> 2, part = lane & 3;
+  // features j and j + 64 together, 16 pairs at a time
 #pragma unroll 1
-    for (int c = 0; c < HALF; c += 32) {
-      uint32_t a[32], b[32];
-      __syncwarp();
-      tmem_ld32(t_head + c, a);
-      tmem_ld32(t_head + HALF + c, b);
-      tmem_ld_wait();
-      if (dst != nullptr || keep != nullptr) {
-        uint32_t o1[16], o2[16];
-        const bool rot = rotates && !(!is_q && !is_k);
-        const float4* cs = rot ? reinterpret_cast<const float4*>(r.cos_table + (size_t)pos * HALF + c) : nullptr;
-        const float4* sn = rot ? reinterpret_cast<const float4*>(r.sin_table + (size_t)pos * HALF + c) : nullptr;
-        const float4* w1 = w ? reinterpret_cast<const float4*>(w + c) : nullptr;
-        const float4* w2 = w ? reinterpret_cast<const float4*>(w + HALF + c) : nullptr;
+  for (int c = 0; c < HALF; c += C) {
+    float4 cv4[C / 4] = {}, sv4[C / 4] = {};
+    if (rotates && r.table_rows > 0) {
+      const size_t at = (size_t)(live && pos_ok ? pos : 0) * HALF + c;
 #pragma unroll
-        for (int q4 = 0; q4 < 8; ++q4) {
-          float x1[4], x2[4];
+      for (int q4 = 0; q4 < C / 4; ++q4) {
+        cv4[q4] = reinterpret_cast<const float4*>(r.cos_table + at)[q4];
+        sv4[q4] = reinterpret_cast<const float4*>(r.sin_table + at)[q4];
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const int col0 = n0 + h * D, head = col0 / D;
+      if (col0 >= p.N || head >= n_cached) continue;
+      const bool is_q = head < r.n_heads, is_k = !is_q && head < r.n_heads + r.n_kv_heads, is_v = !is_q && !is_k;
+      const int kv_head = is_q ? 0 : (is_k ? head - r.n_heads : head - r.n_heads - r.n_kv_heads);
+      const float* w = is_q ? r.q_norm_w : (is_k ? r.k_norm_w : nullptr);
+      const bool unit = r.qk_unit != 0 && !is_v && !w;
+      const bool rot = rotates && !is_v;
+      const size_t v_off = ((size_t)row * r.n_kv_heads + kv_head) * D;
+      const __nv_bfloat16* mix = is_v && r.v_mix && live ? r.v_mix + v_off : nullptr;
+      uint32_t a[C], b[C];
+      __syncwarp();
+      tmem_ld16(t_row + h * D + c, a);
+      tmem_ld16(t_row + h * D + HALF + c, b);
+      tmem_ld_wait();
+      uint32_t o1[C / 2], o2[C / 2];
+#pragma unroll
+      for (int q4 = 0; q4 < C / 4; ++q4) {
+        float x1[4], x2[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          x1[e] = bf16_round(a[4 * q4 + e]);
+          x2[e] = bf16_round(b[4 * q4 + e]);
+        }
+        if (r.bias) {
+          const float4* bias = reinterpret_cast<const float4*>(r.bias + col0);
+          const float4 b1 = bias[c / 4 + q4], b2 = bias[HALF / 4 + c / 4 + q4];
+          x1[0] += b1.x; x1[1] += b1.y; x1[2] += b1.z; x1[3] += b1.w;
+          x2[0] += b2.x; x2[1] += b2.y; x2[2] += b2.z; x2[3] += b2.w;
+        }
+        if (mix) {
+          const float lam = r.v_lambda, left = 1.f - r.v_lambda;
+          const uint2 m1 = *reinterpret_cast<const uint2*>(mix + c + 4 * q4), m2 = *reinterpret_cast<const uint2*>(mix + HALF + c + 4 * q4);
+          const uint32_t mm[4] = {m1.x, m1.y, m2.x, m2.y};
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mm[e]));
+            const float2 f2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mm[2 + e]));
+            x1[2 * e] = left * x1[2 * e] + lam * f1.x; x1[2 * e + 1] = left * x1[2 * e + 1] + lam * f1.y;
+            x2[2 * e] = left * x2[2 * e] + lam * f2.x; x2[2 * e + 1] = left * x2[2 * e + 1] + lam * f2.y;
+          }
+        }
+        if (unit) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) { x1[e] *= inv[h]; x2[e] *= inv[h]; }
+        }
+        if (w) {
+          const float4 wa = reinterpret_cast<const float4*>(w + c)[q4], wb = reinterpret_cast<const float4*>(w + HALF + c)[q4];
+          x1[0] = x1[0] * inv[h] * wa.x; x1[1] = x1[1] * inv[h] * wa.y; x1[2] = x1[2] * inv[h] * wa.z; x1[3] = x1[3] * inv[h] * wa.w;
+          x2[0] = x2[0] * inv[h] * wb.x; x2[1] = x2[1] * inv[h] * wb.y; x2[2] = x2[2] * inv[h] * wb.z; x2[3] = x2[3] * inv[h] * wb.w;
+        }
+        float y1[4], y2[4];
+        if (rot) {
+          const float4 cv = cv4[q4], sv = sv4[q4];
+          const float cc[4] = {cv.x, cv.y, cv.z, cv.w}, ss4[4] = {sv.x, sv.y, sv.z, sv.w};
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            x1[e] = bf16_round(a[4 * q4 + e]);
-            x2[e] = bf16_round(b[4 * q4 + e]);
+            y1[e] = x1[e] * cc[e] - x2[e] * ss4[e];
+            y2[e] = x2[e] * cc[e] + x1[e] * ss4[e];
           }
-          if (bias) {
-            const float4 b1 = bias[c / 4 + q4], b2 = bias[HALF / 4 + c / 4 + q4];
-            x1[0] += b1.x; x1[1] += b1.y; x1[2] += b1.z; x1[3] += b1.w;
-            x2[0] += b2.x; x2[1] += b2.y; x2[2] += b2.z; x2[3] += b2.w;
-          }
-          if (mix) {
-            const float lam = r.v_lambda, rest = 1.f - r.v_lambda;
-            const uint2 m1 = *reinterpret_cast<const uint2*>(mix + c + 4 * q4), m2 = *reinterpret_cast<const uint2*>(mix + HALF + c + 4 * q4);
-            const uint32_t mm[4] = {m1.x, m1.y, m2.x, m2.y};
+        } else {
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mm[e]));
-              const float2 f2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mm[2 + e]));
-              x1[2 * e] = rest * x1[2 * e] + lam * f1.x; x1[2 * e + 1] = rest * x1[2 * e + 1] + lam * f1.y;
-              x2[2 * e] = rest * x2[2 * e] + lam * f2.x; x2[2 * e + 1] = rest * x2[2 * e + 1] + lam * f2.y;
-            }
-          }
-          if (unit && !w) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) { x1[e] *= inv; x2[e] *= inv; }
-          }
-          if (w) {
-            const float4 wa = w1[q4], wb = w2[q4];
-            x1[0] = x1[0] * inv * wa.x; x1[1] = x1[1] * inv * wa.y; x1[2] = x1[2] * inv * wa.z; x1[3] = x1[3] * inv * wa.w;
-            x2[0] = x2[0] * inv * wb.x; x2[1] = x2[1] * inv * wb.y; x2[2] = x2[2] * inv * wb.z; x2[3] = x2[3] * inv * wb.w;
-          }
-          float y1[4], y2[4];
-          if (rot) {
-            const float4 cv = cs[q4], sv = sn[q4];
-            const float cc[4] = {cv.x, cv.y, cv.z, cv.w}, ss4[4] = {sv.x, sv.y, sv.z, sv.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              y1[e] = x1[e] * cc[e] - x2[e] * ss4[e];
-              y2[e] = x2[e] * cc[e] + x1[e] * ss4[e];
-            }
-          } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) { y1[e] = x1[e]; y2[e] = x2[e]; }
-          }
-          o1[2 * q4] = pack2(y1[0], y1[1]); o1[2 * q4 + 1] = pack2(y1[2], y1[3]);
-          o2[2 * q4] = pack2(y2[0], y2[1]); o2[2 * q4 + 1] = pack2(y2[2], y2[3]);
+          for (int e = 0; e < 4; ++e) { y1[e] = x1[e]; y2[e] = x2[e]; }
         }
+        o1[2 * q4] = pack2(y1[0], y1[1]); o1[2 * q4 + 1] = pack2(y1[2], y1[3]);
+        o2[2 * q4] = pack2(y2[0], y2[1]); o2[2 * q4 + 1] = pack2(y2[2], y2[3]);
+      }
+      // out through shared memory: 32 bytes of each half of a row, four lanes a row
+      uint4* mine = reinterpret_cast<uint4*>(out_s + lane * kRopeRow);
+      mine[0] = make_uint4(o1[0], o1[1], o1[2], o1[3]);
+      mine[1] = make_uint4(o1[4], o1[5], o1[6], o1[7]);
+      mine[2] = make_uint4(o2[0], o2[1], o2[2], o2[3]);
+      mine[3] = make_uint4(o2[4], o2[5], o2[6], o2[7]);
+      __syncwarp();
+      const int col = (part & 1) * 8 + (part >> 1) * HALF + c;
+      const bool keeps = is_v && r.v_keep != nullptr;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint4 v1 = make_uint4(o1[4 * j], o1[4 * j + 1], o1[4 * j + 2], o1[4 * j + 3]);
-          const uint4 v2 = make_uint4(o2[4 * j], o2[4 * j + 1], o2[4 * j + 2], o2[4 * j + 3]);
-          if (dst != nullptr) {
-            reinterpret_cast<uint4*>(dst + c)[j] = v1;
-            reinterpret_cast<uint4*>(dst + HALF + c)[j] = v2;
-          }
-          if (keep != nullptr) {
-            reinterpret_cast<uint4*>(keep + c)[j] = v1;
-            reinterpret_cast<uint4*>(keep + HALF + c)[j] = v2;
-          }
+      for (int i = 0; i < 4; ++i) {
+        const int from = 8 * i + sub;
+        const uint4 v = *reinterpret_cast<const uint4*>(out_s + from * kRopeRow + part * 16);
+        __nv_bfloat16* to = reinterpret_cast<__nv_bfloat16*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(dst[h]), from));
+        if (to != nullptr) *reinterpret_cast<uint4*>(to + col) = v;
+        if (keeps) {
+          const int krow = __shfl_sync(0xffffffffu, live ? row : -1, from);
+          if (krow >= 0) *reinterpret_cast<uint4*>(r.v_keep + ((size_t)krow * r.n_kv_heads + kv_head) * D + col) = v;
         }
+      }
+      __syncwarp();
+    }
+  }
+  // columns behind q|k|v
+#pragma unroll 1
+  for (int h = 0; h < H; ++h) {
+    const int col0 = n0 + h * D;
+    if (col0 >= p.N || col0 / D < n_cached) continue;
+#pragma unroll 1
+    for (int c = 0; c < D && col0 + c < p.N; c += 32) {
+      uint32_t v[32];
+      __syncwarp();
+      tmem_ld32(t_row + h * D + c, v);
+      tmem_ld_wait();
+      if (live) {
+        __nv_bfloat16* yrow = reinterpret_cast<__nv_bfloat16*>(p.y) + (size_t)row * p.ldy + col0 + c;
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (col0 + c + j < p.N) yrow[j] = __float2bfloat16_rn(__uint_as_float(v[j]));
       }
     }
   }
 }
 
-// ROPE: the instantiation that carries mode 3's epilogue (it needs 231 registers where the plain epilogues need 94;
+// ROPE: the instantiation that carries mode 3's epilogue (it needs 168 registers, and more threads, where the plain epilogues need 156;
 // the plain products keep a kernel of their own).
 template <bool ROPE>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(ROPE ? kRopeThreads : kThreads, 1)
 gemm_umma2_kernel(Params p, const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap) {
   extern __shared__ char smem_raw[];
   __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
@@ -393,7 +438,7 @@ gemm_umma2_kernel(Params p, const __grid_constant__ CUtensorMap amap, const __gr
     }
     for (int b = 0; b < 2; ++b) {
       tma::mbar_init(&acc_full[b], 1);    // one commit per phase, delivered to both blocks
-      tma::mbar_init(&acc_empty[b], 8);   // the leader's: four epilogue warps of each block
+      tma::mbar_init(&acc_empty[b], ROPE ? 16 : 8);   // the leader's: the epilogue warps of both blocks
     }
     failed = 0;
     tma::fence_barrier_init();
@@ -471,7 +516,7 @@ gemm_umma2_kernel(Params p, const __grid_constant__ CUtensorMap amap, const __gr
       }
     }
   } else {
-    // ---- epilogue: warps 2..5 own TMEM lane quarters 2, 3, 0, 1 of their block ----
+    // ---- epilogue: warps 2..5 own TMEM lane quarters 2, 3, 0, 1 of their block (ROPE: its first head, warps 6..9 its second) ----
     const int quarter = warp & 3;
     int it = 0;
     for (int tile = first_tile; tile < n_tiles_total && !failed; tile += tile_step, ++it) {
@@ -487,7 +532,8 @@ gemm_umma2_kernel(Params p, const __grid_constant__ CUtensorMap amap, const __gr
       const int row = m0 + quarter * 32 + lane;
       const uint32_t t_row = tmem_base + ab * BN + ((uint32_t)(quarter * 32) << 16);
       if (ROPE) {
-        rope_epilogue(p, row, n0, t_row);
+        const int head = (warp - 2) >> 2;
+        rope_epilogue(p, row, n0 + head * 128, t_row + head * 128, smem + STAGES * kStage + (warp - 2) * kRopeWarp, lane);
       } else if (p.mode == 2) {
         __nv_bfloat16* yrow = reinterpret_cast<__nv_bfloat16*>(p.y) + (size_t)row * p.ldy + n0;
 #pragma unroll 1
@@ -676,12 +722,12 @@ static int pe::umma2::launch_pair(Params p, const void* x, long long ldx, const 
   int e = make_map_kblocks(&amap, x, K, M, ldx, BM, KBS);
   if (e == 0) e = make_map_kblocks(&bmap, w, K, w_rows, K, BNH, KBS);
   if (e != 0) return e < 0 ? e : PE_ERR_BAD_ARGUMENT;
-  const size_t smem = 1024 + (size_t)STAGES * kStage;
+  const size_t plain_smem = 1024 + (size_t)STAGES * kStage, rope_smem = plain_smem + 8 * kRopeWarp;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t ce = cudaFuncSetAttribute(gemm_umma2_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t ce = cudaFuncSetAttribute(gemm_umma2_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plain_smem);
     if (ce == cudaSuccess)
-      ce = cudaFuncSetAttribute(gemm_umma2_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      ce = cudaFuncSetAttribute(gemm_umma2_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rope_smem);
     if (ce != cudaSuccess) return (int)ce;
     attr_set = true;
   }
@@ -689,8 +735,8 @@ static int pe::umma2::launch_pair(Params p, const void* x, long long ldx, const 
   const int pairs = tiles < n_sms / 2 ? tiles : n_sms / 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem;
+  cfg.blockDim = dim3(p.mode == 3 ? kRopeThreads : kThreads);
+  cfg.dynamicSmemBytes = p.mode == 3 ? rope_smem : plain_smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
