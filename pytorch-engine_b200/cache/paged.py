@@ -42,16 +42,12 @@ class CacheView:
 
     @property
     def k_pages(self) -> torch.Tensor:
-        g = self.group
-        return g.storage[self.index, 0] if g.paired else g.storage[self.index]
+        return self.group.pages_of_entry(self.index)[0]
 
     @property
     def v_pages(self) -> torch.Tensor:
         """The values' pages; for a group whose values are read out of the key rows, the key pages themselves."""
-        g = self.group
-        if g.paired:
-            return g.storage[self.index, 1]
-        return g.storage[self.index] if g.v_storage is None else g.v_storage[self.index]
+        return self.group.pages_of_entry(self.index)[1]
 
     @property
     def page_table(self) -> torch.Tensor:
@@ -78,6 +74,19 @@ class CacheGroup:
     page_table: Optional[torch.Tensor] = None
     pages_of_slot: Dict[int, List[int]] = field(default_factory=dict)  # logical page -> physical (-1: released)
     state_tensors: Dict[str, torch.Tensor] = field(default_factory=dict)
+    entry_pages: Dict[int, Tuple[torch.Tensor, torch.Tensor]] = field(default_factory=dict)  # views made by pages_of_entry
+
+    def pages_of_entry(self, index: int) -> Tuple[torch.Tensor, torch.Tensor]:
+        """The entry's key pages and value pages: views of the storage, made once (a step asks several times a layer)."""
+        got = self.entry_pages.get(index)
+        if got is None:
+            if self.paired:
+                got = (self.storage[index, 0], self.storage[index, 1])
+            else:
+                keys = self.storage[index]
+                got = (keys, keys if self.v_storage is None else self.v_storage[index])
+            self.entry_pages[index] = got
+        return got
 
 
 class PagedCache:

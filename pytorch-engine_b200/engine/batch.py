@@ -28,10 +28,10 @@ class BufferPool:
         self._views: Dict[tuple, torch.Tensor] = {}   # (name, dtype, shape) -> view of the current buffer
 
     def get(self, name: str, shape: Sequence[int], dtype: torch.dtype) -> torch.Tensor:
-        shape = tuple(int(s) for s in shape)
-        view = self._views.get((name, dtype, shape))
+        view = self._views.get((name, dtype, shape)) if type(shape) is tuple else None
         if view is not None:
             return view
+        shape = tuple(int(s) for s in shape)
         numel = 1
         for s in shape:
             numel *= s

@@ -25,13 +25,14 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)   # tensors exist: CUDA is initialised
 
 
 def _stream() -> int:
     """The current CUDA stream's handle (the raw query is several times cheaper than building a
     ``torch.cuda.Stream`` object, and this runs once per launch)."""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_current_device())
     return torch.cuda.current_stream().cuda_stream
 
 

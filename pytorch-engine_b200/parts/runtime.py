@@ -25,6 +25,12 @@ STATUS_MESSAGES = {
 }
 
 
+# What ``torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction`` reads and sets, without its parsing: (allowed, split-K
+# allowed).  Every library product asks, and a prompt's step has three of them a layer.
+_reduced_reductions = torch._C._get_cublas_allow_bf16_reduced_precision_reduction
+_set_reduced_reductions = torch._C._set_cublas_allow_bf16_reduced_precision_reduction
+
+
 class PendingTokens:
     """Tokens (and the status word) on their way to the host; ``result()`` waits and returns the tokens,
     raising if a kernel reported an error."""
@@ -238,9 +244,9 @@ class Runtime:
                 if prev:
                     torch.backends.cuda.matmul.allow_tf32 = True
         # library product in bfloat16: keep its reductions in float32
-        prev = torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction
-        if prev:
-            torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
+        prev = _reduced_reductions()
+        if prev[0]:
+            _set_reduced_reductions(False, True)
         try:
             if out_dtype is not None and out_dtype != x.dtype:
                 y = torch.mm(x, weight.t(), out_dtype=out_dtype)
@@ -250,5 +256,5 @@ class Runtime:
                 return y
             return torch.mm(x, weight.t(), out=out) if out is not None else torch.mm(x, weight.t())
         finally:
-            if prev:
-                torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = True
+            if prev[0]:
+                _set_reduced_reductions(*prev)
