@@ -133,6 +133,11 @@ int pe_gemm_smallm_glu(const void* x, long long ldx, const void* w, void* y, lon
     cudaStream_t stream);
 int pe_gemm_smallm(const void* x, long long ldx, const void* w, void* y, long long ldy, int M, int N, int K,
     int out_f32, int pair_offset, int n_sms, cudaStream_t stream);
+int pe_gemm_smallm_scaled(const void* x, long long ldx, const void* w, void* y, long long ldy, int M, int N, int K, int pair_offset,
+    int kind, float limit, float alpha, const float* bias, const float* ss, int ss_parts, int dim, float eps, int n_sms,
+    cudaStream_t stream);
+int pe_gemm_smallm_residual(const void* x, long long ldx, const void* w, float* rows, long long rows_ld, int M, int N, int K,
+    const float* next_w, void* next_x, long long next_ld, float* next_ss, int n_sms, cudaStream_t stream);
 int pe_gemm_smallm_grouped(const void* x, long long ldx, long long x_group_stride, int groups, int group_rows,
     const void* w, void* y, long long ldy, int M, int K, int out_f32, int n_sms, cudaStream_t stream);
 

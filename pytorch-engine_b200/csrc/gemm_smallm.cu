@@ -1,10 +1,10 @@
-// y[M, N] = x[M, K] . W[N, K]^T for a handful of rows (M <= 16): the decode-step matrix products.
+// y[M, N] = x[M, K] . W[N, K]^T for a handful of rows (M <= 16, in a chain 32): the decode-step matrix products.
 // bfloat16 operands, float32 accumulation on the tensor cores (mma.sync m16n8k16), output bfloat16 or
 // float32, optionally with the SwiGLU gate fused into the epilogue.
 //
 // With so few rows the product is a stream of the weight matrix through the SMs; everything here
 // serves that stream.  The roles of the MMA operands are swapped: 16 weight rows are the MMA's M
-// dimension, the (up to 8) activation rows are its N dimension.  A warp owns 16 weight rows and a
+// dimension, 8 activation rows (one to four groups of them) are its N dimension.  A warp owns 16 weight rows and a
 // slice of K and loads its fragments straight from global memory with 16-byte loads: lane (g, t)
 // reads elements [8t, 8t+8) of rows g and g+8 of every 32-wide k block.  The contraction index
 // inside a block is permuted accordingly (the same permutation for both operands, so the sum is
@@ -35,6 +35,13 @@ struct Args {
   // in one launch.  0: one input for all rows.
   int group_rows; long long x_group_stride;
   GluEpilogue glu;             // PAIR: what is done with the two sums
+  // CHAIN 1: the input is a residual stream's rows times a norm's weight; outputs are multiplied by rsqrt(mean square + eps) of
+  // their row, whose sum of squares lies in `ss_parts` parts of eight rows each (see CHAIN 2).
+  const float* ss; int ss_parts; float ss_scale, eps;
+  // CHAIN 2: outputs are added to the stream ([M, N], stream_ld apart) and not stored; the new rows times `next_w` (the norm
+  // behind it; null: nobody reads them) go to next_x in bfloat16, and a block leaves its 16 columns' sums of squares in next_ss.
+  float* stream; long long stream_ld;
+  const float* next_w; __nv_bfloat16* next_x; long long next_ld; float* next_ss;
 };
 
 __device__ __forceinline__ uint4 ldg_stream(const uint4* p) {
@@ -52,6 +59,16 @@ __device__ __forceinline__ uint4 ldg_cached(const uint4* p) {
   asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ float4 ldg_f4(const float* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ldg_f1(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];\n" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
@@ -62,16 +79,22 @@ template <typename T> __device__ __forceinline__ void store_out(T* p, float v);
 template <> __device__ __forceinline__ void store_out<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void store_out<__nv_bfloat16>(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 
-// NT: 8-row groups of activations (1: M <= 8, 2: M <= 16).  GLU != 0: two weight-row blocks per warp
+// NT: 8-row groups of activations (1: M <= 8, 2: M <= 16, 4: M <= 32).  GLU != 0: two weight-row blocks per warp
 // (gate and up), combined as silu(gate) * up (1) or as Args::glu says (2; an instantiation of its own, so that the
 // usual one carries nothing of it).  WARPS: warps per block = K slices.  U: k blocks per batch
 // of loads.
 // Registers are capped at 128 per thread for M <= 8 so that 16 warps fit on an SM: what limits this
 // kernel is how many bytes its SM has in flight.  For M <= 16 that cap would spill.
-template <int NT, int GLU, int WARPS, int U, typename OutT>
-__global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 16 / WARPS : 1) gemm_smallm_kernel(Args a) {
+// CHAIN (M <= 32): a pre-norm block's products without kernels for its norms.  An RMSNorm scales a row by one number and a column
+// by its weight; the number can wait until after the product, so the product that writes into the stream leaves the stream times
+// the next norm's weight and the squares' sums, and the product behind reads that as its input and scales what comes out.  One
+// rounding to bfloat16 either way, and the delta is added in float32 (it used to be rounded first).
+template <int NT, int GLU, int WARPS, int U, typename OutT, int CHAIN = 0>
+__global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 16 / WARPS : NT == 4 ? 12 / WARPS : 1) gemm_smallm_kernel(Args a) {
   constexpr bool PAIR = GLU != 0;
   __shared__ float red[WARPS][(PAIR ? 2 : 1) * NT][4][32];
+  __shared__ __align__(16) float squares[CHAIN == 1 ? WARPS : 1][8 * NT];
+  constexpr int SSL = CHAIN == 1 ? 2 : 1;      // 16-byte loads of the squares' sums that a thread has in flight
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int n0 = blockIdx.x * 16;
@@ -156,8 +179,30 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 16 / WARPS : 1) gemm_sma
   // slower: 4.37 and 4.67 ms against 4.34 ms for a decode step of 8 sequences.)
   Batch b0, b1;
   load_w(b0, kb_lo);
+  float next_w[2] = {0.f, 0.f};
+  if (CHAIN == 2 && warp < NT && a.next_w) {      // a norm's weight never changes
+    if (n0 + g < a.N) next_w[0] = a.next_w[n0 + g];
+    if (n0 + g + 8 < a.N) next_w[1] = a.next_w[n0 + g + 8];
+  }
   pdl_wait_block();
   load_x(b0, kb_lo);
+  // the parts of the rows' sums of squares: a thread's are all of the same four rows
+  float4 part[SSL];
+  if (CHAIN == 1) {
+#pragma unroll
+    for (int i = 0; i < SSL; ++i) {
+      const int at = threadIdx.x + i * WARPS * 32;
+      part[i] = at < a.ss_parts * (2 * NT) ? ldg_f4(a.ss + 4 * at) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  float old[4] = {0.f, 0.f, 0.f, 0.f};
+  if (CHAIN == 2 && warp < NT) {      // the rows of the first group that this warp finishes
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int col = n0 + g + ((e >= 2) ? 8 : 0), m = warp * 8 + 2 * t + (e & 1);
+      if (col < a.N && m < a.M) old[e] = ldg_f1(a.stream + (size_t)m * a.stream_ld + col);
+    }
+  }
   for (int kb = kb_lo; kb < kb_hi; kb += 2 * U) {
     load(b1, kb + U);
     fold(b0);
@@ -165,55 +210,126 @@ __global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 16 / WARPS : 1) gemm_sma
     fold(b1);
   }
   pdl_launch_dependents();  // the stream of weights is done: the next kernel may start its own
-  // sum the K slices in warp order
+  if (CHAIN == 1) {
+    float4 sum = part[0];
+#pragma unroll
+    for (int i = 1; i < SSL; ++i) { sum.x += part[i].x; sum.y += part[i].y; sum.z += part[i].z; sum.w += part[i].w; }
+    for (int at = threadIdx.x + SSL * WARPS * 32; at < a.ss_parts * (2 * NT); at += WARPS * 32) {
+      const float4 v = ldg_f4(a.ss + 4 * at);
+      sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+    }
+#pragma unroll
+    for (int o = 2 * NT; o < 32; o <<= 1) {
+      sum.x += __shfl_xor_sync(0xffffffffu, sum.x, o); sum.y += __shfl_xor_sync(0xffffffffu, sum.y, o);
+      sum.z += __shfl_xor_sync(0xffffffffu, sum.z, o); sum.w += __shfl_xor_sync(0xffffffffu, sum.w, o);
+    }
+    if (lane < 2 * NT) *reinterpret_cast<float4*>(&squares[warp][4 * lane]) = sum;
+    if (WARPS == 1) __syncwarp();
+  }
+  // sum the K slices in warp order; a group of eight rows a warp
+  constexpr int P = PAIR ? 2 : 1;
   if (WARPS > 1) {
 #pragma unroll
-    for (int i = 0; i < (PAIR ? 2 : 1) * NT; ++i)
+    for (int i = 0; i < P * NT; ++i)
 #pragma unroll
       for (int e = 0; e < 4; ++e) red[warp][i][e][lane] = c[i][e];
     __syncthreads();
-    if (warp != 0) return;
+  }
+  // v[0]: the group's sums, v[1] those of the paired weight rows.  Element e: weight row n0 + g (+8 for e >= 2), activation row
+  // n * 8 + 2t + (e & 1)
+  OutT* y = reinterpret_cast<OutT*>(a.y);
+  auto finish = [&](int n, float (&v)[P][4]) {
+    if (CHAIN == 1) {
 #pragma unroll
-    for (int i = 0; i < (PAIR ? 2 : 1) * NT; ++i)
+      for (int i = 0; i < 2; ++i) {
+        float total = 0.f;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) total += squares[w][n * 8 + 2 * t + i];
+        const float inv = rsqrtf(total * a.ss_scale + a.eps);
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+          v[k][i] *= inv;
+          v[k][2 + i] *= inv;
+        }
+      }
+    }
+    if constexpr (CHAIN == 2) {
+      float ss[2] = {0.f, 0.f};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        float s = red[0][i][e][lane];
-#pragma unroll
-        for (int w = 1; w < WARPS; ++w) s += red[w][i][e][lane];
-        c[i][e] = s;
+        const int col = n0 + g + ((e >= 2) ? 8 : 0), m = n * 8 + 2 * t + (e & 1);
+        if (col >= a.N || m >= a.M) continue;
+        const float before = n == warp ? old[e] : ldg_f1(a.stream + (size_t)m * a.stream_ld + col);
+        const float h = before + v[0][e];
+        a.stream[(size_t)m * a.stream_ld + col] = h;
+        if (a.next_w) {
+          const float w = WARPS >= NT ? next_w[e >> 1] : a.next_w[col];
+          a.next_x[(size_t)m * a.next_ld + col] = __float2bfloat16_rn(h * w);
+        }
+        ss[e & 1] = fmaf(h, h, ss[e & 1]);
       }
-  }
-  // c[n][e]: weight row n0 + g (+8 for e >= 2), activation row n*8 + 2t + (e & 1)
-  OutT* y = reinterpret_cast<OutT*>(a.y);
+      if (a.next_w) {
 #pragma unroll
-  for (int n = 0; n < NT; ++n)
+        for (int o = 4; o < 32; o <<= 1) {
+          ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], o);
+          ss[1] += __shfl_xor_sync(0xffffffffu, ss[1], o);
+        }
+        if (g == 0) *reinterpret_cast<float2*>(a.next_ss + (size_t)blockIdx.x * (8 * NT) + n * 8 + 2 * t) = make_float2(ss[0], ss[1]);
+      }
+    } else {
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int col = n0 + g + ((e >= 2) ? 8 : 0);
       const int m = n * 8 + 2 * t + (e & 1);
       if (col >= a.N || m >= a.M) continue;
-      float v = c[n][e];
+      float r = v[0][e];
       if (PAIR) {
-        float up = c[NT + n][e];
+        float up = v[P - 1][e];
         if (GLU == 1) {
-          v = sizeof(OutT) == 2 ? silu_mul_fast(v, up) : v / (1.0f + expf(-v)) * up;   // exact for a float32 result
+          r = sizeof(OutT) == 2 ? silu_mul_fast(r, up) : r / (1.0f + expf(-r)) * up;   // exact for a float32 result
         } else {
           if (a.glu.bias) {
-            v += a.glu.bias[col];
+            r += a.glu.bias[col];
             up += a.glu.bias[a.N + col];
           }
-          v = sizeof(OutT) == 2 ? glu_fast(a.glu, v, up) : glu_exact(a.glu.kind, v, up, a.glu.limit, a.glu.alpha);
+          r = sizeof(OutT) == 2 ? glu_fast(a.glu, r, up) : glu_exact(a.glu.kind, r, up, a.glu.limit, a.glu.alpha);
         }
       }
-      store_out<OutT>(y + (size_t)m * a.ldy + col, v);
+      store_out<OutT>(y + (size_t)m * a.ldy + col, r);
     }
+    }
+  };
+  if constexpr (WARPS == 1) {
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      float v[P][4];
+#pragma unroll
+      for (int k = 0; k < P; ++k)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[k][e] = c[k * NT + n][e];
+      finish(n, v);
+    }
+  } else {
+    for (int n = warp; n < NT; n += WARPS) {
+      float v[P][4];
+#pragma unroll
+      for (int k = 0; k < P; ++k)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          v[k][e] = red[0][k * NT + n][e][lane];
+#pragma unroll
+          for (int w = 1; w < WARPS; ++w) v[k][e] += red[w][k * NT + n][e][lane];
+        }
+      finish(n, v);
+    }
+  }
 }
 
-template <int NT, int GLU, typename OutT>
+template <int NT, int GLU, typename OutT, int CHAIN = 0>
 static int launch(const Args& a, int n_sms, cudaStream_t stream) {
   const int blocks = (a.N + 15) / 16;
   const int kblocks = (a.K + 31) / 32;
-  constexpr int U = GLU ? 2 : 4;
+  constexpr int U = (GLU ? 2 : 4) / (NT == 4 ? 2 : 1);
   // K slices per block of 16 weight rows: enough warps in flight over the whole GPU to cover the
   // memory latency, but at least two batches of k blocks per warp.  An SM holds 16 warps of the
   // M <= 8 kernels (128 registers) and 12 of the M <= 16 kernels (up to 168 registers) as long as their
@@ -227,10 +343,10 @@ static int launch(const Args& a, int n_sms, cudaStream_t stream) {
   // (6144 x 4096 at 8 rows: 11.5 us with 8 warps a block, 1.3 waves; 10.2 us with 4).
   if (warps > 1 && (long long)blocks * warps > slots && (long long)blocks * warps * 2 <= slots * 3) warps /= 2;
   switch (warps) {
-    case 1: pe::launch(gemm_smallm_kernel<NT, GLU, 1, U, OutT>, blocks, 32, 0, stream, a); break;
-    case 2: pe::launch(gemm_smallm_kernel<NT, GLU, 2, U, OutT>, blocks, 64, 0, stream, a); break;
-    case 4: pe::launch(gemm_smallm_kernel<NT, GLU, 4, U, OutT>, blocks, 128, 0, stream, a); break;
-    default: pe::launch(gemm_smallm_kernel<NT, GLU, 8, U, OutT>, blocks, 256, 0, stream, a); break;
+    case 1: pe::launch(gemm_smallm_kernel<NT, GLU, 1, U, OutT, CHAIN>, blocks, 32, 0, stream, a); break;
+    case 2: pe::launch(gemm_smallm_kernel<NT, GLU, 2, U, OutT, CHAIN>, blocks, 64, 0, stream, a); break;
+    case 4: pe::launch(gemm_smallm_kernel<NT, GLU, 4, U, OutT, CHAIN>, blocks, 128, 0, stream, a); break;
+    default: pe::launch(gemm_smallm_kernel<NT, GLU, 8, U, OutT, CHAIN>, blocks, 256, 0, stream, a); break;
   }
   PE_LAUNCH_CHECK();
   return PE_OK;
@@ -259,7 +375,7 @@ extern "C" int pe_gemm_smallm_glu(const void* x, long long ldx, const void* w, v
   if (kind < 1 || kind > 3 || (pair_offset <= 0 && bias)) return PE_ERR_BAD_ARGUMENT;
   if (!pe_gemm_smallm_supported(M, N, K)) return PE_ERR_UNSUPPORTED_SIZE;
   if (((uintptr_t)x % 16) || ((uintptr_t)w % 16) || (ldx * 2) % 16) return PE_ERR_BAD_ARGUMENT;
-  pe::smallm::Args a;
+  pe::smallm::Args a = {};
   a.x = (const __nv_bfloat16*)x; a.ldx = ldx; a.w = (const __nv_bfloat16*)w; a.y = y; a.ldy = ldy;
   a.M = M; a.N = N; a.K = K; a.pair_offset = pair_offset;
   a.glu = pe::GluEpilogue{kind, limit, alpha, bias};
@@ -287,7 +403,7 @@ extern "C" int pe_gemm_smallm_grouped(const void* x, long long ldx, long long x_
   const int N = groups * group_rows;
   if (!pe_gemm_smallm_supported(M, N, K)) return PE_ERR_UNSUPPORTED_SIZE;
   if (((uintptr_t)x % 16) || ((uintptr_t)w % 16) || (ldx * 2) % 16 || (x_group_stride * 2) % 16) return PE_ERR_BAD_ARGUMENT;
-  pe::smallm::Args a;
+  pe::smallm::Args a = {};
   a.x = (const __nv_bfloat16*)x; a.ldx = ldx; a.w = (const __nv_bfloat16*)w; a.y = y; a.ldy = ldy;
   a.M = M; a.N = N; a.K = K; a.pair_offset = 0;
   a.glu = pe::GluEpilogue{1, 0.f, 1.f, nullptr};
@@ -296,4 +412,49 @@ extern "C" int pe_gemm_smallm_grouped(const void* x, long long ldx, long long x_
   if (n_sms <= 0) n_sms = pe::kSMs;
   if (M <= 8) return out_f32 ? launch<1, 0, float>(a, n_sms, stream) : launch<1, 0, __nv_bfloat16>(a, n_sms, stream);
   return out_f32 ? launch<2, 0, float>(a, n_sms, stream) : launch<2, 0, __nv_bfloat16>(a, n_sms, stream);
+}
+
+// Up to 32 rows of a pre-norm block's products without kernels for its norms (CHAIN above).
+// pe_gemm_smallm_scaled: y = (x . W^T) * rsqrt(sum of squares / dim + eps) of the row, bfloat16; with pair_offset > 0 the scaled
+// gate and up sums go through the activation as in pe_gemm_smallm_glu.  ss: [ss_parts, 8] float32, 16-byte aligned.
+extern "C" int pe_gemm_smallm_scaled(const void* x, long long ldx, const void* w, void* y, long long ldy, int M, int N, int K,
+                                     int pair_offset, int kind, float limit, float alpha, const float* bias, const float* ss,
+                                     int ss_parts, int dim, float eps, int n_sms, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return PE_OK;
+  if (kind < 1 || kind > 3 || (pair_offset <= 0 && bias) || ss == nullptr || ss_parts <= 0 || dim <= 0) return PE_ERR_BAD_ARGUMENT;
+  if (M > 32 || !pe_gemm_smallm_supported(1, N, K)) return PE_ERR_UNSUPPORTED_SIZE;
+  if (((uintptr_t)x % 16) || ((uintptr_t)w % 16) || (ldx * 2) % 16 || ((uintptr_t)ss % 16)) return PE_ERR_BAD_ARGUMENT;
+  pe::smallm::Args a = {};
+  a.x = (const __nv_bfloat16*)x; a.ldx = ldx; a.w = (const __nv_bfloat16*)w; a.y = y; a.ldy = ldy;
+  a.M = M; a.N = N; a.K = K; a.pair_offset = pair_offset;
+  a.glu = pe::GluEpilogue{kind, limit, alpha, bias};
+  a.ss = ss; a.ss_parts = ss_parts; a.ss_scale = 1.f / (float)dim; a.eps = eps;
+  using namespace pe::smallm;
+  if (n_sms <= 0) n_sms = pe::kSMs;
+  auto go = [&](auto nt) -> int {
+    constexpr int NT = decltype(nt)::value;
+    if (pair_offset <= 0) return launch<NT, 0, __nv_bfloat16, 1>(a, n_sms, stream);
+    if (kind == 1 && bias == nullptr) return launch<NT, 1, __nv_bfloat16, 1>(a, n_sms, stream);
+    return launch<NT, 2, __nv_bfloat16, 1>(a, n_sms, stream);
+  };
+  return M <= 8 ? go(std::integral_constant<int, 1>()) : M <= 16 ? go(std::integral_constant<int, 2>()) : go(std::integral_constant<int, 4>());
+}
+
+// pe_gemm_smallm_residual: stream += x . W^T (float32 [M, N], rows stream_ld apart), and with next_w (float32 [N]) next_x =
+// stream * next_w (bfloat16, rows next_ld apart) and next_ss [(N + 15) / 16, 8] = the parts of the new rows' sums of squares.
+extern "C" int pe_gemm_smallm_residual(const void* x, long long ldx, const void* w, float* rows, long long rows_ld, int M, int N, int K,
+                                       const float* next_w, void* next_x, long long next_ld, float* next_ss, int n_sms, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return PE_OK;
+  if (M > 32 || !pe_gemm_smallm_supported(1, N, K)) return PE_ERR_UNSUPPORTED_SIZE;
+  if (((uintptr_t)x % 16) || ((uintptr_t)w % 16) || (ldx * 2) % 16 || ((uintptr_t)next_ss % 8)) return PE_ERR_BAD_ARGUMENT;
+  if (rows == nullptr || (next_w != nullptr && (next_x == nullptr || next_ss == nullptr))) return PE_ERR_BAD_ARGUMENT;
+  pe::smallm::Args a = {};
+  a.x = (const __nv_bfloat16*)x; a.ldx = ldx; a.w = (const __nv_bfloat16*)w;
+  a.M = M; a.N = N; a.K = K;
+  a.glu = pe::GluEpilogue{1, 0.f, 1.f, nullptr};
+  a.stream = rows; a.stream_ld = rows_ld; a.next_w = next_w; a.next_x = (__nv_bfloat16*)next_x; a.next_ld = next_ld; a.next_ss = next_ss;
+  using namespace pe::smallm;
+  if (n_sms <= 0) n_sms = pe::kSMs;
+  return M <= 8 ? launch<1, 0, __nv_bfloat16, 2>(a, n_sms, stream) : M <= 16 ? launch<2, 0, __nv_bfloat16, 2>(a, n_sms, stream)
+                                                                             : launch<4, 0, __nv_bfloat16, 2>(a, n_sms, stream);
 }

@@ -44,6 +44,10 @@ class DecoderModel:
         self.final_norm = _build_part("norm", plan.final_norm, weights, runtime)
         self.head = _build_part("head", plan.head, weights, runtime)
         runtime.forget_adopted()
+        # per run: the norm that reads the stream next, where it is one that can ride in the products around it
+        firsts = [getattr(self.blocks[run.block], "mixer_norm", None) if hasattr(self.blocks[run.block], "chains") else None
+                  for run in plan.order]
+        self.following_norms = [n if getattr(n, "chains", False) else None for n in firsts[1:]] + [None]
 
     def graph_safe(self) -> bool:
         """Whether a step may be recorded into a CUDA graph: every part must say so itself
@@ -115,9 +119,10 @@ class DecoderModel:
             ctx.embedding_output.copy_(stream)
         ctx.stream_copy = None    # a copy of the stream in the run dtype, if a block has left one (post-norm blocks do)
         pending = None
-        for run in self.plan.order:
+        for run, following in zip(self.plan.order, self.following_norms):
             view = self._view(cache, run)
             block = self.blocks[run.block]
+            ctx.following_norm = following
             if run.writes_cache:
                 pending = block.forward(stream, pending, ctx, view)
             else:

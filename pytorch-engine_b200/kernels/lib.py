@@ -105,6 +105,8 @@ _SIGNATURES = {
     "pe_attention_mma_dims_supported": [I, I, I, I],
     "pe_attention_mma_gated": [I, P, L, P, L, I, I, I, I, I, I, F, I, I, I, I, I, I, I, P, P, I, P, L, P, P, P, P, I, I, P, P, P, I, I, I,
                                P, P],
+    "pe_gemm_smallm_scaled": [P, L, P, P, L, I, I, I, I, I, F, F, P, P, I, I, F, I, P],
+    "pe_gemm_smallm_residual": [P, L, P, P, L, I, I, I, P, P, L, P, I, P],
     "pe_attention_umma_dims_supported": [I, I, I, I],
     "pe_attention_umma_prefill_gated": [P, L, L, P, L, I, I, I, I, I, I, F, I, I, P, P, I, P, L, P, P, P, P, I, I, P, P, I, P, P, P],
     "pe_attention_umma_prefill_parts": [P, L, L, P, L, I, I, I, I, I, I, F, I, I, P, P, I, P, L, P, P, P, P, I, I, P, P, I, P, I, P, P, P],

@@ -475,6 +475,17 @@ def gemm_smallm_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
             and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
 
 
+def gemm_smallm_chained(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """``gemm_smallm_supported`` for the products of a chain, which take up to 32 rows."""
+    return (x.dtype == torch.bfloat16 and x.dim() == 2 and x.shape[0] <= 32 and x.stride(1) == 1 and x.stride(0) % 8 == 0
+            and x.data_ptr() % 16 == 0 and gemm_smallm_weight(weight))
+
+
+def gemm_smallm_weight(weight: torch.Tensor) -> bool:
+    """The part of ``gemm_smallm_supported`` that is the weight's."""
+    return weight.dtype == torch.bfloat16 and weight.is_contiguous() and weight.shape[1] % 8 == 0 and weight.data_ptr() % 16 == 0
+
+
 def gemm_smallm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, pair_offset: int = 0, glu=None) -> None:
     """``out[M, N] = x @ weight^T`` (out bfloat16 or float32).  With ``pair_offset`` = I the weight holds
     gate rows then up rows and ``out[M, I] = silu(x @ gate^T) * (x @ up^T)``, or another activation of the two with
@@ -491,6 +502,46 @@ def gemm_smallm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, pair_o
     _count(1)
 
 
+def chain_rows(rows: int) -> int:
+    """Columns of the squares' parts that ``gemm_smallm_residual`` leaves for so many rows: 8, 16 or 32."""
+    return 8 if rows <= 8 else 16 if rows <= 16 else 32
+
+
+def gemm_smallm_scaled(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, squares: torch.Tensor, eps: float,
+                       pair_offset: int = 0, glu=None) -> None:
+    """``gemm_smallm`` for up to 32 rows of a residual stream times a norm's weight, whose norm's number is still to come:
+    outputs (before the activation) times ``rsqrt(sum of squares / K + eps)``, ``squares`` ``[parts, chain_rows]`` as
+    ``gemm_smallm_residual`` leaves it.  ``out`` bfloat16."""
+    _need(gemm_smallm_chained(x, weight), "gemm_smallm_scaled: needs bfloat16, M <= 32, K % 8 == 0, contiguous rows")
+    _need(out.stride(-1) == 1 and out.dtype == torch.bfloat16, "gemm_smallm_scaled: out bfloat16")
+    _need(squares.dtype == torch.float32 and squares.is_contiguous() and squares.shape[-1] == chain_rows(x.shape[0]), "gemm_smallm_scaled: squares [parts, chain_rows] float32")
+    m, k = x.shape
+    n = out.shape[1]
+    _need(weight.shape[1] == k and weight.shape[0] == (2 * n if pair_offset else n) and out.shape[0] == m and pair_offset in (0, n),
+          "gemm_smallm_scaled: shapes do not match")
+    check(library().pe_gemm_smallm_scaled(_ptr(x), x.stride(0), _ptr(weight), _ptr(out), out.stride(0), m, n, k, pair_offset,
+                                          *_glu_args(glu, n), _ptr(squares), squares.shape[0], k, float(eps), sm_count(x.device),
+                                          _stream()), "gemm_smallm_scaled")
+    _count(1)
+
+
+def gemm_smallm_residual(x: torch.Tensor, weight: torch.Tensor, stream: torch.Tensor, next_weight: Optional[torch.Tensor] = None,
+                         next_x: Optional[torch.Tensor] = None, squares: Optional[torch.Tensor] = None) -> None:
+    """``stream += x @ weight^T`` for up to 32 rows (float32 stream ``[M, N]``); with ``next_weight`` (a norm's, float32)
+    ``next_x = stream * next_weight`` in bfloat16 and ``squares [(N + 15) // 16, chain_rows]`` the parts of its rows' sums of squares."""
+    _need(gemm_smallm_chained(x, weight), "gemm_smallm_residual: needs bfloat16, M <= 32, K % 8 == 0, contiguous rows")
+    m, k = x.shape
+    n = weight.shape[0]
+    _need(stream.dtype == torch.float32 and stream.stride(-1) == 1 and tuple(stream.shape) == (m, n) and weight.shape[1] == k,
+          "gemm_smallm_residual: stream float32 [M, N]")
+    if next_weight is not None:
+        _need(next_weight.dtype == torch.float32 and next_weight.is_contiguous() and next_weight.numel() == n
+              and next_x.dtype == torch.bfloat16 and next_x.stride(-1) == 1 and tuple(next_x.shape) == (m, n)
+              and squares.dtype == torch.float32 and squares.is_contiguous() and tuple(squares.shape) == ((n + 15) // 16, chain_rows(m)),
+              "gemm_smallm_residual: the next norm's weight, input and squares")
+    check(library().pe_gemm_smallm_residual(_ptr(x), x.stride(0), _ptr(weight), _ptr(stream), stream.stride(0), m, n, k,
+                                            _ptr(next_weight), _ptr(next_x), 0 if next_x is None else next_x.stride(0), _ptr(squares),
+                                            sm_count(x.device), _stream()), "gemm_smallm_residual")
     _count(1)
 
 

@@ -190,8 +190,26 @@ class GQAttention:
             self.use_umma_prefill = not self.keep_first and ops.attention_umma_dims_supported(*dims)
         self.generic_attention = bool(getattr(runtime, "generic_attention", False))   # comparisons: the general kernels only
 
-    def forward(self, x: torch.Tensor, ctx, view, writes_cache: bool = True) -> torch.Tensor:
+    def chains(self) -> bool:
+        """Whether ``forward`` takes a ``residual`` (parts/block.py, PreNormBlock)."""
+        return not self.general and ops.gemm_smallm_weight(self.qkv) and ops.gemm_smallm_weight(self.o_proj)
+
+    def forward(self, x, ctx, view, writes_cache: bool = True, residual=None):
+        """``x``: the normed rows; with ``residual`` (few rows) they may be ``ChainedRows``, and the output projection goes where
+        it says."""
         rt = self.runtime
+        if residual is not None:
+            rows = getattr(x, "x", x)
+            n = rows.shape[0]
+            qkv = ctx.buffer("attn.qkv", (n, self.qkv_dim), rt.dtype)
+            if rows is x:
+                rt.linear(x, self.qkv, out=qkv)
+            else:
+                ops.gemm_smallm_scaled(rows, self.qkv, qkv, x.squares, x.norm.eps)
+            out = ctx.buffer("attn.out", (n, self.n_heads * self.head_dim), rt.dtype)
+            self.norm_rotate_append(qkv, n, ctx, view, writes_cache)
+            self.attend(qkv, out, ctx, view)
+            return residual.add_product(out, self.o_proj)
         n = x.shape[0]
         qkv = ctx.buffer("attn.qkv", (n, self.qkv_dim), rt.dtype)
         where = (ctx.token_seq, ctx.token_pos, ctx.seq_slot, ctx.seq_qstart, view.page_table, view.num_pages,

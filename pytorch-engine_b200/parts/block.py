@@ -72,6 +72,36 @@ class StreamsDelta:
         self.write_and_read(self.ones, None, stream)
 
 
+class ChainedRows:
+    """What a pre-norm block hands on where its last product has added its output to the stream itself (few rows, csrc/gemm_smallm.cu):
+    ``x``, the stream times the weight of the norm behind it in the run dtype, and ``squares``, the parts of the rows' sums of
+    squares, from which the next product takes the norm's number.  Nothing is left to be added."""
+
+    def __init__(self, norm, x: Optional[torch.Tensor], squares: Optional[torch.Tensor]) -> None:
+        self.norm, self.x, self.squares = norm, x, squares
+
+    def settle(self, stream: torch.Tensor) -> None:
+        pass
+
+
+class Residual:
+    """Where a part's last product goes in a step without kernels for the norms: into ``stream``, and on to ``norm`` (None: nobody
+    reads it in this form)."""
+
+    def __init__(self, stream: torch.Tensor, norm, ctx) -> None:
+        self.stream, self.norm, self.ctx = stream, norm, ctx
+
+    def add_product(self, x: torch.Tensor, weight: torch.Tensor) -> ChainedRows:
+        n, hidden = self.stream.shape
+        if self.norm is None:
+            ops.gemm_smallm_residual(x, weight, self.stream)
+            return ChainedRows(None, None, None)
+        rows = self.ctx.buffer("block.chained", (n, hidden), x.dtype)
+        squares = self.ctx.buffer("block.squares", ((hidden + 15) // 16, ops.chain_rows(n)), torch.float32)
+        ops.gemm_smallm_residual(x, weight, self.stream, self.norm.weight, rows, squares)
+        return ChainedRows(self.norm, rows, squares)
+
+
 def settle_pending(stream: torch.Tensor, pending) -> None:
     """Add what the block before left to be added (nothing, one delta, several scaled ones, one behind a norm)."""
     if pending is None:
@@ -98,6 +128,13 @@ class PreNormBlock:
         self.ffn = parts["ffn"]
         self.name = spec.name
 
+    def chains(self, n_tokens: int, width: int) -> bool:
+        """Whether a step of so many tokens runs without kernels for the norms: few rows, plain RMSNorms, parts that know how, and
+        all products on csrc/gemm_smallm.cu."""
+        rt = self.runtime
+        return (rt.takes_chained(n_tokens, width) and all(getattr(n, "chains", False) for n in (self.mixer_norm, self.ffn_norm))
+                and all(getattr(p, "chains", None) is not None and p.chains() for p in (self.mixer, self.ffn)))
+
     def forward(self, stream: torch.Tensor, pending: Optional[torch.Tensor], ctx, view, writes_cache: bool = True):
         """``stream``: float32 residual ``[N, hidden]``, updated in place; ``pending``: the previous
         block's delta that is not added yet (or None).  Returns this block's own pending delta."""
@@ -105,14 +142,19 @@ class PreNormBlock:
         if isinstance(pending, NormedDelta):
             pending.settle(stream)
             pending = None
-        normed = ctx.buffer("block.normed", tuple(stream.shape), rt.dtype)
-        self.mixer_norm.add_forward(stream, pending, normed)
-        if writes_cache:
-            mixed = self.mixer.forward(normed, ctx, view)
+        chained = self.chains(*stream.shape)
+        if chained and isinstance(pending, ChainedRows) and pending.norm is self.mixer_norm:
+            x = pending
         else:
-            mixed = self.mixer.forward(normed, ctx, view, writes_cache=False)
-        self.ffn_norm.add_forward(stream, mixed, normed)
-        return self.ffn.forward(normed, ctx)
+            x = ctx.buffer("block.normed", tuple(stream.shape), rt.dtype)
+            self.mixer_norm.add_forward(stream, pending, x)
+        kw = {} if writes_cache else {"writes_cache": False}
+        if chained:
+            rows = self.mixer.forward(x, ctx, view, residual=Residual(stream, self.ffn_norm, ctx), **kw)
+            return self.ffn.forward(rows, ctx, residual=Residual(stream, getattr(ctx, "following_norm", None), ctx))
+        mixed = self.mixer.forward(x, ctx, view, **kw)
+        self.ffn_norm.add_forward(stream, mixed, x)
+        return self.ffn.forward(x, ctx)
 
 
 @register("arrangement", "post_norm")

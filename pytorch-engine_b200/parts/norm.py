@@ -18,6 +18,7 @@ class RMSNorm:
 
     graph_safe = True  # launches only; nothing in forward() waits for the device
     stream_norm = "rms"     # the kernel over several streams (csrc/streams.cu) can end in this norm
+    chains = True           # a weight a column and one number a row: the number can wait until after the next product
 
     @classmethod
     def weight_decls(cls, params) -> Dict[str, WeightDecl]:

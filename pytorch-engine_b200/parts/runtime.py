@@ -103,6 +103,8 @@ class Runtime:
         self.gemm_backend = None  # a callable (x, weight, out, out_dtype) -> tensor or None that takes over products
         self.own_small_gemm = True  # products with few rows run on csrc/gemm_smallm.cu
         self.small_gemm_rows = 8    # up to this many rows (measured: beyond it the library product is faster)
+        self.chain_norms = True     # norms of few rows ride in the products around them (parts/block.py, PreNormBlock): blocks
+        self.chain_widths = (512, {8: 1024, 12: 4096, 32: 2048})   # of this width at least and, by the most rows, at most
         # products with many rows run on csrc/gemm_umma.cu (tcgen05 + TMA); in between, and for shapes it
         # refuses, the library product stands (measured: with fewer rows too few tiles exist to fill the SMs)
         self.own_large_gemm = True
@@ -142,6 +144,18 @@ class Runtime:
     def takes_small_gemm(self, x: torch.Tensor, weight: torch.Tensor) -> bool:
         return (self.own_small_gemm and x.dim() == 2 and x.shape[0] <= self.small_gemm_rows
                 and ops.gemm_smallm_supported(x, weight))
+
+    def takes_chained(self, rows: int, width: int) -> bool:
+        """Whether a step of so many rows of ``width`` may run a pre-norm block as a chain of products (csrc/gemm_smallm.cu, CHAIN).
+        A decode step of 28 layers of width 1,024, chained : with norms of their own: 1 row 698 : 727 us, 8 rows 921 : 964, 9 rows
+        1,143 : 1,632 (where the library's products begin otherwise), 16 rows 1,281 : 1,750, 24 rows 1,635 : 1,922, 32 rows 1,817 :
+        2,090.  Width 2,048: 1 row 463 : 468, 4 rows 649 : 563, 8 rows 765 : 659, 9 rows 779 : 942, 24 rows 1,197 : 1,252, 32 rows 1,373 :
+        1,414.  Width 4,096: 1 row 1,409 : 1,252, 12 rows 1,723 : 1,841, 24 rows 2,147 : 2,004.  A row's squares come in a part per 16
+        features, which every block adds up again, and each block reads its rows from L2.
+        Narrower models keep their norms: a decode step and a prompt of the same tokens then round alike (at width 96 the two were
+        2.4 % of the logits apart after hundreds of chained steps)."""
+        return (self.chain_norms and self.is_cuda and self.dtype == torch.bfloat16 and self.own_small_gemm and self.gemm_backend is None
+                and self.chain_widths[0] <= width <= next((w for r, w in self.chain_widths[1].items() if rows <= r), 0))
 
     def takes_large_gemm(self, x: torch.Tensor, weight: torch.Tensor, pair_offset: int = 0) -> bool:
         rows = 9 if pair_offset else self.large_gemm_rows   # the fused gate wins at every size above the small kernel's

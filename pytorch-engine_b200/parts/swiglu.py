@@ -60,8 +60,16 @@ class SwiGLU:
         self.out_bias_deferred = True
         return self.out_bias
 
-    def forward(self, x: torch.Tensor, ctx) -> torch.Tensor:
+    def chains(self) -> bool:
+        """Whether ``forward`` takes a ``residual`` (parts/block.py, PreNormBlock)."""
+        return self.out_bias is None and ops.gemm_smallm_weight(self.gate_up) and ops.gemm_smallm_weight(self.down)
+
+    def forward(self, x, ctx, residual=None):
         rt = self.runtime
+        if residual is not None:      # x: ChainedRows
+            act = ctx.buffer("ffn.act", (x.x.shape[0], self.intermediate), rt.dtype)
+            ops.gemm_smallm_scaled(x.x, self.gate_up, act, x.squares, x.norm.eps, pair_offset=self.intermediate, glu=self.glu)
+            return residual.add_product(act, self.down)
         n = x.shape[0]
         act = ctx.buffer("ffn.act", (n, self.intermediate), rt.dtype)
         if rt.takes_small_gemm(x, self.gate_up):

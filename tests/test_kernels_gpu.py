@@ -602,6 +602,49 @@ def test_attention_mma_decode_clusters(ops, nh, nkv, d, B, splits, window, keep,
         assert rel_err(outs[0].view(B, nh, d), want) < ATT_TOL[torch.bfloat16]
 
 
+@pytest.mark.parametrize("M", [1, 3, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("hidden,inner", [(16, 8), (100 * 8, 40), (1024, 3072), (4104, 520), (8208, 64)])
+def test_gemm_smallm_chain(ops, M, hidden, inner):
+    """A product into the stream, the stream times the next norm's weight and its squares, and the product that reads them (plain and
+    gated), against the norm and the products in 64 bits on the same rounded inputs."""
+    torch.manual_seed(21)
+    bf = torch.bfloat16
+    x, w = torch.randn(M, inner, device=DEV).to(bf), (torch.randn(hidden, inner, device=DEV) / inner ** 0.5).to(bf)
+    stream0, norm = torch.randn(M, hidden, device=DEV) * 3, 1 + 0.3 * torch.randn(hidden, device=DEV)
+    stream, rows, squares = stream0.clone(), torch.full((M, hidden), float("nan"), device=DEV, dtype=bf), torch.full(((hidden + 15) // 16, ops.chain_rows(M)), float("nan"), device=DEV)
+    ops.gemm_smallm_residual(x, w, stream, norm, rows, squares)
+    want = stream0.double() + x.double() @ w.double().t()
+    size = stream0.double().abs() + x.double().abs() @ w.double().abs().t()
+    assert bool(((stream.double() - want).abs() <= 2.0 ** -22 * size).all())          # float32 sums of exact products
+    assert bool(((rows.double() - stream.double() * norm.double()).abs() <= 2.0 ** -8 * (stream.double() * norm.double()).abs() + 1e-30).all())
+    total = squares.double().sum(0)
+    assert bool(((total[:M] - (stream.double() ** 2).sum(1)).abs() <= 1e-5 * (stream.double() ** 2).sum(1)).all()) and float(total[M:].abs().sum()) == 0
+    again = stream0.clone()
+    ops.gemm_smallm_residual(x, w, again)                                              # nobody reads the rows
+    assert torch.equal(again, stream)
+    eps = 1e-5
+    inv = 1 / ((stream.double() ** 2).mean(1, keepdim=True) + eps).sqrt()
+    for n in (40, 1000):
+        gu = (torch.randn(2 * n, hidden, device=DEV) / hidden ** 0.5).to(bf)
+        y = rows.double() @ gu.double().t() * inv
+        room = rows.double().abs() @ gu.double().abs().t() * inv
+        out = torch.empty(M, 2 * n, device=DEV, dtype=bf)
+        ops.gemm_smallm_scaled(rows, gu, out, squares, eps)
+        assert bool(((out.double() - y).abs() <= 2.0 ** -8 * y.abs() + 1e-5 * room).all())
+        g, u = y[:, :n], y[:, n:]
+        act = torch.empty(M, n, device=DEV, dtype=bf)
+        ops.gemm_smallm_scaled(rows, gu, act, squares, eps, pair_offset=n)
+        want = g / (1 + (-g).exp()) * u
+        slack = 2e-5 * (room[:, :n] * u.abs() * 1.1 + room[:, n:] * g.abs())           # |d silu| <= 1.1
+        assert bool(((act.double() - want).abs() <= 2.0 ** -8 * want.abs() + slack).all())
+        bias = torch.randn(2 * n, device=DEV)
+        ops.gemm_smallm_scaled(rows, gu, act, squares, eps, pair_offset=n, glu=("relu", 0.0, 1.0, bias))
+        g, u = g + bias[:n].double(), u + bias[n:].double()
+        want = g.clamp(min=0) * u
+        slack = 2e-5 * (room[:, :n] * u.abs() + room[:, n:] * g.abs())
+        assert bool(((act.double() - want).abs() <= 2.0 ** -8 * want.abs() + slack).all())
+
+
 @pytest.mark.parametrize("d,dv,kind", [(36, 96, "delta"), (64, 126, "mlstm")])
 def test_recurrences_just_below_48_kb(ops, d, dv, kind):
     """Heads whose dynamic shared memory stays below 48 KB only without the kernel's static part: two tokens in one call as in two."""
