@@ -486,6 +486,87 @@ __device__ __forceinline__ float cluster_load(const float* p, int rank) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(at) : "memory");
   return v;
 }
+// ---- a decode step's q|k|v as the projection left them ------------------------------------------------------
+// APPEND: the decode kernels take q|k|v unnormed and unturned and do what csrc/rope_append.cu does in a kernel of its own that a
+// step waits for once a layer (2.5 us for one sequence, 4.8 for 24): a block norms and turns the query heads of its (sequence,
+// kv head), and the one that holds the sequence's newest page norms and turns the new key, puts it and the new value into the
+// page in shared memory and into the cache.  Formulas and order as there.
+struct Append {
+  const float* q_norm_w; const float* k_norm_w; float eps;    // [HD] or null
+  const float* cos; const float* sin; int rows;                // [rows, HD / 2] or null: no rotation
+  __nv_bfloat16* k_pages; __nv_bfloat16* v_pages;
+};
+
+// Features 2 l, 2 l + 1 and the ones HD / 2 further on, of lane l < HD / 4: what a lane turns.
+template <int HD> struct TurnPair {
+  float2 c, s, w1, w2;
+  __device__ __forceinline__ void weights(const float* w, int lane) {
+    const int j = (lane * 2) % (HD / 2);
+    w1 = w ? *reinterpret_cast<const float2*>(w + j) : make_float2(1.f, 1.f);
+    w2 = w ? *reinterpret_cast<const float2*>(w + j + HD / 2) : make_float2(1.f, 1.f);
+  }
+  __device__ __forceinline__ void angles(const Append& ap, int pos, int lane) {
+    const int j = (lane * 2) % (HD / 2);
+    const bool there = ap.cos != nullptr && pos >= 0 && pos < ap.rows;
+    c = there ? *reinterpret_cast<const float2*>(ap.cos + (size_t)pos * (HD / 2) + j) : make_float2(1.f, 1.f);
+    s = there ? *reinterpret_cast<const float2*>(ap.sin + (size_t)pos * (HD / 2) + j) : make_float2(0.f, 0.f);
+  }
+  // (lo, hi): the two pairs as they lie in q|k|v, and as they come out
+  __device__ __forceinline__ void turn(uint32_t& lo, uint32_t& hi, bool normed, float eps, int lane) const {
+    float2 x1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&lo));
+    float2 x2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hi));
+    if (normed) {
+      float ss = x1.x * x1.x + x1.y * x1.y;
+      ss += x2.x * x2.x + x2.y * x2.y;
+      if (lane * 2 >= HD / 2) ss = 0.f;
+      const float inv = rsqrtf(warp_sum(ss) / (float)HD + eps);
+      x1.x *= inv * w1.x; x1.y *= inv * w1.y; x2.x *= inv * w2.x; x2.y *= inv * w2.y;
+    }
+    lo = pack_bf16(x1.x * c.x - x2.x * s.x, x1.y * c.y - x2.y * s.y);
+    hi = pack_bf16(x2.x * c.x + x1.x * s.x, x2.y * c.y + x1.y * s.y);
+  }
+};
+template <int HD> __device__ __forceinline__ void load_pairs(const __nv_bfloat16* row, int lane, uint32_t& lo, uint32_t& hi) {
+  const int j = (lane * 2) % (HD / 2);
+  lo = *reinterpret_cast<const uint32_t*>(row + j);
+  hi = *reinterpret_cast<const uint32_t*>(row + j + HD / 2);
+}
+// ... and into a swizzled tile of ROWS rows
+template <int HD, int ROWS> __device__ __forceinline__ void store_pairs(char* tile, int row, int lane, uint32_t lo, uint32_t hi) {
+  const int j = lane * 2;
+  if (j >= HD / 2) return;
+  *reinterpret_cast<uint32_t*>(tile + tile_off<HD, ROWS>(row, j / 8) + (j % 8) * 2) = lo;
+  *reinterpret_cast<uint32_t*>(tile + tile_off<HD, ROWS>(row, (j + HD / 2) / 8) + (j % 8) * 2) = hi;
+}
+
+// The new key (warp 0: `lo, hi`, turned) and value (warp 1: as they are) of a sequence of `len` keys go into the newest page's tile
+// and to page `page` of the cache (-1: nowhere).  A page that starts here is cleared behind them: what lies there takes part in
+// products with a probability of zero.  All 128 threads; the caller's barrier follows.
+template <int HD> __device__ __forceinline__ void append_row(const Args& a, const Append& ap, char* stage, int len, int kvh, int page,
+                                                             uint32_t lo, uint32_t hi) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, off = (len - 1) % BN;
+  const size_t at = (((size_t)max(page, 0) * a.n_kv_heads + kvh) * BN + off) * HD;
+  if (warp < 2) {
+    store_pairs<HD, BN>(stage + warp * (BN * HD * 2), off, lane, lo, hi);
+    const int j = lane * 2;
+    if (page >= 0 && j < HD / 2) {
+      __nv_bfloat16* to = (warp ? ap.v_pages : ap.k_pages) + at + j;
+      *reinterpret_cast<uint32_t*>(to) = lo;
+      *reinterpret_cast<uint32_t*>(to + HD / 2) = hi;
+    }
+  }
+  if (off == 0) {
+    constexpr int CPR = HD / 8, N = (BN - 1) * CPR;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < N; i += 128) *reinterpret_cast<uint4*>(stage + BN * HD * 2 + tile_off<HD>(1 + i / CPR, i % CPR)) = zero;
+    if (page >= 0)
+      for (int i = tid; i < N; i += 128) {
+        reinterpret_cast<uint4*>(ap.k_pages + at + HD)[i] = zero;
+        reinterpret_cast<uint4*>(ap.v_pages + at + HD)[i] = zero;
+      }
+  }
+}
+
 // Ranges that one cluster holds at most (the portable size), blocks up to which a step's ranges are clusters.
 constexpr int kClusterRanges = 8, kClusterBlocks = 64;
 
@@ -493,8 +574,8 @@ constexpr int kClusterRanges = 8, kClusterBlocks = 64;
 // CLUSTER: the ranges of a (sequence, kv head) are one cluster, and its blocks put them together through each other's shared
 // memory, a share of the outputs each: no partial results in global memory and no second kernel, which a step waits for
 // once a layer.
-template <int HD, int VD, int STAGES, bool SPLIT_P, bool PAD, bool CLUSTER>
-__global__ void __launch_bounds__(128) decode_split_kernel(Args a, const __grid_constant__ CUtensorMap kmap,
+template <int HD, int VD, int STAGES, bool SPLIT_P, bool PAD, bool CLUSTER, bool APPEND = false>
+__global__ void __launch_bounds__(128) decode_split_kernel(Args a, Append ap, const __grid_constant__ CUtensorMap kmap,
                                                            const __grid_constant__ CUtensorMap vmap) {
   extern __shared__ char smem_raw[];
   __shared__ uint64_t bars[STAGES];
@@ -530,7 +611,23 @@ __global__ void __launch_bounds__(128) decode_split_kernel(Args a, const __grid_
   const int n_tiles = keep_tiles + win_tiles;
   auto tile_k0 = [&](int it) { return it < keep_tiles ? k_lo + it * BN : k_begin + (it - keep_tiles) * BN; };
   const int hole_lo = keep, hole_hi = keep > 0 ? win_lo : 0;
-  const int last_page_k0 = (len - 1) / BN * BN;
+  // (APPEND: this block itself puts the new key into the newest page, which was complete but for it)
+  const int last_page_k0 = APPEND ? -1 : (len - 1) / BN * BN;
+  TurnPair<HD> tq_pair, tk_pair;
+  const bool newest = APPEND && k_hi == len;
+  int new_page = -1;
+  if (APPEND) {
+    tq_pair.weights(ap.q_norm_w, lane);
+    tk_pair.weights(ap.k_norm_w, lane);
+    tq_pair.angles(ap, len - 1, lane);
+    tk_pair.c = tq_pair.c; tk_pair.s = tq_pair.s;
+    if (newest) {
+      if (ap.cos && len > ap.rows && tid == 0) report(a.status, kStatusPositionOutOfRange, tq, len - 1, ap.rows);
+      const int logical = (len - 1) / BN;
+      if (logical < a.table_stride) new_page = a.page_table[(size_t)slot * a.table_stride + logical];
+      if (new_page >= a.num_pages || (ap.cos && len > ap.rows)) new_page = -1;      // issue_page reports the first
+    }
+  }
   if (tid == 0) {
 #pragma unroll
     for (int s = 0; s < STAGES; ++s) tma::mbar_init(&bars[s], 1);
@@ -548,7 +645,24 @@ __global__ void __launch_bounds__(128) decode_split_kernel(Args a, const __grid_
         issue_page<HD, VD>(a, &kmap, &vmap, slot, kvh, tile_k0(s), smem + s * STAGE, &bars[s]);
   }
   constexpr int CPR = HD / 8;
-  for (int i = tid; i < 16 * CPR; i += 128) {
+  uint32_t kv_lo = 0, kv_hi = 0;
+  if (APPEND) {
+    const __nv_bfloat16* row = a.q + (size_t)tq * a.q_ld;
+    uint32_t lo[4], hi[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (warp + 4 * i < group) load_pairs<HD>(row + (size_t)(kvh * group + warp + 4 * i) * HD, lane, lo[i], hi[i]);
+    if (newest && warp < 2) load_pairs<HD>(row + (size_t)(a.n_heads + warp * a.n_kv_heads + kvh) * HD, lane, kv_lo, kv_hi);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = warp + 4 * i;
+      if (r < group) tq_pair.turn(lo[i], hi[i], ap.q_norm_w != nullptr, ap.eps, lane);
+      else lo[i] = hi[i] = 0;
+      store_pairs<HD, 16>(q_s, r, lane, lo[i], hi[i]);
+    }
+    if (newest && warp == 0) tk_pair.turn(kv_lo, kv_hi, ap.k_norm_w != nullptr, ap.eps, lane);
+  }
+  for (int i = tid; !APPEND && i < 16 * CPR; i += 128) {
     const int r = i / CPR, chunk = i % CPR;
     uint4 v = make_uint4(0, 0, 0, 0);
     if (r < group && (!PAD || chunk * 8 < hd))
@@ -578,6 +692,10 @@ __global__ void __launch_bounds__(128) decode_split_kernel(Args a, const __grid_
       return;
     }
     const int k0 = tile_k0(it);
+    if (APPEND && newest && it + 1 == n_tiles) {
+      append_row<HD>(a, ap, smem + (it % STAGES) * STAGE, len, kvh, new_page, kv_lo, kv_hi);
+      __syncthreads();
+    }
     decode_fold_page<HD, VD, SPLIT_P>(smem_u32(smem + (it % STAGES) * STAGE), smem_u32(smem + (it % STAGES) * STAGE) + BN * HD * 2,
                          warp * 16, k0, k_first, k_hi, hole_lo, hole_hi, a.scale_log2, qf, o, m_lo, m_hi, l_lo, l_hi, lane);
     if (CLUSTER) {
@@ -794,7 +912,7 @@ static int opt_in(K kernel, size_t bytes) {
 }
 
 template <int HD, int VD, bool SPLIT_P, bool PAD>
-static int launch(const Args& a, bool decode, int n_seqs, int max_q, cudaStream_t stream) {
+static int launch(const Args& a, bool decode, int n_seqs, int max_q, const Append* append, cudaStream_t stream) {
   constexpr int STAGE = BN * (HD + VD) * 2;
   CUtensorMap kmap, vmap;
   const uint64_t rows = (uint64_t)a.num_pages * a.n_kv_heads * BN;
@@ -823,7 +941,7 @@ static int launch(const Args& a, bool decode, int n_seqs, int max_q, cudaStream_
     int e = opt_in(kern, smem);
     if (e) return e;
     if (!cluster) {
-      pe::launch(kern, grid, 128, smem, stream, a, kmap, vmap);
+      pe::launch(kern, grid, 128, smem, stream, a, Append(), kmap, vmap);
       return 0;
     }
     cudaLaunchConfig_t cfg = {};
@@ -835,15 +953,20 @@ static int launch(const Args& a, bool decode, int n_seqs, int max_q, cudaStream_
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    const cudaError_t ce = cudaLaunchKernelEx(&cfg, kern, a, kmap, vmap);
+    const cudaError_t ce = cudaLaunchKernelEx(&cfg, kern, a, append ? *append : Append(), kmap, vmap);
     return ce == cudaSuccess ? 0 : (int)ce;
   };
   if (cluster_ranges(n_seqs * a.n_kv_heads, a.split_keys, a.max_splits)) {
-    const int e = go(decode_split_kernel<HD, VD, 3, SPLIT_P, PAD, true>, 3, a.max_splits);
+    int e;
+    if constexpr (!SPLIT_P && !PAD)
+      e = append ? go(decode_split_kernel<HD, VD, 3, SPLIT_P, PAD, true, true>, 3, a.max_splits) : go(decode_split_kernel<HD, VD, 3, SPLIT_P, PAD, true>, 3, a.max_splits);
+    else
+      e = go(decode_split_kernel<HD, VD, 3, SPLIT_P, PAD, true>, 3, a.max_splits);
     if (e) return e;
     PE_LAUNCH_CHECK();
     return PE_OK;
   }
+  if (append) return PE_ERR_UNSUPPORTED_SIZE;
   // three stages: two blocks per SM, two pages in flight per block (measured best of 2, 3, 4)
   const int e = go(decode_split_kernel<HD, VD, 3, SPLIT_P, PAD, false>, 3, 0);
   if (e) return e;
@@ -928,16 +1051,16 @@ extern "C" int pe_attention_mma_masked(int decode, const void* q, long long q_ld
                                 split_keys, max_splits, min_range_keys, status, stream);
 }
 
-// The same with values of a size of their own (`v_dim`; the scratch of a decode step then holds v_dim floats per partial
-// row) and, with `gate` (bfloat16, row of token t at gate + t * gate_ld), each head's output times sigmoid(gate[t, head]).
-extern "C" int pe_attention_mma_gated(int decode, const void* q, long long q_ld, void* out, long long out_ld, int n_seqs,
-                                      int max_q, int n_heads, int n_kv_heads, int head_dim, int v_dim, float scale, int window,
-                                      int chunk, int keep_first, int v_heads, int out_f32, int split_p, int sink,
-                                      const float* out_cos, const float* out_sin, int out_rows, const void* gate,
-                                      long long gate_ld, const int* seq_qstart, const int* seq_past, const int* seq_slot,
-                                      const int* page_table, int table_stride, int num_pages, const void* k_pages,
-                                      const void* v_pages, float* scratch, int split_keys, int max_splits, int min_range_keys,
-                                      int* status, cudaStream_t stream) {
+namespace pe {
+namespace fa {
+
+static int run(int decode, const void* q, long long q_ld, void* out, long long out_ld, int n_seqs, int max_q, int n_heads,
+               int n_kv_heads, int head_dim, int v_dim, float scale, int window, int chunk, int keep_first, int v_heads,
+               int out_f32, int split_p, int sink, const float* out_cos, const float* out_sin, int out_rows,
+               const void* gate, long long gate_ld, const int* seq_qstart, const int* seq_past, const int* seq_slot,
+               const int* page_table, int table_stride, int num_pages, const void* k_pages, const void* v_pages,
+               float* scratch, int split_keys, int max_splits, int min_range_keys, const Append* append, int* status,
+               cudaStream_t stream) {
   if (n_seqs <= 0) return PE_OK;
   const bool exact = head_dim == v_dim && (head_dim == 64 || head_dim == 128);
   if (!exact && (split_p || out_cos)) return PE_ERR_UNSUPPORTED_SIZE;
@@ -973,17 +1096,57 @@ extern "C" int pe_attention_mma_gated(int decode, const void* q, long long q_ld,
   const bool dec = decode != 0;
   if (exact) {
     if (split_p) {
-      if (head_dim == 64) return launch<64, 64, true, false>(a, dec, n_seqs, max_q, stream);
-      return launch<128, 128, true, false>(a, dec, n_seqs, max_q, stream);
+      if (head_dim == 64) return launch<64, 64, true, false>(a, dec, n_seqs, max_q, append, stream);
+      return launch<128, 128, true, false>(a, dec, n_seqs, max_q, append, stream);
     }
-    if (head_dim == 64) return launch<64, 64, false, false>(a, dec, n_seqs, max_q, stream);
-    return launch<128, 128, false, false>(a, dec, n_seqs, max_q, stream);
+    if (head_dim == 64) return launch<64, 64, false, false>(a, dec, n_seqs, max_q, append, stream);
+    return launch<128, 128, false, false>(a, dec, n_seqs, max_q, append, stream);
   }
   const bool wide = v_dim > 64;
   switch (pe::fa::tile_of(head_dim)) {
-    case 64: return wide ? launch<64, 128, false, true>(a, dec, n_seqs, max_q, stream) : launch<64, 64, false, true>(a, dec, n_seqs, max_q, stream);
-    case 128: return wide ? launch<128, 128, false, true>(a, dec, n_seqs, max_q, stream) : launch<128, 64, false, true>(a, dec, n_seqs, max_q, stream);
-    case 192: return wide ? launch<192, 128, false, true>(a, dec, n_seqs, max_q, stream) : launch<192, 64, false, true>(a, dec, n_seqs, max_q, stream);
-    default: return wide ? launch<256, 128, false, true>(a, dec, n_seqs, max_q, stream) : launch<256, 64, false, true>(a, dec, n_seqs, max_q, stream);
+    case 64: return wide ? launch<64, 128, false, true>(a, dec, n_seqs, max_q, append, stream) : launch<64, 64, false, true>(a, dec, n_seqs, max_q, append, stream);
+    case 128: return wide ? launch<128, 128, false, true>(a, dec, n_seqs, max_q, append, stream) : launch<128, 64, false, true>(a, dec, n_seqs, max_q, append, stream);
+    case 192: return wide ? launch<192, 128, false, true>(a, dec, n_seqs, max_q, append, stream) : launch<192, 64, false, true>(a, dec, n_seqs, max_q, append, stream);
+    default: return wide ? launch<256, 128, false, true>(a, dec, n_seqs, max_q, append, stream) : launch<256, 64, false, true>(a, dec, n_seqs, max_q, append, stream);
   }
+}
+
+}  // namespace fa
+}  // namespace pe
+
+// The same with values of a size of their own (`v_dim`; the scratch of a decode step then holds v_dim floats per partial
+// row) and, with `gate` (bfloat16, row of token t at gate + t * gate_ld), each head's output times sigmoid(gate[t, head]).
+extern "C" int pe_attention_mma_gated(int decode, const void* q, long long q_ld, void* out, long long out_ld, int n_seqs,
+                                      int max_q, int n_heads, int n_kv_heads, int head_dim, int v_dim, float scale, int window,
+                                      int chunk, int keep_first, int v_heads, int out_f32, int split_p, int sink,
+                                      const float* out_cos, const float* out_sin, int out_rows, const void* gate,
+                                      long long gate_ld, const int* seq_qstart, const int* seq_past, const int* seq_slot,
+                                      const int* page_table, int table_stride, int num_pages, const void* k_pages,
+                                      const void* v_pages, float* scratch, int split_keys, int max_splits, int min_range_keys,
+                                      int* status, cudaStream_t stream) {
+  return pe::fa::run(decode, q, q_ld, out, out_ld, n_seqs, max_q, n_heads, n_kv_heads, head_dim, v_dim, scale, window, chunk,
+                     keep_first, v_heads, out_f32, split_p, sink, out_cos, out_sin, out_rows, gate, gate_ld,
+                     seq_qstart, seq_past, seq_slot, page_table, table_stride, num_pages, k_pages, v_pages,
+                     scratch, split_keys, max_splits, min_range_keys, nullptr, status, stream);
+}
+
+// A decode step of which the projection's q|k|v are given as it left them (rows of (n_heads + 2 n_kv_heads) * head_dim): q/k-norm
+// (weights or null), rotation of the whole head in split halves (tables [table_rows, head_dim / 2] or null) and the append of k and
+// v happen here, as in pe_qk_norm_rope_append, whose alignment rules hold.  head_dim 64 or 128.
+// Ranges of each sequence's own as in pe_attention_mma (split_keys 0), where they are one cluster (pe_attention_mma_decode_launches
+// says 1), else refused.
+extern "C" int pe_attention_mma_append(const void* qkv, long long ld, void* out, long long out_ld, int n_seqs, int n_heads, int n_kv_heads,
+                                       int head_dim, float scale, int window, const float* q_norm_w, const float* k_norm_w, float eps,
+                                       const float* cos_table, const float* sin_table, int table_rows, const int* seq_qstart,
+                                       const int* seq_past, const int* seq_slot, const int* page_table, int table_stride, int num_pages,
+                                       void* k_pages, void* v_pages, float* scratch, int max_splits, int min_range_keys,
+                                       int* status, cudaStream_t stream) {
+  if (head_dim != 64 && head_dim != 128) return PE_ERR_UNSUPPORTED_SIZE;
+  if ((cos_table == nullptr) != (sin_table == nullptr)) return PE_ERR_BAD_ARGUMENT;
+  if (((uintptr_t)q_norm_w % 8) || ((uintptr_t)k_norm_w % 8) || ((uintptr_t)cos_table % 8) || ((uintptr_t)sin_table % 8)) return PE_ERR_BAD_ARGUMENT;
+  if (page_table == nullptr || k_pages == nullptr || v_pages == nullptr) return PE_ERR_BAD_ARGUMENT;
+  const pe::fa::Append append = {q_norm_w, k_norm_w, eps, cos_table, sin_table, table_rows, (__nv_bfloat16*)k_pages, (__nv_bfloat16*)v_pages};
+  return pe::fa::run(1, qkv, ld, out, out_ld, n_seqs, 1, n_heads, n_kv_heads, head_dim, head_dim, scale, window, 0, 0, n_kv_heads, 0, 0, 0,
+                     nullptr, nullptr, 0, nullptr, 0, seq_qstart, seq_past, seq_slot, page_table, table_stride, num_pages, k_pages, v_pages,
+                     scratch, 0, max_splits, min_range_keys, &append, status, stream);
 }

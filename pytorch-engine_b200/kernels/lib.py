@@ -105,6 +105,7 @@ _SIGNATURES = {
     "pe_attention_mma_dims_supported": [I, I, I, I],
     "pe_attention_mma_gated": [I, P, L, P, L, I, I, I, I, I, I, F, I, I, I, I, I, I, I, P, P, I, P, L, P, P, P, P, I, I, P, P, P, I, I, I,
                                P, P],
+    "pe_attention_mma_append": [P, L, P, L, I, I, I, I, F, I, P, P, F, P, P, I, P, P, P, P, I, I, P, P, P, I, I, P, P],
     "pe_gemm_smallm_scaled": [P, L, P, P, L, I, I, I, I, I, F, F, P, P, I, I, F, I, P],
     "pe_gemm_smallm_residual": [P, L, P, P, L, I, I, I, P, P, L, P, I, P],
     "pe_attention_umma_dims_supported": [I, I, I, I],

@@ -426,6 +426,39 @@ def attention_mma_masked(decode: bool, q: torch.Tensor, out: torch.Tensor, n_seq
     _count(_mma_launches(decode, n_seqs * n_kv_heads, split_keys, max_splits))
 
 
+def attention_mma_append_ranges(n_seqs: int, n_kv_heads: int, max_kv_len: int) -> tuple:
+    """(max_splits, least keys) of ``attention_mma_append`` in clusters: ranges of a page, as many as a cluster and a step's blocks
+    allow.  What a short sequence costs is a chain of latencies, and every page a range folds is one more (0.8 us)."""
+    return max(1, min(8, -(-max_kv_len // 64), 64 // (n_seqs * n_kv_heads))), 64
+
+
+def attention_mma_clusters(n_seqs: int, n_kv_heads: int, split_keys: int, max_splits: int) -> bool:
+    """Whether a decode step's ranges are put together inside clusters, with no second kernel."""
+    return int(library().pe_attention_mma_decode_launches(n_seqs * n_kv_heads, split_keys, max_splits)) == 1
+
+
+def attention_mma_append(qkv: torch.Tensor, out: torch.Tensor, n_seqs: int, n_heads: int, n_kv_heads: int, head_dim: int, scale: float,
+                         window: int, q_norm_w: Optional[torch.Tensor], k_norm_w: Optional[torch.Tensor], eps: float,
+                         cos: Optional[torch.Tensor], sin: Optional[torch.Tensor], seq_qstart: torch.Tensor, seq_past: torch.Tensor,
+                         seq_slot: torch.Tensor, page_table: torch.Tensor, num_pages: int, k_pages: torch.Tensor, v_pages: torch.Tensor,
+                         scratch: torch.Tensor, max_splits: int, min_range_keys: int, status: torch.Tensor) -> None:
+    """A decode step's attention on q|k|v as the projection left them: ``qk_norm_rope_append`` (the whole head rotated, or none of
+    it) and ``attention_mma`` in clusters of up to ``max_splits`` ranges in one.  Head size 64 or 128.  ``qkv`` is left as it is."""
+    _need(qkv.stride(-1) == 1 and out.stride(-1) == 1, "attention: rows must be contiguous")
+    _need(qkv.dtype == out.dtype == k_pages.dtype == v_pages.dtype == torch.bfloat16, "attention_mma_append: bfloat16 tensors only")
+    _need(qkv.shape[-1] >= (n_heads + 2 * n_kv_heads) * head_dim, "attention_mma_append: rows of q|k|v")
+    _need((cos is None) == (sin is None) and (cos is None or (cos.dtype == sin.dtype == torch.float32 and cos.is_contiguous()
+          and sin.is_contiguous() and cos.shape == sin.shape and cos.shape[1] * 2 == head_dim)), "attention_mma_append: angle tables")
+    for w in (q_norm_w, k_norm_w):
+        _need(w is None or (w.dtype == torch.float32 and w.is_contiguous() and w.numel() == head_dim), "attention_mma_append: norm weights")
+    check(library().pe_attention_mma_append(
+        _ptr(qkv), qkv.stride(0), _ptr(out), out.stride(0), n_seqs, n_heads, n_kv_heads, head_dim, float(scale), int(window),
+        _ptr(q_norm_w), _ptr(k_norm_w), float(eps), _ptr(cos), _ptr(sin), 0 if cos is None else cos.shape[0], _ptr(seq_qstart),
+        _ptr(seq_past), _ptr(seq_slot), _ptr(page_table), page_table.shape[1], num_pages, _ptr(k_pages), _ptr(v_pages), _ptr(scratch),
+        max_splits, int(min_range_keys), _ptr(status), _stream()), "attention_mma_append")
+    _count(1)
+
+
 def attention_latent_supported(dtype: torch.dtype, row: int, rank: int) -> bool:
     """Whether the tensor-core kernels of csrc/attention_latent.cu take cached rows of ``row`` features whose leading
     ``rank`` are the values (bfloat16; rows up to 576 and values up to 512 features, in steps of 8)."""

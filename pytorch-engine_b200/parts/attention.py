@@ -188,6 +188,9 @@ class GQAttention:
             dims = (runtime.dtype, self.head_dim, self.v_dim, self.n_heads, self.n_kv_heads)
             self.use_mma = ops.attention_mma_dims_supported(*dims)
             self.use_umma_prefill = not self.keep_first and ops.attention_umma_dims_supported(*dims)
+        # norm, rotation and append of a decode step ride in its attention kernels: plain layers, the whole head rotated or none of it
+        self.fuses_append = (not self.general and self.head_dim in (64, 128) and (self.position is None or self.fused_position)
+                             and all(w is None or w.data_ptr() % 8 == 0 for w in (self.q_norm, self.k_norm)))
         self.generic_attention = bool(getattr(runtime, "generic_attention", False))   # comparisons: the general kernels only
 
     def chains(self) -> bool:
@@ -207,8 +210,9 @@ class GQAttention:
             else:
                 ops.gemm_smallm_scaled(rows, self.qkv, qkv, x.squares, x.norm.eps)
             out = ctx.buffer("attn.out", (n, self.n_heads * self.head_dim), rt.dtype)
-            self.norm_rotate_append(qkv, n, ctx, view, writes_cache)
-            self.attend(qkv, out, ctx, view)
+            if not (writes_cache and self.attend_append(qkv, out, ctx, view)):
+                self.norm_rotate_append(qkv, n, ctx, view, writes_cache)
+                self.attend(qkv, out, ctx, view)
             return residual.add_product(out, self.o_proj)
         n = x.shape[0]
         qkv = ctx.buffer("attn.qkv", (n, self.qkv_dim), rt.dtype)
@@ -249,6 +253,11 @@ class GQAttention:
                                     self.eps, cos, sin, rotary_dim, *where, writes_cache, rt.status)
         else:
             rt.linear(x, self.qkv, out=qkv)
+            out = ctx.buffer("attn.out", (n, self.n_heads * self.head_dim), rt.dtype)
+            if writes_cache and self.attend_append(qkv, out, ctx, view):
+                delta = ctx.buffer("attn.delta", (n, self.hidden), rt.dtype)
+                rt.linear(out, self.o_proj, out=delta)
+                return delta
             self.norm_rotate_append(qkv, n, ctx, view, writes_cache)
         out = ctx.buffer("attn.out", (n, self.n_heads * self.head_dim), rt.dtype)
         self.attend(qkv, out, ctx, view)
@@ -443,3 +452,23 @@ class GQAttention:
             return {}
         return dict(parts=parts, scratch=ctx.buffer("attn.parts", (parts * q.shape[0] * self.n_heads * (self.v_dim + 1),), torch.float32))
 
+    def attend_append(self, qkv: torch.Tensor, out: torch.Tensor, ctx, view) -> bool:
+        """A decode step's norm, rotation, append and attention in the attention's kernels, where they can (else False)."""
+        if not (ctx.decode and self.use_mma and self.fuses_append):
+            return False
+        cos = sin = None
+        if self.position is not None:
+            cos, sin, rotary_dim = self.position.tables()
+            if rotary_dim != self.head_dim:
+                return False
+        split_keys, max_splits, _ = ops.attention_mma_decode_ranges(qkv.device, self.head_dim, ctx.n_seqs, self.n_kv_heads, ctx.max_kv_len,
+                                                                    SPLIT_KEYS)
+        if not ops.attention_mma_clusters(ctx.n_seqs, self.n_kv_heads, split_keys, max_splits):
+            return False
+        max_splits, least = ops.attention_mma_append_ranges(ctx.n_seqs, self.n_kv_heads, ctx.max_kv_len)
+        floats = ops.attention_generic_scratch_floats(ctx.n_seqs, self.n_heads, self.head_dim, max_splits)
+        scratch = ctx.buffer("attn.scratch", (floats,), torch.float32)
+        ops.attention_mma_append(qkv, out, ctx.n_seqs, self.n_heads, self.n_kv_heads, self.head_dim, self.scale, self.window, self.q_norm,
+                                 self.k_norm, self.eps, cos, sin, ctx.seq_qstart, ctx.seq_past, ctx.seq_slot, view.page_table,
+                                 view.num_pages, view.k_pages, view.v_pages, scratch, max_splits, least, self.runtime.status)
+        return True

@@ -164,6 +164,8 @@ def test_reference_arm_and_plain_baseline_of_the_benchmark_run(pe):
     assert out["impl"] == "reference" and "unavailable" not in out
     assert out["e2e"]["tokens"] == 12 and out["value"] > 0 and out["config"]["layers"] == 3
     assert "pytorch-engine_b200" not in open(os.path.join(ROOT, "baseline", "reference_arm.py")).read().split('"""', 2)[2]
+
+
 def test_scratch_of_the_sampler_with_groups(pe):
     """Rows with a small top-k leave one float a group of entries: more than 512 groups, and no more than a block holds."""
     f = pe.kernels.lib.library().pe_sample_scratch_bytes
@@ -177,3 +179,16 @@ def test_scratch_of_the_sampler_with_groups(pe):
     assert f(3, 20000, 0.8, 225, 0.95, 0.0) > 0         # chunks and their candidates beyond
 
 
+def test_parts_of_a_prefill_and_ranges_of_a_decode_with_append(pe):
+    """Rules on sizes: a prefill is cut only where its tiles leave half the chip idle and each part keeps at least six pages; a decode
+    step's clusters stay within eight blocks, 64 blocks in all, and the cache's pages."""
+    parts, ranges = pe.kernels.ops.attention_umma_parts, pe.kernels.ops.attention_mma_append_ranges
+    for items in (1, 8, 37, 74, 148, 149, 1000):
+        for pages in (1, 31, 32, 47, 64, 640):
+            n = parts(296, items, pages)
+            assert 1 <= n <= 8 and (n == 1 or (2 * items <= 296 and items * n <= 296 and pages >= 32 and pages // n >= 6)), (items, pages)
+    assert parts(296, 8, 640) == 8 and parts(296, 74, 640) == 4
+    for n_seqs, nkv in ((1, 1), (1, 8), (3, 8), (8, 8), (64, 1)):
+        for keys in (1, 64, 65, 400, 40960):
+            n, least = ranges(n_seqs, nkv, keys)
+            assert 1 <= n <= 8 and n * n_seqs * nkv <= 64 and (n - 1) * least < keys

@@ -645,6 +645,50 @@ def test_gemm_smallm_chain(ops, M, hidden, inner):
         assert bool(((act.double() - want).abs() <= 2.0 ** -8 * want.abs() + slack).all())
 
 
+@pytest.mark.parametrize("nh,nkv,d", [(16, 8, 128), (8, 2, 64), (16, 1, 128), (16, 1, 64), (3, 3, 64)])
+@pytest.mark.parametrize("normed,rotated,window", [(True, True, 0), (False, True, 100), (True, False, 0)])
+def test_attention_mma_append(ops, nh, nkv, d, normed, rotated, window):
+    """Norm, rotation, append and attention in one against the two kernels: outputs, cached rows, and the rest of a page that starts
+    (which holds NaN before)."""
+    torch.manual_seed(23)
+    bf = torch.bfloat16
+    lens = [1, 700, 257, 64, 65, 130][:64 // (4 * nkv) or 1]
+    B = len(lens)
+    qkv = torch.randn(B, (nh + 2 * nkv) * d + 8, device=DEV).to(bf)
+    qw, kw = ((1 + 0.2 * torch.randn(d, device=DEV)) if normed else None for _ in range(2))
+    angles = torch.rand(704, d // 2, device=DEV) * 6
+    cos, sin = (angles.cos(), angles.sin()) if rotated else (None, None)
+    qstart, past = torch.arange(B + 1, dtype=torch.int32, device=DEV), torch.tensor([L - 1 for L in lens], dtype=torch.int32, device=DEV)
+    st = _status()
+    outs, pages = [], []
+    for fused in (True, False):
+        ps = PagedSetup(lens, nkv, d, bf, seed=23, key_scale=2.0)
+        for b, L in enumerate(lens):      # nothing is cached at the new position, and nothing finite behind it in a page that starts
+            page = int(ps.table[ps.slots[b], (L - 1) // 64])
+            ps.k_pages[page, :, (L - 1) % 64:] = ps.v_pages[page, :, (L - 1) % 64:] = float("nan") if L % 64 == 1 else 0.0
+        where = (qstart, past, ps.seq_slot, ps.table, ps.num_pages, ps.k_pages, ps.v_pages)
+        x, out = qkv.clone(), torch.full((B, nh * d), float("nan"), device=DEV, dtype=bf)
+        if fused:
+            floats = ops.attention_generic_scratch_floats(B, nh, d, 4)
+            scratch = torch.full((floats + 64,), float("nan"), device=DEV)
+            ops.attention_mma_append(x, out, B, nh, nkv, d, d ** -0.5, window, qw, kw, 1e-5, cos, sin, *where, scratch, 4, 64, st)
+            assert torch.equal(x, qkv) and bool(scratch[floats:].isnan().all())      # inside the scratch it asked for
+        else:
+            t = torch.arange(B, dtype=torch.int32, device=DEV)
+            ops.qk_norm_rope_append(x, B, nh, nkv, d, qw, kw, 1e-5, cos, sin, d if rotated else 0, t, past, ps.seq_slot, qstart, ps.table,
+                                    ps.num_pages, ps.k_pages, ps.v_pages, True, st)
+            scratch = torch.empty(ops.attention_generic_scratch_floats(B, nh, d, 11), device=DEV)
+            ops.attention_mma(True, x, out, B, 1, nh, nkv, d, d ** -0.5, window, *where, scratch, 64, 11, st)
+        outs.append(out.float())
+        pages.append((ps.k_pages, ps.v_pages))
+    assert st.tolist()[0] == 0
+    assert rel_err(outs[0], outs[1]) < 2 * ATT_TOL[bf]
+    assert torch.equal(pages[0][1], pages[1][1])
+    # a key is one rounding of the same float32 numbers, whose sums may round differently
+    k0, k1 = pages[0][0].double(), pages[1][0].double()
+    assert bool(((k0 - k1).abs() <= 2.0 ** -7 * k1.abs()).all())
+
+
 @pytest.mark.parametrize("d,dv,kind", [(36, 96, "delta"), (64, 126, "mlstm")])
 def test_recurrences_just_below_48_kb(ops, d, dv, kind):
     """Heads whose dynamic shared memory stays below 48 KB only without the kernel's static part: two tokens in one call as in two."""
