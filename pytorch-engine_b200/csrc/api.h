@@ -65,10 +65,13 @@ int pe_attention_mma_gated(int decode, const void* q, long long q_ld, void* out,
     int table_stride, int num_pages, const void* k_pages, const void* v_pages, float* scratch, int split_keys,
     int max_splits, int min_range_keys, int* status, cudaStream_t stream);
 
+int pe_attention_mma_shared_blocks_per_sm(int head_dim);
+long long pe_attention_mma_shared_scratch_floats(int n_seqs, int n_heads, int n_kv_heads, int head_dim, int blocks);
+
 int pe_attention_mma_append(const void* qkv, long long ld, void* out, long long out_ld, int n_seqs, int n_heads, int n_kv_heads,
     int head_dim, float scale, int window, const float* q_norm_w, const float* k_norm_w, float eps, const float* cos_table,
     const float* sin_table, int table_rows, const int* seq_qstart, const int* seq_past, const int* seq_slot,
-    const int* page_table, int table_stride, int num_pages, void* k_pages, void* v_pages, float* scratch,
+    const int* page_table, int table_stride, int num_pages, void* k_pages, void* v_pages, float* scratch, int blocks,
     int max_splits, int min_range_keys, int* status, cudaStream_t stream);
 
 // attention_latent.cu

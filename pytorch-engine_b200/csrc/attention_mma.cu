@@ -879,6 +879,346 @@ __global__ void decode_merge_kernel(Args a) {
   }
 }
 
+// ---- decode, keys shared out over the blocks -----------------------------------------------------------
+// Blocks and ranges above are cut from one sequence each, so the longest sequence sets the time: 24 sequences of 16 to 2,048 keys
+// on 8 kv heads are 192 ranges for 296 places, most of them short.  Here the visible pages of all (sequence, kv head) pairs are
+// one list, sequence after sequence and kv head after kv head, and block i of n takes pages [i T / n, (i + 1) T / n) of its T:
+// every block reads as much as every other, whatever the lengths.  A pair that lies inside one block is finished there; the
+// others leave a partial result a block, number (block + pair) of the list, and a second kernel puts them together.
+//
+// Warp 4 looks pages up, a lane each, and keeps STAGES of them on their way across the pairs' borders; warps 0-3 fold them as
+// above, a quarter of the keys each, and meet only where a pair ends (then they sum through the page they have just read).
+constexpr int kSharedSeqs = 512;       // sequences whose page counts a block holds
+
+struct SharedArgs {
+  int n_seqs;
+  int2* pairs;              // per pair: its first partial result, and how many there are (1: none, it is finished)
+};
+
+// What a decode step's query sees of its sequence: the pages from the window's start.
+struct Visible {
+  int len, win_lo, begin, tiles;
+  __device__ __forceinline__ Visible(const Args& a, int past) {
+    len = past + 1;
+    win_lo = first_visible(a, past);
+    begin = win_lo / BN * BN;
+    tiles = (len - begin + BN - 1) / BN;
+  }
+  __device__ __forceinline__ int key0(int tile) const { return begin + tile * BN; }
+};
+
+// A place in the list of pages.
+struct Place {
+  int b, kvh, tile;
+  __device__ __forceinline__ Place(const int* before, int n_seqs, int n_kv_heads, int at) {
+    int lo = 0, hi = n_seqs;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (before[mid] * n_kv_heads <= at) lo = mid;
+      else hi = mid;
+    }
+    b = lo;
+    const int rest = at - before[b] * n_kv_heads, tiles = before[b + 1] - before[b];
+    kvh = rest / tiles;
+    tile = rest - kvh * tiles;
+  }
+};
+
+__device__ __forceinline__ void bar_sync_consumers() { asm volatile("bar.sync 1, 128;\n" ::: "memory"); }
+
+// Blocks of the shared decode that an SM holds (shared memory; registers are bounded to match).
+__host__ __device__ constexpr int shared_blocks_per_sm(int hd) { return hd <= 64 ? 3 : 2; }
+
+// grid: blocks (any number); block: 160 threads.
+template <int HD, int STAGES>
+__global__ void __launch_bounds__(160, shared_blocks_per_sm(HD)) decode_shared_kernel(Args a, SharedArgs sh, Append ap, const __grid_constant__ CUtensorMap kmap,
+                                                                                      const __grid_constant__ CUtensorMap vmap) {
+  extern __shared__ char smem_raw[];
+  __shared__ uint64_t full[STAGES], empty[STAGES];
+  __shared__ int before[kSharedSeqs + 1];      // pages of one kv head in the sequences before
+  __shared__ int warp_pages[4];
+  __shared__ volatile int failed;
+  __shared__ float ml[4 * 16 * 2];
+  __shared__ int stage_page[STAGES];           // the page of the cache in a stage, -1: outside the pool
+  char* smem = align_1024(smem_raw);
+  constexpr int STAGE = BN * HD * 4;
+  constexpr int KS = HD / 16;
+  constexpr int NO = HD / 8;
+  constexpr int CPR = HD / 8;
+  char* q_s = smem + STAGES * STAGE;           // [16][HD] swizzled
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int group = a.group, n_kv = a.n_kv_heads;
+
+  // the batch description, the page table and all pages but a sequence's last were written before the kernel that precedes this
+  // one started: they are read before the wait
+  constexpr int PER = kSharedSeqs / 128;
+  int mine[PER], sum = 0;
+  if (warp < 4) {
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      const int b = tid * PER + k;
+      mine[k] = b < sh.n_seqs ? Visible(a, a.seq_past[b]).tiles : 0;
+      sum += mine[k];
+    }
+    int up = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, up, o);
+      if (lane >= o) up += v;
+    }
+    if (lane == 31) warp_pages[warp] = up;
+    sum = up - sum;
+  } else if (lane == 0) {
+#pragma unroll
+    for (int s = 0; s < STAGES; ++s) {
+      tma::mbar_init(&full[s], 1);
+      tma::mbar_init(&empty[s], 4);
+    }
+    tma::fence_barrier_init();
+    failed = 0;
+  }
+  __syncthreads();
+  if (warp < 4) {
+    for (int w = 0; w < warp; ++w) sum += warp_pages[w];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      const int b = tid * PER + k;
+      if (b <= sh.n_seqs) before[b] = sum;
+      sum += mine[k];
+    }
+    if (tid == 127 && sh.n_seqs == kSharedSeqs) before[kSharedSeqs] = sum;
+  }
+  __syncthreads();
+  const int total = before[sh.n_seqs] * n_kv, min_pages = max(1, a.min_range_keys / BN);
+  const int n_blocks = max(1, min((int)gridDim.x, total / min_pages)), me = blockIdx.x;
+  if (me >= n_blocks) return;
+  const int x0 = (int)((long long)me * total / n_blocks), x1 = (int)((long long)(me + 1) * total / n_blocks);
+  const int n_tiles = x1 - x0;      // at least 1: n_blocks <= total
+
+  if (warp == 4) {
+    for (int base = 0; base < n_tiles; base += 32) {
+      int y = 0, page = -1;
+      if (base + lane < n_tiles) {
+        const Place p(before, sh.n_seqs, n_kv, x0 + base + lane);
+        const Visible v(a, a.seq_past[p.b]);
+        const int logical = v.key0(p.tile) / BN, slot = a.seq_slot[p.b];
+        if (logical < a.table_stride) page = a.page_table[(size_t)slot * a.table_stride + logical];
+        if (page < 0 || page >= a.num_pages) {
+          report(a.status, kStatusPageOutOfRange, slot, page, logical * BN);
+          page = -1;
+        }
+        y = (max(page, 0) * n_kv + p.kvh) * BN;
+      }
+      const int n = min(32, n_tiles - base);
+      for (int l = 0; l < n; ++l) {
+        const int it = base + l, s = it % STAGES;
+        const int py = __shfl_sync(0xffffffffu, y, l), its_page = __shfl_sync(0xffffffffu, page, l);
+        if (it >= STAGES && !failed && !tma::mbar_wait(&empty[s], (it / STAGES - 1) & 1)) {
+          if (lane == 0) report(a.status, kStatusWaitTimedOut, 3, me, it);
+          failed = 1;
+        }
+        if (failed) break;
+        if (lane == 0) {
+          char* stage = smem + s * STAGE;
+          stage_page[s] = its_page;      // read behind the barrier
+          tma::mbar_expect_tx(&full[s], STAGE);
+#pragma unroll
+          for (int sub = 0; sub < HD / 64; ++sub) {
+            tma::load_2d(stage + sub * (BN * 128), &kmap, sub * 64, py, &full[s]);
+            tma::load_2d(stage + BN * HD * 2 + sub * (BN * 128), &vmap, sub * 64, py, &full[s]);
+          }
+        }
+        __syncwarp();
+      }
+    }
+    if (failed && lane == 0)      // copies still in flight get a bounded chance to land before the block leaves
+      for (int s = 0; s < STAGES; ++s)
+        for (int i = 0; i < 1000; ++i)
+          if (tma::mbar_try_wait(&full[s], 0) && tma::mbar_try_wait(&full[s], 1)) break;
+    return;
+  }
+
+  Place at(before, sh.n_seqs, n_kv, x0);
+  // warp w turns query heads w, w + 4, ..; warp 0 the new key, warp 1 takes the new value
+  uint32_t lo_next[4], hi_next[4], kv_lo_next = 0, kv_hi_next = 0, kv_lo = 0, kv_hi = 0;
+  TurnPair<HD> tq_pair, tk_pair;
+  tq_pair.weights(ap.q_norm_w, lane);
+  tk_pair.weights(ap.k_norm_w, lane);
+  for (int i = tid; i < 16 * CPR; i += 128) *reinterpret_cast<uint4*>(q_s + i * 16) = make_uint4(0, 0, 0, 0);   // rows beyond the group
+  if (warp == 0) pdl_wait();
+  bar_sync_consumers();
+  auto load_q = [&](const Place& p) {
+    const __nv_bfloat16* row = a.q + (size_t)a.seq_qstart[p.b] * a.q_ld;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (warp + 4 * i < group) load_pairs<HD>(row + (size_t)(p.kvh * group + warp + 4 * i) * HD, lane, lo_next[i], hi_next[i]);
+    if (warp < 2) load_pairs<HD>(row + (size_t)(a.n_heads + warp * n_kv + p.kvh) * HD, lane, kv_lo_next, kv_hi_next);
+    tq_pair.angles(ap, a.seq_past[p.b], lane);
+  };
+  uint32_t qf[KS][4];
+  auto take_q = [&]() {      // nobody reads q_s any more
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (warp + 4 * i >= group) break;
+      tq_pair.turn(lo_next[i], hi_next[i], ap.q_norm_w != nullptr, ap.eps, lane);
+      store_pairs<HD, 16>(q_s, warp + 4 * i, lane, lo_next[i], hi_next[i]);
+    }
+    kv_lo = kv_lo_next;
+    kv_hi = kv_hi_next;
+    tk_pair.c = tq_pair.c;
+    tk_pair.s = tq_pair.s;
+    if (warp == 0) tk_pair.turn(kv_lo, kv_hi, ap.k_norm_w != nullptr, ap.eps, lane);
+    bar_sync_consumers();
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      const int r = (lane & 7) + ((lane >> 3) & 1) * 8;
+      ldmatrix_x4(qf[ks], smem_u32(q_s) + tile_off<HD, 16>(r, ks * 2 + (lane >> 4)));
+    }
+  };
+  load_q(at);
+  take_q();
+  float o[NO][4];
+  float m_lo, m_hi, l_lo, l_hi;
+  auto clear = [&]() {
+#pragma unroll
+    for (int n = 0; n < NO; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+    m_lo = m_hi = -INFINITY;
+    l_lo = l_hi = 0.f;
+  };
+  clear();
+  Visible seen(a, a.seq_past[at.b]);
+  int first = at.tile;      // of this pair, in this block
+
+  for (int it = 0; it < n_tiles; ++it) {
+    const int s = it % STAGES;
+    const bool pair_ends = at.tile + 1 == seen.tiles, last = pair_ends || it + 1 == n_tiles;
+    Place next = at;
+    if (pair_ends) {
+      next.tile = 0;
+      if (++next.kvh == n_kv) {
+        next.kvh = 0;
+        ++next.b;
+      }
+      if (it + 1 < n_tiles) load_q(next);      // on its way while this page is folded
+    } else {
+      ++next.tile;
+    }
+    if (!failed && !tma::mbar_wait(&full[s], (it / STAGES) & 1)) {
+      if (lane == 0) report(a.status, kStatusWaitTimedOut, 2, me, it);
+      failed = 1;      // nobody waits any more; what is left is computed from whatever is there, and the step reports the status
+    }
+    char* stage = smem + s * STAGE;
+    if (pair_ends) {
+      const bool known = !ap.cos || seen.len <= ap.rows;
+      if (!known && tid == 0) report(a.status, kStatusPositionOutOfRange, a.seq_qstart[at.b], seen.len - 1, ap.rows);
+      append_row<HD>(a, ap, stage, seen.len, at.kvh, known ? stage_page[s] : -1, kv_lo, kv_hi);
+      bar_sync_consumers();
+    }
+    decode_fold_page<HD, HD, false>(smem_u32(stage), smem_u32(stage) + BN * HD * 2, warp * 16, seen.key0(at.tile), seen.win_lo, seen.len,
+                                    0, 0, a.scale_log2, qf, o, m_lo, m_hi, l_lo, l_hi, lane);
+    if (last) {
+      // the four warps' results summed in warp order, through the page that all of them have read
+      bar_sync_consumers();
+      float* acc = reinterpret_cast<float*>(stage);      // [4 warps][group][HD]
+      if (t == 0) {
+        ml[(warp * 16 + g) * 2] = m_lo;     ml[(warp * 16 + g) * 2 + 1] = l_lo;
+        ml[(warp * 16 + g + 8) * 2] = m_hi; ml[(warp * 16 + g + 8) * 2 + 1] = l_hi;
+      }
+#pragma unroll
+      for (int n = 0; n < NO; ++n) {
+        if (g < group)
+          *reinterpret_cast<float2*>(acc + (size_t)(warp * group + g) * HD + n * 8 + 2 * t) = make_float2(o[n][0], o[n][1]);
+        if (g + 8 < group)
+          *reinterpret_cast<float2*>(acc + (size_t)(warp * group + g + 8) * HD + n * 8 + 2 * t) = make_float2(o[n][2], o[n][3]);
+      }
+      bar_sync_consumers();
+      const bool whole = first == 0 && pair_ends;
+      const int pair = at.b * n_kv + at.kvh, part = me + pair;
+      const int tq = a.seq_qstart[at.b];
+      for (int i = tid; i < group * HD; i += 128) {
+        const int r = i / HD, c = i - r * HD, h = at.kvh * group + r;
+        float mm = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) mm = fmaxf(mm, ml[(w * 16 + r) * 2]);
+        float ll = 0.f, aa = 0.f;
+        if (mm != -INFINITY) {
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            const float mw = ml[(w * 16 + r) * 2];
+            const float f = (mw == -INFINITY) ? 0.f : fast_exp2(mw - mm);
+            ll += ml[(w * 16 + r) * 2 + 1] * f;
+            aa += acc[(size_t)(w * group + r) * HD + c] * f;
+          }
+        }
+        if (!whole) {
+          const size_t pidx = (size_t)part * group + r;
+          a.part_acc[pidx * HD + c] = (ll > 0.f) ? aa / ll : 0.f;
+          if (c == 0) a.part_lse[pidx] = (ll > 0.f) ? (mm + log2f(ll)) * 0.6931471805599453f : -INFINITY;
+          continue;
+        }
+        a.out[(size_t)tq * a.out_ld + (size_t)h * HD + c] = __float2bfloat16_rn(aa / fmaxf(ll, 1e-20f));
+      }
+      if (tid == 0 && first == 0) {
+        // who holds the pair's last page: block i takes pages up to (i + 1) total / n_blocks
+        const long long end = x0 + it + 1 + (long long)(seen.tiles - 1 - at.tile);
+        sh.pairs[pair] = make_int2(part, (int)((end * n_blocks - 1) / total) - me + 1);
+      }
+      tma::fence_proxy_async();      // the page's place is written by TMA next
+      if (it + 1 < n_tiles) {
+        take_q();                    // (its barrier: everyone has read the sums and the old queries)
+        clear();
+        first = 0;
+      }
+    }
+    __syncwarp();
+    if (lane == 0) tma::mbar_arrive(&empty[s]);
+    if (pair_ends && next.b != at.b && it + 1 < n_tiles) seen = Visible(a, a.seq_past[next.b]);
+    at = next;
+  }
+  if (tid == 0) pdl_launch_dependents();
+}
+
+// grid: (n_heads, n_seqs): put a pair's partial results together, in the order of its keys; nothing to do for a pair that one
+// block held.
+template <int HD>
+__global__ void decode_shared_merge_kernel(Args a, SharedArgs sh) {
+  pdl_wait_block();
+  pdl_launch_dependents();
+  const int b = blockIdx.y, h = blockIdx.x, c = threadIdx.x;
+  const int kvh = h / a.group, r = h - kvh * a.group;
+  const int2 parts = sh.pairs[b * a.n_kv_heads + kvh];
+  if (parts.y <= 1) return;
+  const size_t base = (size_t)parts.x * a.group + r;
+  constexpr int G = 8;      // at a time, all their loads before the first is used
+  float mx = -INFINITY, denom = 0.f, v = 0.f;
+  for (int s0 = 0; s0 < parts.y; s0 += G) {
+    float e[G], acc[G];
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      const bool live = s0 + i < parts.y;
+      const size_t at = base + (size_t)(s0 + i) * a.group;
+      e[i] = live ? a.part_lse[at] : -INFINITY;
+      acc[i] = live ? a.part_acc[at * HD + c] : 0.f;
+    }
+    float m_new = mx;
+#pragma unroll
+    for (int i = 0; i < G; ++i) m_new = fmaxf(m_new, e[i]);
+    if (m_new == -INFINITY) continue;
+    const float keep = (mx == -INFINITY) ? 0.f : expf(mx - m_new);
+    denom *= keep;
+    v *= keep;
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      const float w = (e[i] == -INFINITY) ? 0.f : expf(e[i] - m_new);
+      denom += w;
+      v = fmaf(w, acc[i], v);
+    }
+    mx = m_new;
+  }
+  a.out[(size_t)a.seq_qstart[b] * a.out_ld + (size_t)h * HD + c] = __float2bfloat16_rn(v / fmaxf(denom, 1e-20f));
+}
+
 // The tile sizes that rows of these sizes run in.
 static int tile_of(int dim) { return (dim + 63) / 64 * 64; }
 
@@ -909,6 +1249,33 @@ static int opt_in(K kernel, size_t bytes) {
     if (e != cudaSuccess) return (int)e;
   }
   return 0;
+}
+
+// Floats of the shared decode's partial results in front of the pairs' descriptions (on an 8-byte boundary).
+static size_t shared_part_floats(int pairs, int group, int head_dim, int blocks) {
+  const size_t n = (size_t)(pairs + blocks) * group * (head_dim + 1);
+  return n + (n & 1);
+}
+// (A stage has room for four warps' sums of 16 rows: 4 * 16 * HD * 4 bytes are BN * HD * 4.)
+template <int HD>
+static int launch_shared(const Args& a, int n_seqs, int blocks, const Append& append, cudaStream_t stream) {
+  constexpr int STAGES = 3;
+  CUtensorMap kmap, vmap;
+  const uint64_t rows = (uint64_t)a.num_pages * a.n_kv_heads * BN;
+  int e = tma::make_map_2d_bf16(&kmap, a.k_pages, HD, rows, HD, 64, BN);
+  if (e == 0) e = tma::make_map_2d_bf16(&vmap, a.v_pages, HD, rows, HD, 64, BN);
+  if (e != 0) return e < 0 ? e : PE_ERR_BAD_ARGUMENT;
+  if (n_seqs > 65535) return PE_ERR_UNSUPPORTED_SIZE;
+  const SharedArgs sh = {n_seqs, reinterpret_cast<int2*>(a.part_acc + shared_part_floats(n_seqs * a.n_kv_heads, a.group, HD, blocks))};
+  const size_t smem = STAGES * BN * HD * 4 + 16 * HD * 2 + 1024;
+  e = opt_in(decode_shared_kernel<HD, STAGES>, smem);
+  if (e) return e;
+  pe::launch(decode_shared_kernel<HD, STAGES>, blocks, 160, smem, stream, a, sh, append, kmap, vmap);
+  PE_LAUNCH_CHECK();
+  // after the blocks have completed, as below
+  pe::launch_after(decode_shared_merge_kernel<HD>, dim3(a.n_heads, n_seqs), HD, 0, stream, a, sh);
+  PE_LAUNCH_CHECK();
+  return PE_OK;
 }
 
 template <int HD, int VD, bool SPLIT_P, bool PAD>
@@ -1059,7 +1426,7 @@ static int run(int decode, const void* q, long long q_ld, void* out, long long o
                int out_f32, int split_p, int sink, const float* out_cos, const float* out_sin, int out_rows,
                const void* gate, long long gate_ld, const int* seq_qstart, const int* seq_past, const int* seq_slot,
                const int* page_table, int table_stride, int num_pages, const void* k_pages, const void* v_pages,
-               float* scratch, int split_keys, int max_splits, int min_range_keys, const Append* append, int* status,
+               float* scratch, int split_keys, int max_splits, int min_range_keys, int shared_blocks, const Append* append, int* status,
                cudaStream_t stream) {
   if (n_seqs <= 0) return PE_OK;
   const bool exact = head_dim == v_dim && (head_dim == 64 || head_dim == 128);
@@ -1085,7 +1452,15 @@ static int run(int decode, const void* q, long long q_ld, void* out, long long o
   a.chunk = chunk; a.v_heads = v_heads; a.out_f32 = out_f32; a.split_p = split_p;
   a.keep_first = window > 0 ? keep_first : 0;
   a.hd = head_dim; a.vd = v_dim; a.gate = (const __nv_bfloat16*)gate; a.gate_ld = gate_ld;
-  if (decode) {
+  if (shared_blocks > 0) {
+    if (!scratch || ((uintptr_t)scratch % 8) || min_range_keys < 0 || min_range_keys % pe::fa::BN) return PE_ERR_BAD_ARGUMENT;
+    if (n_seqs > kSharedSeqs) return PE_ERR_UNSUPPORTED_SIZE;
+    a.min_range_keys = min_range_keys;
+    a.part_acc = scratch;
+    a.part_lse = scratch + (size_t)(n_seqs * n_kv_heads + shared_blocks) * a.group * v_dim;
+    if (append == nullptr || !exact) return PE_ERR_BAD_ARGUMENT;
+    return head_dim == 64 ? launch_shared<64>(a, n_seqs, shared_blocks, *append, stream) : launch_shared<128>(a, n_seqs, shared_blocks, *append, stream);
+  } else if (decode) {
     if (!scratch || split_keys < 0 || split_keys % pe::fa::BN || max_splits <= 0) return PE_ERR_BAD_ARGUMENT;
     if (min_range_keys < 0 || min_range_keys % pe::fa::BN) return PE_ERR_BAD_ARGUMENT;
     a.split_keys = split_keys; a.max_splits = max_splits; a.min_range_keys = min_range_keys;
@@ -1127,26 +1502,36 @@ extern "C" int pe_attention_mma_gated(int decode, const void* q, long long q_ld,
   return pe::fa::run(decode, q, q_ld, out, out_ld, n_seqs, max_q, n_heads, n_kv_heads, head_dim, v_dim, scale, window, chunk,
                      keep_first, v_heads, out_f32, split_p, sink, out_cos, out_sin, out_rows, gate, gate_ld,
                      seq_qstart, seq_past, seq_slot, page_table, table_stride, num_pages, k_pages, v_pages,
-                     scratch, split_keys, max_splits, min_range_keys, nullptr, status, stream);
+                     scratch, split_keys, max_splits, min_range_keys, 0, nullptr, status, stream);
+}
+
+// Blocks that one SM holds at a time of a decode step whose keys are shared out (pe_attention_mma_append).
+extern "C" int pe_attention_mma_shared_blocks_per_sm(int head_dim) { return pe::fa::shared_blocks_per_sm(head_dim); }
+
+// Floats of scratch for it, 0 where it does not take the step (then the ranges of pe_attention_mma do).
+extern "C" long long pe_attention_mma_shared_scratch_floats(int n_seqs, int n_heads, int n_kv_heads, int head_dim, int blocks) {
+  if (n_seqs <= 0 || n_seqs > pe::fa::kSharedSeqs || blocks <= 0 || (head_dim != 64 && head_dim != 128)) return 0;
+  if (!pe_attention_mma_dims_supported(head_dim, head_dim, n_heads, n_kv_heads)) return 0;
+  return (long long)pe::fa::shared_part_floats(n_seqs * n_kv_heads, n_heads / n_kv_heads, head_dim, blocks) + 2LL * n_seqs * n_kv_heads;
 }
 
 // A decode step of which the projection's q|k|v are given as it left them (rows of (n_heads + 2 n_kv_heads) * head_dim): q/k-norm
 // (weights or null), rotation of the whole head in split halves (tables [table_rows, head_dim / 2] or null) and the append of k and
-// v happen here, as in pe_qk_norm_rope_append, whose alignment rules hold.  head_dim 64 or 128.
-// Ranges of each sequence's own as in pe_attention_mma (split_keys 0), where they are one cluster (pe_attention_mma_decode_launches
-// says 1), else refused.
+// v happen here, as in pe_qk_norm_rope_append, whose alignment rules hold.  head_dim 64 or 128.  blocks > 0: the step's keys shared
+// out evenly over so many blocks, at least min_range_keys each, whichever sequences they belong to; 0: ranges of each sequence's own as in pe_attention_mma (split_keys 0), where they are one cluster
+// (pe_attention_mma_decode_launches says 1), else refused.
 extern "C" int pe_attention_mma_append(const void* qkv, long long ld, void* out, long long out_ld, int n_seqs, int n_heads, int n_kv_heads,
                                        int head_dim, float scale, int window, const float* q_norm_w, const float* k_norm_w, float eps,
                                        const float* cos_table, const float* sin_table, int table_rows, const int* seq_qstart,
                                        const int* seq_past, const int* seq_slot, const int* page_table, int table_stride, int num_pages,
-                                       void* k_pages, void* v_pages, float* scratch, int max_splits, int min_range_keys,
+                                       void* k_pages, void* v_pages, float* scratch, int blocks, int max_splits, int min_range_keys,
                                        int* status, cudaStream_t stream) {
   if (head_dim != 64 && head_dim != 128) return PE_ERR_UNSUPPORTED_SIZE;
   if ((cos_table == nullptr) != (sin_table == nullptr)) return PE_ERR_BAD_ARGUMENT;
   if (((uintptr_t)q_norm_w % 8) || ((uintptr_t)k_norm_w % 8) || ((uintptr_t)cos_table % 8) || ((uintptr_t)sin_table % 8)) return PE_ERR_BAD_ARGUMENT;
-  if (page_table == nullptr || k_pages == nullptr || v_pages == nullptr) return PE_ERR_BAD_ARGUMENT;
+  if (blocks < 0 || page_table == nullptr || k_pages == nullptr || v_pages == nullptr) return PE_ERR_BAD_ARGUMENT;
   const pe::fa::Append append = {q_norm_w, k_norm_w, eps, cos_table, sin_table, table_rows, (__nv_bfloat16*)k_pages, (__nv_bfloat16*)v_pages};
   return pe::fa::run(1, qkv, ld, out, out_ld, n_seqs, 1, n_heads, n_kv_heads, head_dim, head_dim, scale, window, 0, 0, n_kv_heads, 0, 0, 0,
                      nullptr, nullptr, 0, nullptr, 0, seq_qstart, seq_past, seq_slot, page_table, table_stride, num_pages, k_pages, v_pages,
-                     scratch, 0, max_splits, min_range_keys, &append, status, stream);
+                     scratch, 0, max_splits, min_range_keys, blocks, &append, status, stream);
 }

@@ -76,8 +76,8 @@ class ModelRunner:
         else:
             ctx = StepContext(self.runtime, self.pool, n_tokens=n_tokens, n_seqs=n_seqs, max_q=max(q_lens),
                               decode=decode, n_want=n_want,
-                              # decode: the longest sequence the cache allows, as in the captured graphs, so that how a
-                              # sequence's keys are cut into ranges never depends on the other sequences' lengths
+                              # decode: the longest sequence the cache allows, as in the captured graphs, so that both take
+                              # the same kernels and cut keys into the same ranges
                               max_kv_len=self.cache.max_seq_len if decode else max(p + q for p, q in zip(pasts, q_lens)))
             self.stager.send(ints, ctx.meta)
             ops.batch_expand(ctx.seq_qstart, ctx.seq_past, n_seqs, ctx.token_seq, ctx.token_pos)

@@ -105,7 +105,8 @@ _SIGNATURES = {
     "pe_attention_mma_dims_supported": [I, I, I, I],
     "pe_attention_mma_gated": [I, P, L, P, L, I, I, I, I, I, I, F, I, I, I, I, I, I, I, P, P, I, P, L, P, P, P, P, I, I, P, P, P, I, I, I,
                                P, P],
-    "pe_attention_mma_append": [P, L, P, L, I, I, I, I, F, I, P, P, F, P, P, I, P, P, P, P, I, I, P, P, P, I, I, P, P],
+    "pe_attention_mma_shared_blocks_per_sm": [I],
+    "pe_attention_mma_append": [P, L, P, L, I, I, I, I, F, I, P, P, F, P, P, I, P, P, P, P, I, I, P, P, P, I, I, I, P, P],
     "pe_gemm_smallm_scaled": [P, L, P, P, L, I, I, I, I, I, F, F, P, P, I, I, F, I, P],
     "pe_gemm_smallm_residual": [P, L, P, P, L, I, I, I, P, P, L, P, I, P],
     "pe_attention_umma_dims_supported": [I, I, I, I],
@@ -142,6 +143,7 @@ _RESTYPES = {"pe_wait_limit_polls": (L, []),
              "pe_gemm_split32_scratch_floats": (L, [I, I, I, I]),
              "pe_wkv_scratch_floats": (L, [I, I, I, I]),
              "pe_mlstm_walk_scratch_floats": (L, [I, I, I, I]),
+             "pe_attention_mma_shared_scratch_floats": (L, [I, I, I, I, I]),
              "pe_delta_rule_walk_scratch_floats": (L, [I, I, I, I, I]),
              "pe_mlstm_scratch_floats": (L, [I, I, I, I, I]),
              "pe_delta_rule_scratch_floats": (L, [I, I, I, I, I]),

@@ -426,6 +426,19 @@ def attention_mma_masked(decode: bool, q: torch.Tensor, out: torch.Tensor, n_seq
     _count(_mma_launches(decode, n_seqs * n_kv_heads, split_keys, max_splits))
 
 
+def attention_mma_shares(device: torch.device, head_dim: int, n_seqs: int, n_heads: int, n_kv_heads: int, max_kv_len: int) -> tuple:
+    """(blocks, floats of scratch, least keys a block) where ``attention_mma_append`` shares a decode step's keys out over the chip,
+    (0, 0, 0) where ranges of each sequence's own (``attention_mma_decode_ranges``) are the better cut.  Ranges leave places empty where
+    the (sequence, kv head) pairs are between 0.6 and 1 of the chip's places; short caches do not pay for the second kernel.  A step of
+    the 0.6B shape (8 kv heads, 296 places), ranges : shared: 24 sequences of 16 to 2,048 keys 1,913 : 1,788 us, of 2,048 keys 2,558 :
+    2,512, of 300 keys in a cache for as many 1,250 : 1,323; 30 of 2,048 keys 2,954 : 2,861; 20 of 16 to 4,000 keys 2,032 : 2,160."""
+    blocks, pairs = sm_count(device) * int(library().pe_attention_mma_shared_blocks_per_sm(head_dim)), n_seqs * n_kv_heads
+    if pairs > blocks or 5 * pairs < 3 * blocks or max_kv_len <= 512:
+        return 0, 0, 0
+    floats = int(library().pe_attention_mma_shared_scratch_floats(n_seqs, n_heads, n_kv_heads, head_dim, blocks))
+    return (blocks, floats, 128) if floats > 0 else (0, 0, 0)
+
+
 def attention_mma_append_ranges(n_seqs: int, n_kv_heads: int, max_kv_len: int) -> tuple:
     """(max_splits, least keys) of ``attention_mma_append`` in clusters: ranges of a page, as many as a cluster and a step's blocks
     allow.  What a short sequence costs is a chain of latencies, and every page a range folds is one more (0.8 us)."""
@@ -441,9 +454,10 @@ def attention_mma_append(qkv: torch.Tensor, out: torch.Tensor, n_seqs: int, n_he
                          window: int, q_norm_w: Optional[torch.Tensor], k_norm_w: Optional[torch.Tensor], eps: float,
                          cos: Optional[torch.Tensor], sin: Optional[torch.Tensor], seq_qstart: torch.Tensor, seq_past: torch.Tensor,
                          seq_slot: torch.Tensor, page_table: torch.Tensor, num_pages: int, k_pages: torch.Tensor, v_pages: torch.Tensor,
-                         scratch: torch.Tensor, max_splits: int, min_range_keys: int, status: torch.Tensor) -> None:
+                         scratch: torch.Tensor, blocks: int, max_splits: int, min_range_keys: int, status: torch.Tensor) -> None:
     """A decode step's attention on q|k|v as the projection left them: ``qk_norm_rope_append`` (the whole head rotated, or none of
-    it) and ``attention_mma`` in clusters of up to ``max_splits`` ranges in one.  Head size 64 or 128.  ``qkv`` is left as it is."""
+    it) and ``attention_mma`` in one: with the step's keys shared out evenly over ``blocks`` blocks, at least ``min_range_keys`` each,
+    or (``blocks`` 0) in clusters of up to ``max_splits`` ranges.  Head size 64 or 128.  ``qkv`` is left as it is."""
     _need(qkv.stride(-1) == 1 and out.stride(-1) == 1, "attention: rows must be contiguous")
     _need(qkv.dtype == out.dtype == k_pages.dtype == v_pages.dtype == torch.bfloat16, "attention_mma_append: bfloat16 tensors only")
     _need(qkv.shape[-1] >= (n_heads + 2 * n_kv_heads) * head_dim, "attention_mma_append: rows of q|k|v")
@@ -455,8 +469,8 @@ def attention_mma_append(qkv: torch.Tensor, out: torch.Tensor, n_seqs: int, n_he
         _ptr(qkv), qkv.stride(0), _ptr(out), out.stride(0), n_seqs, n_heads, n_kv_heads, head_dim, float(scale), int(window),
         _ptr(q_norm_w), _ptr(k_norm_w), float(eps), _ptr(cos), _ptr(sin), 0 if cos is None else cos.shape[0], _ptr(seq_qstart),
         _ptr(seq_past), _ptr(seq_slot), _ptr(page_table), page_table.shape[1], num_pages, _ptr(k_pages), _ptr(v_pages), _ptr(scratch),
-        max_splits, int(min_range_keys), _ptr(status), _stream()), "attention_mma_append")
-    _count(1)
+        blocks, max_splits, int(min_range_keys), _ptr(status), _stream()), "attention_mma_append")
+    _count(2 if blocks else 1)
 
 
 def attention_latent_supported(dtype: torch.dtype, row: int, rank: int) -> bool:

@@ -461,14 +461,17 @@ class GQAttention:
             cos, sin, rotary_dim = self.position.tables()
             if rotary_dim != self.head_dim:
                 return False
-        split_keys, max_splits, _ = ops.attention_mma_decode_ranges(qkv.device, self.head_dim, ctx.n_seqs, self.n_kv_heads, ctx.max_kv_len,
-                                                                    SPLIT_KEYS)
-        if not ops.attention_mma_clusters(ctx.n_seqs, self.n_kv_heads, split_keys, max_splits):
-            return False
-        max_splits, least = ops.attention_mma_append_ranges(ctx.n_seqs, self.n_kv_heads, ctx.max_kv_len)
-        floats = ops.attention_generic_scratch_floats(ctx.n_seqs, self.n_heads, self.head_dim, max_splits)
+        blocks, floats, least = ops.attention_mma_shares(qkv.device, self.head_dim, ctx.n_seqs, self.n_heads, self.n_kv_heads, ctx.max_kv_len)
+        max_splits = 0
+        if not blocks:
+            split_keys, max_splits, least = ops.attention_mma_decode_ranges(qkv.device, self.head_dim, ctx.n_seqs, self.n_kv_heads,
+                                                                            ctx.max_kv_len, SPLIT_KEYS)
+            if not ops.attention_mma_clusters(ctx.n_seqs, self.n_kv_heads, split_keys, max_splits):
+                return False
+            max_splits, least = ops.attention_mma_append_ranges(ctx.n_seqs, self.n_kv_heads, ctx.max_kv_len)
+            floats = ops.attention_generic_scratch_floats(ctx.n_seqs, self.n_heads, self.head_dim, max_splits)
         scratch = ctx.buffer("attn.scratch", (floats,), torch.float32)
         ops.attention_mma_append(qkv, out, ctx.n_seqs, self.n_heads, self.n_kv_heads, self.head_dim, self.scale, self.window, self.q_norm,
                                  self.k_norm, self.eps, cos, sin, ctx.seq_qstart, ctx.seq_past, ctx.seq_slot, view.page_table,
-                                 view.num_pages, view.k_pages, view.v_pages, scratch, max_splits, least, self.runtime.status)
+                                 view.num_pages, view.k_pages, view.v_pages, scratch, blocks, max_splits, least, self.runtime.status)
         return True

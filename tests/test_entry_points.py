@@ -166,6 +166,18 @@ def test_reference_arm_and_plain_baseline_of_the_benchmark_run(pe):
     assert "pytorch-engine_b200" not in open(os.path.join(ROOT, "baseline", "reference_arm.py")).read().split('"""', 2)[2]
 
 
+def test_scratch_of_the_shared_decode_attention(pe):
+    """Which decode steps can share their keys out over the chip, and their scratch: a partial result a block and pair, and where a pair's lie."""
+    f = pe.kernels.lib.library().pe_attention_mma_shared_scratch_floats
+    for n_seqs, nh, nkv, d, blocks in ((1, 16, 8, 128, 296), (512, 6, 2, 64, 444), (3, 5, 1, 128, 7), (24, 3, 3, 64, 1)):
+        pairs, group = n_seqs * nkv, nh // nkv
+        floats = (pairs + blocks) * group * (d + 1)
+        assert f(n_seqs, nh, nkv, d, blocks) == floats + floats % 2 + 2 * pairs
+    assert f(513, 16, 8, 128, 296) == 0            # more sequences than a block lists
+    assert f(4, 16, 1, 64, 296) > 0 and f(4, 17, 1, 128, 296) == 0 and f(4, 8, 8, 96, 296) == 0
+    assert f(4, 16, 8, 128, 0) == 0 and f(0, 16, 8, 128, 296) == 0
+
+
 def test_scratch_of_the_sampler_with_groups(pe):
     """Rows with a small top-k leave one float a group of entries: more than 512 groups, and no more than a block holds."""
     f = pe.kernels.lib.library().pe_sample_scratch_bytes

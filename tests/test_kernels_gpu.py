@@ -646,13 +646,14 @@ def test_gemm_smallm_chain(ops, M, hidden, inner):
 
 
 @pytest.mark.parametrize("nh,nkv,d", [(16, 8, 128), (8, 2, 64), (16, 1, 128), (16, 1, 64), (3, 3, 64)])
+@pytest.mark.parametrize("blocks,least", [(0, 64), (1, 64), (5, 128), (296, 64), (296, 256)])      # 0: each sequence's ranges as one cluster
 @pytest.mark.parametrize("normed,rotated,window", [(True, True, 0), (False, True, 100), (True, False, 0)])
-def test_attention_mma_append(ops, nh, nkv, d, normed, rotated, window):
+def test_attention_mma_append(ops, nh, nkv, d, blocks, least, normed, rotated, window):
     """Norm, rotation, append and attention in one against the two kernels: outputs, cached rows, and the rest of a page that starts
-    (which holds NaN before)."""
+    (which holds NaN before).  With the keys shared out: pairs that lie inside a block, that end in one, that span many."""
     torch.manual_seed(23)
     bf = torch.bfloat16
-    lens = [1, 700, 257, 64, 65, 130][:64 // (4 * nkv) or 1]
+    lens = [1, 700, 257, 64, 65, 130][:64 // (4 * nkv) or 1] if blocks == 0 else [1, 700, 257, 64, 65, 513, 130]
     B = len(lens)
     qkv = torch.randn(B, (nh + 2 * nkv) * d + 8, device=DEV).to(bf)
     qw, kw = ((1 + 0.2 * torch.randn(d, device=DEV)) if normed else None for _ in range(2))
@@ -670,8 +671,10 @@ def test_attention_mma_append(ops, nh, nkv, d, normed, rotated, window):
         x, out = qkv.clone(), torch.full((B, nh * d), float("nan"), device=DEV, dtype=bf)
         if fused:
             floats = ops.attention_generic_scratch_floats(B, nh, d, 4)
+            if blocks:
+                floats = int(ops.library().pe_attention_mma_shared_scratch_floats(B, nh, nkv, d, blocks))
             scratch = torch.full((floats + 64,), float("nan"), device=DEV)
-            ops.attention_mma_append(x, out, B, nh, nkv, d, d ** -0.5, window, qw, kw, 1e-5, cos, sin, *where, scratch, 4, 64, st)
+            ops.attention_mma_append(x, out, B, nh, nkv, d, d ** -0.5, window, qw, kw, 1e-5, cos, sin, *where, scratch, blocks, 4, least, st)
             assert torch.equal(x, qkv) and bool(scratch[floats:].isnan().all())      # inside the scratch it asked for
         else:
             t = torch.arange(B, dtype=torch.int32, device=DEV)
@@ -687,6 +690,34 @@ def test_attention_mma_append(ops, nh, nkv, d, normed, rotated, window):
     # a key is one rounding of the same float32 numbers, whose sums may round differently
     k0, k1 = pages[0][0].double(), pages[1][0].double()
     assert bool(((k0 - k1).abs() <= 2.0 ** -7 * k1.abs()).all())
+
+
+@pytest.mark.parametrize("B", [129, 512, 513])
+def test_attention_mma_append_of_many_sequences(ops, B):
+    """Batches around the number of sequences whose pages a block lists, keys shared out, against the two kernels."""
+    torch.manual_seed(27)
+    nh, nkv, d, bf = 4, 2, 64, torch.bfloat16
+    lens = [64 * (b % 3) + 1 + b % 64 for b in range(B)]
+    floats = int(ops.library().pe_attention_mma_shared_scratch_floats(B, nh, nkv, d, 444))
+    assert (floats > 0) == (B <= 512)
+    if not floats:
+        return
+    qkv, angles = torch.randn(B, (nh + 2 * nkv) * d, device=DEV).to(bf), torch.rand(256, d // 2, device=DEV) * 6
+    t, qstart = torch.arange(B, dtype=torch.int32, device=DEV), torch.arange(B + 1, dtype=torch.int32, device=DEV)
+    past, st, outs = torch.tensor([L - 1 for L in lens], dtype=torch.int32, device=DEV), _status(), []
+    for fused in (True, False):
+        ps = PagedSetup(lens, nkv, d, bf, seed=27)
+        where = (qstart, past, ps.seq_slot, ps.table, ps.num_pages, ps.k_pages, ps.v_pages)
+        x, out = qkv.clone(), torch.full((B, nh * d), float("nan"), device=DEV, dtype=bf)
+        scratch = torch.empty(max(floats, ops.attention_generic_scratch_floats(B, nh, d, 4)), device=DEV)
+        if fused:
+            ops.attention_mma_append(x, out, B, nh, nkv, d, d ** -0.5, 0, None, None, 1e-5, angles.cos(), angles.sin(), *where, scratch, 444, 0, 64, st)
+        else:
+            ops.qk_norm_rope_append(x, B, nh, nkv, d, None, None, 1e-5, angles.cos(), angles.sin(), d, t, past, ps.seq_slot, qstart, ps.table,
+                                    ps.num_pages, ps.k_pages, ps.v_pages, True, st)
+            ops.attention_mma(True, x, out, B, 1, nh, nkv, d, d ** -0.5, 0, *where, scratch, 64, 4, st)
+        outs.append(out.float())
+    assert st.tolist()[0] == 0 and rel_err(outs[0], outs[1]) < 2 * ATT_TOL[bf]
 
 
 @pytest.mark.parametrize("d,dv,kind", [(36, 96, "delta"), (64, 126, "mlstm")])
