@@ -889,6 +889,7 @@ __global__ void decode_merge_kernel(Args a) {
 // Warp 4 looks pages up, a lane each, and keeps STAGES of them on their way across the pairs' borders; warps 0-3 fold them as
 // above, a quarter of the keys each, and meet only where a pair ends (then they sum through the page they have just read).
 constexpr int kSharedSeqs = 512;       // sequences whose page counts a block holds
+constexpr int kLastPolls = 1000;       // polls that copies in flight get before a block leaves
 
 struct SharedArgs {
   int n_seqs;
@@ -939,7 +940,6 @@ __global__ void __launch_bounds__(160, shared_blocks_per_sm(HD)) decode_shared_k
   __shared__ int warp_pages[4];
   __shared__ volatile int failed;
   __shared__ float ml[4 * 16 * 2];
-  __shared__ int stage_page[STAGES];           // the page of the cache in a stage, -1: outside the pool
   char* smem = align_1024(smem_raw);
   constexpr int STAGE = BN * HD * 4;
   constexpr int KS = HD / 16;
@@ -997,7 +997,8 @@ __global__ void __launch_bounds__(160, shared_blocks_per_sm(HD)) decode_shared_k
   const int n_tiles = x1 - x0;      // at least 1: n_blocks <= total
 
   if (warp == 4) {
-    for (int base = 0; base < n_tiles; base += 32) {
+    int n_issued = n_tiles;      // fewer where a wait ran out
+    for (int base = 0; base < n_issued; base += 32) {
       int y = 0, page = -1;
       if (base + lane < n_tiles) {
         const Place p(before, sh.n_seqs, n_kv, x0 + base + lane);
@@ -1006,22 +1007,25 @@ __global__ void __launch_bounds__(160, shared_blocks_per_sm(HD)) decode_shared_k
         if (logical < a.table_stride) page = a.page_table[(size_t)slot * a.table_stride + logical];
         if (page < 0 || page >= a.num_pages) {
           report(a.status, kStatusPageOutOfRange, slot, page, logical * BN);
-          page = -1;
+          page = 0;
         }
-        y = (max(page, 0) * n_kv + p.kvh) * BN;
+        y = (page * n_kv + p.kvh) * BN;
       }
       const int n = min(32, n_tiles - base);
       for (int l = 0; l < n; ++l) {
         const int it = base + l, s = it % STAGES;
-        const int py = __shfl_sync(0xffffffffu, y, l), its_page = __shfl_sync(0xffffffffu, page, l);
-        if (it >= STAGES && !failed && !tma::mbar_wait(&empty[s], (it / STAGES - 1) & 1)) {
-          if (lane == 0) report(a.status, kStatusWaitTimedOut, 3, me, it);
-          failed = 1;
+        const int py = __shfl_sync(0xffffffffu, y, l);
+        if (it >= STAGES) {      // the warp goes on or gives up as one: lane 0 waits
+          const int free = __shfl_sync(0xffffffffu, lane == 0 ? int(!failed && tma::mbar_wait(&empty[s], (it / STAGES - 1) & 1)) : 0, 0);
+          if (!free) {
+            if (lane == 0 && !failed) report(a.status, kStatusWaitTimedOut, 3, me, it);
+            if (lane == 0) failed = 1;
+            n_issued = it;
+            break;
+          }
         }
-        if (failed) break;
         if (lane == 0) {
           char* stage = smem + s * STAGE;
-          stage_page[s] = its_page;      // read behind the barrier
           tma::mbar_expect_tx(&full[s], STAGE);
 #pragma unroll
           for (int sub = 0; sub < HD / 64; ++sub) {
@@ -1032,10 +1036,11 @@ __global__ void __launch_bounds__(160, shared_blocks_per_sm(HD)) decode_shared_k
         __syncwarp();
       }
     }
-    if (failed && lane == 0)      // copies still in flight get a bounded chance to land before the block leaves
-      for (int s = 0; s < STAGES; ++s)
-        for (int i = 0; i < 1000; ++i)
-          if (tma::mbar_try_wait(&full[s], 0) && tma::mbar_try_wait(&full[s], 1)) break;
+    // A block leaves only when its copies have landed, or have had a bounded chance to: consumers that gave up do not wait for
+    // them.  (A stage's copies follow one another, so it is empty when the last of them is there.)
+    if (lane == 0)
+      for (int it = max(0, n_issued - STAGES); it < n_issued; ++it)
+        for (int i = 0; i < kLastPolls && !tma::mbar_try_wait(&full[it % STAGES], (it / STAGES) & 1); ++i) {}
     return;
   }
 
@@ -1089,12 +1094,19 @@ __global__ void __launch_bounds__(160, shared_blocks_per_sm(HD)) decode_shared_k
   clear();
   Visible seen(a, a.seq_past[at.b]);
   int first = at.tile;      // of this pair, in this block
+  bool gone = false;        // this warp waits no more
 
   for (int it = 0; it < n_tiles; ++it) {
     const int s = it % STAGES;
     const bool pair_ends = at.tile + 1 == seen.tiles, last = pair_ends || it + 1 == n_tiles;
     Place next = at;
+    // Where the new key and value go (-1: nowhere), asked for here so that the page's wait covers it.  The table says it and not the
+    // page ring: it holds whatever has become of the copies.
+    int page = -1;
     if (pair_ends) {
+      const int logical = (seen.len - 1) / BN;
+      if (logical < a.table_stride) page = a.page_table[(size_t)a.seq_slot[at.b] * a.table_stride + logical];
+      if (page >= a.num_pages || (ap.cos && seen.len > ap.rows)) page = -1;      // (the producer reports the first)
       next.tile = 0;
       if (++next.kvh == n_kv) {
         next.kvh = 0;
@@ -1104,15 +1116,16 @@ __global__ void __launch_bounds__(160, shared_blocks_per_sm(HD)) decode_shared_k
     } else {
       ++next.tile;
     }
-    if (!failed && !tma::mbar_wait(&full[s], (it / STAGES) & 1)) {
-      if (lane == 0) report(a.status, kStatusWaitTimedOut, 2, me, it);
-      failed = 1;      // nobody waits any more; what is left is computed from whatever is there, and the step reports the status
+    if (!__all_sync(0xffffffffu, !gone && !failed && tma::mbar_wait(&full[s], (it / STAGES) & 1))) {
+      // nobody waits any more; what is left is computed from whatever is there, and the step reports the status
+      if (lane == 0 && !failed) report(a.status, kStatusWaitTimedOut, 2, me, it);
+      if (lane == 0) failed = 1;
+      gone = true;
     }
     char* stage = smem + s * STAGE;
     if (pair_ends) {
-      const bool known = !ap.cos || seen.len <= ap.rows;
-      if (!known && tid == 0) report(a.status, kStatusPositionOutOfRange, a.seq_qstart[at.b], seen.len - 1, ap.rows);
-      append_row<HD>(a, ap, stage, seen.len, at.kvh, known ? stage_page[s] : -1, kv_lo, kv_hi);
+      if (ap.cos && seen.len > ap.rows && tid == 0) report(a.status, kStatusPositionOutOfRange, a.seq_qstart[at.b], seen.len - 1, ap.rows);
+      append_row<HD>(a, ap, stage, seen.len, at.kvh, page, kv_lo, kv_hi);
       bar_sync_consumers();
     }
     decode_fold_page<HD, HD, false>(smem_u32(stage), smem_u32(stage) + BN * HD * 2, warp * 16, seen.key0(at.tile), seen.win_lo, seen.len,
@@ -1172,7 +1185,7 @@ __global__ void __launch_bounds__(160, shared_blocks_per_sm(HD)) decode_shared_k
       }
     }
     __syncwarp();
-    if (lane == 0) tma::mbar_arrive(&empty[s]);
+    if (lane == 0 && !gone) tma::mbar_arrive(&empty[s]);      // (a page that nobody has waited for keeps its stage)
     if (pair_ends && next.b != at.b && it + 1 < n_tiles) seen = Visible(a, a.seq_past[next.b]);
     at = next;
   }

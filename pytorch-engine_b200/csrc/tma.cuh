@@ -48,7 +48,11 @@ inline int make_map_2d_bf16(CUtensorMap* map, const void* base, uint64_t inner, 
 // ---- device ----------------------------------------------------------------------------------------
 // Polls before a wait gives up.  A poll that finds the phase incomplete comes back after about 2 us (measured: 100,000
 // failing `mbarrier.try_wait` in 198 ms), so this is about two seconds, far beyond any healthy wait inside a kernel.
-constexpr uint32_t kWaitLimit = 1000u * 1000u;
+// (A test compiles a file with none, so that every wait in it runs out.)
+#ifndef PE_WAIT_POLLS
+#define PE_WAIT_POLLS (1000u * 1000u)
+#endif
+constexpr uint32_t kWaitLimit = PE_WAIT_POLLS;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

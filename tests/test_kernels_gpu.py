@@ -1,6 +1,10 @@
 """Each CUDA kernel alone against its plain reference, at sizes other than the engine's."""
+import ctypes
+import importlib
 import math
+import os
 import random
+import subprocess
 
 import pytest
 import torch
@@ -718,6 +722,47 @@ def test_attention_mma_append_of_many_sequences(ops, B):
             ops.attention_mma(True, x, out, B, 1, nh, nkv, d, d ** -0.5, 0, *where, scratch, 64, 4, st)
         outs.append(out.float())
     assert st.tolist()[0] == 0 and rel_err(outs[0], outs[1]) < 2 * ATT_TOL[bf]
+
+
+class _Impatient:
+    """The library, but for the entry points of one file compiled so that every bounded wait runs out at once."""
+
+    def __init__(self, pe, folder, source):
+        build, lib = pe.kernels.build, importlib.import_module("pytorch-engine_b200.kernels.lib")
+        path = os.path.join(str(folder), "impatient.so")
+        subprocess.run([build._find_nvcc(), *build.NVCC_FLAGS, "-DPE_WAIT_POLLS=0", "-I", build.CSRC, "-shared", os.path.join(build.CSRC, source),
+                        "-o", path], check=True)
+        self._usual, self._own = lib.library(), ctypes.CDLL(path)
+        for name, argtypes in lib._SIGNATURES.items():
+            if hasattr(self._own, name):
+                getattr(self._own, name).argtypes = argtypes
+
+    def __getattr__(self, name):
+        return getattr(self._own if name == "pe_attention_mma_append" else self._usual, name)
+
+
+def test_attention_mma_append_whose_waits_run_out(ops, pe, tmp_path, monkeypatch):
+    """Keys shared out, and no wait ends: the step comes back with a status, every sequence's new row is in its own page and no
+    other row of the cache has changed.  (Pages in the ring may then be anybody's; outputs say nothing.)"""
+    torch.manual_seed(31)
+    nh, nkv, d, bf, lens = 8, 2, 128, torch.bfloat16, [700, 1, 65, 64, 513]
+    B, t = len(lens), torch.arange(len(lens), dtype=torch.int32, device=DEV)
+    qkv, angles = torch.randn(B, (nh + 2 * nkv) * d, device=DEV).to(bf), torch.rand(704, d // 2, device=DEV) * 6
+    qstart, past = torch.arange(B + 1, dtype=torch.int32, device=DEV), torch.tensor([L - 1 for L in lens], dtype=torch.int32, device=DEV)
+    usual, impatient = ops.library(), _Impatient(pe, tmp_path, "attention_mma.cu")
+    for blocks in (1, 3, 40):
+        floats = int(usual.pe_attention_mma_shared_scratch_floats(B, nh, nkv, d, blocks))
+        pages = []
+        for library in (impatient, usual):
+            ps, st = PagedSetup(lens, nkv, d, bf, seed=31), _status()
+            scratch, out = torch.full((floats + 64,), float("nan"), device=DEV), torch.empty(B, nh * d, device=DEV, dtype=bf)
+            monkeypatch.setattr(ops, "library", lambda: library)
+            ops.attention_mma_append(qkv, out, B, nh, nkv, d, d ** -0.5, 0, None, None, 1e-5, angles.cos(), angles.sin(), qstart, past,
+                                     ps.seq_slot, ps.table, ps.num_pages, ps.k_pages, ps.v_pages, scratch, blocks, 0, 64, st)
+            assert st.tolist()[0] == (4 if library is impatient else 0)
+            assert bool(scratch[floats:].isnan().all())
+            pages.append((ps.k_pages, ps.v_pages))
+        assert all(torch.equal(a, b) for a, b in zip(*pages))
 
 
 @pytest.mark.parametrize("d,dv,kind", [(36, 96, "delta"), (64, 126, "mlstm")])
