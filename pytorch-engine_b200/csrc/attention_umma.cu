@@ -644,9 +644,10 @@ prefill_umma_kernel(Args a, const __grid_constant__ CUtensorMap qmap, const __gr
         fence_after_sync();
         const int tok = row / group, head = w.kvh * group + row % group;
         if (a.parts > 1) {
-          const float inv = l > 0.f ? 1.f / l : 0.f;
+          // (no visible key where the denominator is 0; one that is NaN goes on to the merge, as it would to the outputs)
+          const float inv = l != 0.f ? 1.f / l : 0.f;
           const size_t at = (size_t)w.part * a.part_rows + (size_t)(w.q0 + tok) * a.n_heads + head;
-          if (live) a.part_lse[at] = l > 0.f ? m_ref + log2f(l) : -INFINITY;
+          if (live) a.part_lse[at] = l != 0.f ? m_ref + log2f(l) : -INFINITY;
           float* dst = a.part_out + at * a.vd;
 #pragma unroll 1
           for (int c = 0; c < a.vd; c += 32) {

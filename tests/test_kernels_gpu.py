@@ -888,6 +888,41 @@ def test_attention_umma_prefill_in_parts(ops, nh, nkv, d, dv, parts, window, sin
     assert rel_err(outs[1], outs[0]) < 2 * ATT_TOL[bf]
 
 
+@pytest.mark.parametrize("parts", [3, 8])
+@pytest.mark.parametrize("where,number", [("key", "nan"), ("key", "inf"), ("value", "nan"), ("value", "inf"), ("query", "nan"), ("query", "inf")])
+def test_attention_umma_prefill_in_parts_keeps_nan_and_infinity(ops, parts, where, number):
+    """One number that is none, in a cached key or value that every row of the first sequence sees or in one query: with parts the same
+    outputs are NaN as with one block a tile, and the rows that do not see it have the bits they have without it."""
+    torch.manual_seed(32)
+    bf, nh, nkv, d = torch.bfloat16, 8, 2, 128
+    q_lens, pasts = [70, 33], [900, 512]
+    N, st = sum(q_lens), _status()
+    q = torch.randn(N, (nh + nkv) * d, device=DEV).to(bf)
+    qstart, past = torch.tensor([0, 70, N], dtype=torch.int32, device=DEV), torch.tensor(pasts, dtype=torch.int32, device=DEV)
+
+    def run(n, poisoned):
+        ps, x = PagedSetup([a + b for a, b in zip(q_lens, pasts)], nkv, d, bf, seed=32, key_scale=2.0), q.clone()
+        page = int(ps.table[ps.slots[0], 300 // 64])
+        if poisoned:
+            row = {"key": ps.k_pages[page, 1, 300 % 64], "value": ps.v_pages[page, 1, 300 % 64], "query": x[5, 2 * d:3 * d]}[where]
+            row[7] = float(number)
+        out = torch.full((N, nh * d), 7.0, device=DEV, dtype=bf)
+        scratch = torch.empty(n * N * nh * (d + 1), device=DEV)
+        ops.attention_umma_prefill(x, out, 2, max(q_lens), nh, nkv, d, d ** -0.5, 0, qstart, past, ps.seq_slot, ps.table, ps.num_pages,
+                                   ps.k_pages, ps.v_pages, st, parts=n, scratch=scratch)
+        assert st.tolist()[0] == 0
+        return out.float().view(N, nh, d)
+
+    one, cut, clean = run(1, True), run(parts, True), run(parts, False)
+    assert torch.equal(one.isfinite(), cut.isfinite()) and not bool(cut.isfinite().all())
+    sees = torch.zeros(N, nh, dtype=torch.bool, device=DEV)
+    if where == "query":
+        sees[5, 2] = True
+    else:
+        sees[:70, nh // 2:] = True
+    assert torch.equal(cut[~sees], clean[~sees]) and bool(clean.isfinite().all())
+
+
 @pytest.mark.parametrize("decode", [False, True])
 def test_attention_mma_finds_a_far_key_and_ignores_what_lies_beyond_the_length(ops, decode):
     nh, nkv, d = 8, 2, 128
