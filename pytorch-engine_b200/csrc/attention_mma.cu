@@ -731,15 +731,13 @@ __global__ void __launch_bounds__(128) decode_split_kernel(Args a, Append ap, co
     float mm = -INFINITY;
 #pragma unroll
     for (int w = 0; w < 4; ++w) mm = fmaxf(mm, ml[(w * 16 + r) * 2]);
-    float ll = 0.f, aa = 0.f;
-    if (mm != -INFINITY) {
+    float ll = 0.f, aa = 0.f;      // (without a visible key: 0; scores that are NaN leave the maximum at -inf and NaN in both)
 #pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        const float mw = ml[(w * 16 + r) * 2];
-        const float f = (mw == -INFINITY) ? 0.f : fast_exp2(mw - mm);
-        ll += ml[(w * 16 + r) * 2 + 1] * f;
-        aa += acc[(size_t)(w * 16 + r) * VD + c] * f;
-      }
+    for (int w = 0; w < 4; ++w) {
+      const float mw = ml[(w * 16 + r) * 2];
+      const float f = (mw == -INFINITY) ? 0.f : fast_exp2(mw - mm);
+      ll += ml[(w * 16 + r) * 2 + 1] * f;
+      aa += acc[(size_t)(w * 16 + r) * VD + c] * f;
     }
     if (CLUSTER) {
       res[r * VD + c] = aa;
@@ -750,9 +748,9 @@ __global__ void __launch_bounds__(128) decode_split_kernel(Args a, Append ap, co
       continue;
     }
     const size_t pidx = ((size_t)b * a.n_heads + (kvh * group + r)) * a.max_splits + split;
-    a.part_acc[pidx * vd + c] = (ll > 0.f) ? aa / ll : 0.f;
+    a.part_acc[pidx * vd + c] = (ll != 0.f) ? aa / ll : 0.f;
     // log-sum-exp in natural units, as the merge kernel expects: (m + log2 l) * ln 2
-    if (c == 0) a.part_lse[pidx] = (ll > 0.f) ? (mm + log2f(ll)) * 0.6931471805599453f : -INFINITY;
+    if (c == 0) a.part_lse[pidx] = (ll != 0.f) ? (mm + log2f(ll)) * 0.6931471805599453f : -INFINITY;
   }
   if (CLUSTER) {
     // the ranges that hold something, and this one's place among them (as in the merge kernel below)
@@ -848,13 +846,12 @@ __global__ void decode_merge_kernel(Args a) {
       float m_new = mx;
 #pragma unroll
       for (int i = 0; i < G; ++i) m_new = fmaxf(m_new, e[i]);
-      if (m_new == -INFINITY) continue;
       const float keep = (mx == -INFINITY) ? 0.f : expf(mx - m_new);
       denom *= keep;
       v *= keep;
 #pragma unroll
       for (int i = 0; i < G; ++i) {
-        const float w = (e[i] == -INFINITY) ? 0.f : expf(e[i] - m_new);
+        const float w = (e[i] == -INFINITY) ? 0.f : expf(e[i] - m_new);      // (NaN: its range's scores were)
         denom += w;
         v = fmaf(w, acc[i], v);
       }
@@ -1154,20 +1151,18 @@ __global__ void __launch_bounds__(160, shared_blocks_per_sm(HD)) decode_shared_k
         float mm = -INFINITY;
 #pragma unroll
         for (int w = 0; w < 4; ++w) mm = fmaxf(mm, ml[(w * 16 + r) * 2]);
-        float ll = 0.f, aa = 0.f;
-        if (mm != -INFINITY) {
+        float ll = 0.f, aa = 0.f;      // (as above: NaN stays NaN)
 #pragma unroll
-          for (int w = 0; w < 4; ++w) {
-            const float mw = ml[(w * 16 + r) * 2];
-            const float f = (mw == -INFINITY) ? 0.f : fast_exp2(mw - mm);
-            ll += ml[(w * 16 + r) * 2 + 1] * f;
-            aa += acc[(size_t)(w * group + r) * HD + c] * f;
-          }
+        for (int w = 0; w < 4; ++w) {
+          const float mw = ml[(w * 16 + r) * 2];
+          const float f = (mw == -INFINITY) ? 0.f : fast_exp2(mw - mm);
+          ll += ml[(w * 16 + r) * 2 + 1] * f;
+          aa += acc[(size_t)(w * group + r) * HD + c] * f;
         }
         if (!whole) {
           const size_t pidx = (size_t)part * group + r;
-          a.part_acc[pidx * HD + c] = (ll > 0.f) ? aa / ll : 0.f;
-          if (c == 0) a.part_lse[pidx] = (ll > 0.f) ? (mm + log2f(ll)) * 0.6931471805599453f : -INFINITY;
+          a.part_acc[pidx * HD + c] = (ll != 0.f) ? aa / ll : 0.f;
+          if (c == 0) a.part_lse[pidx] = (ll != 0.f) ? (mm + log2f(ll)) * 0.6931471805599453f : -INFINITY;
           continue;
         }
         a.out[(size_t)tq * a.out_ld + (size_t)h * HD + c] = __float2bfloat16_rn(aa / fmaxf(ll, 1e-20f));
@@ -1217,13 +1212,12 @@ __global__ void decode_shared_merge_kernel(Args a, SharedArgs sh) {
     float m_new = mx;
 #pragma unroll
     for (int i = 0; i < G; ++i) m_new = fmaxf(m_new, e[i]);
-    if (m_new == -INFINITY) continue;
     const float keep = (mx == -INFINITY) ? 0.f : expf(mx - m_new);
     denom *= keep;
     v *= keep;
 #pragma unroll
     for (int i = 0; i < G; ++i) {
-      const float w = (e[i] == -INFINITY) ? 0.f : expf(e[i] - m_new);
+      const float w = (e[i] == -INFINITY) ? 0.f : expf(e[i] - m_new);      // (NaN: its block's scores were)
       denom += w;
       v = fmaf(w, acc[i], v);
     }

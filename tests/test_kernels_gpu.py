@@ -724,6 +724,48 @@ def test_attention_mma_append_of_many_sequences(ops, B):
     assert st.tolist()[0] == 0 and rel_err(outs[0], outs[1]) < 2 * ATT_TOL[bf]
 
 
+@pytest.mark.parametrize("form", ["ranges", "clusters", 1, 5, 40])      # a number: keys shared out over so many blocks
+@pytest.mark.parametrize("where,number", [("key", "nan"), ("key", "inf"), ("value", "nan"), ("value", "inf"), ("query", "nan"), ("query", "inf")])
+def test_decode_attention_keeps_nan_and_infinity(ops, form, where, number):
+    """One number that is none, in a cached key, value or query: outputs that it reaches are not finite, whichever range, block or warp
+    it falls to, and all others have the bits they have without it."""
+    torch.manual_seed(33)
+    bf, nh, nkv, d, lens = torch.bfloat16, 8, 2, 64, [700, 130]
+    B, st = len(lens), _status()
+    qkv, t = torch.randn(B, (nh + 2 * nkv) * d, device=DEV).to(bf), torch.arange(len(lens), dtype=torch.int32, device=DEV)
+    qstart, past = torch.arange(B + 1, dtype=torch.int32, device=DEV), torch.tensor([L - 1 for L in lens], dtype=torch.int32, device=DEV)
+
+    def run(poisoned):
+        ps, x = PagedSetup(lens, nkv, d, bf, seed=33), qkv.clone()
+        page = int(ps.table[ps.slots[0], 300 // 64])
+        if poisoned:
+            {"key": ps.k_pages[page, 1, 300 % 64], "value": ps.v_pages[page, 1, 300 % 64], "query": x[0, 2 * d:3 * d]}[where][7] = float(number)
+        out, blocks = torch.full((B, nh * d), 7.0, device=DEV, dtype=bf), form if isinstance(form, int) else 0
+        floats = int(ops.library().pe_attention_mma_shared_scratch_floats(B, nh, nkv, d, max(blocks, 1)))
+        scratch = torch.empty(max(floats, ops.attention_generic_scratch_floats(B, nh, d, 11)), device=DEV)
+        where_to = (qstart, past, ps.seq_slot, ps.table, ps.num_pages, ps.k_pages, ps.v_pages)
+        if form == "ranges":
+            ops.qk_norm_rope_append(x, B, nh, nkv, d, None, None, 1e-5, None, None, 0, t, past, ps.seq_slot, qstart, ps.table, ps.num_pages,
+                                    ps.k_pages, ps.v_pages, True, st)
+            ops.attention_mma(True, x, out, B, 1, nh, nkv, d, d ** -0.5, 0, *where_to, scratch, 64, 11, st)
+        else:
+            ops.attention_mma_append(x, out, B, nh, nkv, d, d ** -0.5, 0, None, None, 1e-5, None, None, *where_to, scratch, blocks, 4, 64, st)
+        assert st.tolist()[0] == 0
+        return out.float().view(B, nh, d)
+
+    reached = torch.zeros(B, nh, d, dtype=torch.bool, device=DEV)
+    if where == "query":
+        reached[0, 2] = True
+    elif where == "value":
+        reached[0, nh // 2:, 7] = True
+    else:      # a score of minus infinity weighs nothing
+        reached[0, nh // 2:] = (qkv[0, nh // 2 * d:nh * d].view(-1, d)[:, 7:8] > 0) | (number == "nan")
+    got, clean = run(True), run(False)
+    assert torch.equal(got.isfinite(), ~reached)
+    if number == "nan":
+        assert torch.equal(got[~reached], clean[~reached]) and bool(clean.isfinite().all())
+
+
 class _Impatient:
     """The library, but for the entry points of one file compiled so that every bounded wait runs out at once."""
 
