@@ -17,7 +17,8 @@
 // of a row, which hold every entry that the row's top-k can keep.
 //   top-k up to kTopMax: the first leaves the largest value of every group of 8 to 512 neighbouring entries and nothing else
 //     (sample_maxima_kernel); the second bounds the row's k-th value by the k-th of the maxima, which has k entries at or above
-//     it, and reads again only the groups whose maximum reaches it.
+//     it, and reads again only the groups whose maximum reaches it.  A row whose groups tie (most entries one and the same
+//     number) is searched whole.
 //   larger top-k: chunks of kChunk entries in shared memory, threshold search (sample_chunks_kernel).
 // A threshold search over a row takes 8 sweeps of 4 bits with per-thread counters (no atomics, fixed
 // summation order) instead of 32 sweeps of one bit.
@@ -32,9 +33,8 @@ constexpr int kChunk = 4096;        // entries of a row per block of the first k
 constexpr int kChunkThreads = 256;
 constexpr int kMaxChunks = 64;
 constexpr int kMaxCandidates = 3072;  // candidates of a row that the second kernel takes
-constexpr int kGroupThreads = 512;      // threads of the second kernel where the first left groups' maxima
-constexpr int kGroupsPer = 5;           // maxima a thread of it holds
-constexpr int kMaxGroups = kGroupThreads * kGroupsPer;
+constexpr int kMaxGroups = 2560;        // groups of a row whose maxima the second kernel holds, in registers
+constexpr int kGroupsPer = (kMaxGroups + kSampleThreads - 1) / kSampleThreads;
 constexpr int kMaximaThreads = 256;
 constexpr int kMaximaTask = 1024;       // entries a warp of the first kernel takes: eight 16-byte loads a lane
 constexpr int kMaxGroupList = 1024;     // groups that the second kernel reads again
@@ -368,15 +368,15 @@ __global__ void __launch_bounds__(kChunkThreads) sample_chunks_kernel(SampleArgs
 }
 
 // The second kernel, or the only one.  GROUPS: the first left groups' maxima.
-template <int THREADS, bool GROUPS>
-__global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
-  constexpr int kSampleThreads = THREADS;
+template <bool GROUPS>
+__global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleArgs a) {
   __shared__ float red_f[33 * 16];
   __shared__ int red_i[33 * 16];
   __shared__ ArgBest red_b[32];
   __shared__ float c_val[kMaxCompact];
   __shared__ int c_idx[kMaxCompact];
-  __shared__ int scan[kMaxGroupList > kSampleThreads ? kMaxGroupList : kSampleThreads];
+  __shared__ int scan[kSampleThreads];      // (GROUPS: the list of groups, later of kept entries)
+  static_assert(kMaxGroupList <= kSampleThreads && kMaxRanked <= kSampleThreads, "lists in `scan`");
   __shared__ float l_val[kMaxCandidates];
   __shared__ int l_idx[kMaxCandidates];
   __shared__ int chunk_base[kMaxChunks], chunk_cnt[kMaxChunks];
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
     unsigned gkey[kGroupsPer];
 #pragma unroll
     for (int j = 0; j < kGroupsPer; ++j) {
-      const int g = j * THREADS + tid;
+      const int g = j * kSampleThreads + tid;
       gkey[j] = g < a.n_chunks ? ordered_key(scaled(maxima[g], mult)) : 0u;
     }
     const int k = min(a.top_k, V), slack = k / 8 + 8;
@@ -421,10 +421,10 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
     for (int j = 0; j < kGroupsPer; ++j) mine += gkey[j] >= bound;
     int pos = block_offset(mine, red_i, &n_list);
     if (n_list <= kMaxGroupList) {      // (more only where groups tie)
-      int* list = scan;                 // in c_idx's place would do as well: neither is in use yet
+      int* list = scan;
 #pragma unroll
       for (int j = 0; j < kGroupsPer; ++j)
-        if (gkey[j] >= bound) list[pos++] = j * THREADS + tid;
+        if (gkey[j] >= bound) list[pos++] = j * kSampleThreads + tid;
       __syncthreads();
       // the groups' entries that reach the bound, a thread's quads one after the other: counted, then written (from the L1)
       const int quads = a.group / 4, n_quads = n_list * quads;
@@ -432,16 +432,37 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
         i = list[e / quads] * a.group + e % quads * 4;
         return load_quad(src, i, V, a.vec);
       };
-      mine = 0;
-      for (int e = tid; e < n_quads; e += THREADS) {
-        int i;
-        const float4 q = quad_at(e, i);
+      auto reach = [&](unsigned least) {      // this thread's entries that reach `least`
+        int n_reach = 0;
+        for (int e = tid; e < n_quads; e += kSampleThreads) {
+          int i;
+          const float4 q = quad_at(e, i);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) mine += i + c < V && ordered_key(scaled((&q.x)[c], mult)) >= bound;
-      }
+          for (int c = 0; c < 4; ++c) n_reach += i + c < V && ordered_key(scaled((&q.x)[c], mult)) >= least;
+        }
+        return n_reach;
+      };
+      mine = reach(bound);
       pos = block_offset(mine, red_i, &total);
+      if (total > kMaxCandidates) {
+        // Large entries next to each other (a row masked to one range, logits that fall with the id): the maxima bound the k-th value
+        // from too far below, and the bound is raised bit by bit on the groups' entries until few enough reach it.  64 rows of
+        // 151,936 falling logits, GPU time of a draw: 57 and 76 us at top-k 50 and 200 (a search over the whole row 818, other rows
+        // 53 and 59).
+        unsigned raised = 0u;
+        for (int bit = 31; bit >= 0; --bit) {
+          const unsigned cand = raised | (1u << bit);
+          int count = kMaxCandidates;
+          if (cand > bound && (count = block_count(reach(cand), red_i)) < k) continue;
+          raised = cand;
+          if (count <= kMaxRanked) break;
+        }
+        bound = max(bound, raised);
+        mine = reach(bound);
+        pos = block_offset(mine, red_i, &total);
+      }
       if (total <= kMaxCandidates) {
-        for (int e = tid; e < n_quads; e += THREADS) {
+        for (int e = tid; e < n_quads; e += kSampleThreads) {
           int i;
           const float4 q = quad_at(e, i);
 #pragma unroll
@@ -511,10 +532,10 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
   if (GROUPS && idxs != nullptr && n <= kMaxRanked) {
     // few candidates: the k-th key is the smallest that fewer than k others exceed
     if (tid == 0) red_i[0] = -1;        // as unsigned the largest key there is
-    for (int i = tid; i < n; i += THREADS) c_idx[i] = (int)ordered_key(l_val[i]);
+    for (int i = tid; i < n; i += kSampleThreads) c_idx[i] = (int)ordered_key(l_val[i]);
     __syncthreads();
     const int k = min(a.top_k, n);
-    for (int i = tid; i < n; i += THREADS) {
+    for (int i = tid; i < n; i += kSampleThreads) {
       const unsigned own = (unsigned)c_idx[i];
       int more = 0;
       for (int j = 0; j < n; ++j) more += (unsigned)c_idx[j] > own;
@@ -523,9 +544,9 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
     __syncthreads();
     keep_key = max((unsigned)red_i[0], kFirstKey);
     int mine = 0, total;
-    for (int i = tid; i < n; i += THREADS) mine += (unsigned)c_idx[i] >= keep_key;
+    for (int i = tid; i < n; i += kSampleThreads) mine += (unsigned)c_idx[i] >= keep_key;
     int pos = block_offset(mine, red_i, &total);
-    for (int i = tid; i < n; i += THREADS)
+    for (int i = tid; i < n; i += kSampleThreads)
       if ((unsigned)c_idx[i] >= keep_key) {
         c_val[pos] = l_val[i];
         scan[pos++] = l_idx[i];
@@ -629,14 +650,14 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
     unsigned J = 0u;
     if (listed) {
       // few entries: each adds up the mass above itself; J is the smallest key that stays
-      for (int i = tid; i < n; i += THREADS) {
+      for (int i = tid; i < n; i += kSampleThreads) {
         const float v = vals[i];
         l_val[i] = ordered_key(v) >= kk ? expf(v - mx) : 0.f;
         l_idx[i] = (int)ordered_key(v);
       }
       if (tid == 0) red_i[0] = -1;   // as unsigned the largest key there is
       __syncthreads();
-      for (int i = tid; i < n; i += THREADS) {
+      for (int i = tid; i < n; i += kSampleThreads) {
         const unsigned own = (unsigned)l_idx[i];
         float mass = 0.f;
         for (int j = 0; j < n; ++j) mass += (unsigned)l_idx[j] > own ? l_val[j] : 0.f;
@@ -766,14 +787,14 @@ extern "C" int pe_sample(const float* logits, long long ld, int n_rows, int voca
       const int tasks = (vocab + pe::kMaximaTask - 1) / pe::kMaximaTask, warps = pe::kMaximaThreads / 32;
       pe::launch(pe::sample_maxima_kernel, dim3((tasks + warps - 1) / warps, n_rows), pe::kMaximaThreads, 0, stream, a);
       PE_LAUNCH_CHECK();
-      pe::launch(pe::sample_kernel<pe::kGroupThreads, true>, n_rows, pe::kGroupThreads, 0, stream, a);
+      pe::launch(pe::sample_kernel<true>, n_rows, pe::kSampleThreads, 0, stream, a);
       PE_LAUNCH_CHECK();
       return PE_OK;
     }
     pe::launch(pe::sample_chunks_kernel, dim3(a.n_chunks, n_rows), pe::kChunkThreads, 0, stream, a);
     PE_LAUNCH_CHECK();
   }
-  pe::launch(pe::sample_kernel<pe::kSampleThreads, false>, n_rows, pe::kSampleThreads, 0, stream, a);
+  pe::launch(pe::sample_kernel<false>, n_rows, pe::kSampleThreads, 0, stream, a);
   PE_LAUNCH_CHECK();
   return PE_OK;
 }

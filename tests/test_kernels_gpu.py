@@ -1385,6 +1385,45 @@ def test_sampler_top_k_at_the_edges_of_its_chunks(ops, V, k):
             assert probs[a[r]] > 0
 
 
+@pytest.mark.parametrize("V,k", [(50001, 50), (50001, 200), (151936, 1), (151936, 224)])
+def test_sampler_large_entries_side_by_side(ops, V, k):
+    """Rows whose largest entries fill a few groups, so that their maxima bound the k-th value from far below, and rows of ties: the
+    same draws as one kernel over the whole row, and (but for the ties) in a few times what other rows take."""
+    torch.manual_seed(34)
+    x = torch.randn(8, V, device=DEV) * 2.5
+    rows = torch.arange(V, device=DEV) * -1e-3 + 5e-4 * x     # fall with the id
+    rows[1] = x[1].sort(descending=True)[0]
+    rows[2] = torch.full_like(x[2], -float("inf"))
+    rows[2, 20000:25000] = x[2, 20000:25000]                  # some thousand entries of one range
+    rows[3] = x[3].sort()[0]                                  # the last, ragged group holds the largest
+    rows[4, ::7] = float("nan")
+    rows[5, 1000:1000 + 2 * k] = 6.0                          # ties at the top
+    rows[6] = 0.25                                            # nothing but ties
+    rows[7] = torch.where(rows[2].isinf(), torch.full_like(x[7], -1e9), x[7])
+    req, step = torch.arange(8, dtype=torch.int32, device=DEV), torch.zeros(8, dtype=torch.int32, device=DEV)
+    scratch = torch.empty(ops.sample_scratch_bytes(8, V, 0.8, k, 0.95, 0.0), dtype=torch.uint8, device=DEV)
+    a, b = (torch.empty(8, dtype=torch.int32, device=DEV) for _ in range(2))
+    for top_p, min_p in ((1.0, 0.0), (0.95, 0.0), (0.7, 0.02)):
+        ops.sample(rows, 0.8, k, top_p, min_p, 3, req, step, a, scratch=scratch)
+        ops.sample(rows, 0.8, k, top_p, min_p, 3, req, step, b)
+        assert a.tolist() == b.tolist(), (top_p, min_p)
+
+    def took(logits):
+        times = []
+        for _ in range(9):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda._sleep(100000)                         # the launches are queued behind this
+            start.record()
+            ops.sample(logits, 0.8, k, 0.95, 0.0, 3, req, step, a, scratch=scratch)
+            end.record()
+            torch.cuda.synchronize()
+            times.append(start.elapsed_time(end))
+        return sorted(times)[4]
+
+    # a search over the whole row takes some fifteen times as long as a draw from other rows
+    assert took(rows[:6].repeat(2, 1)[:8]) < 6 * took(x)
+
+
 def test_sampler_with_scratch_unfiltered_draw_is_the_single_kernels(ops):
     torch.manual_seed(13)
     rows, V = 12, 30000
