@@ -28,7 +28,9 @@ class BufferPool:
         self._views: Dict[tuple, torch.Tensor] = {}   # (name, dtype, shape) -> view of the current buffer
 
     def get(self, name: str, shape: Sequence[int], dtype: torch.dtype) -> torch.Tensor:
-        view = self._views.get((name, dtype, shape)) if type(shape) is tuple else None
+        if type(shape) is not tuple:
+            shape = tuple(int(s) for s in shape)
+        view = self._views.get((name, dtype, shape))
         if view is not None:
             return view
         shape = tuple(int(s) for s in shape)

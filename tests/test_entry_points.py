@@ -204,3 +204,11 @@ def test_parts_of_a_prefill_and_ranges_of_a_decode_with_append(pe):
         for keys in (1, 64, 65, 400, 40960):
             n, least = ranges(n_seqs, nkv, keys)
             assert 1 <= n <= 8 and n * n_seqs * nkv <= 64 and (n - 1) * least < keys
+
+
+def test_buffers_are_asked_for_by_any_sequence_of_sizes(pe):
+    """The same view again for a tuple, a list and a ``torch.Size``; a larger buffer replaces the views of the smaller one."""
+    pool = pe.engine.BufferPool("cpu")
+    view = pool.get("x", (2, 3), torch.float32)
+    assert all(pool.get("x", shape, torch.float32) is view for shape in ([2, 3], torch.Size([2, 3]), (2, 3)))
+    assert pool.get("x", [4, 3], torch.float32).data_ptr() == pool.get("x", (2, 3), torch.float32).data_ptr() and pool.nbytes() == 48
