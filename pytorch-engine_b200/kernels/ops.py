@@ -465,6 +465,11 @@ def attention_mma_append(qkv: torch.Tensor, out: torch.Tensor, n_seqs: int, n_he
           and sin.is_contiguous() and cos.shape == sin.shape and cos.shape[1] * 2 == head_dim)), "attention_mma_append: angle tables")
     for w in (q_norm_w, k_norm_w):
         _need(w is None or (w.dtype == torch.float32 and w.is_contiguous() and w.numel() == head_dim), "attention_mma_append: norm weights")
+    _need(n_seqs <= min(seq_qstart.numel(), seq_past.numel(), seq_slot.numel()), "attention_mma_append: a number for each sequence")
+    _need(scratch.dtype == torch.float32 and scratch.is_contiguous(), "attention_mma_append: scratch float32")
+    if blocks:
+        floats = int(library().pe_attention_mma_shared_scratch_floats(n_seqs, n_heads, n_kv_heads, head_dim, blocks))
+        _need(0 < floats <= scratch.numel(), "attention_mma_append: scratch of the blocks' partial results")
     check(library().pe_attention_mma_append(
         _ptr(qkv), qkv.stride(0), _ptr(out), out.stride(0), n_seqs, n_heads, n_kv_heads, head_dim, float(scale), int(window),
         _ptr(q_norm_w), _ptr(k_norm_w), float(eps), _ptr(cos), _ptr(sin), 0 if cos is None else cos.shape[0], _ptr(seq_qstart),

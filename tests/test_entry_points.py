@@ -212,3 +212,34 @@ def test_buffers_are_asked_for_by_any_sequence_of_sizes(pe):
     view = pool.get("x", (2, 3), torch.float32)
     assert all(pool.get("x", shape, torch.float32) is view for shape in ([2, 3], torch.Size([2, 3]), (2, 3)))
     assert pool.get("x", [4, 3], torch.float32).data_ptr() == pool.get("x", (2, 3), torch.float32).data_ptr() and pool.nbytes() == 48
+
+
+def test_shared_decode_attention_refuses_a_scratch_that_is_too_small(pe, monkeypatch):
+    """Too few floats for the blocks asked for, another type, or fewer lengths than sequences: an error before anything is launched."""
+    ops, bf = pe.kernels.ops, torch.bfloat16
+    n_seqs, nh, nkv, d, blocks = 3, 4, 2, 64, 10
+    floats = int(ops.library().pe_attention_mma_shared_scratch_floats(n_seqs, nh, nkv, d, blocks))
+    qkv, out, pages = torch.zeros(n_seqs, (nh + 2 * nkv) * d, dtype=bf), torch.zeros(n_seqs, nh * d, dtype=bf), torch.zeros(4, nkv, 64, d, dtype=bf)
+    ints = [torch.zeros(n, dtype=torch.int32) for n in (n_seqs + 1, n_seqs, n_seqs)]
+    launched = []
+    monkeypatch.setattr(ops, "_stream", lambda: launched.append(1) or 0)
+    monkeypatch.setattr(ops, "_ptr", lambda t: None)
+    monkeypatch.setattr(ops, "check", lambda code, what: None)
+
+    def call(scratch, ints=ints, blocks=blocks):
+        class Library:
+            pe_attention_mma_shared_scratch_floats = ops_library.pe_attention_mma_shared_scratch_floats
+            pe_attention_mma_append = staticmethod(lambda *a: 0)
+        monkeypatch.setattr(ops, "library", Library)
+        ops.attention_mma_append(qkv, out, n_seqs, nh, nkv, d, 0.125, 0, None, None, 1e-6, None, None, *ints, torch.zeros(4, 2, dtype=torch.int32),
+                                 4, pages, pages, scratch, blocks, 0, 64, torch.zeros(4, dtype=torch.int32))
+
+    ops_library = ops.library()
+    call(torch.zeros(floats))
+    call(torch.zeros(1), blocks=0)      # clusters keep no partial results
+    assert len(launched) == 2
+    for bad in (dict(scratch=torch.zeros(floats - 1)), dict(scratch=torch.zeros(floats, dtype=torch.float64)), dict(scratch=torch.zeros(floats), blocks=11),
+                dict(scratch=torch.zeros(floats), ints=[ints[0], ints[1][:2], ints[2]])):
+        with pytest.raises(pe.kernels.lib.KernelError):
+            call(**bad)
+    assert len(launched) == 2
