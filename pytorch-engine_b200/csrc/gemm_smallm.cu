@@ -36,7 +36,7 @@ struct Args {
   int group_rows; long long x_group_stride;
   GluEpilogue glu;             // PAIR: what is done with the two sums
   // CHAIN 1: the input is a residual stream's rows times a norm's weight; outputs are multiplied by rsqrt(mean square + eps) of
-  // their row, whose sum of squares lies in `ss_parts` parts of eight rows each (see CHAIN 2).
+  // their row, whose sum of squares lies in `ss_parts` parts of 8 * NT rows each (see CHAIN 2).
   const float* ss; int ss_parts; float ss_scale, eps;
   // CHAIN 2: outputs are added to the stream ([M, N], stream_ld apart) and not stored; the new rows times `next_w` (the norm
   // behind it; null: nobody reads them) go to next_x in bfloat16, and a block leaves its 16 columns' sums of squares in next_ss.
@@ -416,7 +416,8 @@ extern "C" int pe_gemm_smallm_grouped(const void* x, long long ldx, long long x_
 
 // Up to 32 rows of a pre-norm block's products without kernels for its norms (CHAIN above).
 // pe_gemm_smallm_scaled: y = (x . W^T) * rsqrt(sum of squares / dim + eps) of the row, bfloat16; with pair_offset > 0 the scaled
-// gate and up sums go through the activation as in pe_gemm_smallm_glu.  ss: [ss_parts, 8] float32, 16-byte aligned.
+// gate and up sums go through the activation as in pe_gemm_smallm_glu.  ss: float32, 16-byte aligned, [ss_parts, 8] for M <= 8,
+// [ss_parts, 16] for M <= 16, [ss_parts, 32] beyond.
 extern "C" int pe_gemm_smallm_scaled(const void* x, long long ldx, const void* w, void* y, long long ldy, int M, int N, int K,
                                      int pair_offset, int kind, float limit, float alpha, const float* bias, const float* ss,
                                      int ss_parts, int dim, float eps, int n_sms, cudaStream_t stream) {
@@ -441,7 +442,8 @@ extern "C" int pe_gemm_smallm_scaled(const void* x, long long ldx, const void* w
 }
 
 // pe_gemm_smallm_residual: stream += x . W^T (float32 [M, N], rows stream_ld apart), and with next_w (float32 [N]) next_x =
-// stream * next_w (bfloat16, rows next_ld apart) and next_ss [(N + 15) / 16, 8] = the parts of the new rows' sums of squares.
+// stream * next_w (bfloat16, rows next_ld apart) and next_ss = the parts of the new rows' sums of squares: [(N + 15) / 16, 8] for
+// M <= 8, [(N + 15) / 16, 16] for M <= 16, [(N + 15) / 16, 32] beyond.
 extern "C" int pe_gemm_smallm_residual(const void* x, long long ldx, const void* w, float* rows, long long rows_ld, int M, int N, int K,
                                        const float* next_w, void* next_x, long long next_ld, float* next_ss, int n_sms, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return PE_OK;

@@ -562,12 +562,13 @@ def chain_rows(rows: int) -> int:
 def gemm_smallm_scaled(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, squares: torch.Tensor, eps: float,
                        pair_offset: int = 0, glu=None) -> None:
     """``gemm_smallm`` for up to 32 rows of a residual stream times a norm's weight, whose norm's number is still to come:
-    outputs (before the activation) times ``rsqrt(sum of squares / K + eps)``, ``squares`` ``[parts, chain_rows]`` as
+    outputs (before the activation) times ``rsqrt(sum of squares / K + eps)``, ``squares`` ``[(K + 15) // 16, chain_rows]`` as
     ``gemm_smallm_residual`` leaves it.  ``out`` bfloat16."""
     _need(gemm_smallm_chained(x, weight), "gemm_smallm_scaled: needs bfloat16, M <= 32, K % 8 == 0, contiguous rows")
     _need(out.stride(-1) == 1 and out.dtype == torch.bfloat16, "gemm_smallm_scaled: out bfloat16")
-    _need(squares.dtype == torch.float32 and squares.is_contiguous() and squares.shape[-1] == chain_rows(x.shape[0]), "gemm_smallm_scaled: squares [parts, chain_rows] float32")
     m, k = x.shape
+    _need(squares.dtype == torch.float32 and squares.is_contiguous() and tuple(squares.shape) == ((k + 15) // 16, chain_rows(m)),
+          "gemm_smallm_scaled: squares [(K + 15) // 16, chain_rows] float32")
     n = out.shape[1]
     _need(weight.shape[1] == k and weight.shape[0] == (2 * n if pair_offset else n) and out.shape[0] == m and pair_offset in (0, n),
           "gemm_smallm_scaled: shapes do not match")

@@ -243,3 +243,21 @@ def test_shared_decode_attention_refuses_a_scratch_that_is_too_small(pe, monkeyp
         with pytest.raises(pe.kernels.lib.KernelError):
             call(**bad)
     assert len(launched) == 2
+
+
+@pytest.mark.parametrize("rows,columns", [(1, 8), (8, 8), (9, 16), (16, 16), (17, 32), (32, 32)])
+def test_chained_products_refuse_squares_of_another_width(pe, monkeypatch, rows, columns):
+    """The squares' parts are one per 16 features of the stream and 8, 16 or 32 rows wide: any other shape is an error."""
+    ops, bf, k, n = pe.kernels.ops, torch.bfloat16, 72, 24
+    launched = []
+    monkeypatch.setattr(ops, "_ptr", lambda t: None)
+    monkeypatch.setattr(ops, "_stream", lambda: launched.append(1) or 0)
+    monkeypatch.setattr(ops, "sm_count", lambda device: 148)
+    monkeypatch.setattr(ops, "check", lambda code, what: None)
+    monkeypatch.setattr(ops, "library", lambda: type("L", (), {"pe_gemm_smallm_scaled": staticmethod(lambda *a: 0)}))
+    x, weight, out = torch.zeros(rows, k, dtype=bf), torch.zeros(n, k, dtype=bf), torch.zeros(rows, n, dtype=bf)
+    ops.gemm_smallm_scaled(x, weight, out, torch.zeros(5, columns), 1e-6)
+    for shape in ((4, columns), (6, columns), (5, 2 * columns), (5, columns // 2), (5 * columns,)):
+        with pytest.raises(pe.kernels.lib.KernelError):
+            ops.gemm_smallm_scaled(x, weight, out, torch.zeros(*shape), 1e-6)
+    assert len(launched) == 1
