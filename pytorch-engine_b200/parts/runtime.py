@@ -25,10 +25,20 @@ STATUS_MESSAGES = {
 }
 
 
-# What ``torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction`` reads and sets, without its parsing: (allowed, split-K
-# allowed).  Every library product asks, and a prompt's step has three of them a layer.
-_reduced_reductions = torch._C._get_cublas_allow_bf16_reduced_precision_reduction
-_set_reduced_reductions = torch._C._set_cublas_allow_bf16_reduced_precision_reduction
+def _reductions_switch() -> tuple:
+    """How ``torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction`` is read and set: as (allowed, split-K allowed) and
+    without its parsing where this PyTorch has the calls behind it (every library product asks, and a prompt's step has three of
+    them a layer), else as the attribute itself."""
+    read = getattr(torch._C, "_get_cublas_allow_bf16_reduced_precision_reduction", None)
+    write = getattr(torch._C, "_set_cublas_allow_bf16_reduced_precision_reduction", None)
+    if read is not None and write is not None and isinstance(read(), tuple) and len(read()) == 2:
+        return read, write
+    matmul = torch.backends.cuda.matmul
+    return (lambda: (matmul.allow_bf16_reduced_precision_reduction, True),
+            lambda allowed, split_k: setattr(matmul, "allow_bf16_reduced_precision_reduction", allowed))
+
+
+_reduced_reductions, _set_reduced_reductions = _reductions_switch()
 
 
 class PendingTokens:

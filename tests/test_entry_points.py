@@ -261,3 +261,28 @@ def test_chained_products_refuse_squares_of_another_width(pe, monkeypatch, rows,
         with pytest.raises(pe.kernels.lib.KernelError):
             ops.gemm_smallm_scaled(x, weight, out, torch.zeros(*shape), 1e-6)
     assert len(launched) == 1
+
+
+@pytest.mark.parametrize("behind", ["as it is", "one flag", "nothing"])
+def test_the_switch_of_bf16_reductions_with_any_pytorch(pe, monkeypatch, behind):
+    """The setting is read and written whether PyTorch has a pair behind it, a single flag or no such calls."""
+    from importlib import import_module
+    runtime = import_module("pytorch-engine_b200.parts.runtime")
+    matmul = torch.backends.cuda.matmul
+    usual = matmul.allow_bf16_reduced_precision_reduction
+    if behind != "as it is":      # a PyTorch whose attribute is one flag
+        monkeypatch.setattr(torch.backends.cuda, "matmul", type("Matmul", (), {"allow_bf16_reduced_precision_reduction": usual})())
+        for name in ("_get_cublas_allow_bf16_reduced_precision_reduction", "_set_cublas_allow_bf16_reduced_precision_reduction"):
+            if behind == "nothing":
+                monkeypatch.delattr(torch._C, name)
+            else:
+                monkeypatch.setattr(torch._C, name, lambda *a: usual)
+    read, write = runtime._reductions_switch()
+    before = read()
+    try:
+        for allowed in (False, True, False):
+            write(allowed, True)
+            assert read()[0] is allowed and torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction is allowed
+    finally:
+        write(*before)
+    assert read() == before
