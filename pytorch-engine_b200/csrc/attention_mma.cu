@@ -880,8 +880,8 @@ __global__ void decode_merge_kernel(Args a) {
 // Blocks and ranges above are cut from one sequence each, so the longest sequence sets the time: 24 sequences of 16 to 2,048 keys
 // on 8 kv heads are 192 ranges for 296 places, most of them short.  Here the visible pages of all (sequence, kv head) pairs are
 // one list, sequence after sequence and kv head after kv head, and block i of n takes pages [i T / n, (i + 1) T / n) of its T:
-// every block reads as much as every other, whatever the lengths.  A pair that lies inside one block is finished there; the
-// others leave a partial result a block, number (block + pair) of the list, and a second kernel puts them together.
+// every block reads as much as every other, whatever the lengths (or one pair, where that is the better cut: takes_whole_pairs).  A
+// pair that lies inside one block is finished there; the others leave a partial result a block, number (block + pair) of the list, and a second kernel puts them together.
 //
 // Warp 4 looks pages up, a lane each, and keeps STAGES of them on their way across the pairs' borders; warps 0-3 fold them as
 // above, a quarter of the keys each, and meet only where a pair ends (then they sum through the page they have just read).
@@ -922,6 +922,15 @@ struct Place {
   }
 };
 
+// Whether each block takes one pair and no more, instead of an even share of the pages: where pairs are short or of about the same
+// length, what an even cut saves (0.3 to 0.4 us for a page that the busiest block has less of) is less than what its partial results
+// and their merge cost (2.7 us a layer).  A step of the 0.6B shape in us, even : a pair a block: 24 sequences of 40 keys 1,144 : 1,071,
+// of 300 1,306 : 1,214, of 1,000 1,582 : 1,539, of 2,048 2,512 : 2,438, of 16 to 500 1,318 : 1,288; of 16 to 1,000 1,477 : 1,490 and of
+// 16 to 2,048 1,849 : 1,995 (even).
+__device__ __forceinline__ bool takes_whole_pairs(int longest, int total, int n_pairs, int even_blocks, int max_blocks) {
+  return n_pairs <= max_blocks && (longest - total / even_blocks <= 8 || (long long)longest * n_pairs <= total + total / 4);
+}
+
 __device__ __forceinline__ void bar_sync_consumers() { asm volatile("bar.sync 1, 128;\n" ::: "memory"); }
 
 // Blocks of the shared decode that an SM holds (shared memory; registers are bounded to match).
@@ -934,7 +943,7 @@ __global__ void __launch_bounds__(160, shared_blocks_per_sm(HD)) decode_shared_k
   extern __shared__ char smem_raw[];
   __shared__ uint64_t full[STAGES], empty[STAGES];
   __shared__ int before[kSharedSeqs + 1];      // pages of one kv head in the sequences before
-  __shared__ int warp_pages[4];
+  __shared__ int warp_pages[4], warp_longest[4];
   __shared__ volatile int failed;
   __shared__ float ml[4 * 16 * 2];
   char* smem = align_1024(smem_raw);
@@ -950,21 +959,26 @@ __global__ void __launch_bounds__(160, shared_blocks_per_sm(HD)) decode_shared_k
   // the batch description, the page table and all pages but a sequence's last were written before the kernel that precedes this
   // one started: they are read before the wait
   constexpr int PER = kSharedSeqs / 128;
-  int mine[PER], sum = 0;
+  int mine[PER], sum = 0, longest = 0;
   if (warp < 4) {
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
       const int b = tid * PER + k;
       mine[k] = b < sh.n_seqs ? Visible(a, a.seq_past[b]).tiles : 0;
       sum += mine[k];
+      longest = max(longest, mine[k]);
     }
+    longest = __reduce_max_sync(0xffffffffu, longest);
     int up = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int v = __shfl_up_sync(0xffffffffu, up, o);
       if (lane >= o) up += v;
     }
-    if (lane == 31) warp_pages[warp] = up;
+    if (lane == 31) {
+      warp_pages[warp] = up;
+      warp_longest[warp] = longest;
+    }
     sum = up - sum;
   } else if (lane == 0) {
 #pragma unroll
@@ -988,9 +1002,18 @@ __global__ void __launch_bounds__(160, shared_blocks_per_sm(HD)) decode_shared_k
   }
   __syncthreads();
   const int total = before[sh.n_seqs] * n_kv, min_pages = max(1, a.min_range_keys / BN);
-  const int n_blocks = max(1, min((int)gridDim.x, total / min_pages)), me = blockIdx.x;
+  longest = max(max(warp_longest[0], warp_longest[1]), max(warp_longest[2], warp_longest[3]));
+  const int n_pairs = sh.n_seqs * n_kv, me = blockIdx.x;
+  int n_blocks = max(1, min((int)gridDim.x, total / min_pages));
+  const bool whole_pairs = takes_whole_pairs(longest, total, n_pairs, n_blocks, (int)gridDim.x);
+  if (whole_pairs) n_blocks = n_pairs;
   if (me >= n_blocks) return;
-  const int x0 = (int)((long long)me * total / n_blocks), x1 = (int)((long long)(me + 1) * total / n_blocks);
+  int x0 = (int)((long long)me * total / n_blocks), x1 = (int)((long long)(me + 1) * total / n_blocks);
+  if (whole_pairs) {
+    const int b = me / n_kv, tiles = before[b + 1] - before[b];
+    x0 = before[b] * n_kv + (me - b * n_kv) * tiles;
+    x1 = x0 + tiles;
+  }
   const int n_tiles = x1 - x0;      // at least 1: n_blocks <= total
 
   if (warp == 4) {
@@ -1168,9 +1191,9 @@ __global__ void __launch_bounds__(160, shared_blocks_per_sm(HD)) decode_shared_k
         a.out[(size_t)tq * a.out_ld + (size_t)h * HD + c] = __float2bfloat16_rn(aa / fmaxf(ll, 1e-20f));
       }
       if (tid == 0 && first == 0) {
-        // who holds the pair's last page: block i takes pages up to (i + 1) total / n_blocks
+        // who holds the pair's last page: this block, or with even shares block i takes pages up to (i + 1) total / n_blocks
         const long long end = x0 + it + 1 + (long long)(seen.tiles - 1 - at.tile);
-        sh.pairs[pair] = make_int2(part, (int)((end * n_blocks - 1) / total) - me + 1);
+        sh.pairs[pair] = make_int2(part, pair_ends ? 1 : (int)((end * n_blocks - 1) / total) - me + 1);
       }
       tma::fence_proxy_async();      // the page's place is written by TMA next
       if (it + 1 < n_tiles) {

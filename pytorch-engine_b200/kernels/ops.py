@@ -429,9 +429,11 @@ def attention_mma_masked(decode: bool, q: torch.Tensor, out: torch.Tensor, n_seq
 def attention_mma_shares(device: torch.device, head_dim: int, n_seqs: int, n_heads: int, n_kv_heads: int, max_kv_len: int) -> tuple:
     """(blocks, floats of scratch, least keys a block) where ``attention_mma_append`` shares a decode step's keys out over the chip,
     (0, 0, 0) where ranges of each sequence's own (``attention_mma_decode_ranges``) are the better cut.  Ranges leave places empty where
-    the (sequence, kv head) pairs are between 0.6 and 1 of the chip's places; short caches do not pay for the second kernel.  A step of
-    the 0.6B shape (8 kv heads, 296 places), ranges : shared: 24 sequences of 16 to 2,048 keys 1,913 : 1,788 us, of 2,048 keys 2,558 :
-    2,512, of 300 keys in a cache for as many 1,250 : 1,323; 30 of 2,048 keys 2,954 : 2,861; 20 of 16 to 4,000 keys 2,032 : 2,160."""
+    the (sequence, kv head) pairs are between 0.6 and 1 of the chip's places; short caches do not pay for the second kernel.  (The
+    limit is the cache's; the lengths themselves decide on the device whether pairs are cut at all.)  A step of the 0.6B shape (8 kv
+    heads, 296 places) in us, ranges : shared: 24 sequences of 300 keys 1,220 : 1,214, of 1,000 1,543 : 1,539, of 2,048 2,519 : 2,438,
+    of 16 to 500 1,275 : 1,288, of 16 to 2,048 1,907 : 1,841; 30 of 16 to 2,048 1,970 : 1,831; 37 of 300 1,607 : 1,574; 20 of 16 to
+    4,000 keys, cut evenly, 2,032 : 2,160."""
     blocks, pairs = sm_count(device) * int(library().pe_attention_mma_shared_blocks_per_sm(head_dim)), n_seqs * n_kv_heads
     if pairs > blocks or 5 * pairs < 3 * blocks or max_kv_len <= 512:
         return 0, 0, 0

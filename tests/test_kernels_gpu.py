@@ -696,6 +696,39 @@ def test_attention_mma_append(ops, nh, nkv, d, blocks, least, normed, rotated, w
     assert bool(((k0 - k1).abs() <= 2.0 ** -7 * k1.abs()).all())
 
 
+@pytest.mark.parametrize("nh,nkv,d", [(16, 8, 128), (6, 2, 64)])
+@pytest.mark.parametrize("lens,others", [([300, 1, 64, 65, 130], [2, 512, 100, 449, 7]), ([520, 513], [576, 515]), ([2000, 1900, 2048], [1990, 2048, 1921])])
+def test_attention_mma_append_takes_whole_pairs(ops, nh, nkv, d, lens, others):
+    """Short sequences, or such of about the same length, are not cut: no partial results, and a sequence's output has the same bits
+    whatever the others' lengths; with a block too few for that, and by the two kernels, the same within rounding."""
+    torch.manual_seed(35)
+    bf, B = torch.bfloat16, len(lens)
+    qkv, angles = torch.randn(B, (nh + 2 * nkv) * d, device=DEV).to(bf), torch.rand(2112, d // 2, device=DEV) * 6
+    t, qstart, st, outs = torch.arange(B, dtype=torch.int32, device=DEV), torch.arange(B + 1, dtype=torch.int32, device=DEV), _status(), []
+    whole = PagedSetup(lens, nkv, d, bf, seed=35)
+    for seen, blocks in ((lens, 296), (lens, B * nkv), (lens, B * nkv - 1), (lens, 0), ([lens[0]] + others[1:], 296)):
+        ps = PagedSetup(seen, nkv, d, bf, seed=36)
+        for i in range(-(-lens[0] // 64)):      # the first sequence's pages are the same in every run
+            page, as_in = int(ps.table[ps.slots[0], i]), int(whole.table[whole.slots[0], i])
+            ps.k_pages[page], ps.v_pages[page] = whole.k_pages[as_in], whole.v_pages[as_in]
+        past = torch.tensor([L - 1 for L in seen], dtype=torch.int32, device=DEV)
+        where = (qstart, past, ps.seq_slot, ps.table, ps.num_pages, ps.k_pages, ps.v_pages)
+        x, out = qkv.clone(), torch.full((B, nh * d), float("nan"), device=DEV, dtype=bf)
+        if blocks:
+            scratch = torch.full((int(ops.library().pe_attention_mma_shared_scratch_floats(B, nh, nkv, d, blocks)),), float("nan"), device=DEV)
+            ops.attention_mma_append(x, out, B, nh, nkv, d, d ** -0.5, 0, None, None, 1e-5, angles.cos(), angles.sin(), *where, scratch, blocks, 0, 128, st)
+            assert bool(scratch[:(B * nkv + blocks) * (nh // nkv) * (d + 1)].isnan().all()) == (blocks >= B * nkv)
+        else:
+            ops.qk_norm_rope_append(x, B, nh, nkv, d, None, None, 1e-5, angles.cos(), angles.sin(), d, t, past, ps.seq_slot, qstart, ps.table,
+                                    ps.num_pages, ps.k_pages, ps.v_pages, True, st)
+            scratch = torch.empty(ops.attention_generic_scratch_floats(B, nh, d, 32), device=DEV)
+            ops.attention_mma(True, x, out, B, 1, nh, nkv, d, d ** -0.5, 0, *where, scratch, 64, 32, st)
+        outs.append(out)
+    assert st.tolist()[0] == 0
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0][0], outs[4][0])
+    assert all(rel_err(outs[0].float(), o.float()) < 2 * ATT_TOL[bf] for o in outs[2:4])
+
+
 @pytest.mark.parametrize("B", [129, 512, 513])
 def test_attention_mma_append_of_many_sequences(ops, B):
     """Batches around the number of sequences whose pages a block lists, keys shared out, against the two kernels."""
