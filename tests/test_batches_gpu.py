@@ -236,3 +236,92 @@ def test_greedy_tokens_alone_and_in_a_batch_of_64(pe, big_engines, oracles, mode
           f"({agree32:.1%} of tokens before a first difference); bfloat16 {same16:.0%} ({agree16:.1%})")
     assert same32 >= 0.95 and agree32 >= 0.97
     assert agree16 > 0.5
+
+
+# ---- steps of few rows without kernels for the norms, and decode steps whose attention appends -----------------------------
+FEW_ROWS = (1, 8, 9, 12, 13, 16, 17, 24, 32, 33)     # either side of every bound of ``Runtime.takes_chained``; keys shared out at 24 to 33
+# How far bfloat16 logits are off the float32 engine's, in the 2-norm over that of the latter: TOL, some 25 roundings of 2^-9 (three
+# layers have eight each).  Measured: 0.5 % at width 512, 0.7 % at 1,024, 1.2 % at 2,048, with or without kernels for the norms; the two
+# ways are 0.4, 0.6 and 0.8 % apart, a decode step and the prompt of the same tokens 0.4, 0.6 and 0.9 %.
+
+
+class _FewRows:
+    """Three layers of 8 kv heads of 128 features in several engines on the same weights, each for sequences of up to 1,024 tokens."""
+
+    def __init__(self, pe, width):
+        self.pe = pe
+        self.config = pe.preset("qwen3_0_6b", num_hidden_layers=3, hidden_size=width, intermediate_size=2 * width, vocab_size=3000)
+        rng = random.Random(width)
+        self.prompts = [_tokens(3000, n, n + width) for n in [700] + [rng.randint(16, 600) for _ in range(max(FEW_ROWS) - 1)]]
+        self.next = [_tokens(3000, 3, 7 * i + width) for i in range(len(self.prompts))]
+
+    def engine(self, dtype="bfloat16", usual=True, graphs=True, without=()):
+        """``usual`` False: norms, rotation and append in kernels of their own; ``without``: layers that do not take part."""
+        eng = self.pe.Engine.from_random(self.config, seed=5, dtype=dtype, max_context_len=1024, max_cache_tokens=64 * 384, max_batch=33,
+                                         enable_cuda_graph=graphs)
+        eng.runtime.chain_norms = usual
+        for i, run in enumerate(eng.model.plan.order):
+            block = eng.model.blocks[run.block]
+            block.mixer.fuses_append = block.mixer.fuses_append and usual
+            if i in without:
+                block.chains = lambda *a: False
+        return eng
+
+    def decode(self, eng, n):
+        """Logits of three decode steps of the first ``n`` sequences, and of the first made once more."""
+        entry, slots = self.pe.StepEntry, [eng.alloc_slot() for _ in range(n)]
+        eng.step([entry(s, p) for s, p in zip(slots, self.prompts)])
+        out = []
+        for k in (0, 1, 2, 0):
+            out.append(eng.step([entry(s, [t[k]], (0,)) for s, t in zip(slots, self.next)]).float().clone())
+            if k == 2:
+                for s, p in zip(slots, self.prompts):
+                    eng.cache.truncate(s, len(p))
+        for s in slots:
+            eng.free_slot(s)
+        assert eng.runtime.status.tolist()[0] == 0
+        return out
+
+
+def _off(got, ref):
+    return float((got.double() - ref.double()).norm() / ref.double().norm())
+
+
+@pytest.mark.parametrize("width", [512, 1024, 2048])
+def test_steps_of_few_rows_with_and_without_kernels_for_the_norms(pe, width):
+    """Decode steps around every batch size at which other kernels take over, eager and captured, against the same engine with a kernel
+    for each norm and append and against float32: as far off, the captured step's bits those of the eager one, and the prompt of the same
+    tokens within the same bound."""
+    few = _FewRows(pe, width)
+    usual, eager, plainer, exact = few.engine(), few.engine(graphs=False), few.engine(usual=False), few.engine("float32")
+    entry = pe.StepEntry
+    for n in FEW_ROWS:
+        chained = usual.runtime.takes_chained(n, width)
+        assert chained == (n <= 32 if width < 2048 else 8 < n <= 32)
+        got, again, other, ref = few.decode(usual, n), few.decode(eager, n), few.decode(plainer, n), few.decode(exact, n)
+        assert torch.equal(got[0], got[3]) and all(torch.equal(a, b) for a, b in zip(got, again)), n
+        errors, others = [_off(a, r) for a, r in zip(got, ref)], [_off(a, r) for a, r in zip(other, ref)]
+        print(f"width {width} x {n}: off float32 {max(errors):.4f}, with kernels for the norms {max(others):.4f}, from each other "
+              f"{max(_off(a, b) for a, b in zip(got, other)):.4f}")
+        assert max(errors) < TOL["bfloat16"] and max(others) < TOL["bfloat16"]
+        assert sum(errors) < 1.1 * sum(others)
+    slots = [usual.alloc_slot() for _ in few.prompts]
+    whole = usual.step([entry(s, p + t[:1], (len(p),)) for s, p, t in zip(slots, few.prompts, few.next)]).float().clone()
+    for s in slots:
+        usual.free_slot(s)
+    for n in FEW_ROWS:
+        drift = _off(few.decode(usual, n)[0], whole[:n])
+        print(f"width {width} x {n}: step and prompt {drift:.4f} apart")
+        assert drift < TOL["bfloat16"]
+
+
+@pytest.mark.parametrize("without", [(0,), (1,), (2,), (0, 2)])
+def test_a_block_that_cannot_chain_behind_and_before_one_that_can(pe, without):
+    """What a chained block hands on has been added to the stream already: any other block reads it, and the final norm does."""
+    few = _FewRows(pe, 512)
+    mixed, plainer, exact = few.engine(without=without), few.engine(usual=False), few.engine("float32")
+    for n in (1, 9, 24):
+        got, other, ref = few.decode(mixed, n), few.decode(plainer, n), few.decode(exact, n)
+        assert torch.equal(got[0], got[3])
+        assert max(_off(a, r) for a, r in zip(got, ref)) < TOL["bfloat16"]
+        assert sum(_off(a, r) for a, r in zip(got, ref)) < 1.1 * sum(_off(a, r) for a, r in zip(other, ref))
