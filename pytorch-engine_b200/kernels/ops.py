@@ -770,8 +770,9 @@ def attention_mma_decode_ranges(device: torch.device, head_dim: int, n_seqs: int
 
 
 def mma_decode_ranges(slots: int, pairs: int, max_kv_len: int, split_keys: int) -> tuple:
-    """``decode_ranges`` with a case of its own.  How a sequence's keys are cut depends on its own length, the cache's limit
-    ``max_kv_len`` and the number of sequences, never on the other sequences' lengths.
+    """``decode_ranges`` with a case of its own.  How a sequence's keys are cut into ranges depends on its own length, the cache's limit
+    ``max_kv_len`` and the number of sequences, never on the other sequences' lengths.  (A step whose keys are shared out over the chip,
+    ``attention_mma_shares``, has no ranges, and there the lengths of all its sequences decide.)
 
     Room for two or more ranges a pair: a block takes about 0.8 us a page and the chip is mostly empty, so ranges of two pages
     or more, 16 of them or as many as ranges of ``split_keys`` keys would be, whichever is more, while one wave holds them.
