@@ -246,7 +246,7 @@ __device__ __forceinline__ int block_offset(int mine, int* scratch, int* total) 
 
 // First kernel for top-k up to kTopMax.  grid: (tasks of eight warps, rows).  The largest value of every group, as it is in the row
 // (NaN counts as -infinity); the reads are all it does.  A call for 64 rows of 151,936
-// entries, top-k 50: 9.9 us, 12.3 the second kernel, 78 a call with its copies (26.1, 17.5 and 95 with chunks of which the first
+// entries, top-k 50: 9.9 us, 12.3 the second kernel, 82 a call with its copies (26.1, 17.5 and 94 with chunks of which the first
 // kernel also took the k-th value and the candidates).
 __global__ void __launch_bounds__(kMaximaThreads) sample_maxima_kernel(SampleArgs a) {
   pdl_wait_block();
